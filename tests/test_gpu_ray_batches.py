@@ -1,0 +1,76 @@
+"""Ray batches at the edges of the trace kernels' warp chunks, and trees at the edges of their
+stacks: a single leaf, and chains deeper than the part of the stack kept in shared memory."""
+import numpy as np
+import pytest
+
+import oracle_bind as ob
+from test_gpu_trace import compare_hits, random_rays
+from x3dcore2_gb300 import abi
+from x3dcore2_gb300 import scene as S
+
+pytestmark = pytest.mark.gpu
+LAYOUTS = [abi.BVH_SAH, abi.BVH_WIDE]
+
+
+def check(ctx, sc, layout, rays):
+    ctx.upload(sc, layout=layout)
+    osc = ob.OracleScene(sc)
+    o = osc.trace_closest(rays)
+    compare_hits(ctx.trace_closest(rays), o["mesh"], o["tri"], o["t"])
+    tmin = np.full(len(rays), 1e-4, np.float32)
+    tmax = np.random.default_rng(len(rays)).uniform(1e-3, 2.5, len(rays)).astype(np.float32)
+    assert np.mean(ctx.trace_any(rays, tmin, tmax) == osc.trace_any(rays, tmin, tmax)) >= 0.9999
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("n", [1, 31, 33, 4097, 155_649, 400_003])
+def test_batch_sizes(ctx, layout, n):
+    """One ray, part of a warp, one ray per lane, and chunks of 64 and 96 rays per warp with a ragged last one."""
+    check(ctx, S.soup(3000, seed=7, width=64, height=64), layout, random_rays(max(n, 64), -1.0, 1.0, seed=n)[-n:])
+
+
+def mesh_scene(tris):
+    """Triangles (T, 3, 3) as one mesh, with a small light above them."""
+    def mesh(t):
+        t = np.asarray(t, np.float32)
+        n = np.cross(t[:, 1] - t[:, 0], t[:, 2] - t[:, 0])
+        n /= np.linalg.norm(n, axis=1, keepdims=True)
+        return S.Mesh(t.reshape(-1, 3), np.repeat(n, 3, axis=0), np.arange(3 * len(t)).reshape(-1, 3))
+    m = S.material(abi.MAT_OREN_NAYAR, albedo=(0.5, 0.5, 0.5))
+    light = abi.Light()
+    light.mesh = 1
+    light.radiance[:] = [1.0, 1.0, 1.0]
+    lamp = mesh([[[0.0, 0.0, 5.0], [0.0, 0.1, 5.0], [0.1, 0.0, 5.0]]])
+    cam = S.soup(10, seed=1, width=32, height=32).camera
+    return S.from_meshes([mesh(tris), lamp], [0, 0], [m], [light], cam)
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("count", [1, 6])
+def test_tree_of_few_triangles(ctx, layout, count):
+    r = np.random.default_rng(count)
+    check(ctx, mesh_scene(r.uniform(-1, 1, (count, 3, 3))), layout, random_rays(2000, -1.0, 1.0, seed=count))
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_stack_beyond_its_shared_part(ctx, layout):
+    """Sheets whose spacing doubles along x: the tree is a chain, and a ray along it that hits none
+    of the nearer sheets keeps a far child per level."""
+    tris = []
+    for k in range(20):
+        x = 2.0 ** (k - 18)
+        for j in range(12):
+            y = -1.0 + j / 6.0
+            tris.append([[x, y, -1.0], [x, y + 0.16, -1.0], [x, y, 1.0]])
+    r = np.random.default_rng(3)
+    n = 4000
+    o = np.stack([np.full(n, -1.0), r.uniform(-1, 1, n), r.uniform(-1, 1, n)], axis=1)
+    d = np.stack([np.ones(n), r.normal(0, 0.05, n), r.normal(0, 0.05, n)], axis=1)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    back = np.stack([o[:, 0] + 4.0, o[:, 1], o[:, 2]], axis=1)
+    rays = np.concatenate([ob.rays_array(o.astype(np.float32), d.astype(np.float32)),
+                           ob.rays_array(back.astype(np.float32), -d.astype(np.float32))])
+    sc = mesh_scene(tris)
+    check(ctx, sc, layout, rays)
+    if layout == abi.BVH_SAH:
+        assert ctx.bvh_stats()["max_depth"] > 9

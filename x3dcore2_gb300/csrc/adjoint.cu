@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kBlock) k_adjoint(DevScene S, RenderArgs A, Fi
                                                     float const *__restrict__ dl_dimage, float inv_spp,
                                                     unsigned long long *work, float *d_albedo, float *d_rough,
                                                     float *path_rgb) {
-    __shared__ uint32_t stk_all[kStackWords * kBlock];
+    __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
     extern __shared__ float sgrad[];
     GradAcc g{sgrad, sgrad + 3 * S.nmat, S.nmat};
     for (uint32_t k = threadIdx.x; k < 4 * S.nmat; k += blockDim.x)

@@ -108,8 +108,8 @@ template <class T> static cudaError_t upload(dev_buffer &b, std::vector<T> const
 void fill_dev_scene(e8g_ctx *c) {
     DevScene &S = c->dev;
     packed_scene &p = c->pack;
-    S.nlo = static_cast<float4 const *>(c->b_nlo.ptr);
-    S.nhi = static_cast<float4 const *>(c->b_nhi.ptr);
+    S.nlo.p = static_cast<float4 const *>(c->b_nodes.ptr) + kNodeShift;
+    S.nhi.p = S.nlo.p + 1;
     S.wnodes = static_cast<uint4 const *>(c->b_wide.ptr);
     S.tri = static_cast<float4 const *>(c->b_tri.ptr);
     S.tidx = static_cast<uint4 const *>(c->b_tidx.ptr);
@@ -244,9 +244,7 @@ e8g_status build_on_device(e8g_ctx *c, bool *built) {
     uint32_t nt = p.nt;
     bvh_build_opts const &o = c->bvh_opts;
     fill_dev_scene(c);
-    cudaError_t e = c->b_nlo.reserve(32 * static_cast<size_t>(nt));
-    if (e == cudaSuccess)
-        e = c->b_nhi.reserve(32 * static_cast<size_t>(nt));
+    cudaError_t e = c->b_nodes.reserve(node_buffer_bytes(2 * static_cast<size_t>(nt)));
     if (e == cudaSuccess)
         e = c->b_tri.reserve(48 * static_cast<size_t>(nt));
     if (e == cudaSuccess)
@@ -264,8 +262,8 @@ e8g_status build_on_device(e8g_ctx *c, bool *built) {
     in.num_sms = c->num_sms;
     in.scratch = c->b_gbuild.ptr;
     in.host_pinned = c->host_pinned;
-    in.nlo = static_cast<float4 *>(c->b_nlo.ptr);
-    in.nhi = static_cast<float4 *>(c->b_nhi.ptr);
+    in.nlo.p = static_cast<float4 *>(c->b_nodes.ptr) + kNodeShift;
+    in.nhi.p = in.nlo.p + 1;
     in.tri = static_cast<float4 *>(c->b_tri.ptr);
     GpuBuildOut out;
     auto t0 = std::chrono::steady_clock::now();
@@ -300,8 +298,8 @@ e8g_status build_on_device(e8g_ctx *c, bool *built) {
         for (int k = 0; k < 3; k++)
             max_abs = std::max(max_abs, std::fabs(p.cam.origin[k]));
         GpuWideIn wi{};
-        wi.nlo = in.nlo;
-        wi.nhi = in.nhi;
+        wi.nlo.p = in.nlo.p;
+        wi.nhi.p = in.nhi.p;
         wi.tri = in.tri;
         wi.num_tris = nt;
         wi.max_abs = max_abs;
@@ -365,9 +363,13 @@ e8g_status build_tree(e8g_ctx *c) {
             c->built = false;
             return fail(c, E8G_ERR_UNSUPPORTED, "reference BVH deeper than the traversal stack (63 levels)");
         }
-        cudaError_t e = upload(c->b_nlo, p.bvh.lo, c->stream);
-        if (e == cudaSuccess)
-            e = upload(c->b_nhi, p.bvh.hi, c->stream);
+        std::vector<float> nodes;
+        try {
+            interleave_nodes(p.bvh, nodes);
+        } catch (std::bad_alloc const &) {
+            return fail(c, E8G_ERR_OUT_OF_MEMORY, "host allocation failed while building the BVH");
+        }
+        cudaError_t e = upload(c->b_nodes, nodes, c->stream);
         if (e == cudaSuccess)
             e = upload(c->b_wide, p.wide, c->stream);
         if (e == cudaSuccess)
@@ -629,16 +631,29 @@ e8g_status e8g_bvh_read(e8g_ctx *c, void *nodes_out, void *tris_out) {
     if (nodes_out && p.layout == E8G_BVH_WIDE) {
         e = cudaMemcpyAsync(nodes_out, c->b_wide.ptr, nn * 4 * kWideWords, cudaMemcpyDeviceToHost, c->stream);
     } else if (nodes_out && nn) {
-        e = cudaMemcpyAsync(nodes_out, c->b_nlo.ptr, nn * 16, cudaMemcpyDeviceToHost, c->stream);
+        std::vector<float> nodes;
+        try {
+            nodes.resize(8 * nn);
+        } catch (std::bad_alloc const &) {
+            return fail(c, E8G_ERR_OUT_OF_MEMORY, "host allocation failed while reading the BVH back");
+        }
+        e = cudaMemcpyAsync(nodes.data(), static_cast<float4 *>(c->b_nodes.ptr) + kNodeShift, nn * 32,
+                            cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(static_cast<char *>(nodes_out) + nn * 16, c->b_nhi.ptr, nn * 16,
-                                cudaMemcpyDeviceToHost, c->stream);
+            e = cudaStreamSynchronize(c->stream);
+        auto *lo = static_cast<char *>(nodes_out), *hi = lo + nn * 16;
+        for (size_t i = 0; i < nn && e == cudaSuccess; i++) {
+            std::memcpy(lo + 16 * i, &nodes[8 * i], 16);
+            std::memcpy(hi + 16 * i, &nodes[8 * i + 4], 16);
+        }
     }
     if (e == cudaSuccess && tris_out && p.nt)
         e = cudaMemcpyAsync(tris_out, c->b_tri.ptr, static_cast<size_t>(p.nt) * 48, cudaMemcpyDeviceToHost,
                             c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
+    for (size_t k = 0; tris_out && e == cudaSuccess && k < p.nt; k++) // the leaves' end marks are the traversal's own
+        static_cast<float *>(tris_out)[12 * k + 7] = 0.0f;
     return e == cudaSuccess ? E8G_OK : cuda_fail(c, e, "tree read-back");
 }
 
@@ -676,7 +691,8 @@ e8g_status e8g_trace_closest_dev(e8g_ctx *c, e8g_ray const *d_rays, uint32_t n, 
         return fail(c, E8G_ERR_INVALID_ARG, "NULL buffers");
     cudaSetDevice(c->device);
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
-    launch_trace_closest(c->dev, reinterpret_cast<float const *>(d_rays), n, reinterpret_cast<float *>(d_hits), st);
+    launch_trace_closest(c->dev, reinterpret_cast<float const *>(d_rays), n, reinterpret_cast<float *>(d_hits), c->num_sms,
+                         st);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? E8G_OK : cuda_fail(c, e, "trace_closest launch");
 }
@@ -699,7 +715,7 @@ e8g_status e8g_trace_closest(e8g_ctx *c, e8g_ray const *rays, uint32_t n, e8g_hi
     if (e != cudaSuccess)
         return cuda_fail(c, e, "trace_closest upload");
     launch_trace_closest(c->dev, static_cast<float const *>(c->b_io0.ptr), n, static_cast<float *>(c->b_io1.ptr),
-                         c->stream);
+                         c->num_sms, c->stream);
     e = cudaMemcpyAsync(hits, c->b_io1.ptr, hb, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
@@ -730,7 +746,7 @@ e8g_status e8g_trace_any(e8g_ctx *c, e8g_ray const *rays, float const *t_min, fl
         e = cudaMemcpyAsync(dtmax, t_max, tb, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "trace_any upload");
-    launch_trace_any(c->dev, reinterpret_cast<float const *>(base), dtmin, dtmax, n, docc, c->stream);
+    launch_trace_any(c->dev, reinterpret_cast<float const *>(base), dtmin, dtmax, n, docc, c->num_sms, c->stream);
     e = cudaMemcpyAsync(occluded, docc, n, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);

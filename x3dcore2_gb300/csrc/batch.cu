@@ -64,7 +64,7 @@ extern "C" e8g_status e8g_batch_render(e8g_ctx *c, e8g_batch_item const *items, 
     // host: pack, build, stage
     staged st;
     struct offs {
-        size_t nlo, nhi, wide, tri, tidx, vpos, vnrm, vtx, mesh_mat, mesh_light, mesh_toff, mesh_area, tri_cum, mats, light_mesh,
+        size_t nodes, wide, tri, tidx, vpos, vnrm, vtx, mesh_mat, mesh_light, mesh_toff, mesh_area, tri_cum, mats, light_mesh,
             light_rad, light_cum, light_pnorm;
     };
     std::vector<offs> off(n);
@@ -91,8 +91,9 @@ extern "C" e8g_status e8g_batch_render(e8g_ctx *c, e8g_batch_item const *items, 
         for (uint32_t k = 0; k < n; k++) {
             packed_scene &p = packs[k];
             offs &o = off[k];
-            o.nlo = st.put(p.bvh.lo);
-            o.nhi = st.put(p.bvh.hi);
+            std::vector<float> nodes;
+            interleave_nodes(p.bvh, nodes);
+            o.nodes = st.put(nodes);
             o.wide = st.put(p.wide);
             o.tri = st.put(p.tri);
             o.tidx = st.put(p.tidx);
@@ -136,8 +137,8 @@ extern "C" e8g_status e8g_batch_render(e8g_ctx *c, e8g_batch_item const *items, 
         packed_scene &p = packs[k];
         offs &o = off[k];
         DevScene S{};
-        S.nlo = reinterpret_cast<float4 const *>(base + o.nlo);
-        S.nhi = reinterpret_cast<float4 const *>(base + o.nhi);
+        S.nlo.p = reinterpret_cast<float4 const *>(base + o.nodes) + kNodeShift;
+        S.nhi.p = S.nlo.p + 1;
         S.wnodes = reinterpret_cast<uint4 const *>(base + o.wide);
         S.tri = reinterpret_cast<float4 const *>(base + o.tri);
         S.tidx = reinterpret_cast<uint4 const *>(base + o.tidx);

@@ -231,4 +231,14 @@ flat_bvh build_bvh(float const *pos, uint32_t const *tris, uint32_t num_tris, bv
     return out;
 }
 
+void interleave_nodes(flat_bvh const &b, std::vector<float> &out) {
+    const size_t n = b.lo.size() / 4;
+    out.resize(n ? 8 * (n + 1) : 0);
+    for (size_t i = 0; i < n; i++)
+        for (int k = 0; k < 4; k++) {
+            out[8 * (i + 1) + k] = b.lo[4 * i + k];
+            out[8 * (i + 1) + 4 + k] = b.hi[4 * i + k];
+        }
+}
+
 } // namespace e8g

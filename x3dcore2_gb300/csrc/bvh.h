@@ -1,5 +1,5 @@
 // Host BVH builder: binned SAH over triangles, flattened to 32-byte nodes in two
-// structure-of-arrays halves (lo: min xyz + link, hi: max xyz + count), children stored as
+// halves (lo: min xyz + link, hi: max xyz + count), children stored as
 // adjacent pairs so one interior visit reads 64 contiguous bytes per half-array pair.
 #pragma once
 
@@ -48,6 +48,10 @@ struct flat_bvh {
 
 // tris: 3 global vertex indices per triangle; pos: 3 floats per vertex.
 flat_bvh build_bvh(float const *pos, uint32_t const *tris, uint32_t num_tris, bvh_build_opts const &o);
+
+// The tree as the device keeps it: eight floats before node 0, then 32 bytes per node, (min xyz |
+// link) and (max xyz | count).
+void interleave_nodes(flat_bvh const &b, std::vector<float> &out);
 
 // The reference's tree (bvh_path_space_layout::commit) in depth-first order: node n's left child
 // is n + 1, its right child `link`; boxes are the reference's, uninflated.

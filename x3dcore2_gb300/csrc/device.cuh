@@ -29,9 +29,19 @@ constexpr uint32_t kHardDepth = 1024;
 
 // ------------------------------------------------------------------ data layout ----
 
+// One half of the nodes of a binary tree, indexed by node: node i is the 32 bytes [2i] = (min xyz |
+// link), [2i + 1] = (max xyz | count). The array starts 32 bytes into its buffer, so that the
+// child pair of an interior node (nodes 2k + 1 and 2k + 2) fills one aligned 64-byte half line.
+template <class T> struct NodeHalf {
+    T *p;
+    __host__ __device__ __forceinline__ T &operator[](size_t i) const { return p[2 * i]; }
+};
+constexpr size_t kNodeShift = 2; // float4 before node 0
+inline size_t node_buffer_bytes(size_t n) { return 32 * n + 16 * kNodeShift; }
+
 struct DevScene {
-    const float4 *nlo;      // node min xyz | link
-    const float4 *nhi;      // node max xyz | count
+    NodeHalf<const float4> nlo; // node min xyz | link
+    NodeHalf<const float4> nhi; // node max xyz | count
     const uint4 *wnodes;    // eight-wide layout: 6 uint4 per node (bvh_wide.h)
     const float4 *tri;      // 3 float4 per BVH position: (v0 | global tri id), (v1 - v0), (v2 - v0)
     const uint4 *tidx;      // per global triangle: global vertex indices, mesh
@@ -257,110 +267,196 @@ struct TraceCounters {
     uint32_t rays; // counted by the callers that trace (the bidirectional kernels)
 };
 
-// Slab test of a node box against [tmin, tmax] (aabb::intersect, tensor.h:815-840, with the
-// box inflated by the builder so rounding never culls a triangle the exact test would hit).
-__device__ __forceinline__ bool slab(float4 lo, float4 hi, float3 o, float3 inv, float tmin, float tmax,
-                                     float &tnear) {
-    float x0 = (lo.x - o.x) * inv.x, x1 = (hi.x - o.x) * inv.x;
-    float y0 = (lo.y - o.y) * inv.y, y1 = (hi.y - o.y) * inv.y;
-    float z0 = (lo.z - o.z) * inv.z, z1 = (hi.z - o.z) * inv.z;
-    float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-    float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), tmax));
-    tnear = tn;
-    return tn <= tf;
-}
-
 // ray::intersect (tensor.h:688-725) on a triangle stored as (v0, v1 - v0, v2 - v0).
 __device__ __forceinline__ bool tri_test(float3 o, float3 d, float4 a, float4 b, float4 c, float tmin,
                                          float tmax, float &t0, float &b1o, float &b2o) {
     return hd_tri_test(o, d, a, b, c, tmin, tmax, t0, b1o, b2o);
 }
 
-// SAH child-pair tree. Closest hit (any = false) with the reference's strict `t0 < t`
-// (pathspace.cpp:330-413) or any hit (has_intersect, pathspace.cpp:415-456) on [tmin, tmax]:
-// ordered child visits, far children and their entry distances kept on a per-thread stack in
-// shared memory (stack entries of one thread are kBlock words apart, so lanes never conflict);
-// the closest-hit query culls boxes beyond its best hit.
+// ---- SAH child-pair tree ----
+// Closest hit (any = false) with the reference's strict `t0 < t` (pathspace.cpp:330-413) or any hit
+// (has_intersect, pathspace.cpp:415-456) on [tmin, tmax]: the nearer child first, the farther one
+// with its entry distance on a per-thread stack, boxes beyond the closest hit culled. The walk is
+// resumable one node at a time, so that a persistent kernel can give a lane a new ray as soon as
+// its ray is done.
+//
+// The next node is one word: the index of a child pair (interior), or bit 31 and the first triangle
+// record of a leaf, whose last record is marked (w of its second float4). A pop therefore fetches
+// no node, and a leaf needs no count. Stack entries of one thread are kBlock words apart, so lanes
+// never share a bank; the first kSahFast live in shared memory, the rest (deep trees only) in the
+// thread's local memory: 8 KB a block instead of 32 KB leave the L1 cache to the tree (fast entries
+// 4 / 6 / 8 / 16: 20.4 / 19.9 / 19.5 / 19.7 ms for the pooled megakernel's 1080p, 16-spp frame).
+constexpr int kSahFast = 8;
+constexpr uint32_t kSahLeaf = 0x80000000u;
+struct SahOverflow {
+    uint32_t w[kStack - kSahFast];
+    float t[kStack - kSahFast];
+};
+struct SahWalk {
+    float3 o, d;
+    float3 inv, oi; // box tests: reciprocal direction, -o * inv
+    float tmin, cull; // cull: the best hit so far, at most tmax (any hit: tmax)
+    uint32_t w;       // the next node
+    int sp;
+    Hit h;
+    __device__ __forceinline__ bool leaf() const { return static_cast<int32_t>(w) < 0; }
+};
+
+__device__ __forceinline__ uint32_t sah_word(float lo_w, float hi_w) {
+    uint32_t link = __float_as_uint(lo_w);
+    return __float_as_uint(hi_w) == 0u ? link >> 1 : link | kSahLeaf;
+}
+
+// Box tests use direction components at least 1e-30 in magnitude, so that a parallel ray's plane
+// distances stay finite; its triangles are tested with the direction as given.
+__device__ __forceinline__ float box_rcp(float d) { return 1.0f / (fabsf(d) < 1e-30f ? copysignf(1e-30f, d) : d); }
+
+__device__ __forceinline__ void sah_begin(DevScene const &S, SahWalk &T, float3 o, float3 d, float tmin, float tmax) {
+    T.o = o;
+    T.d = d;
+    T.inv = f3(box_rcp(d.x), box_rcp(d.y), box_rcp(d.z));
+    T.oi = f3(-(o.x * T.inv.x), -(o.y * T.inv.y), -(o.z * T.inv.z));
+    T.tmin = tmin;
+    T.cull = tmax;
+    T.sp = 0;
+    T.h.t = INFINITY;
+    T.h.tri = 0xFFFFFFFFu;
+    T.h.b1 = T.h.b2 = 0.0f;
+    T.w = S.nnodes == 1 ? kSahLeaf : 0u; // the root: pair 0, or a leaf of every triangle
+}
+
+// A node's 32 bytes in one load.
+__device__ __forceinline__ void ldg_node(float4 const *p, float4 &lo, float4 &hi) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w)
+        : "l"(p));
+}
+
+// Slab test of a node box against [tmin, tmax] (aabb::intersect, tensor.h:815-840), one FMA a
+// plane. The builder pushes boxes out by about 1e-6 of the scene's extent, several times the
+// rounding of lo * inv - o * inv, so no box that a triangle hit lies in is culled.
+__device__ __forceinline__ bool sah_slab(float4 lo, float4 hi, float3 inv, float3 oi, float tmin, float tmax,
+                                         float &tnear) {
+    float x0 = __fmaf_rn(lo.x, inv.x, oi.x), x1 = __fmaf_rn(hi.x, inv.x, oi.x);
+    float y0 = __fmaf_rn(lo.y, inv.y, oi.y), y1 = __fmaf_rn(hi.y, inv.y, oi.y);
+    float z0 = __fmaf_rn(lo.z, inv.z, oi.z), z1 = __fmaf_rn(hi.z, inv.z, oi.z);
+    float tn = fmaxf(hd_max3(fminf(x0, x1), fminf(y0, y1), fminf(z0, z1)), tmin);
+    float tf = fminf(hd_min3(fmaxf(x0, x1), fmaxf(y0, y1), fmaxf(z0, z1)), tmax);
+    tnear = tn;
+    return tn <= tf;
+}
+
+// The next box still in front of the closest hit; true when there is none (the ray is done).
+__device__ __forceinline__ bool sah_pop(SahWalk &T, uint32_t *stk, SahOverflow const &ov) {
+    while (T.sp > 0) {
+        T.sp--;
+        uint32_t w;
+        float tn;
+        if (T.sp < kSahFast) {
+            w = stk[2 * T.sp * kBlock];
+            tn = __uint_as_float(stk[(2 * T.sp + 1) * kBlock]);
+        } else {
+            w = ov.w[T.sp - kSahFast];
+            tn = ov.t[T.sp - kSahFast];
+        }
+        if (tn <= T.cull) {
+            T.w = w;
+            return false;
+        }
+    }
+    return true;
+}
+
+// Visits the interior node T.w: tests its child pair (one 64-byte half line, two loads) and keeps
+// the farther hit child on the stack. Returns true when the ray is done.
+__device__ __forceinline__ bool sah_interior(DevScene const &S, SahWalk &T, uint32_t *stk, SahOverflow &ov) {
+    if (!E8G_CHK(S.check, 2 * static_cast<uint64_t>(T.w) + 2 < S.nnodes, kChkNode, T.w))
+        return true;
+    float4 l0, h0, l1, h1;
+    float4 const *pair = S.nlo.p + 4 * static_cast<size_t>(T.w) + 2;
+    ldg_node(pair, l0, h0);
+    ldg_node(pair + 2, l1, h1);
+    float tn0, tn1;
+    const bool hit0 = sah_slab(l0, h0, T.inv, T.oi, T.tmin, T.cull, tn0);
+    const bool hit1 = sah_slab(l1, h1, T.inv, T.oi, T.tmin, T.cull, tn1);
+    if (!hit0 && !hit1)
+        return sah_pop(T, stk, ov);
+    const uint32_t w0 = sah_word(l0.w, h0.w), w1 = sah_word(l1.w, h1.w);
+    const bool second = hit1 && (!hit0 || tn1 < tn0);
+    if (hit0 && hit1) {
+        if (!E8G_CHK(S.check, T.sp < kStack, kChkStack, T.w))
+            return true;
+        const uint32_t w = second ? w0 : w1;
+        const float tf = second ? tn0 : tn1;
+        if (T.sp < kSahFast) {
+            stk[2 * T.sp * kBlock] = w;
+            stk[(2 * T.sp + 1) * kBlock] = __float_as_uint(tf);
+        } else {
+            ov.w[T.sp - kSahFast] = w;
+            ov.t[T.sp - kSahFast] = tf;
+        }
+        T.sp++;
+    }
+    T.w = second ? w1 : w0;
+    return false;
+}
+
+// Tests the triangles of the leaf T.w. Returns true when the ray is done.
+__device__ __forceinline__ bool sah_leaf(DevScene const &S, SahWalk &T, bool any, uint32_t *stk, SahOverflow const &ov,
+                                         uint32_t *cnt_tris = nullptr) {
+    uint32_t k = T.w & ~kSahLeaf;
+    bool last;
+    do {
+        if (!E8G_CHK(S.check, k < S.ntris, kChkTri, k))
+            break;
+        float4 const *rec = S.tri + 3 * static_cast<size_t>(k);
+        float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
+        k++;
+        if (cnt_tris)
+            (*cnt_tris)++;
+        last = b.w != 0.0f;
+        float t0, b1, b2;
+        if (tri_test(T.o, T.d, a, b, c, T.tmin, T.cull, t0, b1, b2) && t0 < T.h.t) {
+            T.h.t = t0;
+            T.h.tri = __float_as_uint(a.w);
+            T.h.b1 = b1;
+            T.h.b2 = b2;
+            if (any)
+                return true;
+            T.cull = t0;
+        }
+    } while (!last);
+    return sah_pop(T, stk, ov);
+}
+
+// Kernels that walk a warp's rays step by step let lanes that reached a leaf wait until this many of
+// them (or every busy lane) can test triangles together (4 / 8 / 16 lanes: 11.5 / 11.2 / 12.0 ms of
+// tracing in the wavefront's 1080p, 16-spp frame).
+constexpr uint32_t kLeafMin = 8;
+
+// The whole walk of one ray.
 template <bool COUNT>
 __device__ __forceinline__ Hit trace_sah(const DevScene &S, float3 o, float3 d, float tmin, float tmax, bool any,
                                          uint32_t *stk, TraceCounters *cnt) {
-    uint32_t *sn = stk;
-    float *st = reinterpret_cast<float *>(stk + kStack * kBlock);
-    Hit h;
-    h.t = INFINITY;
-    h.tri = 0xFFFFFFFFu;
-    h.b1 = h.b2 = 0.0f;
-    if (S.nnodes == 0)
-        return h;
-    float3 inv = f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-    float cull = tmax;
-    uint32_t link = __float_as_uint(__ldg(&S.nlo[0].w));
-    uint32_t count = __float_as_uint(__ldg(&S.nhi[0].w));
-    int sp = 0;
-    while (true) {
-        if (count == 0) {
-            if (!E8G_CHK(S.check, link + 1 < S.nnodes, kChkNode, link))
-                break;
-            float4 l0 = __ldg(&S.nlo[link]), h0 = __ldg(&S.nhi[link]);
-            float4 l1 = __ldg(&S.nlo[link + 1]), h1 = __ldg(&S.nhi[link + 1]);
+    SahWalk T;
+    SahOverflow ov;
+    sah_begin(S, T, o, d, tmin, tmax);
+    bool done = S.nnodes == 0;
+    while (!done) {
+        while (!done && !T.leaf()) {
             if (COUNT)
                 cnt->nodes += 2;
-            float tn0, tn1;
-            bool hit0 = slab(l0, h0, o, inv, tmin, cull, tn0);
-            bool hit1 = slab(l1, h1, o, inv, tmin, cull, tn1);
-            if (hit0 && hit1) {
-                bool swap = tn1 < tn0;
-                if (!E8G_CHK(S.check, sp < kStack, kChkStack, link))
-                    break;
-                sn[sp * kBlock] = swap ? link : link + 1;
-                st[sp * kBlock] = swap ? tn0 : tn1;
-                sp++;
-                float4 nl = swap ? l1 : l0, nh = swap ? h1 : h0;
-                link = __float_as_uint(nl.w);
-                count = __float_as_uint(nh.w);
-                continue;
-            } else if (hit0 || hit1) {
-                link = __float_as_uint(hit0 ? l0.w : l1.w);
-                count = __float_as_uint(hit0 ? h0.w : h1.w);
-                continue;
-            }
-        } else {
-            if (!E8G_CHK(S.check, link + count <= S.ntris, kChkTri, link + count - 1))
-                count = 0;
-            for (uint32_t k = link; k < link + count; k++) {
-                float4 a = __ldg(&S.tri[3 * k]), b = __ldg(&S.tri[3 * k + 1]), c = __ldg(&S.tri[3 * k + 2]);
-                if (COUNT)
-                    cnt->tris++;
-                float t0, b1, b2;
-                if (tri_test(o, d, a, b, c, tmin, tmax, t0, b1, b2) && t0 < h.t) {
-                    h.t = t0;
-                    h.tri = __float_as_uint(a.w);
-                    h.b1 = b1;
-                    h.b2 = b2;
-                    if (any)
-                        return h;
-                    cull = fminf(t0, tmax);
-                }
-            }
+            done = sah_interior(S, T, stk, ov);
         }
-        // pop the next box still in front of the closest hit
-        bool found = false;
-        while (sp > 0) {
-            sp--;
-            uint32_t node = sn[sp * kBlock];
-            float tn = st[sp * kBlock];
-            if (tn <= cull) {
-                link = __float_as_uint(__ldg(&S.nlo[node].w));
-                count = __float_as_uint(__ldg(&S.nhi[node].w));
-                found = true;
-                break;
-            }
-        }
-        if (!found)
-            break;
+        if (!done)
+            done = sah_leaf(S, T, any, stk, ov, COUNT ? &cnt->tris : nullptr);
     }
-    return h;
+    return T.h;
 }
+
+// Shared words per thread of a layout's traversal stack.
+template <int LAYOUT>
+constexpr int kStackOf = LAYOUT == 0 ? 2 * kSahFast : LAYOUT == 2 ? 2 * kWideStack : LAYOUT == 1 ? kStackWords : 1;
 
 // ---- the reference's tree, visited in the reference's order ----
 // bvh_path_space_layout::intersect / has_intersect (pathspace.cpp:330-456): depth-first with an
@@ -539,91 +635,6 @@ __device__ __forceinline__ bool trace_any(const DevScene &S, float3 o, float3 d,
     if (S.layout == 3)
         return trace_linear<COUNT>(S, o, d, tmin, tmax, true, cnt).tri != 0xFFFFFFFFu;
     return trace_l<0, COUNT>(S, o, d, tmin, tmax, true, stk, cnt).tri != 0xFFFFFFFFu;
-}
-
-// ---- resumable traversal (SAH layout): one node per call ----
-// Lets a persistent trace kernel give a lane a new ray as soon as its ray is done, instead of
-// holding the lane until the warp's slowest ray finishes.
-struct TravState {
-    float3 o, d, inv;
-    float tmin, cull;     // closest: min(best, 1000); any: tmax
-    uint32_t link, count; // current node (count == 0: interior)
-    int sp;
-    bool found;           // any-hit: an occluder was found
-    Hit best;
-};
-
-__device__ __forceinline__ void trav_begin(const DevScene &S, TravState &T, float3 o, float3 d, float tmin, float tmax) {
-    T.o = o;
-    T.d = d;
-    T.inv = f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-    T.tmin = tmin;
-    T.cull = tmax;
-    T.sp = 0;
-    T.found = false;
-    T.best.t = INFINITY;
-    T.best.tri = 0xFFFFFFFFu;
-    T.best.b1 = T.best.b2 = 0.0f;
-    T.link = __float_as_uint(__ldg(&S.nlo[0].w));
-    T.count = __float_as_uint(__ldg(&S.nhi[0].w));
-}
-
-// Visits one node; returns true when the ray is finished (stack empty, or any-hit found).
-// Same tests, order and culling as trace_closest_sah / trace_any_sah.
-template <bool ANY>
-__device__ __forceinline__ bool trav_step(const DevScene &S, TravState &T, uint32_t *stk) {
-    uint32_t *sn = stk;
-    float *st = reinterpret_cast<float *>(stk + kStack * kBlock);
-    if (T.count == 0) {
-        float4 l0 = __ldg(&S.nlo[T.link]), h0 = __ldg(&S.nhi[T.link]);
-        float4 l1 = __ldg(&S.nlo[T.link + 1]), h1 = __ldg(&S.nhi[T.link + 1]);
-        float tn0, tn1;
-        bool hit0 = slab(l0, h0, T.o, T.inv, T.tmin, T.cull, tn0);
-        bool hit1 = slab(l1, h1, T.o, T.inv, T.tmin, T.cull, tn1);
-        if (hit0 && hit1) {
-            bool swap = tn1 < tn0;
-            sn[T.sp * kBlock] = swap ? T.link : T.link + 1;
-            if (!ANY)
-                st[T.sp * kBlock] = swap ? tn0 : tn1;
-            T.sp++;
-            float4 nl = swap ? l1 : l0, nh = swap ? h1 : h0;
-            T.link = __float_as_uint(nl.w);
-            T.count = __float_as_uint(nh.w);
-            return false;
-        }
-        if (hit0 || hit1) {
-            T.link = __float_as_uint(hit0 ? l0.w : l1.w);
-            T.count = __float_as_uint(hit0 ? h0.w : h1.w);
-            return false;
-        }
-    } else {
-        for (uint32_t k = T.link; k < T.link + T.count; k++) {
-            float4 a = __ldg(&S.tri[3 * k]), b = __ldg(&S.tri[3 * k + 1]), c = __ldg(&S.tri[3 * k + 2]);
-            float t0, b1, b2;
-            if (ANY) {
-                if (tri_test(T.o, T.d, a, b, c, T.tmin, T.cull, t0, b1, b2)) {
-                    T.found = true;
-                    return true;
-                }
-            } else if (tri_test(T.o, T.d, a, b, c, T.tmin, 1000.0f, t0, b1, b2) && t0 < T.best.t) {
-                T.best.t = t0;
-                T.best.tri = __float_as_uint(a.w);
-                T.best.b1 = b1;
-                T.best.b2 = b2;
-                T.cull = fminf(t0, 1000.0f);
-            }
-        }
-    }
-    while (T.sp > 0) {
-        T.sp--;
-        uint32_t node = sn[T.sp * kBlock];
-        if (ANY || st[T.sp * kBlock] <= T.cull) {
-            T.link = __float_as_uint(__ldg(&S.nlo[node].w));
-            T.count = __float_as_uint(__ldg(&S.nhi[node].w));
-            return false;
-        }
-    }
-    return true;
 }
 
 // ------------------------------------------------------------------ surfaces ----

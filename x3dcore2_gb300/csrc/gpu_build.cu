@@ -558,7 +558,7 @@ __global__ void k_flat_flags(FlatItem const *items, uint32_t f, uint8_t const *l
 __global__ void k_flat_emit(FlatItem const *items, uint32_t f, uint32_t const *iscan, uint32_t n, int2 const *child,
                             uint8_t const *leaf, uint32_t const *ntris, uint32_t const *icount, float4 const *blo,
                             float4 const *bhi, uint32_t const *order, uint4 const *tidx, float4 const *vpos,
-                            uint32_t const *red, float4 *nlo, float4 *nhi, float4 *tri, FlatItem *next,
+                            uint32_t const *red, NodeHalf<float4> nlo, NodeHalf<float4> nhi, float4 *tri, FlatItem *next,
                             unsigned long long *leaf_stats) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= f)
@@ -587,7 +587,8 @@ __global__ void k_flat_emit(FlatItem const *items, uint32_t f, uint32_t const *i
                 float4 p0 = vpos[g.x], p1 = vpos[g.y], p2 = vpos[g.z];
                 size_t r = 3 * static_cast<size_t>(it.tri_start + k);
                 tri[r] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(t));
-                tri[r + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z, 0.0f);
+                tri[r + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z,
+                                         k + 1 == static_cast<int>(count) ? 1.0f : 0.0f); // the leaf's last record
                 tri[r + 2] = make_float4(p2.x - p0.x, p2.y - p0.y, p2.z - p0.z, 0.0f);
                 k++;
             } else if (sp + 2 <= kLeafStack) {
@@ -710,7 +711,7 @@ __device__ __forceinline__ float wide_area(float4 lo, float4 hi) {
 // Children of one wide node in slot order (binary node ids, kNone for an empty slot).
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
-__device__ void wide_children(uint32_t bn, float4 const *nlo, float4 const *nhi, uint32_t slots[8]) {
+__device__ void wide_children(uint32_t bn, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi, uint32_t slots[8]) {
     uint32_t ch[8];
     int n = 0;
     if (__float_as_uint(nhi[bn].w) == 0) {
@@ -785,7 +786,7 @@ __device__ void wide_children(uint32_t bn, float4 const *nlo, float4 const *nhi,
         slots[s] = child_in[s] < 0 ? kNone : ch[child_in[s]];
 }
 
-__global__ void k_wide_plan(WideItem const *items, uint32_t f, float4 const *nlo, float4 const *nhi,
+__global__ void k_wide_plan(WideItem const *items, uint32_t f, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
                             uint32_t *slots_out, uint32_t *n_int, uint32_t *n_tri) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= f)
@@ -808,8 +809,8 @@ __global__ void k_wide_plan(WideItem const *items, uint32_t f, float4 const *nlo
 }
 
 __global__ void k_wide_emit(WideItem const *items, uint32_t f, uint32_t const *slots_in, uint32_t const *int_scan,
-                            uint32_t const *tri_scan, uint32_t next_base, uint32_t tri_running, float4 const *nlo,
-                            float4 const *nhi, float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide,
+                            uint32_t const *tri_scan, uint32_t next_base, uint32_t tri_running, NodeHalf<const float4> nlo,
+                            NodeHalf<const float4> nhi, float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide,
                             WideItem *next) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= f)

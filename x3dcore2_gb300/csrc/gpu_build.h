@@ -16,7 +16,7 @@ struct GpuBuildIn {
     int num_sms;
     void *scratch;       // gpu_build_scratch_bytes(num_tris) bytes of device memory
     void *host_pinned;   // 32 bytes of pinned host memory
-    float4 *nlo, *nhi;   // 2 * num_tris nodes each
+    NodeHalf<float4> nlo, nhi; // 2 * num_tris nodes
     float4 *tri;         // 3 * num_tris triangle records
 };
 
@@ -36,7 +36,7 @@ cudaError_t gpu_build_sah_pairs(GpuBuildIn const &in, GpuBuildOut &out, cudaStre
 // device: the same nodes, byte for byte, as the host collapse (bvh_wide.cpp) of that tree. The
 // triangle records are reordered in place. Uses the scratch of the build that made the tree.
 struct GpuWideIn {
-    float4 const *nlo, *nhi; // the binary tree
+    NodeHalf<const float4> nlo, nhi; // the binary tree
     float4 *tri;             // its triangle records; the wide order on success
     uint32_t num_tris;
     float max_abs;           // largest |coordinate| of the vertices and the camera

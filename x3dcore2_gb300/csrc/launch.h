@@ -17,11 +17,10 @@ void launch_camera_rays(DevScene const &S, uint32_t w, uint32_t h, float *rays6,
 // pixel[i] = i, samples[i] = sample.
 void launch_first_hits_rays(DevScene const &S, float const *rays6, uint32_t n, FirstHit *out, uint32_t sample,
                             uint32_t *pixel, uint32_t *samples, cudaStream_t st);
-void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, float *hits5, cudaStream_t st);
+void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, float *hits5, int num_sms,
+                          cudaStream_t st);
 void launch_trace_any(DevScene const &S, float const *rays6, float const *tmin, float const *tmax, uint32_t n,
-                      uint8_t *occ, cudaStream_t st);
-void launch_trace_closest_counted(DevScene const &S, float const *rays6, uint32_t n, float *hits5,
-                                  unsigned long long *counters, cudaStream_t st);
+                      uint8_t *occ, int num_sms, cudaStream_t st);
 void launch_resolve(float4 const *accum, uint32_t npix, float inv_spp, float *rgba, cudaStream_t st);
 // Firefly clamp of K sample-major per-sample images (W*H rgb each), added to accum in sample order.
 void launch_firefly(float const *est, uint32_t K, uint32_t w, uint32_t h, float4 *accum, cudaStream_t st);

@@ -279,7 +279,7 @@ template <class R, bool COUNT, int LAYOUT>
 __global__ void __launch_bounds__(kBlock, kMegaBlocksPerSm) k_mega(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh,
                                                  float4 *accum, float *path_rgb, unsigned long long *work,
                                                  unsigned long long *counters) {
-    __shared__ uint32_t stk_all[kStackWords * kBlock];
+    __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
     uint32_t *sn = stk_all + threadIdx.x;
     TraceCounters cnt{0, 0};
     uint32_t rays = 0;
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kBlock, kMegaBlocksPerSm) k_mega(DevScene S, R
 template <class R, int LAYOUT>
 __global__ void __launch_bounds__(kBlock, kMegaBlocksPerSm) k_plain(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh,
                                                                    float4 *accum, float *path_rgb) {
-    __shared__ uint32_t stk_all[kStackWords * kBlock];
+    __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
     uint32_t *sn = stk_all + threadIdx.x;
     uint64_t idx = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x;
     uint32_t pixel, sample, out;
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kBlock, kMegaBlocksPerSm) k_plain(DevScene S, 
 template <class R>
 __global__ void __launch_bounds__(kBlock, kMegaBlocksPerSm) k_mega_batch(BatchDev B, FirstHit const *__restrict__ fh_all, float4 *accum_all,
                                                        unsigned long long *work) {
-    __shared__ uint32_t stk_all[kStackWords * kBlock];
+    __shared__ uint32_t stk_all[kStackOf<0> * kBlock];
     uint32_t *sn = stk_all + threadIdx.x;
     TraceCounters cnt{0, 0};
     uint32_t rays = 0;

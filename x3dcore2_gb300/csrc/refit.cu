@@ -103,7 +103,8 @@ __global__ void __launch_bounds__(kRefitBlock) k_refit_tris(float4 *tri, uint4 c
         uint4 g = tidx[__float_as_uint(w)];
         float4 p0 = vpos[g.x], p1 = vpos[g.y], p2 = vpos[g.z];
         tri[3 * static_cast<size_t>(k)] = make_float4(p0.x, p0.y, p0.z, w);
-        tri[3 * static_cast<size_t>(k) + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z, 0.0f);
+        float last = tri[3 * static_cast<size_t>(k) + 1].w; // the leaf's end mark stays
+        tri[3 * static_cast<size_t>(k) + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z, last);
         tri[3 * static_cast<size_t>(k) + 2] = make_float4(p2.x - p0.x, p2.y - p0.y, p2.z - p0.z, 0.0f);
         tlo[k] = make_float4(fminf(fminf(p0.x, p1.x), p2.x), fminf(fminf(p0.y, p1.y), p2.y),
                              fminf(fminf(p0.z, p1.z), p2.z), 0.0f);
@@ -150,7 +151,7 @@ __device__ __forceinline__ void range_box(float4 const *tlo, float4 const *thi, 
 
 // ---------------------------------------------------------------- SAH child pairs ----
 
-__global__ void k_parents_pairs(float4 const *nlo, float4 const *nhi, uint32_t nn, uint32_t *parent) {
+__global__ void k_parents_pairs(NodeHalf<const float4> nlo, NodeHalf<const float4> nhi, uint32_t nn, uint32_t *parent) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nn || __float_as_uint(nhi[i].w) != 0)
         return;
@@ -159,7 +160,7 @@ __global__ void k_parents_pairs(float4 const *nlo, float4 const *nhi, uint32_t n
     parent[link + 1] = i;
 }
 
-__device__ __forceinline__ void store_pair_node(float4 *nlo, float4 *nhi, uint32_t n, float const lo[3],
+__device__ __forceinline__ void store_pair_node(NodeHalf<float4> nlo, NodeHalf<float4> nhi, uint32_t n, float const lo[3],
                                                 float const hi[3], float eps, float4 *ex_lo, float4 *ex_hi) {
     ex_lo[n] = make_float4(lo[0], lo[1], lo[2], 0.0f);
     ex_hi[n] = make_float4(hi[0], hi[1], hi[2], 0.0f);
@@ -169,7 +170,7 @@ __device__ __forceinline__ void store_pair_node(float4 *nlo, float4 *nhi, uint32
 }
 
 __global__ void __launch_bounds__(kRefitBlock)
-    k_refit_pairs(float4 *nlo, float4 *nhi, uint32_t nn, float4 const *tlo, float4 const *thi, uint32_t const *parent,
+    k_refit_pairs(NodeHalf<float4> nlo, NodeHalf<float4> nhi, uint32_t nn, float4 const *tlo, float4 const *thi, uint32_t const *parent,
                   uint32_t *counter, float4 *ex_lo, float4 *ex_hi, uint32_t const *red) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nn)
@@ -344,7 +345,7 @@ void launch_refit(DevScene const &S, RefitScratch const &R, uint32_t nv, float c
                                                                               R.red, cam_abs);
         }
     } else
-        k_refit_pairs<<<blocks_for(nn), kRefitBlock, 0, st>>>(const_cast<float4 *>(S.nlo), const_cast<float4 *>(S.nhi),
+        k_refit_pairs<<<blocks_for(nn), kRefitBlock, 0, st>>>(NodeHalf<float4>{const_cast<float4 *>(S.nlo.p)}, NodeHalf<float4>{const_cast<float4 *>(S.nhi.p)},
                                                                 nn, R.tlo, R.thi, R.parent, R.counter, R.ex_lo,
                                                                 R.ex_hi, R.red);
 }

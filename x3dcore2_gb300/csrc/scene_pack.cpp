@@ -213,6 +213,15 @@ void write_tri_records(packed_scene &s, std::vector<float> const &p3, std::vecto
         }
         std::memcpy(&dst[3], &t, 4);
     }
+    if (s.layout != 0)
+        return;
+    for (size_t n = 0; n < s.bvh.hi.size() / 4; n++) { // the last record of every leaf of child pairs is marked
+        uint32_t link, count;
+        std::memcpy(&link, &s.bvh.lo[4 * n + 3], 4);
+        std::memcpy(&count, &s.bvh.hi[4 * n + 3], 4);
+        if (count)
+            s.tri[12 * (static_cast<size_t>(link) + count - 1) + 7] = 1.0f;
+    }
 }
 
 } // namespace

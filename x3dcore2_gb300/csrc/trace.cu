@@ -1,18 +1,22 @@
 // Primary-hit, ray-batch traversal and resolve kernels.
 #include "launch.h"
 
+#include <algorithm>
+
 namespace e8g {
 
 // compute_first_hit (pathtracer.cpp:456-472): camera ray, closest hit, back-facing hits become
 // misses, emitter lookup.
-__global__ void __launch_bounds__(kBlock) k_first_hits(DevScene S, uint32_t w, uint32_t h, FirstHit *out) {
-    __shared__ uint32_t stk[kStackWords * kBlock];
+template <int LAYOUT>
+__global__ void __launch_bounds__(kBlock) k_first_hits(const __grid_constant__ DevScene S, uint32_t w, uint32_t h,
+                                                       FirstHit *out) {
+    __shared__ uint32_t stk[kStackOf<LAYOUT> * kBlock];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= w * h)
         return;
     float3 o, d;
     camera_ray(S.cam, i % w, i / w, w, h, o, d);
-    Hit hit = trace_closest<false>(S, o, d, stk + threadIdx.x, nullptr);
+    Hit hit = trace_l<LAYOUT, false>(S, o, d, 1e-4f, 1000.0f, false, stk + threadIdx.x, nullptr);
     FirstHit f;
     f.d = make_float4(d.x, d.y, d.z, 0.0f);
     int32_t mesh = -1, light = -1;
@@ -32,15 +36,16 @@ __global__ void __launch_bounds__(kBlock) k_first_hits(DevScene S, uint32_t w, u
 }
 
 // compute_first_hit for explicit rays: ray i's first hit into out[i].
-__global__ void __launch_bounds__(kBlock) k_first_hits_rays(DevScene S, float const *rays6, uint32_t n,
-                                                             FirstHit *out) {
-    __shared__ uint32_t stk[kStackWords * kBlock];
+template <int LAYOUT>
+__global__ void __launch_bounds__(kBlock) k_first_hits_rays(const __grid_constant__ DevScene S, float const *rays6,
+                                                             uint32_t n, FirstHit *out) {
+    __shared__ uint32_t stk[kStackOf<LAYOUT> * kBlock];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
     float3 o = f3(rays6[6 * i], rays6[6 * i + 1], rays6[6 * i + 2]);
     float3 d = f3(rays6[6 * i + 3], rays6[6 * i + 4], rays6[6 * i + 5]);
-    Hit hit = trace_closest<false>(S, o, d, stk + threadIdx.x, nullptr);
+    Hit hit = trace_l<LAYOUT, false>(S, o, d, 1e-4f, 1000.0f, false, stk + threadIdx.x, nullptr);
     FirstHit f;
     f.d = make_float4(d.x, d.y, d.z, 0.0f);
     int32_t mesh = -1, light = -1;
@@ -83,54 +88,111 @@ __global__ void k_camera_rays(DevScene S, uint32_t w, uint32_t h, float *rays6) 
     r[5] = d.z;
 }
 
-template <bool COUNT>
-__global__ void __launch_bounds__(kBlock) k_trace_closest(DevScene S, float const *rays6, uint32_t n, float *hits5,
-                                                          unsigned long long *counters) {
-    __shared__ uint32_t stk[kStackWords * kBlock];
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    TraceCounters c{0, 0};
-    if (i < n) {
-        float const *r = rays6 + 6 * static_cast<size_t>(i);
-        float3 o = f3(r[0], r[1], r[2]), d = f3(r[3], r[4], r[5]);
-        Hit h = trace_closest<COUNT>(S, o, d, stk + threadIdx.x, &c);
-        float *out = hits5 + 5 * static_cast<size_t>(i);
-        if (h.tri == 0xFFFFFFFFu) {
-            out[0] = 0.0f;
-            out[1] = __int_as_float(-1);
-            out[2] = __int_as_float(-1);
-            out[3] = 0.0f;
-            out[4] = 0.0f;
-        } else {
-            uint4 ti = __ldg(&S.tidx[h.tri]);
-            out[0] = h.t;
-            out[1] = __int_as_float(static_cast<int>(ti.w));
-            out[2] = __int_as_float(static_cast<int>(h.tri - __ldg(&S.mesh_toff[ti.w])));
-            out[3] = h.b1;
-            out[4] = h.b2;
-        }
+__device__ __forceinline__ void store_hit(DevScene const &S, Hit const &h, float *out) {
+    if (h.tri == 0xFFFFFFFFu) {
+        out[0] = 0.0f;
+        out[1] = __int_as_float(-1);
+        out[2] = __int_as_float(-1);
+        out[3] = 0.0f;
+        out[4] = 0.0f;
+    } else {
+        uint4 ti = __ldg(&S.tidx[h.tri]);
+        out[0] = h.t;
+        out[1] = __int_as_float(static_cast<int>(ti.w));
+        out[2] = __int_as_float(static_cast<int>(h.tri - __ldg(&S.mesh_toff[ti.w])));
+        out[3] = h.b1;
+        out[4] = h.b2;
     }
-    if (COUNT) {
-        unsigned long long a = c.nodes, b = c.tris;
-        for (int off = 16; off > 0; off >>= 1) {
-            a += __shfl_down_sync(~0u, a, off);
-            b += __shfl_down_sync(~0u, b, off);
+}
+
+// Ray batches on the SAH pairs and the eight-wide tree. Each warp owns `chunk` consecutive rays and
+// gives an idle lane the next of them once kRayRefill lanes are idle: a batch's rays have no order,
+// and with one ray per lane the warp waits for its longest (3.3 of 32 lanes active on 300,000 random
+// rays against the 1.3M-triangle icosphere). The chunks are fixed, so calls on several streams
+// share nothing. ANY: any-hit on [tmin[i], tmax[i]] into occ, else the closest hit into hits5.
+constexpr uint32_t kRayRefill = 8;
+constexpr int kRayBlocks = 8; // blocks of 128 threads per SM (64 registers), as the wavefront's trace kernel
+
+template <int LAYOUT, bool ANY>
+__global__ void __launch_bounds__(kBlock, kRayBlocks)
+    k_trace_rays(const __grid_constant__ DevScene S, float const *__restrict__ rays6, float const *__restrict__ tmin,
+                 float const *__restrict__ tmax, uint32_t n, uint32_t chunk, float *hits5, uint8_t *occ) {
+    __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
+    uint32_t *stk = stk_all + threadIdx.x;
+    const uint32_t lane = lane_id();
+    const uint64_t first = static_cast<uint64_t>(blockIdx.x * (kBlock / 32) + threadIdx.x / 32) * chunk;
+    if (first >= n)
+        return;
+    uint32_t next = static_cast<uint32_t>(first); // the warp's next ray, up to `end` (the same in every lane)
+    const uint32_t end = static_cast<uint32_t>(first + chunk < n ? first + chunk : n);
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    uint32_t cur = kNone;
+    const WideView WV{S.wnodes, S.tri, S.nnodes, S.ntris, S.check};
+    SahWalk T;
+    SahOverflow ov;
+    WideTrav TW;
+    while (true) {
+        uint32_t busy = __ballot_sync(~0u, cur != kNone);
+        const uint32_t idle = ~busy;
+        if (next < end && (busy == 0 || static_cast<uint32_t>(__popc(idle)) >= kRayRefill)) {
+            const uint32_t r = __popc(idle & ((1u << lane) - 1u));
+            if (cur == kNone && r < end - next) {
+                cur = next + r;
+                float const *q = rays6 + 6 * static_cast<size_t>(cur);
+                float3 o = f3(q[0], q[1], q[2]), d = f3(q[3], q[4], q[5]);
+                float t0 = ANY ? tmin[cur] : 1e-4f, t1 = ANY ? tmax[cur] : 1000.0f;
+                if (LAYOUT == 2)
+                    wide_begin(TW, o, d, t0, t1, ANY);
+                else
+                    sah_begin(S, T, o, d, t0, t1);
+            }
+            const uint32_t k = static_cast<uint32_t>(__popc(idle));
+            next = k < end - next ? next + k : end;
+            busy = __ballot_sync(~0u, cur != kNone);
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&counters[1], a);
-            atomicAdd(&counters[2], b);
+        if (busy == 0)
+            break;
+        bool done = false;
+        if (S.nnodes == 0) {
+            done = cur != kNone;
+        } else if (LAYOUT == 2) {
+            if (cur != kNone)
+                done = wide_step(WV, TW, stk, kBlock, nullptr, nullptr);
+        } else {
+            if (cur != kNone && !T.leaf())
+                done = sah_interior(S, T, stk, ov);
+            const bool leaf = cur != kNone && !done && T.leaf();
+            const uint32_t lf = __ballot_sync(~0u, leaf);
+            if (lf && (static_cast<uint32_t>(__popc(lf)) >= kLeafMin || lf == busy)) {
+                if (leaf)
+                    done = sah_leaf(S, T, ANY, stk, ov);
+            }
+        }
+        if (done) {
+            const Hit h = LAYOUT == 2 ? TW.h : T.h;
+            if (ANY)
+                occ[cur] = h.tri != 0xFFFFFFFFu ? 1 : 0;
+            else
+                store_hit(S, h, hits5 + 5 * static_cast<size_t>(cur));
+            cur = kNone;
         }
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_trace_any(DevScene S, float const *rays6, float const *tmin,
-                                                      float const *tmax, uint32_t n, uint8_t *occ) {
+// One ray per thread: the reference's tree and the linear layout.
+template <bool ANY>
+__global__ void __launch_bounds__(kBlock) k_trace_plain(DevScene S, float const *rays6, float const *tmin,
+                                                        float const *tmax, uint32_t n, float *hits5, uint8_t *occ) {
     __shared__ uint32_t stk[kStackWords * kBlock];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
     float const *r = rays6 + 6 * static_cast<size_t>(i);
     float3 o = f3(r[0], r[1], r[2]), d = f3(r[3], r[4], r[5]);
-    occ[i] = trace_any<false>(S, o, d, tmin[i], tmax[i], stk + threadIdx.x, nullptr) ? 1 : 0;
+    if (ANY)
+        occ[i] = trace_any<false>(S, o, d, tmin[i], tmax[i], stk + threadIdx.x, nullptr) ? 1 : 0;
+    else
+        store_hit(S, trace_closest<false>(S, o, d, stk + threadIdx.x, nullptr), hits5 + 5 * static_cast<size_t>(i));
 }
 
 __global__ void k_resolve(float4 const *accum, uint32_t npix, float inv_spp, float *rgba) {
@@ -189,31 +251,48 @@ __global__ void k_firefly(float const *__restrict__ est, uint32_t K, uint32_t w,
 static inline int blocks(uint32_t n, int b) { return static_cast<int>((n + b - 1) / b); }
 
 void launch_first_hits(DevScene const &S, uint32_t w, uint32_t h, FirstHit *out, cudaStream_t st) {
-    k_first_hits<<<blocks(w * h, kBlock), kBlock, 0, st>>>(S, w, h, out);
+    auto *kern = S.layout == 0 ? k_first_hits<0> : S.layout == 1 ? k_first_hits<1> : S.layout == 2 ? k_first_hits<2> : k_first_hits<3>;
+    kern<<<blocks(w * h, kBlock), kBlock, 0, st>>>(S, w, h, out);
 }
 void launch_first_hits_rays(DevScene const &S, float const *rays6, uint32_t n, FirstHit *out, uint32_t sample,
                             uint32_t *pixel, uint32_t *samples, cudaStream_t st) {
     if (!n)
         return;
-    k_first_hits_rays<<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, n, out);
+    auto *kern = S.layout == 0   ? k_first_hits_rays<0>
+                 : S.layout == 1 ? k_first_hits_rays<1>
+                 : S.layout == 2 ? k_first_hits_rays<2>
+                                 : k_first_hits_rays<3>;
+    kern<<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, n, out);
     k_ray_lists<<<blocks(n, 256), 256, 0, st>>>(n, sample, pixel, samples);
 }
 void launch_camera_rays(DevScene const &S, uint32_t w, uint32_t h, float *rays6, cudaStream_t st) {
     k_camera_rays<<<blocks(w * h, 256), 256, 0, st>>>(S, w, h, rays6);
 }
-void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, float *hits5, cudaStream_t st) {
-    if (n)
-        k_trace_closest<false><<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, n, hits5, nullptr);
+// Rays per warp: one per lane while the batch is smaller than the GPU's lanes, else an equal share
+// of the batch for every resident warp (a multiple of 32).
+template <bool ANY>
+static void trace_rays(DevScene const &S, float const *rays6, float const *tmin, float const *tmax, uint32_t n,
+                       float *hits5, uint8_t *occ, int num_sms, cudaStream_t st) {
+    if (!n)
+        return;
+    if (S.layout != 0 && S.layout != 2) {
+        k_trace_plain<ANY><<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, tmin, tmax, n, hits5, occ);
+        return;
+    }
+    const uint32_t warps = static_cast<uint32_t>(num_sms) * kRayBlocks * (kBlock / 32);
+    const uint32_t chunk = std::max(32u, ((n - 1) / warps + 1 + 31) / 32 * 32);
+    const uint32_t g = ((n - 1) / chunk) / (kBlock / 32) + 1;
+    if (S.layout == 2)
+        k_trace_rays<2, ANY><<<g, kBlock, 0, st>>>(S, rays6, tmin, tmax, n, chunk, hits5, occ);
+    else
+        k_trace_rays<0, ANY><<<g, kBlock, 0, st>>>(S, rays6, tmin, tmax, n, chunk, hits5, occ);
 }
-void launch_trace_closest_counted(DevScene const &S, float const *rays6, uint32_t n, float *hits5,
-                                  unsigned long long *counters, cudaStream_t st) {
-    if (n)
-        k_trace_closest<true><<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, n, hits5, counters);
+void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, float *hits5, int num_sms, cudaStream_t st) {
+    trace_rays<false>(S, rays6, nullptr, nullptr, n, hits5, nullptr, num_sms, st);
 }
 void launch_trace_any(DevScene const &S, float const *rays6, float const *tmin, float const *tmax, uint32_t n,
-                      uint8_t *occ, cudaStream_t st) {
-    if (n)
-        k_trace_any<<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, tmin, tmax, n, occ);
+                      uint8_t *occ, int num_sms, cudaStream_t st) {
+    trace_rays<true>(S, rays6, tmin, tmax, n, nullptr, occ, num_sms, st);
 }
 void launch_resolve(float4 const *accum, uint32_t npix, float inv_spp, float *rgba, cudaStream_t st) {
     k_resolve<<<blocks(npix, 256), 256, 0, st>>>(accum, npix, inv_spp, rgba);

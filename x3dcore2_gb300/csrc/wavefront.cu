@@ -377,15 +377,11 @@ __global__ void __launch_bounds__(256, 8)
     }
 }
 
-// Persistent trace kernel with per-lane dynamic fetch: a lane whose ray is finished takes the
-// next queue entry; lanes are refilled together (one atomic) once at least `threshold` of them
-// are idle, or when none is busy. WIDE: the eight-wide tree (one node visit per step), else the
-// SAH child pairs.
-// The wide tree's stack takes 2 * kWideStack words per thread (16 KB per block), so its kernels
-// fit eight blocks per SM when they are held to 64 registers. Measured on the 1080p, 64-spp
+// Resident blocks of the trace kernels. The wide tree's stack takes 2 * kWideStack words per thread
+// (16 KB per block), so they fit eight blocks per SM when they are held to 64 registers. Measured on the 1080p, 64-spp
 // frame of the 1.3M-triangle scene: 6 blocks (75 registers, no spills) 72.1 ms, 7 (70) 67.9 ms,
 // 8 (64) 66.3 ms, 9 (56, 64-byte spills) 69.9 ms, 10 (48) 76.9 ms.
-constexpr int kWfWideBlocks = 8;
+constexpr int kWfTraceBlocks = 8;
 
 // Queue entries a warp reserves with one atomic on the queue head; its idle lanes take entries
 // from that reserve first. Measured on the 1080p, 64-spp frame: one atomic per refill (the
@@ -394,115 +390,21 @@ constexpr int kWfWideBlocks = 8;
 // make refills cheap enough for warps to refill sooner.
 constexpr uint32_t kWarpChunk = 32;
 
-template <bool ANY, bool WIDE>
-__global__ void __launch_bounds__(kBlock, WIDE ? kWfWideBlocks : 1)
-    k_wf_trace_dyn(DevScene S, RenderArgs A, WfSlots W, Counters *cnt, float4 *accum, float *path_rgb,
-                   uint32_t threshold) {
-    __shared__ uint32_t stk_all[(WIDE ? 2 * kWideStack : kStackWords) * kBlock];
-    uint32_t *stk = stk_all + threadIdx.x;
-    const uint32_t n = ANY ? cnt->shadow_n : cnt->ext_n;
-    uint32_t *head = ANY ? &cnt->shadow_head : &cnt->ext_head;
-    const uint32_t lane = lane_id();
-    constexpr uint32_t kNone = 0xFFFFFFFFu;
-    const WideView WV{S.wnodes, S.tri, S.nnodes, S.ntris, S.check};
-    uint32_t q = kNone;
-    bool exhausted = false;  // the same in every lane: the queue and the warp's reserve are empty
-    uint32_t wb = 0, we = 0; // the warp's reserved entries [wb, we)
-    bool gdrained = false;
-    uint32_t qw = 0; // the lane's ray's output (shadow) or slot (extension), kept from the refill
-    TravState T;
-    WideTrav TW;
-    while (true) {
-        bool idle = q == kNone && !exhausted;
-        uint32_t im = __ballot_sync(~0u, idle);
-        uint32_t busy = __ballot_sync(~0u, q != kNone);
-        if (im && (__popc(im) >= threshold || busy == 0)) {
-            const uint32_t k = static_cast<uint32_t>(__popc(im));
-            const uint32_t avail = we - wb;
-            uint32_t nb = 0, ne = 0;
-            if (avail < k && !gdrained) {
-                uint32_t want = kWarpChunk > k ? kWarpChunk : k;
-                if (lane == 0)
-                    nb = atomicAdd(head, want);
-                nb = __shfl_sync(~0u, nb, 0);
-                ne = nb + want < n ? nb + want : n;
-                if (nb >= n) {
-                    gdrained = true;
-                    ne = nb;
-                }
-            }
-            const uint32_t r = __popc(im & ((1u << lane) - 1u));
-            uint32_t qq = kNone;
-            if (r < avail)
-                qq = wb + r;
-            else if (r - avail < ne - nb)
-                qq = nb + (r - avail);
-            const uint32_t t_old = k < avail ? k : avail;
-            wb += t_old;
-            if (ne > nb) {
-                uint32_t t_new = k - t_old < ne - nb ? k - t_old : ne - nb;
-                wb = nb + t_new;
-                we = ne;
-            }
-            exhausted = gdrained && wb >= we;
-            if (idle) {
-                if (qq != kNone) {
-                    q = qq;
-                    float3 ro, rd;
-                    float tmax;
-                    if (ANY) {
-                        float4 so = W.sh_o[q], sd = W.sh_d[q];
-                        ro = xyz(so);
-                        rd = xyz(sd);
-                        tmax = sd.w;
-                        qw = __float_as_uint(so.w);
-                    } else {
-                        float4 eo = W.ext_o[q];
-                        ro = xyz(eo);
-                        rd = xyz(W.ext_d[q]);
-                        tmax = 1000.0f;
-                        qw = __float_as_uint(eo.w);
-                    }
-                    if (WIDE)
-                        wide_begin(TW, ro, rd, 1e-4f, tmax, ANY);
-                    else
-                        trav_begin(S, T, ro, rd, 1e-4f, tmax);
-                }
-            }
-            busy = __ballot_sync(~0u, q != kNone);
-        }
-        if (busy == 0) {
-            if (__ballot_sync(~0u, !exhausted) == 0)
-                break;
-            continue;
-        }
-        if (q == kNone)
-            continue;
-        bool done = WIDE ? wide_step(WV, TW, stk, kBlock, nullptr, nullptr) : trav_step<ANY>(S, T, stk);
-        if (done) {
-            if (ANY) {
-                bool occluded = WIDE ? TW.h.tri != 0xFFFFFFFFu : T.found;
-                if (!occluded)
-                    emit_to(A, accum, path_rgb, qw, xyz(W.sh_c[q]));
-            } else {
-                Hit b = WIDE ? TW.h : T.best;
-                W.hit[qw] = make_float4(b.t, __uint_as_float(b.tri), b.b1, b.b2);
-            }
-            q = kNone;
-        }
-    }
-}
-
-// Both queues of a bounce in one launch on the eight-wide tree: queue positions below ext_n are
-// extension rays (closest hit), the rest shadow rays (any hit), so a bounce has one kernel tail
-// instead of two. Per-lane dynamic fetch like k_wf_trace_dyn's, from warp reserves. MULTI: each
-// ray carries its scene index (w of its direction or of its contribution) and traces that
-// scene's tree.
-template <bool MULTI>
-__global__ void __launch_bounds__(kBlock, kWfWideBlocks)
-    k_wf_trace_wide_both(const __grid_constant__ DevScene S0, RenderArgs A, BatchDev B, WfSlots W, Counters *cnt,
-                         float4 *accum, float *path_rgb, uint32_t threshold) {
-    __shared__ uint32_t stk_all[2 * kWideStack * kBlock];
+// Both queues of a bounce in one launch, so that a bounce has one kernel tail instead of two:
+// queue positions below ext_n are extension rays (closest hit), the rest shadow rays (any hit).
+// Persistent, with per-lane dynamic fetch: idle lanes are refilled together, from the warp's
+// reserve, once at least `threshold` of them are idle. WIDE: the eight-wide tree, else the SAH
+// child pairs, whose leaves wait for kLeafMin lanes. MULTI: each ray carries its scene index (w of
+// its direction or of its contribution) and traces that scene's tree.
+// Bound by issue slots and the L1 data pipe together (58% each in the SAH pairs' first bounce, 15
+// of 32 lanes active). On the 1080p, 16-spp frame of the 1.3M-triangle scene with 2^23 slots the
+// SAH pairs trace in 10.7 ms (two kernels of one node a step with 32 KB stacks: 17.5 ms), the
+// eight-wide tree in 9.7.
+template <bool MULTI, bool WIDE>
+__global__ void __launch_bounds__(kBlock, kWfTraceBlocks)
+    k_wf_trace_both(const __grid_constant__ DevScene S0, RenderArgs A, BatchDev B, WfSlots W, Counters *cnt,
+                    float4 *accum, float *path_rgb, uint32_t threshold) {
+    __shared__ uint32_t stk_all[kStackOf<WIDE ? 2 : 0> * kBlock];
     uint32_t *stk = stk_all + threadIdx.x;
     const uint32_t n_ext = cnt->ext_n, n = n_ext + cnt->shadow_n;
     uint32_t *head = &cnt->ext_head;
@@ -517,6 +419,8 @@ __global__ void __launch_bounds__(kBlock, kWfWideBlocks)
     // from the queue at the ray's end cost 3.6% of the kernel's time
     uint32_t qw = 0;
     WideTrav T;
+    SahWalk TS;
+    SahOverflow ov;
     while (true) {
         uint32_t busy = __ballot_sync(~0u, q != kNone);
         uint32_t im = drained ? 0u : ~busy; // idle lanes
@@ -557,12 +461,18 @@ __global__ void __launch_bounds__(kBlock, kWfWideBlocks)
                         float4 ed = W.ext_d[q], eo = W.ext_o[q];
                         sid = __float_as_uint(ed.w);
                         qw = __float_as_uint(eo.w);
-                        wide_begin(T, xyz(eo), xyz(ed), 1e-4f, 1000.0f, false);
+                        if (WIDE)
+                            wide_begin(T, xyz(eo), xyz(ed), 1e-4f, 1000.0f, false);
+                        else
+                            sah_begin(S0, TS, xyz(eo), xyz(ed), 1e-4f, 1000.0f);
                     } else {
                         float4 sd = W.sh_d[q - n_ext], so = W.sh_o[q - n_ext];
                         sid = MULTI ? __float_as_uint(W.sh_c[q - n_ext].w) : 0;
                         qw = __float_as_uint(so.w);
-                        wide_begin(T, xyz(so), xyz(sd), 1e-4f, sd.w, true);
+                        if (WIDE)
+                            wide_begin(T, xyz(so), xyz(sd), 1e-4f, sd.w, true);
+                        else
+                            sah_begin(S0, TS, xyz(so), xyz(sd), 1e-4f, sd.w);
                     }
                     if (MULTI) {
                         DevScene const &S = B.scenes[sid];
@@ -577,14 +487,28 @@ __global__ void __launch_bounds__(kBlock, kWfWideBlocks)
                 break;
             continue;
         }
-        if (q == kNone)
-            continue;
-        if (wide_step(WV, T, stk, kBlock, nullptr, nullptr)) {
+        bool done = false;
+        if (WIDE) {
+            if (q == kNone)
+                continue;
+            done = wide_step(WV, T, stk, kBlock, nullptr, nullptr);
+        } else {
+            if (q != kNone && !TS.leaf())
+                done = sah_interior(S0, TS, stk, ov);
+            const bool leaf = q != kNone && !done && TS.leaf();
+            const uint32_t lf = __ballot_sync(~0u, leaf);
+            if (lf && (static_cast<uint32_t>(__popc(lf)) >= kLeafMin || lf == busy)) {
+                if (leaf)
+                    done = sah_leaf(S0, TS, q >= n_ext, stk, ov);
+            }
+        }
+        if (done) {
+            const Hit h = WIDE ? T.h : TS.h;
             if (q < n_ext) {
                 uint32_t slot = qw;
                 if (E8G_CHK(S0.check, slot < W.capacity, kChkSlot, slot))
-                    W.hit[slot] = make_float4(T.h.t, __uint_as_float(T.h.tri), T.h.b1, T.h.b2);
-            } else if (T.h.tri == 0xFFFFFFFFu) {
+                    W.hit[slot] = make_float4(h.t, __uint_as_float(h.tri), h.b1, h.b2);
+            } else if (h.tri == 0xFFFFFFFFu) {
                 uint32_t sq = q - n_ext;
                 emit_to(A, accum, path_rgb, qw, xyz(W.sh_c[sq]));
             }
@@ -652,11 +576,11 @@ size_t wf_total_bytes(uint32_t capacity) {
 int wf_trace_blocks_per_sm(uint32_t layout, uint32_t threshold) {
     int a = 0, b = 0;
     if (threshold > 0 && layout == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_wf_trace_dyn<true, false>, kBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_wf_trace_dyn<false, false>, kBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_wf_trace_both<false, false>, kBlock, 0);
+        b = a;
     } else if (threshold > 0 && layout == 2) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_wf_trace_wide_both<false>, kBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_wf_trace_wide_both<true>, kBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_wf_trace_both<false, true>, kBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_wf_trace_both<true, true>, kBlock, 0);
     } else {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_wf_extend, kBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_wf_shadow, kBlock, 0);
@@ -739,7 +663,7 @@ void wf_enqueue_bounce(DevScene const &S, RenderArgs const &A, FirstHit const *f
             k_wf_shade<RngPhilox, true, 256, 4, false><<<shade_grid, 256, 0, st>>>(S, A, *B, fh, W, cnt, accum, nullptr,
                                                                                     total_paths);
         mark(1);
-        k_wf_trace_wide_both<true><<<trace_grid, kBlock, 0, st>>>(S, A, *B, W, cnt, accum, nullptr, threshold);
+        k_wf_trace_both<true, true><<<trace_grid, kBlock, 0, st>>>(S, A, *B, W, cnt, accum, nullptr, threshold);
         mark(2);
         return;
     }
@@ -750,10 +674,9 @@ void wf_enqueue_bounce(DevScene const &S, RenderArgs const &A, FirstHit const *f
         launch_shade<RngPhilox>(shade_variant, shade_grid, st, S, A, fh, W, cnt, accum, path_rgb, total_paths);
     mark(1);
     if (threshold > 0 && S.layout == 0) {
-        k_wf_trace_dyn<true, false><<<trace_grid, kBlock, 0, st>>>(S, A, W, cnt, accum, path_rgb, threshold);
-        k_wf_trace_dyn<false, false><<<trace_grid, kBlock, 0, st>>>(S, A, W, cnt, accum, path_rgb, threshold);
+        k_wf_trace_both<false, false><<<trace_grid, kBlock, 0, st>>>(S, A, none, W, cnt, accum, path_rgb, threshold);
     } else if (threshold > 0 && S.layout == 2) {
-        k_wf_trace_wide_both<false><<<trace_grid, kBlock, 0, st>>>(S, A, none, W, cnt, accum, path_rgb, threshold);
+        k_wf_trace_both<false, true><<<trace_grid, kBlock, 0, st>>>(S, A, none, W, cnt, accum, path_rgb, threshold);
     } else {
         k_wf_shadow<<<trace_grid, kBlock, 0, st>>>(S, A, W, cnt, accum, path_rgb);
         k_wf_extend<<<trace_grid, kBlock, 0, st>>>(S, W, cnt);
@@ -778,10 +701,9 @@ void wf_enqueue_trace(DevScene const &S, RenderArgs const &A, WfSlots const &W, 
     auto *cnt = reinterpret_cast<Counters *>(W.counters);
     BatchDev none{};
     if (threshold > 0 && S.layout == 0) {
-        k_wf_trace_dyn<true, false><<<trace_grid, kBlock, 0, st>>>(S, A, W, cnt, accum, path_rgb, threshold);
-        k_wf_trace_dyn<false, false><<<trace_grid, kBlock, 0, st>>>(S, A, W, cnt, accum, path_rgb, threshold);
+        k_wf_trace_both<false, false><<<trace_grid, kBlock, 0, st>>>(S, A, none, W, cnt, accum, path_rgb, threshold);
     } else if (threshold > 0 && S.layout == 2) {
-        k_wf_trace_wide_both<false><<<trace_grid, kBlock, 0, st>>>(S, A, none, W, cnt, accum, path_rgb, threshold);
+        k_wf_trace_both<false, true><<<trace_grid, kBlock, 0, st>>>(S, A, none, W, cnt, accum, path_rgb, threshold);
     } else {
         k_wf_shadow<<<trace_grid, kBlock, 0, st>>>(S, A, W, cnt, accum, path_rgb);
         k_wf_extend<<<trace_grid, kBlock, 0, st>>>(S, W, cnt);
