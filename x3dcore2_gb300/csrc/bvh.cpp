@@ -234,11 +234,10 @@ flat_bvh build_bvh(float const *pos, uint32_t const *tris, uint32_t num_tris, bv
 void interleave_nodes(flat_bvh const &b, std::vector<float> &out) {
     const size_t n = b.lo.size() / 4;
     out.resize(n ? 8 * (n + 1) : 0);
-    for (size_t i = 0; i < n; i++)
-        for (int k = 0; k < 4; k++) {
-            out[8 * (i + 1) + k] = b.lo[4 * i + k];
-            out[8 * (i + 1) + 4 + k] = b.hi[4 * i + k];
-        }
+    for (size_t i = 0; i < n; i++) {
+        std::memcpy(&out[8 * (i + 1)], &b.lo[4 * i], 16);
+        std::memcpy(&out[8 * (i + 1) + 4], &b.hi[4 * i], 16);
+    }
 }
 
 } // namespace e8g

@@ -32,6 +32,16 @@ void launch_megakernel(DevScene const &S, RenderArgs const &A, FirstHit const *f
                        unsigned long long *work, unsigned long long *counters, int grid, cudaStream_t st,
                        bool plain = false);
 int megakernel_blocks_per_sm();
+// The megakernel over block-local path pools (mega_pool.cuh): whether it takes this scene and
+// estimator, the bytes of its slots, and the launch (work and per-path output zeroed beforehand).
+bool mega_pool_takes(DevScene const &S, RenderArgs const &A);
+size_t mega_pool_bytes(RenderArgs const &A, int num_sms);
+void launch_mega_pool(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
+                      unsigned long long *work, void *pool, int num_sms, cudaStream_t st);
+void launch_mega_pool_l0(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
+                         unsigned long long *work, float4 *pool, int num_sms, cudaStream_t st);
+void launch_mega_pool_l2(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
+                         unsigned long long *work, float4 *pool, int num_sms, cudaStream_t st);
 // The same for one tree layout (mega_l0.cu: SAH pairs, mega_l1.cu: reference, mega_l2.cu: wide,
 // mega_l3.cu: linear).
 void launch_mega_l0(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,

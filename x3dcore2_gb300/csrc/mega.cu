@@ -40,4 +40,21 @@ void launch_megakernel(DevScene const &S, RenderArgs const &A, FirstHit const *f
         launch_mega_l0(S, A, fh, accum, path_rgb, work, counters, grid, plain, st);
 }
 
+// The estimators with a random walk on their default streams, on the two fast trees, from 2^19 paths
+// on (five per lane of the GPU): below that the pools hardly refill and k_mega is as fast or faster
+// (640 x 360, 1 spp: 0.49 ms against 0.58; 16 spp of 256 x 256: 1.21 against 0.91).
+bool mega_pool_takes(DevScene const &S, RenderArgs const &A) {
+    return (S.layout == 0 || S.layout == 2) && A.total_paths >= (1u << 19) &&
+           ((A.mode == E8G_MODE_MIS && A.rng == E8G_RNG_PHILOX) ||
+            ((A.mode == E8G_MODE_REF_LT1 || A.mode == E8G_MODE_REF_UNI) && A.rng == E8G_RNG_MINSTD));
+}
+
+void launch_mega_pool(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
+                      unsigned long long *work, void *pool, int num_sms, cudaStream_t st) {
+    if (S.layout == 0)
+        launch_mega_pool_l0(S, A, fh, accum, path_rgb, work, static_cast<float4 *>(pool), num_sms, st);
+    else
+        launch_mega_pool_l2(S, A, fh, accum, path_rgb, work, static_cast<float4 *>(pool), num_sms, st);
+}
+
 } // namespace e8g

@@ -1,5 +1,7 @@
 // Megakernel integrators (templates; mega_l0/l1/l2.cu instantiate one tree layout each so the
-// three compile in parallel, mega.cu holds the many-scene kernel and the dispatch).
+// three compile in parallel, mega.cu holds the many-scene kernel and the dispatch). Large renders on
+// the fast trees run mega_pool.cuh instead; k_mega has the other estimators and trees, counted runs,
+// small renders and contexts with a memory limit.
 //
 // One thread carries one path at a time; threads are persistent and a
 // lane whose path ended takes the next path in the same loop iteration, the lanes of a warp

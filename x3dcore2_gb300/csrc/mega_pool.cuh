@@ -1,0 +1,426 @@
+// Megakernel over block-local path pools (templates; mega_l0.cu and mega_l2.cu instantiate the SAH
+// pairs and the eight-wide tree): the persistent megakernel of large renders.
+//
+// One thread per path (mega.cuh's k_mega) holds a warp for the longest of its 32 rays at every
+// vertex: 5.4 of 32 lanes active on the 1.3M-triangle frame. Here a block owns a pool of path slots
+// in device memory and alternates between two phases: every slot whose rays are back is shaded
+// (vertices, emission, light sample, BSDF sample, a new path for a free slot), then the block's
+// warps trace the extension and shadow rays of all slots from a queue in shared memory, a lane
+// taking the next ray as soon as its own is done. Rays still on their way when the queue is empty
+// stay in their lanes over the next shading phase, so no block waits for its longest ray. No phase
+// leaves the kernel: no launches, no host synchronisation, and small renders keep the GPU as busy
+// as large ones.
+//
+// Measured on one GB300, device time of the integrator: the 1080p, 16-spp MIS frame of that scene
+// 26.3 (k_mega) -> 18.8 ms on the pairs and 30.8 -> 19.1 on the eight-wide tree, the 720p lt1 frame
+// 11.4 -> 8.1, a 1080p one-sample unidirectional frame 0.97 -> 0.90, the Cornell room at 256 x 256,
+// 16 spp 1.21 -> 0.91, a 50,000-triangle soup 4.13 -> 2.67. What bounds it now: issue slots (0.5 per
+// cycle and scheduler) shared with memory latency at 28 warps per SM; three quarters of the time is
+// tracing.
+#pragma once
+
+#include "mega.cuh"
+#include "wavefront.h"
+
+#include <algorithm>
+
+namespace e8g {
+
+namespace {
+
+// Blocks per SM (72 registers): 6 / 7 / 8 blocks take 21.5 / 19.6 / 20.0 ms per 16-spp frame.
+constexpr int kPoolBlocks = 7;
+// Slots per block at most (pool_slots).
+constexpr uint32_t kPoolSlots = 1024;
+// Idle lanes of a warp that wait for each other before they take new rays (4 / 8 / 16: within 2%).
+constexpr uint32_t kPoolRefill = 8;
+
+// State of a slot's ray: none, on its way (or queued), back with its hit.
+enum : uint8_t { kRayNone = 0, kRayOut = 1, kRayHit = 2 };
+
+// A block's slots: arrays of float4, kPoolSlots each.
+enum { kPoolIds = 0, kPoolBeta, kPoolDir, kPoolHit, kPoolPos, kPoolShDir, kPoolShAdd, kPoolArrays };
+
+// One contribution of a path to the image (or to its entry of the per-path output, which the host
+// zeroed); nothing when it is exactly zero.
+__device__ __forceinline__ void pool_add(float4 *accum, float *path_rgb, uint32_t out, float3 c) {
+    if (c.x == 0.0f && c.y == 0.0f && c.z == 0.0f)
+        return;
+    if (path_rgb) {
+        float *o = path_rgb + 3 * static_cast<size_t>(out);
+        atomicAdd(o, c.x);
+        atomicAdd(o + 1, c.y);
+        atomicAdd(o + 2, c.z);
+    } else {
+        atomicAdd(&accum[out], make_float4(c.x, c.y, c.z, 0.0f));
+    }
+}
+
+struct PoolVertex {
+    float3 beta, p, n, o;
+    int32_t mesh;
+    uint32_t depth;
+};
+
+struct PoolRays {
+    float3 add;        // contribution that needs no shadow ray
+    float3 sd, vis;    // shadow ray direction, contribution when unoccluded
+    float st;          // shadow ray length
+    uint32_t occ_nan;  // channels that an occluded sample turns into NaN (reference estimators)
+    float3 i;          // extension direction
+    float pdf;
+    bool shadow, extend;
+};
+
+// One vertex up to its rays (mega_step's draws and arithmetic): v.beta becomes the throughput
+// after the extension.
+template <int MODE, class R>
+__device__ __forceinline__ void pool_shade(DevScene const &S, RenderArgs const &A, PoolVertex &v, R &rng, PoolRays &q) {
+    q.add = q.vis = f3(0, 0, 0);
+    q.sd = q.i = f3(0, 0, 1);
+    q.st = q.pdf = 0.0f;
+    q.occ_nan = 0;
+    q.shadow = q.extend = false;
+    const DevMaterial &m = vert_mat(S, v.mesh);
+    float3 bl = v.beta;
+    if (MODE != E8G_MODE_REF_DIRECT) {
+        if ((A.max_depth && v.depth >= A.max_depth) || v.depth >= kHardDepth)
+            return;
+        float surv = A.rr_prob;
+        if (v.depth >= A.rr_start) {
+            if (rng.next() >= surv)
+                return;
+        }
+        if (MODE == E8G_MODE_MIS) {
+            if (v.depth >= A.rr_start)
+                v.beta = divs(v.beta, surv);
+            bl = v.beta;
+        } else {
+            bl = divs(v.beta, v.depth >= A.rr_start ? surv : 1.0f);
+        }
+    }
+    if (MODE == E8G_MODE_REF_LT1) { // transport_direct_illum with one light sample (pathtracer.cpp:152-242)
+        float pmf;
+        int light = sample_light(S, rng, pmf);
+        Surf ls = mesh_sample(S, __ldg(&S.light_mesh[light]), rng, false);
+        ls.area_dens *= pmf;
+        float3 l = sub(v.p, ls.p);
+        float3 illum = light_eval(S, light, l, ls.n, v.n);
+        float3 occ = mul(bl, divs(divs(f3(0, 0, 0), ls.area_dens), 1.0f)); // zero, or NaN
+        if (!vequals0(illum)) {
+            float dist = norm(l);
+            q.sd = divs(neg(l), dist);
+            q.st = dist - 1e-3f;
+            q.vis = mul(bl, divs(divs(mul(illum, bsdf_eval(S, m, v.n, v.o, q.sd)), ls.area_dens), 1.0f));
+            q.occ_nan = (occ.x == 0.0f ? 0u : 1u) | (occ.y == 0.0f ? 0u : 2u) | (occ.z == 0.0f ? 0u : 4u);
+            q.shadow = true;
+        } else {
+            q.add = occ;
+        }
+    } else if (MODE == E8G_MODE_MIS) {
+        float pmf;
+        int light = sample_light(S, rng, pmf);
+        Surf ls = mesh_sample(S, __ldg(&S.light_mesh[light]), rng, true);
+        float3 l = sub(v.p, ls.p);
+        float r2 = dot(l, l);
+        float dist = sqrtf(r2);
+        float3 ln = divs(l, dist);
+        float cos_l = dot(ls.n, ln);
+        float3 wi = neg(ln);
+        float cos_x = dot(v.n, wi);
+        if (cos_l > 0.0f && cos_x > 0.0f) {
+            float3 f = bsdf_eval(S, m, v.n, v.o, wi);
+            if (!vequals0(f)) {
+                float p_l = pmf * ls.area_dens * r2 / cos_l;
+                float p_b = bsdf_pdf(S, m, v.n, v.o, wi);
+                float w = power_heuristic(p_l, p_b);
+                q.vis = scale(mul(mul(v.beta, f), light_rad(S, light)), cos_x * w / p_l);
+                q.sd = wi;
+                q.st = dist - 1e-3f;
+                q.shadow = true;
+            }
+        }
+    } else if (MODE == E8G_MODE_REF_UNI) { // emission at every vertex (pathtracer.cpp:543-547)
+        int32_t light = __ldg(&S.mesh_light[v.mesh]);
+        if (light >= 0)
+            q.add = mul(bl, light_radiance(S, light, v.o, v.n));
+    }
+    if (MODE == E8G_MODE_MIS) {
+        q.i = bsdf_sample_mis(S, m, rng, q.pdf, v.n, v.o);
+        if (q.pdf > 0.0f) {
+            float cw = dot(v.n, q.i);
+            if (cw > 0.0f) {
+                float3 f = bsdf_eval(S, m, v.n, v.o, q.i);
+                v.beta = mul(v.beta, scale(f, cw / q.pdf));
+                q.extend = true;
+            }
+        }
+    } else {
+        q.i = bsdf_sample_ref(S, m, rng, q.pdf, v.n, v.o);
+        if (q.pdf != 0.0f) {
+            float3 f = bsdf_eval(S, m, v.n, v.o, q.i);
+            v.beta = divs(scale(mul(bl, f), dot(v.n, q.i)), q.pdf);
+            q.extend = true;
+        }
+    }
+}
+
+template <class R, int LAYOUT, int MODE>
+__global__ void __launch_bounds__(kBlock, kPoolBlocks)
+    k_mega_pool(const __grid_constant__ DevScene S, const __grid_constant__ RenderArgs A,
+                FirstHit const *__restrict__ fh, float4 *accum, float *path_rgb, unsigned long long *work, float4 *pool,
+                uint32_t slots, uint32_t keep) {
+    __shared__ uint32_t stk_all[(LAYOUT == 2 ? 2 * kWideStack : 2 * kSahFast) * kBlock];
+    __shared__ uint16_t queue[2 * kPoolSlots];
+    __shared__ uint8_t ext_st[kPoolSlots], sh_st[kPoolSlots]; // the slot's rays: kRayNone, ...
+    __shared__ uint32_t n_ext, n_sh, head, over;
+    uint32_t *stk = stk_all + threadIdx.x;
+    const uint64_t mix = splitmix64(A.seed);
+    const uint32_t lane = lane_id();
+    float4 *P = pool + static_cast<size_t>(blockIdx.x) * kPoolArrays * slots;
+    for (uint32_t s = threadIdx.x; s < slots; s += kBlock)
+        ext_st[s] = sh_st[s] = kRayNone;
+    if (threadIdx.x == 0) {
+        n_ext = n_sh = head = 0;
+        over = 0;
+    }
+    __syncthreads();
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    const WideView WV{S.wnodes, S.tri, S.nnodes, S.ntris, S.check};
+    uint32_t cur = kNone; // the slot of the lane's ray; rays on their way stay over a shading phase
+    bool any = false;
+    SahWalk T;
+    WideTrav TW;
+    SahOverflow ov;
+    while (true) {
+        // ---- shade every slot ----
+        for (uint32_t s0 = 0; s0 < slots; s0 += kBlock) {
+            const uint32_t s = s0 + threadIdx.x;
+            bool at_vertex = false, fresh = false;
+            PoolVertex v;
+            R rng;
+            uint32_t pixel = 0, sample = 0, out = 0;
+            float3 add = f3(0, 0, 0);
+            const uint32_t es = ext_st[s];
+            const bool open = es != kRayOut && sh_st[s] == kRayNone;
+            if (open && es == kRayHit) {
+                float4 hv = P[kPoolHit * slots + s], ids = P[kPoolIds * slots + s];
+                out = __float_as_uint(ids.z);
+                Hit h;
+                h.t = hv.x;
+                h.tri = __float_as_uint(hv.y);
+                h.b1 = hv.z;
+                h.b2 = hv.w;
+                if (h.tri != 0xFFFFFFFFu) {
+                    float4 dd = P[kPoolDir * slots + s], bp = P[kPoolBeta * slots + s];
+                    Vert nv = make_vert(S, h);
+                    v.o = neg(xyz(dd));
+                    if (!(dot(nv.n, v.o) <= 0.0f)) {
+                        v.beta = xyz(bp);
+                        if (MODE == E8G_MODE_MIS) {
+                            int32_t hl = __ldg(&S.mesh_light[nv.mesh]);
+                            if (hl >= 0) {
+                                float cos_l2 = dot(nv.n, v.o);
+                                float pl = __ldg(&S.light_pnorm[hl]) / S.total_power;
+                                float inv_area = 1.0f / __ldg(&S.mesh_area[__ldg(&S.light_mesh[hl])]);
+                                float p_l = pl * inv_area * (nv.t * nv.t) / cos_l2;
+                                float w = power_heuristic(bp.w, p_l);
+                                add = scale(mul(v.beta, light_rad(S, hl)), w);
+                            }
+                        }
+                        pixel = __float_as_uint(ids.x);
+                        sample = __float_as_uint(ids.y);
+                        rng = RngSlot<R>::load(A, pixel, sample, __float_as_uint(ids.w));
+                        v.p = nv.p;
+                        v.n = nv.n;
+                        v.mesh = nv.mesh;
+                        v.depth = __float_as_uint(dd.w) + 1u;
+                        at_vertex = true;
+                    }
+                }
+            }
+            // a path for every free slot; paths without a first hit end at once
+            bool want = open && !at_vertex && over == 0;
+            while (true) {
+                const uint32_t mask = __ballot_sync(~0u, want);
+                if (!mask)
+                    break;
+                const int leader = __ffs(mask) - 1;
+                unsigned long long base = 0;
+                if (static_cast<int>(lane) == leader)
+                    base = atomicAdd(work, static_cast<unsigned long long>(__popc(mask)));
+                base = __shfl_sync(~0u, base, leader);
+                if (want) {
+                    const uint64_t idx = base + __popc(mask & ((1u << lane) - 1u));
+                    if (idx >= A.total_paths) {
+                        want = false;
+                        over = 1;
+                    } else if (path_coords(A, idx, pixel, sample, out)) {
+                        FirstHit f = fh[pixel];
+                        if (__float_as_int(f.p.w) >= 0) {
+                            v.p = xyz(f.p);
+                            v.n = xyz(f.n);
+                            v.o = neg(xyz(f.d));
+                            v.mesh = __float_as_int(f.p.w);
+                            v.depth = 0;
+                            v.beta = f3(1.0f, 1.0f, 1.0f);
+                            rng = RngSlot<R>::fresh(A, mix, pixel, sample);
+                            int32_t light = __float_as_int(f.n.w);
+                            if ((MODE == E8G_MODE_MIS || MODE == E8G_MODE_REF_LT1) && light >= 0)
+                                add = light_radiance(S, light, v.o, v.n);
+                            at_vertex = fresh = true;
+                            want = false;
+                        }
+                    }
+                }
+            }
+            bool shadow = false, extend = false;
+            if (at_vertex) {
+                pool_add(accum, path_rgb, out, add);
+                PoolRays q;
+                pool_shade<MODE>(S, A, v, rng, q);
+                if (MODE != E8G_MODE_MIS)
+                    pool_add(accum, path_rgb, out, q.add);
+                shadow = q.shadow;
+                extend = q.extend;
+                if (extend) {
+                    P[kPoolBeta * slots + s] = make_float4(v.beta.x, v.beta.y, v.beta.z, q.pdf);
+                    P[kPoolDir * slots + s] = make_float4(q.i.x, q.i.y, q.i.z, __uint_as_float(v.depth));
+                }
+                if (shadow) {
+                    P[kPoolShDir * slots + s] = make_float4(q.sd.x, q.sd.y, q.sd.z, q.st);
+                    P[kPoolShAdd * slots + s] = make_float4(q.vis.x, q.vis.y, q.vis.z, __uint_as_float(q.occ_nan));
+                }
+                if (shadow || extend) {
+                    P[kPoolPos * slots + s] = make_float4(v.p.x, v.p.y, v.p.z, 0.0f);
+                    if (fresh)
+                        P[kPoolIds * slots + s] = make_float4(__uint_as_float(pixel), __uint_as_float(sample),
+                                                              __uint_as_float(out), __uint_as_float(RngSlot<R>::store(rng)));
+                    else if (extend)
+                        reinterpret_cast<uint32_t *>(&P[kPoolIds * slots + s])[3] = RngSlot<R>::store(rng);
+                }
+            }
+            if (open) {
+                ext_st[s] = extend ? kRayOut : kRayNone;
+                sh_st[s] = shadow ? kRayOut : kRayNone;
+            }
+            const uint32_t me = __ballot_sync(~0u, extend), ms = __ballot_sync(~0u, shadow);
+            uint32_t be = 0, bs = 0;
+            if (lane == 0 && me)
+                be = atomicAdd(&n_ext, static_cast<uint32_t>(__popc(me)));
+            if (lane == 0 && ms)
+                bs = atomicAdd(&n_sh, static_cast<uint32_t>(__popc(ms)));
+            be = __shfl_sync(~0u, be, 0);
+            bs = __shfl_sync(~0u, bs, 0);
+            const uint32_t below = (1u << lane) - 1u;
+            if (extend)
+                queue[be + __popc(me & below)] = static_cast<uint16_t>(s);
+            if (shadow)
+                queue[2 * kPoolSlots - 1 - (bs + __popc(ms & below))] = static_cast<uint16_t>(s);
+        }
+        const int out_rays = __syncthreads_or(cur != kNone);
+        const uint32_t ne = n_ext, n = ne + n_sh;
+        if (n == 0 && over && !out_rays)
+            break;
+        // ---- trace the block's rays: extension rays, then shadow rays ----
+        {
+            bool drained = n == 0;
+            for (uint32_t steps = 0;; steps++) {
+                uint32_t busy = __ballot_sync(~0u, cur != kNone);
+                uint32_t idle = drained ? 0u : ~busy;
+                if (idle && (static_cast<uint32_t>(__popc(idle)) >= kPoolRefill || busy == 0)) {
+                    const uint32_t k = static_cast<uint32_t>(__popc(idle));
+                    uint32_t b = 0;
+                    if (lane == 0)
+                        b = atomicAdd(&head, k);
+                    b = __shfl_sync(~0u, b, 0);
+                    drained = b + k >= n;
+                    const uint32_t idx = b + __popc(idle & ((1u << lane) - 1u));
+                    if (cur == kNone && idx < n) {
+                        any = idx >= ne;
+                        cur = queue[any ? 2 * kPoolSlots - 1 - (idx - ne) : idx];
+                        float4 o = P[kPoolPos * slots + cur];
+                        float4 d = P[(any ? kPoolShDir : kPoolDir) * slots + cur];
+                        float tmax = any ? d.w : 1000.0f;
+                        if (LAYOUT == 2)
+                            wide_begin(TW, xyz(o), xyz(d), 1e-4f, tmax, any);
+                        else
+                            sah_begin(S, T, xyz(o), xyz(d), 1e-4f, tmax);
+                    }
+                    busy = __ballot_sync(~0u, cur != kNone);
+                }
+                if (drained && (busy == 0 || (static_cast<uint32_t>(__popc(busy)) <= keep && steps >= 16)))
+                    break;
+                bool done = false;
+                if (LAYOUT == 2) {
+                    if (cur != kNone)
+                        done = wide_step(WV, TW, stk, kBlock, nullptr, nullptr);
+                } else {
+                    if (cur != kNone && !T.leaf())
+                        done = sah_interior(S, T, stk, ov);
+                    const bool leaf = cur != kNone && !done && T.leaf();
+                    const uint32_t lf = __ballot_sync(~0u, leaf);
+                    if (lf && (static_cast<uint32_t>(__popc(lf)) >= kLeafMin || lf == busy)) {
+                        if (leaf)
+                            done = sah_leaf(S, T, any, stk, ov);
+                    }
+                }
+                if (done) {
+                    Hit h = LAYOUT == 2 ? TW.h : T.h;
+                    if (!any) {
+                        ext_st[cur] = kRayHit;
+                        P[kPoolHit * slots + cur] = make_float4(h.t, __uint_as_float(h.tri), h.b1, h.b2);
+                    } else {
+                        sh_st[cur] = kRayNone;
+                        float4 c = P[kPoolShAdd * slots + cur];
+                        float3 add = f3(0, 0, 0);
+                        if (h.tri == 0xFFFFFFFFu) {
+                            add = xyz(c);
+                        } else if (MODE == E8G_MODE_REF_LT1 && __float_as_uint(c.w)) {
+                            uint32_t f = __float_as_uint(c.w);
+                            float nan = __uint_as_float(0x7FFFFFFFu);
+                            add = f3(f & 1u ? nan : 0.0f, f & 2u ? nan : 0.0f, f & 4u ? nan : 0.0f);
+                        }
+                        pool_add(accum, path_rgb, __float_as_uint(P[kPoolIds * slots + cur].z), add);
+                    }
+                    cur = kNone;
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            n_ext = n_sh = head = 0;
+        __syncthreads();
+    }
+}
+
+} // namespace
+
+// Slots per block: about sixteen paths each, since a pool that the render fills only a few times
+// spends its time in the end, when slots run empty (2 M paths: 256 / 512 / 1024 slots 0.89 / 0.92 /
+// 1.05 ms; 33 M: 19.9 / 19.4 / 18.8).
+inline uint32_t pool_slots(RenderArgs const &A, int num_sms) {
+    const uint64_t per_block = A.total_paths / (static_cast<uint64_t>(num_sms) * kPoolBlocks);
+    const uint64_t want = (per_block / 16 + kBlock - 1) / kBlock * kBlock;
+    return static_cast<uint32_t>(std::min<uint64_t>(std::max<uint64_t>(want, 256), kPoolSlots));
+}
+
+template <int LAYOUT>
+inline void launch_pool(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
+                        unsigned long long *work, float4 *pool, int num_sms, cudaStream_t st) {
+    const int grid = num_sms * kPoolBlocks;
+    const uint32_t slots = pool_slots(A, num_sms);
+    // A warp leaves the trace phase with up to 8 rays on their way (0 / 8 / 16: 21.8 / 18.8 / 18.9 ms
+    // per frame); in a tiny tree rays are short and of one length, and leaving slots out of the next
+    // shading costs more than their wait (Cornell: 0.91 ms with 0, 0.96 with 8).
+    const uint32_t keep = S.nnodes >= 1024 ? 8u : 0u;
+    auto go = [&](auto *kern) { kern<<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, pool, slots, keep); };
+    if (A.mode == E8G_MODE_MIS)
+        go(k_mega_pool<RngPhilox, LAYOUT, E8G_MODE_MIS>);
+    else if (A.mode == E8G_MODE_REF_LT1)
+        go(k_mega_pool<RngMinstd, LAYOUT, E8G_MODE_REF_LT1>);
+    else
+        go(k_mega_pool<RngMinstd, LAYOUT, E8G_MODE_REF_UNI>);
+}
+
+} // namespace e8g

@@ -174,6 +174,19 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
     return E8G_OK;
 }
 
+// Whether the megakernel runs over block-local path pools: an estimator and a tree that kernel
+// has, and its slots allocated. A context with a memory limit keeps the kernel without slots, so
+// that what fitted the limit still fits; so does one whose allocation fails.
+bool use_mega_pool(e8g_ctx *c, e8g_render_params const *p, RenderArgs const &A) {
+    if (p->integrator == E8G_INTEGRATOR_PLAIN || c->budget.cap != 0 || !mega_pool_takes(c->dev, A))
+        return false;
+    if (c->b_pool.reserve(mega_pool_bytes(A, c->num_sms)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 e8g_status run_integrator(e8g_ctx *c, e8g_render_params const *p, RenderArgs const &A, float4 *accum, float *path_rgb,
                           unsigned long long *d_counts) {
     // the counted run traces the same rays one thread per path
@@ -191,6 +204,8 @@ e8g_status run_integrator(e8g_ctx *c, e8g_render_params const *p, RenderArgs con
     if (A.mode == E8G_MODE_REF_BDPT || A.mode == E8G_MODE_BDPT_POWER || A.mode == E8G_MODE_REF_LT2) {
         launch_bdpt(c->dev, A, fh, accum, path_rgb, work, persistent_grid(c, bdpt_blocks_per_sm()), c->stream,
                     d_counts);
+    } else if (!d_counts && use_mega_pool(c, p, A)) {
+        launch_mega_pool(c->dev, A, fh, accum, path_rgb, work, c->b_pool.ptr, c->num_sms, c->stream);
     } else {
         int grid = persistent_grid(c, megakernel_blocks_per_sm());
         launch_megakernel(c->dev, A, fh, accum, path_rgb, work, d_counts, grid, c->stream,
@@ -540,7 +555,7 @@ e8g_status render_list(e8g_ctx *c, e8g_render_params const *p, uint32_t const *d
     A.list_pixel = d_pixel;
     A.list_sample = d_sample;
     A.total_paths = n;
-    if (p->integrator == E8G_INTEGRATOR_WAVEFRONT && p->mode == E8G_MODE_MIS) {
+    if (p->integrator != E8G_INTEGRATOR_PLAIN) { // integrators that add to a path's output
         cudaError_t e = cudaMemsetAsync(d_rgb, 0, static_cast<size_t>(n) * 3 * sizeof(float), c->stream);
         if (e != cudaSuccess)
             return cuda_fail(c, e, "path output clear");
