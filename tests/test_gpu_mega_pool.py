@@ -63,3 +63,29 @@ def test_memory_limit_keeps_the_kernel_without_pools(lib):
         c.upload(sc)
         np.testing.assert_allclose(c.render(p), want, rtol=RTOL, atol=1e-12)
         assert c.memory_used() < pooled
+
+
+@pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE])
+@pytest.mark.parametrize("kind,depth,rr", [("cornell", 6, 3), ("cornell", 20, 20), ("ico", 9, 9)])
+def test_backward_is_the_one_path_per_lane_kernels(lib, kind, depth, rr, layout):
+    """Gradients of the pooled backward against those of the kernel a context with a memory limit
+    keeps: paths within the scatter list, far beyond it (a second walk), and one vertex beyond.
+    The image gradient is positive, so albedo terms do not cancel: a block sums at most about 10,000
+    of them per material, in any order, within 10,000 x 2^-24 of their sum."""
+    from x3dcore2_gb300.core import Context
+    w, h = 257, 255
+    sc = (S.cornell(w, h) if kind == "cornell"
+          else S.displaced_icosphere(level=5, seed=2, num_materials=16, width=w, height=h))
+    p = default_params(abi.MODE_MIS, w, h, 8, seed=5, max_depth=depth, rr_start=rr)
+    dl = np.random.default_rng(2).uniform(0.5, 1.0, (h, w, 3)).astype(np.float32)
+    got = []
+    for limit in (0, 4 << 30):
+        with Context(0) as c:
+            c.set_memory_limit(limit)
+            c.upload(sc, layout=layout)
+            c.forward(p)
+            got.append(c.backward(dl))
+    (da, dr), (wa, wr) = got
+    assert np.abs(wa).sum() > 0
+    np.testing.assert_allclose(da, wa, rtol=1e-3, atol=1e-6 * np.abs(wa).max())
+    assert np.linalg.norm(dr - wr) <= 1e-3 * max(np.linalg.norm(wr), 1e-12)

@@ -35,8 +35,9 @@ constexpr uint32_t kPoolSlots = 1024;
 // Idle lanes of a warp that wait for each other before they take new rays (4 / 8 / 16: within 2%).
 constexpr uint32_t kPoolRefill = 8;
 
-// State of a slot's ray: none, on its way (or queued), back with its hit.
-enum : uint8_t { kRayNone = 0, kRayOut = 1, kRayHit = 2 };
+// State of a slot's ray: none, on its way (or queued), back with its hit; kRayEnd: no extension ray, but
+// an end still to be handled (the backward's).
+enum : uint8_t { kRayNone = 0, kRayOut = 1, kRayHit = 2, kRayEnd = 3 };
 
 // A block's slots: arrays of float4, kPoolSlots each.
 enum { kPoolIds = 0, kPoolBeta, kPoolDir, kPoolHit, kPoolPos, kPoolShDir, kPoolShAdd, kPoolArrays };
@@ -165,33 +166,179 @@ __device__ __forceinline__ void pool_shade(DevScene const &S, RenderArgs const &
     }
 }
 
+// A block's ray queue and slot states (shared memory): extension rays from the front, shadow rays
+// from the back.
+struct PoolQueue {
+    uint16_t slot[2 * kPoolSlots];
+    uint8_t ext_st[kPoolSlots], sh_st[kPoolSlots];
+    uint32_t n_ext, n_sh, head;
+    uint32_t over; // no path is left
+};
+
+// Appends a warp's rays of slot s.
+__device__ __forceinline__ void pool_push(PoolQueue &Q, uint32_t s, bool extend, bool shadow) {
+    const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
+    const uint32_t me = __ballot_sync(~0u, extend), ms = __ballot_sync(~0u, shadow);
+    uint32_t be = 0, bs = 0;
+    if (lane == 0 && me)
+        be = atomicAdd(&Q.n_ext, static_cast<uint32_t>(__popc(me)));
+    if (lane == 0 && ms)
+        bs = atomicAdd(&Q.n_sh, static_cast<uint32_t>(__popc(ms)));
+    be = __shfl_sync(~0u, be, 0);
+    bs = __shfl_sync(~0u, bs, 0);
+    if (extend)
+        Q.slot[be + __popc(me & below)] = static_cast<uint16_t>(s);
+    if (shadow)
+        Q.slot[2 * kPoolSlots - 1 - (bs + __popc(ms & below))] = static_cast<uint16_t>(s);
+}
+
+// A lane's ray: kept over a shading phase when it is still on its way.
+constexpr uint32_t kPoolNone = 0xFFFFFFFFu;
+struct PoolLane {
+    uint32_t cur; // its slot, or kPoolNone
+    bool any;
+    SahWalk T;
+    WideTrav TW;
+    SahOverflow ov;
+};
+
+// Traces the block's queue: ne extension rays, then shadow rays, n in all. A warp leaves when the
+// queue is empty and at most `keep` of its rays are on their way, after 16 steps at least.
+// shadow_done(slot, visible) takes a finished shadow ray and gives its slot's new shadow state.
+template <int LAYOUT, class F>
+__device__ __forceinline__ void pool_trace(DevScene const &S, PoolLane &L, float4 *P, uint32_t slots, PoolQueue &Q,
+                                           uint32_t ne, uint32_t n, uint32_t *stk, uint32_t keep, F &&shadow_done) {
+    const uint32_t lane = lane_id();
+    const WideView WV{S.wnodes, S.tri, S.nnodes, S.ntris, S.check};
+    bool drained = n == 0;
+    for (uint32_t steps = 0;; steps++) {
+        uint32_t busy = __ballot_sync(~0u, L.cur != kPoolNone);
+        uint32_t idle = drained ? 0u : ~busy;
+        if (idle && (static_cast<uint32_t>(__popc(idle)) >= kPoolRefill || busy == 0)) {
+            const uint32_t k = static_cast<uint32_t>(__popc(idle));
+            uint32_t b = 0;
+            if (lane == 0)
+                b = atomicAdd(&Q.head, k);
+            b = __shfl_sync(~0u, b, 0);
+            drained = b + k >= n;
+            const uint32_t idx = b + __popc(idle & ((1u << lane) - 1u));
+            if (L.cur == kPoolNone && idx < n) {
+                L.any = idx >= ne;
+                L.cur = Q.slot[L.any ? 2 * kPoolSlots - 1 - (idx - ne) : idx];
+                float4 o = P[kPoolPos * slots + L.cur];
+                float4 d = P[(L.any ? kPoolShDir : kPoolDir) * slots + L.cur];
+                float tmax = L.any ? d.w : 1000.0f;
+                if (LAYOUT == 2)
+                    wide_begin(L.TW, xyz(o), xyz(d), 1e-4f, tmax, L.any);
+                else
+                    sah_begin(S, L.T, xyz(o), xyz(d), 1e-4f, tmax);
+            }
+            busy = __ballot_sync(~0u, L.cur != kPoolNone);
+        }
+        if (drained && (busy == 0 || (static_cast<uint32_t>(__popc(busy)) <= keep && steps >= 16)))
+            break;
+        bool done = false;
+        if (LAYOUT == 2) {
+            if (L.cur != kPoolNone)
+                done = wide_step(WV, L.TW, stk, kBlock, nullptr, nullptr);
+        } else {
+            if (L.cur != kPoolNone && !L.T.leaf())
+                done = sah_interior(S, L.T, stk, L.ov);
+            const bool leaf = L.cur != kPoolNone && !done && L.T.leaf();
+            const uint32_t lf = __ballot_sync(~0u, leaf);
+            if (lf && (static_cast<uint32_t>(__popc(lf)) >= kLeafMin || lf == busy)) {
+                if (leaf)
+                    done = sah_leaf(S, L.T, L.any, stk, L.ov);
+            }
+        }
+        if (done) {
+            const Hit h = LAYOUT == 2 ? L.TW.h : L.T.h;
+            if (!L.any) {
+                P[kPoolHit * slots + L.cur] = make_float4(h.t, __uint_as_float(h.tri), h.b1, h.b2);
+                Q.ext_st[L.cur] = kRayHit;
+            } else {
+                Q.sh_st[L.cur] = shadow_done(L.cur, h.tri == 0xFFFFFFFFu);
+            }
+            L.cur = kPoolNone;
+        }
+    }
+}
+
+// Finishes a slot's extension ray: its vertex and the emission there with the MIS weight (add).
+// False when the path ends (miss or back face).
+template <int MODE>
+__device__ __forceinline__ bool pool_complete(DevScene const &S, float4 hv, float4 dd, float4 bp, PoolVertex &v,
+                                              float3 &add) {
+    Hit h;
+    h.t = hv.x;
+    h.tri = __float_as_uint(hv.y);
+    h.b1 = hv.z;
+    h.b2 = hv.w;
+    Vert nv = make_vert(S, h);
+    v.o = neg(xyz(dd));
+    if (dot(nv.n, v.o) <= 0.0f)
+        return false;
+    v.beta = xyz(bp);
+    if (MODE == E8G_MODE_MIS) {
+        int32_t hl = __ldg(&S.mesh_light[nv.mesh]);
+        if (hl >= 0) {
+            float cos_l2 = dot(nv.n, v.o);
+            float pl = __ldg(&S.light_pnorm[hl]) / S.total_power;
+            float inv_area = 1.0f / __ldg(&S.mesh_area[__ldg(&S.light_mesh[hl])]);
+            float p_l = pl * inv_area * (nv.t * nv.t) / cos_l2;
+            float w = power_heuristic(bp.w, p_l);
+            add = scale(mul(v.beta, light_rad(S, hl)), w);
+        }
+    }
+    v.p = nv.p;
+    v.n = nv.n;
+    v.mesh = nv.mesh;
+    v.depth = __float_as_uint(dd.w) + 1u;
+    return true;
+}
+
+// Starts a path at its cached first hit. False when the camera ray has none.
+__device__ __forceinline__ bool pool_start(FirstHit const &f, PoolVertex &v) {
+    if (__float_as_int(f.p.w) < 0)
+        return false;
+    v.p = xyz(f.p);
+    v.n = xyz(f.n);
+    v.o = neg(xyz(f.d));
+    v.mesh = __float_as_int(f.p.w);
+    v.depth = 0;
+    v.beta = f3(1.0f, 1.0f, 1.0f);
+    return true;
+}
+
+// The next path index of every lane that wants one, one atomic per warp.
+__device__ __forceinline__ uint64_t pool_next_path(unsigned long long *work, uint32_t mask) {
+    const uint32_t lane = lane_id();
+    const int leader = __ffs(mask) - 1;
+    unsigned long long base = 0;
+    if (static_cast<int>(lane) == leader)
+        base = atomicAdd(work, static_cast<unsigned long long>(__popc(mask)));
+    base = __shfl_sync(~0u, base, leader);
+    return base + __popc(mask & ((1u << lane) - 1u));
+}
+
 template <class R, int LAYOUT, int MODE>
 __global__ void __launch_bounds__(kBlock, kPoolBlocks)
     k_mega_pool(const __grid_constant__ DevScene S, const __grid_constant__ RenderArgs A,
                 FirstHit const *__restrict__ fh, float4 *accum, float *path_rgb, unsigned long long *work, float4 *pool,
                 uint32_t slots, uint32_t keep) {
-    __shared__ uint32_t stk_all[(LAYOUT == 2 ? 2 * kWideStack : 2 * kSahFast) * kBlock];
-    __shared__ uint16_t queue[2 * kPoolSlots];
-    __shared__ uint8_t ext_st[kPoolSlots], sh_st[kPoolSlots]; // the slot's rays: kRayNone, ...
-    __shared__ uint32_t n_ext, n_sh, head, over;
+    __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
+    __shared__ PoolQueue Q;
     uint32_t *stk = stk_all + threadIdx.x;
     const uint64_t mix = splitmix64(A.seed);
-    const uint32_t lane = lane_id();
     float4 *P = pool + static_cast<size_t>(blockIdx.x) * kPoolArrays * slots;
     for (uint32_t s = threadIdx.x; s < slots; s += kBlock)
-        ext_st[s] = sh_st[s] = kRayNone;
-    if (threadIdx.x == 0) {
-        n_ext = n_sh = head = 0;
-        over = 0;
-    }
+        Q.ext_st[s] = Q.sh_st[s] = kRayNone;
+    if (threadIdx.x == 0)
+        Q.n_ext = Q.n_sh = Q.head = Q.over = 0;
     __syncthreads();
-    constexpr uint32_t kNone = 0xFFFFFFFFu;
-    const WideView WV{S.wnodes, S.tri, S.nnodes, S.ntris, S.check};
-    uint32_t cur = kNone; // the slot of the lane's ray; rays on their way stay over a shading phase
-    bool any = false;
-    SahWalk T;
-    WideTrav TW;
-    SahOverflow ov;
+    PoolLane L;
+    L.cur = kPoolNone;
+    L.any = false;
     while (true) {
         // ---- shade every slot ----
         for (uint32_t s0 = 0; s0 < slots; s0 += kBlock) {
@@ -201,69 +348,31 @@ __global__ void __launch_bounds__(kBlock, kPoolBlocks)
             R rng;
             uint32_t pixel = 0, sample = 0, out = 0;
             float3 add = f3(0, 0, 0);
-            const uint32_t es = ext_st[s];
-            const bool open = es != kRayOut && sh_st[s] == kRayNone;
+            const uint32_t es = Q.ext_st[s];
+            const bool open = es != kRayOut && Q.sh_st[s] == kRayNone;
             if (open && es == kRayHit) {
                 float4 hv = P[kPoolHit * slots + s], ids = P[kPoolIds * slots + s];
-                out = __float_as_uint(ids.z);
-                Hit h;
-                h.t = hv.x;
-                h.tri = __float_as_uint(hv.y);
-                h.b1 = hv.z;
-                h.b2 = hv.w;
-                if (h.tri != 0xFFFFFFFFu) {
-                    float4 dd = P[kPoolDir * slots + s], bp = P[kPoolBeta * slots + s];
-                    Vert nv = make_vert(S, h);
-                    v.o = neg(xyz(dd));
-                    if (!(dot(nv.n, v.o) <= 0.0f)) {
-                        v.beta = xyz(bp);
-                        if (MODE == E8G_MODE_MIS) {
-                            int32_t hl = __ldg(&S.mesh_light[nv.mesh]);
-                            if (hl >= 0) {
-                                float cos_l2 = dot(nv.n, v.o);
-                                float pl = __ldg(&S.light_pnorm[hl]) / S.total_power;
-                                float inv_area = 1.0f / __ldg(&S.mesh_area[__ldg(&S.light_mesh[hl])]);
-                                float p_l = pl * inv_area * (nv.t * nv.t) / cos_l2;
-                                float w = power_heuristic(bp.w, p_l);
-                                add = scale(mul(v.beta, light_rad(S, hl)), w);
-                            }
-                        }
+                if (__float_as_uint(hv.y) != 0xFFFFFFFFu) {
+                    at_vertex = pool_complete<MODE>(S, hv, P[kPoolDir * slots + s], P[kPoolBeta * slots + s], v, add);
+                    if (at_vertex) {
                         pixel = __float_as_uint(ids.x);
                         sample = __float_as_uint(ids.y);
+                        out = __float_as_uint(ids.z);
                         rng = RngSlot<R>::load(A, pixel, sample, __float_as_uint(ids.w));
-                        v.p = nv.p;
-                        v.n = nv.n;
-                        v.mesh = nv.mesh;
-                        v.depth = __float_as_uint(dd.w) + 1u;
-                        at_vertex = true;
                     }
                 }
             }
             // a path for every free slot; paths without a first hit end at once
-            bool want = open && !at_vertex && over == 0;
-            while (true) {
-                const uint32_t mask = __ballot_sync(~0u, want);
-                if (!mask)
-                    break;
-                const int leader = __ffs(mask) - 1;
-                unsigned long long base = 0;
-                if (static_cast<int>(lane) == leader)
-                    base = atomicAdd(work, static_cast<unsigned long long>(__popc(mask)));
-                base = __shfl_sync(~0u, base, leader);
+            bool want = open && !at_vertex && Q.over == 0;
+            while (const uint32_t mask = __ballot_sync(~0u, want)) {
+                const uint64_t idx = pool_next_path(work, mask);
                 if (want) {
-                    const uint64_t idx = base + __popc(mask & ((1u << lane) - 1u));
                     if (idx >= A.total_paths) {
                         want = false;
-                        over = 1;
+                        Q.over = 1;
                     } else if (path_coords(A, idx, pixel, sample, out)) {
                         FirstHit f = fh[pixel];
-                        if (__float_as_int(f.p.w) >= 0) {
-                            v.p = xyz(f.p);
-                            v.n = xyz(f.n);
-                            v.o = neg(xyz(f.d));
-                            v.mesh = __float_as_int(f.p.w);
-                            v.depth = 0;
-                            v.beta = f3(1.0f, 1.0f, 1.0f);
+                        if (pool_start(f, v)) {
                             rng = RngSlot<R>::fresh(A, mix, pixel, sample);
                             int32_t light = __float_as_int(f.n.w);
                             if ((MODE == E8G_MODE_MIS || MODE == E8G_MODE_REF_LT1) && light >= 0)
@@ -301,95 +410,31 @@ __global__ void __launch_bounds__(kBlock, kPoolBlocks)
                 }
             }
             if (open) {
-                ext_st[s] = extend ? kRayOut : kRayNone;
-                sh_st[s] = shadow ? kRayOut : kRayNone;
+                Q.ext_st[s] = extend ? kRayOut : kRayNone;
+                Q.sh_st[s] = shadow ? kRayOut : kRayNone;
             }
-            const uint32_t me = __ballot_sync(~0u, extend), ms = __ballot_sync(~0u, shadow);
-            uint32_t be = 0, bs = 0;
-            if (lane == 0 && me)
-                be = atomicAdd(&n_ext, static_cast<uint32_t>(__popc(me)));
-            if (lane == 0 && ms)
-                bs = atomicAdd(&n_sh, static_cast<uint32_t>(__popc(ms)));
-            be = __shfl_sync(~0u, be, 0);
-            bs = __shfl_sync(~0u, bs, 0);
-            const uint32_t below = (1u << lane) - 1u;
-            if (extend)
-                queue[be + __popc(me & below)] = static_cast<uint16_t>(s);
-            if (shadow)
-                queue[2 * kPoolSlots - 1 - (bs + __popc(ms & below))] = static_cast<uint16_t>(s);
+            pool_push(Q, s, extend, shadow);
         }
-        const int out_rays = __syncthreads_or(cur != kNone);
-        const uint32_t ne = n_ext, n = ne + n_sh;
-        if (n == 0 && over && !out_rays)
+        const int out_rays = __syncthreads_or(L.cur != kPoolNone);
+        const uint32_t ne = Q.n_ext, n = ne + Q.n_sh;
+        if (n == 0 && Q.over && !out_rays)
             break;
-        // ---- trace the block's rays: extension rays, then shadow rays ----
-        {
-            bool drained = n == 0;
-            for (uint32_t steps = 0;; steps++) {
-                uint32_t busy = __ballot_sync(~0u, cur != kNone);
-                uint32_t idle = drained ? 0u : ~busy;
-                if (idle && (static_cast<uint32_t>(__popc(idle)) >= kPoolRefill || busy == 0)) {
-                    const uint32_t k = static_cast<uint32_t>(__popc(idle));
-                    uint32_t b = 0;
-                    if (lane == 0)
-                        b = atomicAdd(&head, k);
-                    b = __shfl_sync(~0u, b, 0);
-                    drained = b + k >= n;
-                    const uint32_t idx = b + __popc(idle & ((1u << lane) - 1u));
-                    if (cur == kNone && idx < n) {
-                        any = idx >= ne;
-                        cur = queue[any ? 2 * kPoolSlots - 1 - (idx - ne) : idx];
-                        float4 o = P[kPoolPos * slots + cur];
-                        float4 d = P[(any ? kPoolShDir : kPoolDir) * slots + cur];
-                        float tmax = any ? d.w : 1000.0f;
-                        if (LAYOUT == 2)
-                            wide_begin(TW, xyz(o), xyz(d), 1e-4f, tmax, any);
-                        else
-                            sah_begin(S, T, xyz(o), xyz(d), 1e-4f, tmax);
-                    }
-                    busy = __ballot_sync(~0u, cur != kNone);
-                }
-                if (drained && (busy == 0 || (static_cast<uint32_t>(__popc(busy)) <= keep && steps >= 16)))
-                    break;
-                bool done = false;
-                if (LAYOUT == 2) {
-                    if (cur != kNone)
-                        done = wide_step(WV, TW, stk, kBlock, nullptr, nullptr);
-                } else {
-                    if (cur != kNone && !T.leaf())
-                        done = sah_interior(S, T, stk, ov);
-                    const bool leaf = cur != kNone && !done && T.leaf();
-                    const uint32_t lf = __ballot_sync(~0u, leaf);
-                    if (lf && (static_cast<uint32_t>(__popc(lf)) >= kLeafMin || lf == busy)) {
-                        if (leaf)
-                            done = sah_leaf(S, T, any, stk, ov);
-                    }
-                }
-                if (done) {
-                    Hit h = LAYOUT == 2 ? TW.h : T.h;
-                    if (!any) {
-                        ext_st[cur] = kRayHit;
-                        P[kPoolHit * slots + cur] = make_float4(h.t, __uint_as_float(h.tri), h.b1, h.b2);
-                    } else {
-                        sh_st[cur] = kRayNone;
-                        float4 c = P[kPoolShAdd * slots + cur];
-                        float3 add = f3(0, 0, 0);
-                        if (h.tri == 0xFFFFFFFFu) {
-                            add = xyz(c);
-                        } else if (MODE == E8G_MODE_REF_LT1 && __float_as_uint(c.w)) {
-                            uint32_t f = __float_as_uint(c.w);
-                            float nan = __uint_as_float(0x7FFFFFFFu);
-                            add = f3(f & 1u ? nan : 0.0f, f & 2u ? nan : 0.0f, f & 4u ? nan : 0.0f);
-                        }
-                        pool_add(accum, path_rgb, __float_as_uint(P[kPoolIds * slots + cur].z), add);
-                    }
-                    cur = kNone;
-                }
+        pool_trace<LAYOUT>(S, L, P, slots, Q, ne, n, stk, keep, [&](uint32_t slot, bool visible) {
+            float4 c = P[kPoolShAdd * slots + slot];
+            float3 add = f3(0, 0, 0);
+            if (visible) {
+                add = xyz(c);
+            } else if (MODE == E8G_MODE_REF_LT1 && __float_as_uint(c.w)) {
+                uint32_t f = __float_as_uint(c.w);
+                float nan = __uint_as_float(0x7FFFFFFFu);
+                add = f3(f & 1u ? nan : 0.0f, f & 2u ? nan : 0.0f, f & 4u ? nan : 0.0f);
             }
-        }
+            pool_add(accum, path_rgb, __float_as_uint(P[kPoolIds * slots + slot].z), add);
+            return kRayNone;
+        });
         __syncthreads();
         if (threadIdx.x == 0)
-            n_ext = n_sh = head = 0;
+            Q.n_ext = Q.n_sh = Q.head = 0;
         __syncthreads();
     }
 }
@@ -405,15 +450,17 @@ inline uint32_t pool_slots(RenderArgs const &A, int num_sms) {
     return static_cast<uint32_t>(std::min<uint64_t>(std::max<uint64_t>(want, 256), kPoolSlots));
 }
 
+// Rays a warp may leave the trace phase with (0 / 8 / 16: 21.8 / 18.8 / 18.9 ms per 16-spp frame); in a
+// tiny tree rays are short and of one length, and leaving slots out of the next shading costs more
+// than their wait (Cornell: 0.91 ms with 0, 0.96 with 8).
+inline uint32_t pool_keep(DevScene const &S) { return S.nnodes >= 1024 ? 8u : 0u; }
+
 template <int LAYOUT>
 inline void launch_pool(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
                         unsigned long long *work, float4 *pool, int num_sms, cudaStream_t st) {
     const int grid = num_sms * kPoolBlocks;
     const uint32_t slots = pool_slots(A, num_sms);
-    // A warp leaves the trace phase with up to 8 rays on their way (0 / 8 / 16: 21.8 / 18.8 / 18.9 ms
-    // per frame); in a tiny tree rays are short and of one length, and leaving slots out of the next
-    // shading costs more than their wait (Cornell: 0.91 ms with 0, 0.96 with 8).
-    const uint32_t keep = S.nnodes >= 1024 ? 8u : 0u;
+    const uint32_t keep = pool_keep(S);
     auto go = [&](auto *kern) { kern<<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, pool, slots, keep); };
     if (A.mode == E8G_MODE_MIS)
         go(k_mega_pool<RngPhilox, LAYOUT, E8G_MODE_MIS>);

@@ -909,9 +909,19 @@ e8g_status e8g_backward(e8g_ctx *c, float const *dl_dimage, float *d_albedo, flo
         return s;
     RenderArgs A = make_args(&p);
     cudaEventRecord(c->ev2, c->stream);
-    e = launch_adjoint(c->dev, A, static_cast<FirstHit const *>(c->b_fh.ptr), d_dl,
-                       p.spp ? 1.0f / static_cast<float>(p.spp) : 0.0f, static_cast<unsigned long long *>(c->b_work.ptr),
-                       d_a, d_r, nullptr, c->num_sms, c->stream);
+    // pools as in use_mega_pool: not under a memory limit, nor when their allocation fails
+    AdjointPool pool = c->budget.cap == 0 ? adjoint_pool(c->dev, A, c->num_sms) : AdjointPool{};
+    if (pool.slots && c->b_pool.reserve(pool.bytes) != cudaSuccess) {
+        cudaGetLastError();
+        pool.slots = 0;
+    }
+    const float inv_spp = p.spp ? 1.0f / static_cast<float>(p.spp) : 0.0f;
+    auto *work = static_cast<unsigned long long *>(c->b_work.ptr);
+    auto const *fh = static_cast<FirstHit const *>(c->b_fh.ptr);
+    if (pool.slots)
+        e = launch_adjoint_pool(c->dev, A, fh, d_dl, inv_spp, work, d_a, d_r, pool, c->b_pool.ptr, c->stream);
+    else
+        e = launch_adjoint(c->dev, A, fh, d_dl, inv_spp, work, d_a, d_r, nullptr, c->num_sms, c->stream);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "adjoint launch");
     cudaEventRecord(c->ev3, c->stream);
