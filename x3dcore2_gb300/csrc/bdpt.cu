@@ -10,10 +10,39 @@
 #include "launch.h"
 #include "wavefront.h"
 
+#include <algorithm>
+
 namespace e8g {
 
 namespace {
 
+// One out-of-line traversal for a kernel's five call sites: inlined, with every layout behind a
+// run-time test, they overflowed the instruction cache (7.7 of 15 stall cycles per instruction in
+// k_bdpt_ref, 166 registers): with it, eight blocks per SM and no walk for paths without a camera
+// vertex that frame takes 3.2 ms against 7.3. LAYOUT -1: the scene's layout at run time (the reference's tree, the linear layout, and
+// the counted runs).
+template <int LAYOUT, bool COUNT>
+__device__ __noinline__ Hit trace_call(DevScene const &S, float3 o, float3 d, float tmin, float tmax, bool any,
+                                       uint32_t *stk, TraceCounters *cnt) {
+    if constexpr (LAYOUT == 0) {
+        return trace_sah<COUNT, false>(S, o, d, tmin, tmax, any, stk, cnt);
+    } else if constexpr (LAYOUT > 0) {
+        return trace_l<LAYOUT, COUNT>(S, o, d, tmin, tmax, any, stk, cnt);
+    } else {
+        if (S.layout == 1)
+            return trace_l<1, COUNT>(S, o, d, tmin, tmax, any, stk, cnt);
+        if (S.layout == 2)
+            return trace_l<2, COUNT>(S, o, d, tmin, tmax, any, stk, cnt);
+        if (S.layout == 3)
+            return trace_l<3, COUNT>(S, o, d, tmin, tmax, any, stk, cnt);
+        return trace_sah<COUNT, false>(S, o, d, tmin, tmax, any, stk, cnt);
+    }
+}
+
+// Blocks per SM of the one-thread-per-path kernels (64 registers; the subpaths are in local memory):
+// 4 / 5 / 6 / 7 / 8 blocks take 3.49 / 3.51 / 3.41 / 3.37 / 3.21 ms on a 641 x 361, 8-spp frame of the
+// 82,000-triangle scene with the reference's weights.
+constexpr int kBdptBlocks = 8;
 constexpr int kMaxSub = 16; // longest subpath the ABI accepts (bdpt_max_len <= 16)
 
 struct PV { // sampled_pathlet (pathtracer.cpp:12-40)
@@ -24,7 +53,7 @@ struct PV { // sampled_pathlet (pathtracer.cpp:12-40)
     int32_t light;
 };
 
-template <bool COUNT, class R>
+template <int LAYOUT, bool COUNT, class R>
 __device__ __forceinline__ uint32_t sample_subpath(DevScene const &S, R &rng, PV *path, uint32_t depth,
                                                    uint32_t max_len, uint32_t *stk, TraceCounters *cnt) {
     while (depth != max_len) { // sample_path, pathtracer.cpp:73-95
@@ -35,7 +64,7 @@ __device__ __forceinline__ uint32_t sample_subpath(DevScene const &S, R &rng, PV
             return depth;
         if (COUNT)
             cnt->rays++;
-        Hit h = trace_closest<COUNT>(S, prev.p, i, stk, cnt);
+        Hit h = trace_call<LAYOUT, COUNT>(S, prev.p, i, 1e-4f, 1000.0f, false, stk, cnt);
         if (h.tri == 0xFFFFFFFFu)
             return depth;
         Vert nv = make_vert(S, h);
@@ -54,7 +83,7 @@ __device__ __forceinline__ uint32_t sample_subpath(DevScene const &S, R &rng, PV
 }
 
 // transport_illum_source (pathtracer.cpp:152-176)
-template <bool COUNT>
+template <int LAYOUT, bool COUNT>
 __device__ __forceinline__ float3 illum_source(DevScene const &S, int light, float3 pl, float3 nl, PV const &tv,
                                                uint32_t *stk, TraceCounters *cnt) {
     float3 l = sub(tv.p, pl);
@@ -65,13 +94,13 @@ __device__ __forceinline__ float3 illum_source(DevScene const &S, int light, flo
     float3 i = divs(neg(l), dist);
     if (COUNT)
         cnt->rays++;
-    if (!trace_any<COUNT>(S, tv.p, i, 1e-4f, dist - 1e-3f, stk, cnt))
+    if (trace_call<LAYOUT, COUNT>(S, tv.p, i, 1e-4f, dist - 1e-3f, true, stk, cnt).tri == 0xFFFFFFFFu)
         return mul(illum, bsdf_eval<true>(S, vert_mat(S, tv.mesh), tv.n, tv.v, i));
     return f3(0, 0, 0);
 }
 
 // transport_all_connectible_subpaths (pathtracer.cpp:351-452)
-template <bool COUNT>
+template <int LAYOUT, bool COUNT>
 __device__ float3 connect_all(DevScene const &S, PV const *cam, uint32_t clen, PV const *lp, uint32_t llen, float3 em_p,
                               float3 em_n, float em_area_dens, int light, uint32_t *stk, TraceCounters *cnt) {
     if (clen == 0)
@@ -109,7 +138,7 @@ __device__ float3 connect_all(DevScene const &S, PV const *cam, uint32_t clen, P
                 wsum += cw;
             } else if (light_plen == 0) {
                 PV const &cj = cam[cam_plen - 1];
-                float3 ti = divs(illum_source<COUNT>(S, light, em_p, em_n, cj, stk, cnt), em_area_dens);
+                float3 ti = divs(illum_source<LAYOUT, COUNT>(S, light, em_p, em_n, cj, stk, cnt), em_area_dens);
                 float3 pr = divs(mul(ti, cam_pre[cam_plen - 1]), cam[0].dens);
                 psum = add(psum, scale(pr, cw));
                 wsum += cw;
@@ -123,7 +152,7 @@ __device__ float3 connect_all(DevScene const &S, PV const *cam, uint32_t clen, P
                 float cos_wi = dot(cj.n, neg(join));
                 if (COUNT && cos_wo > 0.0f && cos_wi > 0.0f)
                     cnt->rays++;
-                if (cos_wo > 0.0f && cos_wi > 0.0f && !trace_any<COUNT>(S, lj.p, join, 1e-3f, jd - 1e-3f, stk, cnt)) {
+                if (cos_wo > 0.0f && cos_wi > 0.0f && trace_call<LAYOUT, COUNT>(S, lj.p, join, 1e-3f, jd - 1e-3f, true, stk, cnt).tri == 0xFFFFFFFFu) {
                     float3 le = divs(light_projected(S, light, neg(lp[0].v), em_n), lp[0].dens * em_area_dens);
                     float3 lsi = mul(le, light_pre[light_plen - 1]);
                     float to_area = cos_wi * cos_wo / (jd * jd);
@@ -171,7 +200,7 @@ __device__ __forceinline__ float vpdf(DevScene const &S, BV const &v, float3 wo,
     return bsdf_pdf<true>(S, vert_mat(S, v.mesh), v.n, wo, wi);
 }
 
-template <bool COUNT, class R>
+template <int LAYOUT, bool COUNT, class R>
 __device__ uint32_t bdp_walk(DevScene const &S, R &rng, BV *path, uint32_t len, uint32_t max_len, float3 wo,
                              uint32_t *stk, TraceCounters *cnt) {
     while (len < max_len) {
@@ -187,7 +216,7 @@ __device__ uint32_t bdp_walk(DevScene const &S, R &rng, BV *path, uint32_t len, 
         float3 f = bsdf_eval<true>(S, m, cur.n, wo, i);
         if (COUNT)
             cnt->rays++;
-        Hit h = trace_closest<COUNT>(S, cur.p, i, stk, cnt);
+        Hit h = trace_call<LAYOUT, COUNT>(S, cur.p, i, 1e-4f, 1000.0f, false, stk, cnt);
         if (h.tri == 0xFFFFFFFFu)
             break;
         Vert nv = make_vert(S, h);
@@ -209,7 +238,7 @@ __device__ uint32_t bdp_walk(DevScene const &S, R &rng, BV *path, uint32_t len, 
     return len;
 }
 
-template <bool COUNT>
+template <int LAYOUT, bool COUNT>
 __device__ float3 connect_power(DevScene const &S, BV *cam, uint32_t clen, BV *lp, uint32_t llen, uint32_t maxlen,
                                 float3 o0, int light, uint32_t *stk, TraceCounters *cnt) {
     float3 L = f3(0, 0, 0);
@@ -260,7 +289,7 @@ __device__ float3 connect_power(DevScene const &S, BV *cam, uint32_t clen, BV *l
                     continue;
                 if (COUNT)
                     cnt->rays++;
-                if (trace_any<COUNT>(S, cv.p, dir, 1e-4f, dist - 1e-3f, stk, cnt))
+                if (trace_call<LAYOUT, COUNT>(S, cv.p, dir, 1e-4f, dist - 1e-3f, true, stk, cnt).tri != 0xFFFFFFFFu)
                     continue;
                 float G = cos_c * cos_l / d2;
                 contrib = scale(mul(mul(mul(cv.beta, fc), fl), lv.beta), G);
@@ -332,28 +361,55 @@ __device__ __forceinline__ void flush_counts(TraceCounters const &cnt, unsigned 
     }
 }
 
+// A path for every lane of the warp (false: none left). A path without a camera vertex (its camera
+// ray left the scene) has no connection, so its light subpath is not walked: its output is zero and
+// the lane draws again.
+__device__ __forceinline__ bool next_bdpt_path(RenderArgs const &A, FirstHit const *fh, uint32_t max_len,
+                                               unsigned long long *work, float *path_rgb, uint32_t &pixel,
+                                               uint32_t &sample, uint32_t &out) {
+    const uint32_t lane = lane_id();
+    bool want = true, have = false;
+    while (const uint32_t mask = __ballot_sync(~0u, want)) {
+        const int leader = __ffs(mask) - 1;
+        unsigned long long base = 0;
+        if (static_cast<int>(lane) == leader)
+            base = atomicAdd(work, static_cast<unsigned long long>(__popc(mask)));
+        base = __shfl_sync(~0u, base, leader);
+        if (want) {
+            const uint64_t idx = base + __popc(mask & ((1u << lane) - 1u));
+            if (idx >= A.total_paths) {
+                want = false;
+            } else if (path_coords(A, idx, pixel, sample, out)) {
+                have = max_len != 0 && __float_as_int(fh[pixel].p.w) >= 0;
+                want = !have;
+                if (want && path_rgb) {
+                    float *o = path_rgb + 3 * static_cast<size_t>(out);
+                    o[0] = o[1] = o[2] = 0.0f;
+                }
+            }
+        }
+    }
+    return have;
+}
+
 // COUNT: the instrumented instantiation that counts traversal work into counters[0..2].
-template <class R, bool COUNT>
-__global__ void __launch_bounds__(kBlock) k_bdpt_ref(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh,
+template <class R, int LAYOUT, bool COUNT>
+__global__ void __launch_bounds__(kBlock, COUNT || LAYOUT < 0 ? 1 : kBdptBlocks) k_bdpt_ref(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh,
                                                      float4 *accum, float *path_rgb, unsigned long long *work,
                                                      unsigned long long *counters) {
     TraceCounters cnt{0, 0, 0};
-    __shared__ uint32_t stk_all[kStackWords * kBlock];
+    __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
     uint32_t *stk = stk_all + threadIdx.x;
     const uint64_t mix = splitmix64(A.seed);
     const uint32_t lane = lane_id();
     const uint32_t max_len = A.bdpt_max_len < kMaxSub ? A.bdpt_max_len : kMaxSub;
     PV cam[kMaxSub], lp[kMaxSub];
     while (true) {
-        unsigned long long base = 0;
-        if (lane == 0)
-            base = atomicAdd(work, 32ull);
-        base = __shfl_sync(~0u, base, 0);
-        if (base >= A.total_paths)
+        uint32_t pixel = 0, sample = 0, out = 0;
+        const bool have = next_bdpt_path(A, fh, max_len, work, path_rgb, pixel, sample, out);
+        if (!__any_sync(~0u, have))
             break;
-        uint64_t idx = base + lane;
-        uint32_t pixel, sample, out;
-        if (idx < A.total_paths && path_coords(A, idx, pixel, sample, out)) {
+        if (have) {
             R rng;
             seed_path(rng, A, mix, pixel, sample);
             FirstHit f = fh[pixel];
@@ -366,7 +422,7 @@ __global__ void __launch_bounds__(kBlock) k_bdpt_ref(DevScene S, RenderArgs A, F
                 cam[0].n = xyz(f.n);
                 cam[0].mesh = mesh;
                 cam[0].light = __float_as_int(f.n.w);
-                clen = sample_subpath<COUNT>(S, rng, cam, 1, max_len, stk, &cnt);
+                clen = sample_subpath<LAYOUT, COUNT>(S, rng, cam, 1, max_len, stk, &cnt);
             }
             // sample_illum_source (:754-767), area_light::sample_emssion (light.cpp:26-32)
             float pmf;
@@ -378,7 +434,7 @@ __global__ void __launch_bounds__(kBlock) k_bdpt_ref(DevScene S, RenderArgs A, F
             uint32_t llen = 0;
             if (COUNT)
                 cnt.rays++;
-            Hit h = trace_closest<COUNT>(S, em.p, w, stk, &cnt); // sample_path from r0 (:109-120)
+            Hit h = trace_call<LAYOUT, COUNT>(S, em.p, w, 1e-4f, 1000.0f, false, stk, &cnt); // sample_path from r0 (:109-120)
             if (h.tri != 0xFFFFFFFFu && max_len != 0) {
                 Vert v0 = make_vert(S, h);
                 if (!(dot(v0.n, neg(w)) <= 0.0f)) {
@@ -388,10 +444,10 @@ __global__ void __launch_bounds__(kBlock) k_bdpt_ref(DevScene S, RenderArgs A, F
                     lp[0].n = v0.n;
                     lp[0].mesh = v0.mesh;
                     lp[0].light = -1;
-                    llen = sample_subpath<COUNT>(S, rng, lp, 1, max_len, stk, &cnt);
+                    llen = sample_subpath<LAYOUT, COUNT>(S, rng, lp, 1, max_len, stk, &cnt);
                 }
             }
-            float3 L = connect_all<COUNT>(S, cam, clen, lp, llen, em.p, em.n, em.area_dens, light, stk, &cnt);
+            float3 L = connect_all<LAYOUT, COUNT>(S, cam, clen, lp, llen, em.p, em.n, em.area_dens, light, stk, &cnt);
             if (path_rgb) {
                 path_rgb[3 * static_cast<size_t>(out)] = L.x;
                 path_rgb[3 * static_cast<size_t>(out) + 1] = L.y;
@@ -408,7 +464,7 @@ __global__ void __launch_bounds__(kBlock) k_bdpt_ref(DevScene S, RenderArgs A, F
 // Both subpaths of one path (the draw order of k_bdpt_power): the camera subpath from the cached
 // first hit f, then the light pick, the emission point and direction and the light subpath.
 // Returns the light's index; clen = 0 when the camera ray missed.
-template <bool COUNT, class R>
+template <int LAYOUT, bool COUNT, class R>
 __device__ __forceinline__ int sample_subpaths(DevScene const &S, R &rng, FirstHit const &f, uint32_t max_len, BV *cam,
                                                BV *lp, uint32_t &clen, uint32_t &llen, uint32_t *stk,
                                                TraceCounters *cnt) {
@@ -423,7 +479,7 @@ __device__ __forceinline__ int sample_subpaths(DevScene const &S, R &rng, FirstH
         cam[0].beta = f3(1.0f, 1.0f, 1.0f);
         cam[0].fwd = 1.0f;
         cam[0].rev = 0.0f;
-        clen = bdp_walk<COUNT>(S, rng, cam, 1, max_len, o0, stk, cnt);
+        clen = bdp_walk<LAYOUT, COUNT>(S, rng, cam, 1, max_len, o0, stk, cnt);
     }
     float pmf;
     int light = sample_light(S, rng, pmf);
@@ -443,7 +499,7 @@ __device__ __forceinline__ int sample_subpaths(DevScene const &S, R &rng, FirstH
         if (pdf_w > 0.0f && max_len > 1) {
             if (COUNT)
                 cnt->rays++;
-            Hit h = trace_closest<COUNT>(S, em.p, w, stk, cnt);
+            Hit h = trace_call<LAYOUT, COUNT>(S, em.p, w, 1e-4f, 1000.0f, false, stk, cnt);
             if (h.tri != 0xFFFFFFFFu) {
                 Vert v0 = make_vert(S, h);
                 if (dot(v0.n, neg(w)) > 0.0f) {
@@ -453,7 +509,7 @@ __device__ __forceinline__ int sample_subpaths(DevScene const &S, R &rng, FirstH
                     lp[1].beta = scale(light_rad(S, light), dot(em.n, w) / (pdf_w * lp[0].fwd));
                     lp[1].fwd = to_area(pdf_w, em.p, lp[1].p, lp[1].n);
                     lp[1].rev = 0.0f;
-                    llen = bdp_walk<COUNT>(S, rng, lp, 2, max_len, neg(w), stk, cnt);
+                    llen = bdp_walk<LAYOUT, COUNT>(S, rng, lp, 2, max_len, neg(w), stk, cnt);
                 }
             }
         }
@@ -461,33 +517,29 @@ __device__ __forceinline__ int sample_subpaths(DevScene const &S, R &rng, FirstH
     return light;
 }
 
-template <class R, bool COUNT>
-__global__ void __launch_bounds__(kBlock) k_bdpt_power(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh,
+template <class R, int LAYOUT, bool COUNT>
+__global__ void __launch_bounds__(kBlock, COUNT || LAYOUT < 0 ? 1 : kBdptBlocks) k_bdpt_power(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh,
                                                        float4 *accum, float *path_rgb, unsigned long long *work,
                                                        unsigned long long *counters) {
     TraceCounters cnt{0, 0, 0};
-    __shared__ uint32_t stk_all[kStackWords * kBlock];
+    __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
     uint32_t *stk = stk_all + threadIdx.x;
     const uint64_t mix = splitmix64(A.seed);
     const uint32_t lane = lane_id();
     const uint32_t max_len = A.bdpt_max_len < kMaxSub ? A.bdpt_max_len : kMaxSub;
     BV cam[kMaxSub], lp[kMaxSub];
     while (true) {
-        unsigned long long base = 0;
-        if (lane == 0)
-            base = atomicAdd(work, 32ull);
-        base = __shfl_sync(~0u, base, 0);
-        if (base >= A.total_paths)
+        uint32_t pixel = 0, sample = 0, out = 0;
+        const bool have = next_bdpt_path(A, fh, max_len, work, path_rgb, pixel, sample, out);
+        if (!__any_sync(~0u, have))
             break;
-        uint64_t idx = base + lane;
-        uint32_t pixel, sample, out;
-        if (idx < A.total_paths && path_coords(A, idx, pixel, sample, out)) {
+        if (have) {
             R rng;
             seed_path(rng, A, mix, pixel, sample);
             FirstHit f = fh[pixel];
             uint32_t clen, llen;
-            int light = sample_subpaths<COUNT>(S, rng, f, max_len, cam, lp, clen, llen, stk, &cnt);
-            float3 L = clen ? connect_power<COUNT>(S, cam, clen, lp, llen, max_len, neg(xyz(f.d)), light, stk, &cnt)
+            int light = sample_subpaths<LAYOUT, COUNT>(S, rng, f, max_len, cam, lp, clen, llen, stk, &cnt);
+            float3 L = clen ? connect_power<LAYOUT, COUNT>(S, cam, clen, lp, llen, max_len, neg(xyz(f.d)), light, stk, &cnt)
                             : f3(0, 0, 0);
             if (path_rgb) {
                 path_rgb[3 * static_cast<size_t>(out)] = L.x;
@@ -587,17 +639,25 @@ __device__ __forceinline__ bool walk_complete(DevScene const &S, float4 *sub, ui
 // the camera subpath's length in bits 7-11.
 enum : uint32_t { kWkEmpty = 0, kWkCam = 1, kWkLight = 2 };
 constexpr int kWalkRounds = 4; // paths a slot may start and finish without a ray in one bounce
+constexpr int kWalkDraws = 8;  // paths without a first hit a slot may pass over in one round
+
+constexpr int kWalkBlock = 512;
 
 // One bounce of the walk over every slot. range: the chunk's first path index and path count
 // (device memory, so one captured graph serves every chunk). W.next_path: the chunk's path
 // counter; W.sid: the slot's path (index in the chunk), W.out: its light, W.beta_pdf: throughput
 // of the pending vertex | sampling density, W.o: ray direction | reverse density.
-// The materials' code is out of line and the kernel held to 64 registers (four blocks of 256 per
-// SM): the walk stalled on instruction fetch with it inlined, and at three blocks per SM (80
-// registers, no spills) it took 52.1 ms per 1280x720, 32-spp frame against 47.6 ms at four.
+// The materials' code is out of line and the kernel held to 64 registers (32 warps per SM): the walk
+// stalled on instruction fetch with it inlined, and at 24 warps per SM (80 registers, no spills) it
+// took 52.1 ms per 1280x720, 32-spp frame against 47.6 ms.
+// It is bound by instruction fetch (9.7 of 22 stall cycles per instruction waited for it): every warp
+// runs some tens of kilobytes of code per group of slots. The barriers keep a block's warps in the
+// same part of it, so that a fetched line serves all of them: blocks of 256 threads without barriers
+// 36.0 ms per frame, with one / three barriers per group of slots 34.2 / 33.7, blocks of 512 33.2 /
+// 33.0, of 1024 33.0.
 template <class R>
-__global__ void __launch_bounds__(256, 4)
-    k_bdw_walk(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh, float *path_rgb, BdwChunk C, WfSlots W,
+__global__ void __launch_bounds__(kWalkBlock, 1024 / kWalkBlock)
+    k_bdw_walk(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh, BdwChunk C, WfSlots W,
                uint64_t const *range, uint32_t *ext_n, uint32_t *busy) {
     const uint64_t mix = splitmix64(A.seed);
     const uint32_t max_len = C.max_len;
@@ -606,6 +666,7 @@ __global__ void __launch_bounds__(256, 4)
     const uint32_t lane = lane_id();
     uint32_t busy_local = 0;
     for (uint32_t s0 = blockIdx.x * blockDim.x; s0 < W.capacity; s0 += gridDim.x * blockDim.x) {
+        __syncthreads();
         const uint32_t s = s0 + threadIdx.x;
         const bool in = s < W.capacity;
         const uint32_t st = in ? W.state[s] : kWkEmpty;
@@ -635,14 +696,18 @@ __global__ void __launch_bounds__(256, 4)
                 at_vertex = true;
             }
         }
+        __syncthreads();
         // once the chunk's path counter has passed its last path (it only grows), no slot takes a
         // path for the rest of the chunk: the tail bounces skip the refill atomics
         bool emitted = false, paths_left = __ldcg(W.next_path) < count;
         for (int round = 0; round < kWalkRounds; round++) {
-            // a new path for every empty slot, one atomic per warp
+            // a new path for every empty slot, one atomic per warp and draw; a path whose camera ray
+            // left the scene has no camera vertex and contributes nothing, so the lane draws again
             bool want = in && stage == kWkEmpty && paths_left;
-            uint32_t mask = __ballot_sync(~0u, want);
-            if (mask) {
+            for (int draw = 0; draw < kWalkDraws; draw++) {
+                const uint32_t mask = __ballot_sync(~0u, want);
+                if (!mask)
+                    break;
                 int leader = __ffs(mask) - 1;
                 unsigned long long base = 0;
                 if (static_cast<int>(lane) == leader)
@@ -652,18 +717,16 @@ __global__ void __launch_bounds__(256, 4)
                     uint64_t idx = base + __popc(mask & ((1u << lane) - 1u));
                     uint32_t out;
                     if (idx >= count) {
-                        paths_left = false;
+                        paths_left = want = false;
                     } else if (path_coords(A, first + idx, pixel, sample, out)) {
-                        path = static_cast<uint32_t>(idx);
-                        seed_path(rng, A, mix, pixel, sample);
                         FirstHit f = fh[pixel];
-                        const float3 o0 = neg(xyz(f.d));
-                        C.o0[path] = make_float4(o0.x, o0.y, o0.z, 0.0f);
-                        stage = kWkCam;
-                        len = 0;
-                        at_vertex = false;
                         int32_t mesh = __float_as_int(f.p.w);
                         if (mesh >= 0 && max_len) {
+                            path = static_cast<uint32_t>(idx);
+                            seed_path(rng, A, mix, pixel, sample);
+                            const float3 o0 = neg(xyz(f.d));
+                            C.o0[path] = make_float4(o0.x, o0.y, o0.z, 0.0f);
+                            stage = kWkCam;
                             BV v0;
                             v0.p = xyz(f.p);
                             v0.n = xyz(f.n);
@@ -676,6 +739,7 @@ __global__ void __launch_bounds__(256, 4)
                             len = 1;
                             wo = o0;
                             at_vertex = true;
+                            want = false;
                         }
                     }
                 }
@@ -734,11 +798,6 @@ __global__ void __launch_bounds__(256, 4)
                 path_coords(A, first + path, px, smp, out);
                 C.info[path] = make_int4(static_cast<int>(clen | len << 8), static_cast<int>(light),
                                          static_cast<int>(out), 0);
-                if (path_rgb) {
-                    path_rgb[3 * static_cast<size_t>(out)] = 0.0f;
-                    path_rgb[3 * static_cast<size_t>(out) + 1] = 0.0f;
-                    path_rgb[3 * static_cast<size_t>(out) + 2] = 0.0f;
-                }
                 for (uint32_t t = 1; t <= clen; t++)
                     n_conn += len + (__ldg(&S.mesh_light[__float_as_int(cam[3 * (t - 1)].w)]) >= 0 ? 1u : 0u);
             }
@@ -767,6 +826,7 @@ __global__ void __launch_bounds__(256, 4)
             if (__ballot_sync(~0u, in && stage == kWkEmpty && paths_left) == 0)
                 break;
         }
+        __syncthreads();
         // the slot's ray to the extension queue, one atomic per warp
         uint32_t mask = __ballot_sync(~0u, emitted);
         uint32_t base = 0;
@@ -949,12 +1009,6 @@ __global__ void __launch_bounds__(kBlock, 6) k_bdw_eval(DevScene S, float4 *accu
 
 } // namespace
 
-int bdpt_blocks_per_sm() {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_bdpt_ref<RngMinstd, false>, kBlock, 0);
-    return n > 0 ? n : 1;
-}
-
 // ---- bidirect_lt2_path_tracer (pathtracer.cpp:655-752) ----
 
 // join_with_light_paths (pathtracer.cpp:655-699): one light sample (transport_direct_illum)
@@ -965,7 +1019,7 @@ __device__ __forceinline__ float3 lt2_join(DevScene const &S, R &rng, PV const &
     int light = sample_light(S, rng, pmf);
     Surf ls = mesh_sample(S, __ldg(&S.light_mesh[light]), rng, false);
     ls.area_dens *= pmf;
-    float3 p1 = divs(add(f3(0, 0, 0), divs(illum_source<false>(S, light, ls.p, ls.n, tv, stk, nullptr), ls.area_dens)), 1.0f);
+    float3 p1 = divs(add(f3(0, 0, 0), divs(illum_source<-1, false>(S, light, ls.p, ls.n, tv, stk, nullptr), ls.area_dens)), 1.0f);
     float pmf2;
     int light2 = sample_light(S, rng, pmf2);
     Surf em = mesh_sample(S, __ldg(&S.light_mesh[light2]), rng, false); // area_light::sample_emssion
@@ -1081,12 +1135,18 @@ int bdpt_eval_blocks_per_sm() {
     return n > 0 ? n : 1;
 }
 
-void launch_bdpt_walk(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float *path_rgb, BdwChunk const &C,
+// Two rounds of the resident blocks, or a block per group of slots.
+int bdpt_walk_grid(uint32_t slots, int num_sms) {
+    return static_cast<int>(std::min<uint64_t>((slots + kWalkBlock - 1) / kWalkBlock,
+                                               static_cast<uint64_t>(num_sms) * 2 * (1024 / kWalkBlock)));
+}
+
+void launch_bdpt_walk(DevScene const &S, RenderArgs const &A, FirstHit const *fh, BdwChunk const &C,
                       WfSlots const &W, uint64_t const *range, int grid, cudaStream_t st) {
     if (A.rng == E8G_RNG_MINSTD)
-        k_bdw_walk<RngMinstd><<<grid, 256, 0, st>>>(S, A, fh, path_rgb, C, W, range, wf_ext_count_ptr(W), wf_busy_ptr(W));
+        k_bdw_walk<RngMinstd><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_ext_count_ptr(W), wf_busy_ptr(W));
     else
-        k_bdw_walk<RngPhilox><<<grid, 256, 0, st>>>(S, A, fh, path_rgb, C, W, range, wf_ext_count_ptr(W), wf_busy_ptr(W));
+        k_bdw_walk<RngPhilox><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_ext_count_ptr(W), wf_busy_ptr(W));
 }
 
 void launch_bdpt_eval(DevScene const &S, float4 *accum, float *path_rgb, BdwChunk const &C, WfSlots const &Q,
@@ -1095,34 +1155,35 @@ void launch_bdpt_eval(DevScene const &S, float4 *accum, float *path_rgb, BdwChun
 }
 
 void launch_bdpt(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
-                 unsigned long long *work, int grid, cudaStream_t st, unsigned long long *counters) {
-    bool minstd = A.rng == E8G_RNG_MINSTD;
-    if (A.mode == E8G_MODE_BDPT_POWER) {
-        if (counters && minstd)
-            k_bdpt_power<RngMinstd, true><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, counters);
-        else if (counters)
-            k_bdpt_power<RngPhilox, true><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, counters);
-        else if (minstd)
-            k_bdpt_power<RngMinstd, false><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, nullptr);
-        else
-            k_bdpt_power<RngPhilox, false><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, nullptr);
-        return;
-    }
+                 unsigned long long *work, int num_sms, cudaStream_t st, unsigned long long *counters) {
+    const bool minstd = A.rng == E8G_RNG_MINSTD;
+    auto blocks = [&](auto *kern) {
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kBlock, 0);
+        return num_sms * std::max(n, 1);
+    };
     if (A.mode == E8G_MODE_REF_LT2) {
-        if (minstd)
-            k_lt2<RngMinstd><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work);
-        else
-            k_lt2<RngPhilox><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work);
+        auto *kern = minstd ? k_lt2<RngMinstd> : k_lt2<RngPhilox>;
+        kern<<<blocks(kern), kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work);
         return;
     }
-    if (counters && minstd)
-        k_bdpt_ref<RngMinstd, true><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, counters);
-    else if (counters)
-        k_bdpt_ref<RngPhilox, true><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, counters);
-    else if (minstd)
-        k_bdpt_ref<RngMinstd, false><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, nullptr);
-    else
-        k_bdpt_ref<RngPhilox, false><<<grid, kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, nullptr);
+    auto go = [&](auto *kern) { kern<<<blocks(kern), kBlock, 0, st>>>(S, A, fh, accum, path_rgb, work, counters); };
+    const int layout = counters || S.layout == 1 || S.layout == 3 ? -1 : static_cast<int>(S.layout);
+#define E8G_BDPT(KERN)                                                                                                 \
+    if (counters)                                                                                                      \
+        minstd ? go(KERN<RngMinstd, -1, true>) : go(KERN<RngPhilox, -1, true>);                                        \
+    else if (layout == 0)                                                                                              \
+        minstd ? go(KERN<RngMinstd, 0, false>) : go(KERN<RngPhilox, 0, false>);                                        \
+    else if (layout == 2)                                                                                              \
+        minstd ? go(KERN<RngMinstd, 2, false>) : go(KERN<RngPhilox, 2, false>);                                        \
+    else                                                                                                               \
+        minstd ? go(KERN<RngMinstd, -1, false>) : go(KERN<RngPhilox, -1, false>);
+    if (A.mode == E8G_MODE_BDPT_POWER) {
+        E8G_BDPT(k_bdpt_power)
+    } else {
+        E8G_BDPT(k_bdpt_ref)
+    }
+#undef E8G_BDPT
 }
 
 } // namespace e8g

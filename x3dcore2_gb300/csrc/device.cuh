@@ -325,8 +325,14 @@ __device__ __forceinline__ void sah_begin(DevScene const &S, SahWalk &T, float3 
     T.w = S.nnodes == 1 ? kSahLeaf : 0u; // the root: pair 0, or a leaf of every triangle
 }
 
-// A node's 32 bytes in one load.
-__device__ __forceinline__ void ldg_node(float4 const *p, float4 &lo, float4 &hi) {
+// A node's 32 bytes in one load (V8), or in two: in an out-of-line function ptxas 13.0 does not take the
+// 256-bit form.
+template <bool V8 = true> __device__ __forceinline__ void ldg_node(float4 const *p, float4 &lo, float4 &hi) {
+    if (!V8) {
+        lo = __ldg(p);
+        hi = __ldg(p + 1);
+        return;
+    }
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w)
         : "l"(p));
@@ -369,13 +375,14 @@ __device__ __forceinline__ bool sah_pop(SahWalk &T, uint32_t *stk, SahOverflow c
 
 // Visits the interior node T.w: tests its child pair (one 64-byte half line, two loads) and keeps
 // the farther hit child on the stack. Returns true when the ray is done.
+template <bool V8 = true>
 __device__ __forceinline__ bool sah_interior(DevScene const &S, SahWalk &T, uint32_t *stk, SahOverflow &ov) {
     if (!E8G_CHK(S.check, 2 * static_cast<uint64_t>(T.w) + 2 < S.nnodes, kChkNode, T.w))
         return true;
     float4 l0, h0, l1, h1;
     float4 const *pair = S.nlo.p + 4 * static_cast<size_t>(T.w) + 2;
-    ldg_node(pair, l0, h0);
-    ldg_node(pair + 2, l1, h1);
+    ldg_node<V8>(pair, l0, h0);
+    ldg_node<V8>(pair + 2, l1, h1);
     float tn0, tn1;
     const bool hit0 = sah_slab(l0, h0, T.inv, T.oi, T.tmin, T.cull, tn0);
     const bool hit1 = sah_slab(l1, h1, T.inv, T.oi, T.tmin, T.cull, tn1);
@@ -435,7 +442,7 @@ __device__ __forceinline__ bool sah_leaf(DevScene const &S, SahWalk &T, bool any
 constexpr uint32_t kLeafMin = 8;
 
 // The whole walk of one ray.
-template <bool COUNT>
+template <bool COUNT, bool V8 = true>
 __device__ __forceinline__ Hit trace_sah(const DevScene &S, float3 o, float3 d, float tmin, float tmax, bool any,
                                          uint32_t *stk, TraceCounters *cnt) {
     SahWalk T;
@@ -446,7 +453,7 @@ __device__ __forceinline__ Hit trace_sah(const DevScene &S, float3 o, float3 d, 
         while (!done && !T.leaf()) {
             if (COUNT)
                 cnt->nodes += 2;
-            done = sah_interior(S, T, stk, ov);
+            done = sah_interior<V8>(S, T, stk, ov);
         }
         if (!done)
             done = sah_leaf(S, T, any, stk, ov, COUNT ? &cnt->tris : nullptr);
@@ -456,7 +463,7 @@ __device__ __forceinline__ Hit trace_sah(const DevScene &S, float3 o, float3 d, 
 
 // Shared words per thread of a layout's traversal stack.
 template <int LAYOUT>
-constexpr int kStackOf = LAYOUT == 0 ? 2 * kSahFast : LAYOUT == 2 ? 2 * kWideStack : LAYOUT == 1 ? kStackWords : 1;
+constexpr int kStackOf = LAYOUT == 0 ? 2 * kSahFast : LAYOUT == 2 ? 2 * kWideStack : LAYOUT == 3 ? 1 : kStackWords;
 
 // ---- the reference's tree, visited in the reference's order ----
 // bvh_path_space_layout::intersect / has_intersect (pathspace.cpp:330-456): depth-first with an

@@ -79,8 +79,7 @@ cudaError_t launch_composite(float const *d_rgba, uint32_t w, uint32_t h, e8g_co
 // Bidirectional path tracing (uniform or power-heuristic weights), one thread per path.
 // counters (or null): the instrumented run (bidirectional modes; rays, node boxes, triangles).
 void launch_bdpt(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum, float *path_rgb,
-                 unsigned long long *work, int grid, cudaStream_t st, unsigned long long *counters = nullptr);
-int bdpt_blocks_per_sm();
+                 unsigned long long *work, int num_sms, cudaStream_t st, unsigned long long *counters = nullptr);
 
 // The split form of E8G_MODE_BDPT_POWER (E8G_INTEGRATOR_WAVEFRONT): a chunk of `count` paths
 // starting at path index `first` (at most kBdwMaxChunk), subpaths of at most max_len vertices.

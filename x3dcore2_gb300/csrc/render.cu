@@ -89,7 +89,7 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
     // refill threshold of the trace kernels (threshold 8 against 16: 42.3 against 43.0 ms per
     // 1280x720, 32-spp frame)
     const uint32_t threshold = c->dev.layout == 0 || c->dev.layout == 2 ? 8u : 0u;
-    const int grid_walk = static_cast<int>(std::min<uint64_t>((slots + 255) / 256, static_cast<uint64_t>(c->num_sms) * 8));
+    const int grid_walk = bdpt_walk_grid(slots, c->num_sms);
     const int grid_eval = persistent_grid(c, bdpt_eval_blocks_per_sm());
     const int grid_trace = persistent_grid(c, wf_trace_blocks_per_sm(c->dev.layout, threshold));
     auto const *fh = static_cast<FirstHit const *>(c->b_fh.ptr);
@@ -101,7 +101,7 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
         return cuda_fail(c, e, "bidirectional walk capture");
     for (uint32_t k = 0; k < kBounces; k++) {
         wf_enqueue_reset(W, c->stream);
-        launch_bdpt_walk(c->dev, A, fh, path_rgb, C, W, range, grid_walk, c->stream);
+        launch_bdpt_walk(c->dev, A, fh, C, W, range, grid_walk, c->stream);
         wf_enqueue_trace(c->dev, A, W, nullptr, nullptr, grid_trace, threshold, c->stream);
     }
     e = cudaStreamEndCapture(c->stream, &graph);
@@ -202,7 +202,7 @@ e8g_status run_integrator(e8g_ctx *c, e8g_render_params const *p, RenderArgs con
     auto *work = static_cast<unsigned long long *>(c->b_work.ptr);
     auto const *fh = static_cast<FirstHit const *>(c->b_fh.ptr);
     if (A.mode == E8G_MODE_REF_BDPT || A.mode == E8G_MODE_BDPT_POWER || A.mode == E8G_MODE_REF_LT2) {
-        launch_bdpt(c->dev, A, fh, accum, path_rgb, work, persistent_grid(c, bdpt_blocks_per_sm()), c->stream,
+        launch_bdpt(c->dev, A, fh, accum, path_rgb, work, c->num_sms, c->stream,
                     d_counts);
     } else if (!d_counts && use_mega_pool(c, p, A)) {
         launch_mega_pool(c->dev, A, fh, accum, path_rgb, work, c->b_pool.ptr, c->num_sms, c->stream);

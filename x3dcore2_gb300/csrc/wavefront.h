@@ -92,10 +92,11 @@ void wf_enqueue_reset(WfSlots const &W, cudaStream_t st);
 // count in device memory. The connections: one thread per entry [first, first + n) of the chunk's
 // list into the shadow queue of Q (its counters zeroed beforehand, sh_* arrays sized for n
 // entries), which wf_enqueue_trace then drains.
-void launch_bdpt_walk(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float *path_rgb, BdwChunk const &C,
+void launch_bdpt_walk(DevScene const &S, RenderArgs const &A, FirstHit const *fh, BdwChunk const &C,
                       WfSlots const &W, uint64_t const *range, int grid, cudaStream_t st);
 void launch_bdpt_eval(DevScene const &S, float4 *accum, float *path_rgb, BdwChunk const &C, WfSlots const &Q,
                       uint32_t first, uint32_t n, int grid, cudaStream_t st);
+int bdpt_walk_grid(uint32_t slots, int num_sms);
 int bdpt_eval_blocks_per_sm();
 unsigned long long *wf_next_ptr(WfSlots const &W);
 // The two halves of a bounce, for pools that interleave on two streams (concurrent wavefront):
