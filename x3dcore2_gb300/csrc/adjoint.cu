@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(kBlock, kAdjBlocks)
     L.any = false;
     while (true) {
         for (uint32_t s0 = 0; s0 < slots; s0 += kBlock) {
+            __syncthreads(); // warps together in the code, as in k_mega_pool
             const uint32_t s = s0 + threadIdx.x;
             bool at_vertex = false, fresh = false, second = false;
             PoolVertex v;
@@ -409,6 +410,7 @@ __global__ void __launch_bounds__(kBlock, kAdjBlocks)
                     }
                 }
             }
+            __syncthreads();
             if (fresh) {
                 const FirstHit f = fh[pixel];
                 pool_start(f, v);
