@@ -245,7 +245,7 @@ __device__ __forceinline__ void pool_trace(DevScene const &S, PoolLane &L, float
         bool done = false;
         if (LAYOUT == 2) {
             if (cur != kPoolNone)
-                done = wide_step(WV, TW, stk, kBlock, nullptr, nullptr);
+                done = wide_step<true>(WV, TW, stk, kBlock, nullptr, nullptr);
         } else {
             if (cur != kPoolNone && !T.leaf())
                 done = sah_interior(S, T, stk, L.ov);

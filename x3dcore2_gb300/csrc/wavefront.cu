@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kBlock, kWfTraceBlocks)
         if (WIDE) {
             if (q == kNone)
                 continue;
-            done = wide_step(WV, T, stk, kBlock, nullptr, nullptr);
+            done = wide_step<true>(WV, T, stk, kBlock, nullptr, nullptr);
         } else {
             if (q != kNone && !TS.leaf())
                 done = sah_interior(S0, TS, stk, ov);
