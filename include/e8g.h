@@ -295,6 +295,9 @@ void e8g_default_bvh_opts(e8g_bvh_opts *opts);
 e8g_status e8g_camera_rays(e8g_ctx *ctx, uint32_t width, uint32_t height, e8g_ray *rays_out);
 
 e8g_status e8g_trace_closest(e8g_ctx *ctx, const e8g_ray *rays, uint32_t n, e8g_hit *hits);
+/* The same hits as arrays, 5 n words: n t, n mesh, n tri, then n pairs (b1, b2); mesh and tri are
+ * int32. */
+e8g_status e8g_trace_closest_arrays(e8g_ctx *ctx, const e8g_ray *rays, uint32_t n, float *hits);
 e8g_status e8g_trace_any(e8g_ctx *ctx, const e8g_ray *rays, const float *t_min, const float *t_max,
                          uint32_t n, uint8_t *occluded);
 e8g_status e8g_trace_closest_dev(e8g_ctx *ctx, const e8g_ray *d_rays, uint32_t n, e8g_hit *d_hits,

@@ -74,3 +74,19 @@ def test_stack_beyond_its_shared_part(ctx, layout):
     check(ctx, sc, layout, rays)
     if layout == abi.BVH_SAH:
         assert ctx.bvh_stats()["max_depth"] > 9
+
+
+@pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE, abi.BVH_REFERENCE, abi.BVH_LINEAR])
+@pytest.mark.parametrize("n", [1, 33, 5000])
+def test_hit_records_equal_hit_arrays(ctx, layout, n):
+    """e8g_trace_closest's records and e8g_trace_closest_arrays (which Context.trace_closest uses) are
+    the same hits, misses among them; the arrays are contiguous."""
+    ctx.upload(S.displaced_icosphere(level=3, seed=2, num_materials=16, width=64, height=36), layout=layout)
+    rays = random_rays(max(n, 64), -2.0, 2.0, seed=n)[-n:]
+    g = ctx.trace_closest(rays)
+    raw = np.zeros((n, 5), np.float32)
+    ctx._check(ctx.lib.e8g_trace_closest(ctx.h, rays.ctypes.data, n, raw.ctypes.data), "e8g_trace_closest")
+    assert all(g[k].flags["C_CONTIGUOUS"] and g[k].flags["WRITEABLE"] for k in g)
+    assert np.array_equal(g["t"], raw[:, 0]) and np.array_equal(g["b"], raw[:, 3:])
+    assert np.array_equal(g["mesh"], raw[:, 1].view(np.int32)) and np.array_equal(g["tri"], raw[:, 2].view(np.int32))
+    assert n == 1 or (g["mesh"] < 0).any()

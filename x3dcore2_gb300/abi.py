@@ -155,6 +155,7 @@ SIGNATURES = {
     "e8g_bvh_read": (_ST, [_P, _P, _P]),
     "e8g_camera_rays": (_ST, [_P, _U32, _U32, _P]),
     "e8g_trace_closest": (_ST, [_P, _P, _U32, _P]),
+    "e8g_trace_closest_arrays": (_ST, [_P, _P, _U32, _P]),
     "e8g_trace_any": (_ST, [_P, _P, _P, _P, _U32, _P]),
     "e8g_trace_closest_dev": (_ST, [_P, _P, _U32, _P, _P]),
     "e8g_render": (_ST, [_P, C.POINTER(RenderParams), _P]),

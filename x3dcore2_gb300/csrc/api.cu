@@ -691,13 +691,13 @@ e8g_status e8g_trace_closest_dev(e8g_ctx *c, e8g_ray const *d_rays, uint32_t n, 
         return fail(c, E8G_ERR_INVALID_ARG, "NULL buffers");
     cudaSetDevice(c->device);
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
-    launch_trace_closest(c->dev, reinterpret_cast<float const *>(d_rays), n, reinterpret_cast<float *>(d_hits), c->num_sms,
-                         st);
+    launch_trace_closest(c->dev, reinterpret_cast<float const *>(d_rays), n, hit_records(reinterpret_cast<float *>(d_hits)),
+                         c->num_sms, st);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? E8G_OK : cuda_fail(c, e, "trace_closest launch");
 }
 
-e8g_status e8g_trace_closest(e8g_ctx *c, e8g_ray const *rays, uint32_t n, e8g_hit *hits) {
+static e8g_status trace_closest_host(e8g_ctx *c, e8g_ray const *rays, uint32_t n, void *hits, bool arrays) {
     e8g_status s = check_ready(c);
     if (s != E8G_OK)
         return s;
@@ -714,12 +714,21 @@ e8g_status e8g_trace_closest(e8g_ctx *c, e8g_ray const *rays, uint32_t n, e8g_hi
         e = cudaMemcpyAsync(c->b_io0.ptr, rays, rb, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "trace_closest upload");
-    launch_trace_closest(c->dev, static_cast<float const *>(c->b_io0.ptr), n, static_cast<float *>(c->b_io1.ptr),
-                         c->num_sms, c->stream);
-    e = cudaMemcpyAsync(hits, c->b_io1.ptr, hb, cudaMemcpyDeviceToHost, c->stream);
+    auto *out = static_cast<float *>(c->b_io1.ptr);
+    launch_trace_closest(c->dev, static_cast<float const *>(c->b_io0.ptr), n,
+                         arrays ? hit_arrays(out, n) : hit_records(out), c->num_sms, c->stream);
+    e = cudaMemcpyAsync(hits, out, hb, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
     return e == cudaSuccess ? read_checks(c) : cuda_fail(c, e, "trace_closest");
+}
+
+e8g_status e8g_trace_closest(e8g_ctx *c, e8g_ray const *rays, uint32_t n, e8g_hit *hits) {
+    return trace_closest_host(c, rays, n, hits, false);
+}
+
+e8g_status e8g_trace_closest_arrays(e8g_ctx *c, e8g_ray const *rays, uint32_t n, float *hits) {
+    return trace_closest_host(c, rays, n, hits, true);
 }
 
 e8g_status e8g_trace_any(e8g_ctx *c, e8g_ray const *rays, float const *t_min, float const *t_max, uint32_t n,

@@ -17,7 +17,14 @@ void launch_camera_rays(DevScene const &S, uint32_t w, uint32_t h, float *rays6,
 // pixel[i] = i, samples[i] = sample.
 void launch_first_hits_rays(DevScene const &S, float const *rays6, uint32_t n, FirstHit *out, uint32_t sample,
                             uint32_t *pixel, uint32_t *samples, cudaStream_t st);
-void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, float *hits5, int num_sms,
+// Where the words of hit i go: t, mesh and tri at i * stride, the two barycentrics at i * b_stride.
+struct HitOut {
+    float *t, *mesh, *tri, *b;
+    uint32_t stride, b_stride;
+};
+inline HitOut hit_records(float *hits5) { return HitOut{hits5, hits5 + 1, hits5 + 2, hits5 + 3, 5, 5}; }
+inline HitOut hit_arrays(float *words, size_t n) { return HitOut{words, words + n, words + 2 * n, words + 3 * n, 1, 2}; }
+void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, HitOut const &hits, int num_sms,
                           cudaStream_t st);
 void launch_trace_any(DevScene const &S, float const *rays6, float const *tmin, float const *tmax, uint32_t n,
                       uint8_t *occ, int num_sms, cudaStream_t st);

@@ -88,35 +88,38 @@ __global__ void k_camera_rays(DevScene S, uint32_t w, uint32_t h, float *rays6) 
     r[5] = d.z;
 }
 
-__device__ __forceinline__ void store_hit(DevScene const &S, Hit const &h, float *out) {
-    if (h.tri == 0xFFFFFFFFu) {
-        out[0] = 0.0f;
-        out[1] = __int_as_float(-1);
-        out[2] = __int_as_float(-1);
-        out[3] = 0.0f;
-        out[4] = 0.0f;
-    } else {
+__device__ __forceinline__ void store_hit(DevScene const &S, Hit const &h, HitOut const &out, uint32_t i) {
+    float t = 0.0f, b1 = 0.0f, b2 = 0.0f;
+    int mesh = -1, tri = -1;
+    if (h.tri != 0xFFFFFFFFu) {
         uint4 ti = __ldg(&S.tidx[h.tri]);
-        out[0] = h.t;
-        out[1] = __int_as_float(static_cast<int>(ti.w));
-        out[2] = __int_as_float(static_cast<int>(h.tri - __ldg(&S.mesh_toff[ti.w])));
-        out[3] = h.b1;
-        out[4] = h.b2;
+        t = h.t;
+        mesh = static_cast<int>(ti.w);
+        tri = static_cast<int>(h.tri - __ldg(&S.mesh_toff[ti.w]));
+        b1 = h.b1;
+        b2 = h.b2;
     }
+    const size_t k = static_cast<size_t>(i) * out.stride;
+    out.t[k] = t;
+    out.mesh[k] = __int_as_float(mesh);
+    out.tri[k] = __int_as_float(tri);
+    float *b = out.b + static_cast<size_t>(i) * out.b_stride;
+    b[0] = b1;
+    b[1] = b2;
 }
 
 // Ray batches on the SAH pairs and the eight-wide tree. Each warp owns `chunk` consecutive rays and
 // gives an idle lane the next of them once kRayRefill lanes are idle: a batch's rays have no order,
 // and with one ray per lane the warp waits for its longest (3.3 of 32 lanes active on 300,000 random
 // rays against the 1.3M-triangle icosphere). The chunks are fixed, so calls on several streams
-// share nothing. ANY: any-hit on [tmin[i], tmax[i]] into occ, else the closest hit into hits5.
+// share nothing. ANY: any-hit on [tmin[i], tmax[i]] into occ, else the closest hit into hits.
 constexpr uint32_t kRayRefill = 8;
 constexpr int kRayBlocks = 8; // blocks of 128 threads per SM (64 registers), as the wavefront's trace kernel
 
 template <int LAYOUT, bool ANY>
 __global__ void __launch_bounds__(kBlock, kRayBlocks)
     k_trace_rays(const __grid_constant__ DevScene S, float const *__restrict__ rays6, float const *__restrict__ tmin,
-                 float const *__restrict__ tmax, uint32_t n, uint32_t chunk, float *hits5, uint8_t *occ) {
+                 float const *__restrict__ tmax, uint32_t n, uint32_t chunk, HitOut hits, uint8_t *occ) {
     __shared__ uint32_t stk_all[kStackOf<LAYOUT> * kBlock];
     uint32_t *stk = stk_all + threadIdx.x;
     const uint32_t lane = lane_id();
@@ -157,13 +160,13 @@ __global__ void __launch_bounds__(kBlock, kRayBlocks)
             done = cur != kNone;
         } else if (LAYOUT == 2) {
             if (cur != kNone)
-                done = wide_step(WV, TW, stk, kBlock, nullptr, nullptr);
+                done = wide_step<true>(WV, TW, stk, kBlock, nullptr, nullptr);
         } else {
             if (cur != kNone && !T.leaf())
                 done = sah_interior(S, T, stk, ov);
             const bool leaf = cur != kNone && !done && T.leaf();
             const uint32_t lf = __ballot_sync(~0u, leaf);
-            if (lf && (static_cast<uint32_t>(__popc(lf)) >= kLeafMin || lf == busy)) {
+            if (lf && 4 * __popc(lf) >= __popc(busy)) {
                 if (leaf)
                     done = sah_leaf(S, T, ANY, stk, ov);
             }
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(kBlock, kRayBlocks)
             if (ANY)
                 occ[cur] = h.tri != 0xFFFFFFFFu ? 1 : 0;
             else
-                store_hit(S, h, hits5 + 5 * static_cast<size_t>(cur));
+                store_hit(S, h, hits, cur);
             cur = kNone;
         }
     }
@@ -182,7 +185,7 @@ __global__ void __launch_bounds__(kBlock, kRayBlocks)
 // One ray per thread: the reference's tree and the linear layout.
 template <bool ANY>
 __global__ void __launch_bounds__(kBlock) k_trace_plain(DevScene S, float const *rays6, float const *tmin,
-                                                        float const *tmax, uint32_t n, float *hits5, uint8_t *occ) {
+                                                        float const *tmax, uint32_t n, HitOut hits, uint8_t *occ) {
     __shared__ uint32_t stk[kStackWords * kBlock];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(kBlock) k_trace_plain(DevScene S, float const 
     if (ANY)
         occ[i] = trace_any<false>(S, o, d, tmin[i], tmax[i], stk + threadIdx.x, nullptr) ? 1 : 0;
     else
-        store_hit(S, trace_closest<false>(S, o, d, stk + threadIdx.x, nullptr), hits5 + 5 * static_cast<size_t>(i));
+        store_hit(S, trace_closest<false>(S, o, d, stk + threadIdx.x, nullptr), hits, i);
 }
 
 __global__ void k_resolve(float4 const *accum, uint32_t npix, float inv_spp, float *rgba) {
@@ -268,31 +271,34 @@ void launch_first_hits_rays(DevScene const &S, float const *rays6, uint32_t n, F
 void launch_camera_rays(DevScene const &S, uint32_t w, uint32_t h, float *rays6, cudaStream_t st) {
     k_camera_rays<<<blocks(w * h, 256), 256, 0, st>>>(S, w, h, rays6);
 }
-// Rays per warp: one per lane while the batch is smaller than the GPU's lanes, else an equal share
-// of the batch for every resident warp (a multiple of 32).
+// Rays per warp: an equal share of the batch for every resident warp. A small batch then has few rays
+// in each warp, whose steps follow each other sooner than 32 lanes' would: a closest-hit and an
+// any-hit query of 1,500 rays against a 1,000-triangle soup take 250 us in 47 warps and 179 us with a
+// warp each (of 1,000,003 rays against the 327,690-triangle icosphere 0.85 ms).
 template <bool ANY>
 static void trace_rays(DevScene const &S, float const *rays6, float const *tmin, float const *tmax, uint32_t n,
-                       float *hits5, uint8_t *occ, int num_sms, cudaStream_t st) {
+                       HitOut const &hits, uint8_t *occ, int num_sms, cudaStream_t st) {
     if (!n)
         return;
     if (S.layout != 0 && S.layout != 2) {
-        k_trace_plain<ANY><<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, tmin, tmax, n, hits5, occ);
+        k_trace_plain<ANY><<<blocks(n, kBlock), kBlock, 0, st>>>(S, rays6, tmin, tmax, n, hits, occ);
         return;
     }
     const uint32_t warps = static_cast<uint32_t>(num_sms) * kRayBlocks * (kBlock / 32);
-    const uint32_t chunk = std::max(32u, ((n - 1) / warps + 1 + 31) / 32 * 32);
+    const uint32_t chunk = (n - 1) / warps + 1;
     const uint32_t g = ((n - 1) / chunk) / (kBlock / 32) + 1;
     if (S.layout == 2)
-        k_trace_rays<2, ANY><<<g, kBlock, 0, st>>>(S, rays6, tmin, tmax, n, chunk, hits5, occ);
+        k_trace_rays<2, ANY><<<g, kBlock, 0, st>>>(S, rays6, tmin, tmax, n, chunk, hits, occ);
     else
-        k_trace_rays<0, ANY><<<g, kBlock, 0, st>>>(S, rays6, tmin, tmax, n, chunk, hits5, occ);
+        k_trace_rays<0, ANY><<<g, kBlock, 0, st>>>(S, rays6, tmin, tmax, n, chunk, hits, occ);
 }
-void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, float *hits5, int num_sms, cudaStream_t st) {
-    trace_rays<false>(S, rays6, nullptr, nullptr, n, hits5, nullptr, num_sms, st);
+void launch_trace_closest(DevScene const &S, float const *rays6, uint32_t n, HitOut const &hits, int num_sms,
+                          cudaStream_t st) {
+    trace_rays<false>(S, rays6, nullptr, nullptr, n, hits, nullptr, num_sms, st);
 }
 void launch_trace_any(DevScene const &S, float const *rays6, float const *tmin, float const *tmax, uint32_t n,
                       uint8_t *occ, int num_sms, cudaStream_t st) {
-    trace_rays<true>(S, rays6, tmin, tmax, n, nullptr, occ, num_sms, st);
+    trace_rays<true>(S, rays6, tmin, tmax, n, HitOut{}, occ, num_sms, st);
 }
 void launch_resolve(float4 const *accum, uint32_t npix, float inv_spp, float *rgba, cudaStream_t st) {
     k_resolve<<<blocks(npix, 256), 256, 0, st>>>(accum, npix, inv_spp, rgba);
