@@ -190,3 +190,24 @@ def test_refit_of_device_wide_tree_keeps_its_bytes(ctx, name):
     nodes1, tris1 = ctx.bvh_read()
     assert np.array_equal(nodes0, nodes1)
     assert np.array_equal(tris0.view(np.uint32), tris1.view(np.uint32))
+
+
+@pytest.mark.parametrize("tris", [1, 2, 7, 2047, 2049, 4097, 40_000])
+@pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE])
+def test_build_sizes(ctx, tris, layout):
+    """Sizes around the one-block clustering's 2,048 clusters, a scan tile and several batches of
+    rounds: every triangle once, and the hits of the host-built tree."""
+    sc = S.soup(tris, seed=tris, width=64, height=64)
+    r = np.random.default_rng(tris)
+    o = r.uniform(-0.9, 0.9, (5000, 3))
+    d = r.normal(size=(5000, 3))
+    rays = np.concatenate([o, d / np.linalg.norm(d, axis=1, keepdims=True)], axis=1).astype(np.float32)
+    ctx.upload(sc, layout=layout)
+    want = ctx.trace_closest(rays)
+    ctx.upload(sc, layout=layout, builder=abi.BUILDER_DEVICE)
+    assert ctx.bvh_stats()["layout"] == layout
+    _, rec = ctx.bvh_read()
+    assert np.array_equal(np.sort(rec.view(np.uint32)[:, 3]), np.arange(sc.num_tris))
+    got = ctx.trace_closest(rays)
+    assert np.array_equal(got["t"].view(np.uint32), want["t"].view(np.uint32))
+    assert np.mean(got["tri"] == want["tri"]) >= 0.999

@@ -305,7 +305,7 @@ e8g_status build_on_device(e8g_ctx *c, bool *built) {
         wi.max_abs = max_abs;
         wi.max_depth = kWideMaxDepth;
         wi.scratch = in.scratch;
-        wi.host_pinned = c->host_pinned;
+        wi.num_sms = c->num_sms;
         wi.wide = static_cast<uint4 *>(c->b_wide.ptr);
         GpuWideOut wo;
         e = gpu_collapse_wide(wi, wo, c->stream);

@@ -17,7 +17,12 @@
 //    pushed out exactly as the host builder pushes them out, bvh_boxes.h) at its depth-first
 //    preorder slot (the host builder's order: children adjacent, the k-th interior node's at 1 + 2k,
 //    from interior-node counts of the subtrees), leaves write their triangles' records.
-// Everything is deterministic: scans, not atomics, decide every position.
+// Every byte of the tree is deterministic: scans decide the clusters' and wide nodes' positions, and the
+// flattening's items carry theirs (only the order of a level's work list comes from an atomic).
+// Counts stay on the device: rounds and levels follow each other in the stream with grids for the
+// most they can hold, and the host reads back every few rounds and at the end. 525 launches and about
+// 70 reads made 5.7 ms of the 1.3M-triangle scene's eight-wide build; it is 236 launches, a dozen
+// reads and 3.1 ms (pairs 4.3 -> 2.3).
 #include "bvh_boxes.h"
 #include "gpu_build.h"
 #include "launch.h"
@@ -35,6 +40,7 @@ constexpr int kSortTile = kGB * kSortItems;
 constexpr int kScanItems = 4;     // elements per thread in the device-wide scan
 constexpr int kScanTile = 1024 * kScanItems;
 constexpr int kPlocRadius = 24;
+constexpr int kLevels = 40;       // entries of the per-level states (trees are at most 32 levels deep)
 constexpr int kLeafStack = 16;    // subtree walk of a leaf (at most 15 triangles)
 
 __device__ __forceinline__ uint32_t ord_key(float f) {
@@ -46,11 +52,11 @@ __device__ __forceinline__ float key_float(uint32_t u) {
 }
 
 // Inclusive scan of one value per thread over a block of `threads` threads (a multiple of 32).
-template <int THREADS> __device__ __forceinline__ uint32_t block_inclusive(uint32_t v, uint32_t *sh) {
+template <int THREADS, class T> __device__ __forceinline__ T block_inclusive(T v, T *sh) {
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t x = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        T x = __shfl_up_sync(0xFFFFFFFFu, v, o);
         if (lane >= o)
             v += x;
     }
@@ -58,10 +64,10 @@ template <int THREADS> __device__ __forceinline__ uint32_t block_inclusive(uint3
         sh[warp] = v;
     __syncthreads();
     if (warp == 0) {
-        uint32_t w = lane < THREADS / 32 ? sh[lane] : 0;
+        T w = lane < THREADS / 32 ? sh[lane] : T(0);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t x = __shfl_up_sync(0xFFFFFFFFu, w, o);
+            T x = __shfl_up_sync(0xFFFFFFFFu, w, o);
             if (lane >= o)
                 w += x;
         }
@@ -69,7 +75,7 @@ template <int THREADS> __device__ __forceinline__ uint32_t block_inclusive(uint3
             sh[lane] = w;
     }
     __syncthreads();
-    uint32_t r = v + (warp ? sh[warp - 1] : 0);
+    T r = v + (warp ? sh[warp - 1] : T(0));
     __syncthreads();
     return r;
 }
@@ -324,8 +330,27 @@ __device__ __forceinline__ float union_area(float4 a0, float4 a1, float4 b0, flo
     return dx * dy + dy * dz + dz * dx;
 }
 
-__global__ void __launch_bounds__(kGB) k_ploc_nn(uint32_t const *clus, uint32_t m, float4 const *blo,
-                                                  float4 const *bhi, int32_t *nn) {
+// A round: neighbours, a scan of the merge and keep flags (two counts in one 64-bit word, tile by
+// tile), the tile totals, and the merges. The cluster count stays on the device: round r reads
+// state[r & 1] and writes the other one, so the host looks only every few rounds (kPlocBatch), with
+// grids for the count it last saw. Once kPlocSmall clusters are left a round does nothing.
+struct PlocState {
+    uint32_t m, base;  // clusters, next tree node
+    uint32_t cur;      // which cluster array holds them
+    uint32_t rounds;
+    uint32_t stuck;    // a round found no mutual pair (non-finite boxes)
+};
+constexpr int kPlocSmall = 2048; // clusters the one-block kernel takes over at
+constexpr int kPlocBatch = 4;
+
+__global__ void k_ploc_start(PlocState *state, uint32_t n) { state[0] = PlocState{n, n, 0, 0, 0}; }
+
+__global__ void __launch_bounds__(kGB) k_ploc_nn(PlocState const *state, uint32_t const *c0, uint32_t const *c1,
+                                                  float4 const *blo, float4 const *bhi, int32_t *nn) {
+    const uint32_t m = state->m;
+    if (m <= static_cast<uint32_t>(kPlocSmall) || blockIdx.x * kGB >= m)
+        return;
+    uint32_t const *clus = state->cur ? c1 : c0;
     __shared__ float4 slo[kGB + 2 * kPlocRadius], shi[kGB + 2 * kPlocRadius];
     int s0 = static_cast<int>(blockIdx.x * kGB) - kPlocRadius;
     for (int k = threadIdx.x; k < kGB + 2 * kPlocRadius; k += kGB) {
@@ -356,40 +381,100 @@ __global__ void __launch_bounds__(kGB) k_ploc_nn(uint32_t const *clus, uint32_t 
     nn[i] = bj;
 }
 
-__global__ void k_ploc_flags(int32_t const *nn, uint32_t m, uint32_t *merged, uint32_t *keep) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m)
-        return;
+// Cluster i's flags: merged in the high word (the lower position of a mutual pair), kept in the low.
+__device__ __forceinline__ uint64_t ploc_flags(int32_t const *nn, uint32_t i) {
     int32_t j = nn[i];
     bool mutual = j >= 0 && nn[j] == static_cast<int32_t>(i);
-    merged[i] = mutual && static_cast<int32_t>(i) < j;
-    keep[i] = !(mutual && static_cast<int32_t>(i) > j);
+    uint64_t merged = mutual && static_cast<int32_t>(i) < j, keep = !(mutual && static_cast<int32_t>(i) > j);
+    return merged << 32 | keep;
 }
 
-__global__ void k_ploc_apply(uint32_t const *clus, uint32_t *clus_out, int32_t const *nn, uint32_t m,
-                             uint32_t const *mscan, uint32_t const *kscan, uint32_t const *mflag,
-                             uint32_t const *kflag, uint32_t base, float4 *blo, float4 *bhi, int2 *child) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || !kflag[i])
+__global__ void __launch_bounds__(1024) k_ploc_tiles(PlocState const *state, int32_t const *nn, uint64_t *scan,
+                                                     uint64_t *sums) {
+    const uint32_t m = state->m;
+    if (m <= static_cast<uint32_t>(kPlocSmall) || blockIdx.x * kScanTile >= m)
         return;
-    if (mflag[i]) {
-        uint32_t node = base + mscan[i]; // < 2n - 1: every merge removes one cluster
+    __shared__ uint64_t sh[32];
+    uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    uint64_t v[kScanItems], t = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        v[k] = base + k < m ? ploc_flags(nn, base + k) : 0;
+        t += v[k];
+    }
+    uint64_t incl = block_inclusive<1024>(t, sh);
+    uint64_t run = incl - t;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (base + k < m)
+            scan[base + k] = run;
+        run += v[k];
+    }
+    if (threadIdx.x == 1023)
+        sums[blockIdx.x] = incl;
+}
+
+// Exclusive scan of m tile totals in place, one block; the grand total in every thread.
+__device__ __forceinline__ uint64_t scan_totals(uint64_t *sums, uint32_t m, uint64_t *sh) {
+    uint64_t carry = 0;
+    for (uint32_t b = 0; b < m; b += 1024) {
+        uint32_t i = b + threadIdx.x;
+        uint64_t v = i < m ? sums[i] : 0;
+        uint64_t incl = block_inclusive<1024>(v, sh);
+        if (i < m)
+            sums[i] = carry + incl - v;
+        carry += sh[31]; // the block's total
+        __syncthreads();
+    }
+    return carry;
+}
+
+__global__ void __launch_bounds__(1024) k_ploc_sums(PlocState const *state, PlocState *next, uint64_t *sums) {
+    __shared__ uint64_t sh[32];
+    PlocState s = *state;
+    if (s.m > static_cast<uint32_t>(kPlocSmall)) {
+        uint64_t total = scan_totals(sums, (s.m - 1) / kScanTile + 1, sh);
+        uint32_t merged = static_cast<uint32_t>(total >> 32);
+        s.stuck |= merged == 0;
+        s.m = static_cast<uint32_t>(total);
+        s.base += merged;
+        s.cur ^= 1u;
+        s.rounds++;
+    }
+    if (threadIdx.x == 0)
+        *next = s;
+}
+
+__global__ void __launch_bounds__(kGB) k_ploc_apply(PlocState const *state, uint32_t *c0, uint32_t *c1,
+                                                     int32_t const *nn, uint64_t const *scan, uint64_t const *sums,
+                                                     float4 *blo, float4 *bhi, int2 *child) {
+    const uint32_t m = state->m, i = blockIdx.x * kGB + threadIdx.x;
+    if (m <= static_cast<uint32_t>(kPlocSmall) || i >= m)
+        return;
+    uint32_t const *clus = state->cur ? c1 : c0;
+    uint32_t *clus_out = state->cur ? c0 : c1;
+    const uint64_t f = ploc_flags(nn, i), at = scan[i] + sums[i / kScanTile];
+    if (!static_cast<uint32_t>(f))
+        return;
+    if (f >> 32) {
+        uint32_t node = state->base + static_cast<uint32_t>(at >> 32); // < 2n - 1: every merge removes one cluster
         uint32_t a = clus[i], b = clus[nn[i]];
         child[node] = make_int2(static_cast<int>(a), static_cast<int>(b));
         float4 a0 = blo[a], a1 = bhi[a], b0 = blo[b], b1 = bhi[b];
         blo[node] = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.0f);
         bhi[node] = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), 0.0f);
-        clus_out[kscan[i]] = node;
+        clus_out[static_cast<uint32_t>(at)] = node;
     } else {
-        clus_out[kscan[i]] = clus[i];
+        clus_out[static_cast<uint32_t>(at)] = clus[i];
     }
 }
 
 // The last rounds, once few clusters are left, in one block: the same rounds as the kernels above
-// (same neighbour search, tie-breaks and node numbering), without a launch and a host read per
-// round.
-constexpr int kPlocSmall = 2048;  // clusters the one-block kernel takes over at
+// (same neighbour search, tie-breaks and node numbering), without launches between them. The
+// clusters' boxes stay in shared memory (279 -> 180 us from 2,048 clusters on, against reading them
+// through L1 for every neighbour).
 constexpr int kPlocSmallThreads = 1024;
+constexpr size_t kPlocFinishShared = 4 * kPlocSmall * sizeof(float4);
 
 __global__ void __launch_bounds__(kPlocSmallThreads)
     k_ploc_finish(uint32_t const *clus_in, uint32_t m, uint32_t base, float4 *blo, float4 *bhi, int2 *child,
@@ -399,23 +484,26 @@ __global__ void __launch_bounds__(kPlocSmallThreads)
     __shared__ uint32_t ms[kPlocSmall], ks[kPlocSmall];
     __shared__ uint32_t sh[32];
     constexpr int per = kPlocSmall / kPlocSmallThreads; // elements per thread in the scans
-    for (uint32_t i = threadIdx.x; i < m; i += kPlocSmallThreads)
+    extern __shared__ float4 boxes[];
+    float4 *lo = boxes, *hi = boxes + kPlocSmall, *lo2 = hi + kPlocSmall, *hi2 = lo2 + kPlocSmall;
+    for (uint32_t i = threadIdx.x; i < m; i += kPlocSmallThreads) {
         ca[i] = clus_in[i];
+        lo[i] = blo[clus_in[i]];
+        hi[i] = bhi[clus_in[i]];
+    }
     __syncthreads();
     uint32_t *cur = ca, *nxt = cb;
     int rounds = 0;
     while (m > 1 && rounds++ < 1000000) {
         for (uint32_t i = threadIdx.x; i < m; i += kPlocSmallThreads) {
-            uint32_t node = cur[i];
-            float4 a0 = blo[node], a1 = bhi[node];
+            float4 a0 = lo[i], a1 = hi[i];
             float best = INFINITY;
             int bj = -1;
             for (int d = -kPlocRadius; d <= kPlocRadius; d++) {
                 int j = static_cast<int>(i) + d;
                 if (d == 0 || j < 0 || j >= static_cast<int>(m))
                     continue;
-                uint32_t o = cur[j];
-                float area = union_area(a0, a1, blo[o], bhi[o]);
+                float area = union_area(a0, a1, lo[j], hi[j]);
                 if (area < best) {
                     best = area;
                     bj = j;
@@ -466,12 +554,16 @@ __global__ void __launch_bounds__(kPlocSmallThreads)
                 uint32_t node = base + ms[i];
                 uint32_t a = cur[i], b = cur[nn[i]];
                 child[node] = make_int2(static_cast<int>(a), static_cast<int>(b));
-                float4 a0 = blo[a], a1 = bhi[a], b0 = blo[b], b1 = bhi[b];
-                blo[node] = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.0f);
-                bhi[node] = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), 0.0f);
+                float4 a0 = lo[i], a1 = hi[i], b0 = lo[nn[i]], b1 = hi[nn[i]];
+                float4 u0 = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.0f);
+                float4 u1 = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), 0.0f);
+                blo[node] = lo2[ks[i]] = u0;
+                bhi[node] = hi2[ks[i]] = u1;
                 nxt[ks[i]] = node;
             } else {
                 nxt[ks[i]] = cur[i];
+                lo2[ks[i]] = lo[i];
+                hi2[ks[i]] = hi[i];
             }
         }
         __syncthreads();
@@ -482,7 +574,9 @@ __global__ void __launch_bounds__(kPlocSmallThreads)
         uint32_t *t = cur;
         cur = nxt;
         nxt = t;
-        __threadfence_block();
+        float4 *x = lo, *y = hi;
+        lo = lo2, hi = hi2;
+        lo2 = x, hi2 = y;
         __syncthreads();
     }
     if (threadIdx.x == 0)
@@ -549,69 +643,97 @@ struct WideItem {
     uint32_t bn, wn; // binary node, wide node index
 };
 
-__global__ void k_flat_flags(FlatItem const *items, uint32_t f, uint8_t const *leaf, uint32_t *interior) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < f)
-        interior[i] = leaf[items[i].node] ? 0u : 1u;
+__global__ void k_flat_start(FlatItem *items, uint32_t *lvl, unsigned long long *leaf_stats, uint32_t root) {
+    if (threadIdx.x < kLevels)
+        lvl[threadIdx.x] = threadIdx.x == 0;
+    if (threadIdx.x < 2)
+        leaf_stats[threadIdx.x] = 0;
+    if (threadIdx.x == 0)
+        items[0] = FlatItem{root, 0, 0, 0};
 }
 
-__global__ void k_flat_emit(FlatItem const *items, uint32_t f, uint32_t const *iscan, uint32_t n, int2 const *child,
-                            uint8_t const *leaf, uint32_t const *ntris, uint32_t const *icount, float4 const *blo,
-                            float4 const *bhi, uint32_t const *order, uint4 const *tidx, float4 const *vpos,
-                            uint32_t const *red, NodeHalf<float4> nlo, NodeHalf<float4> nhi, float4 *tri, FlatItem *next,
-                            unsigned long long *leaf_stats) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= f)
-        return;
-    FlatItem it = items[i];
+// One level: lvl[level] frontier items (any order: an item carries its node slot and triangle start)
+// into lvl[level + 1] items of the next. Grids are for any count, so the levels follow each other
+// without the host.
+__global__ void __launch_bounds__(kGB)
+    k_flat_level(FlatItem const *items, FlatItem *next, uint32_t *lvl, uint32_t level, uint32_t n, int2 const *child,
+                 uint8_t const *leaf, uint32_t const *ntris, uint32_t const *icount, float4 const *blo,
+                 float4 const *bhi, uint32_t const *order, uint4 const *tidx, float4 const *vpos, uint32_t const *red,
+                 NodeHalf<float4> nlo, NodeHalf<float4> nhi, float4 *tri, unsigned long long *leaf_stats) {
+    const uint32_t f = lvl[level], lane = threadIdx.x & 31u;
     float lo[3], hi[3];
     for (int a = 0; a < 3; a++) {
         lo[a] = key_float(red[a]);
         hi[a] = key_float(red[3 + a]);
     }
-    float eps = scene_eps(lo, hi);
-    float4 b0 = blo[it.node], b1 = bhi[it.node];
-    uint32_t link, count;
-    if (leaf[it.node]) {
-        link = it.tri_start;
-        count = ntris[it.node];
-        // the leaf's triangles, left to right
-        uint32_t stack[kLeafStack];
-        int sp = 0, k = 0;
-        stack[sp++] = it.node;
-        while (sp > 0) {
-            uint32_t x = stack[--sp];
-            if (x < n) {
-                uint32_t t = order[x];
-                uint4 g = tidx[t];
-                float4 p0 = vpos[g.x], p1 = vpos[g.y], p2 = vpos[g.z];
-                size_t r = 3 * static_cast<size_t>(it.tri_start + k);
-                tri[r] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(t));
-                tri[r + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z,
-                                         k + 1 == static_cast<int>(count) ? 1.0f : 0.0f); // the leaf's last record
-                tri[r + 2] = make_float4(p2.x - p0.x, p2.y - p0.y, p2.z - p0.z, 0.0f);
-                k++;
-            } else if (sp + 2 <= kLeafStack) {
-                int2 c = child[x];
-                stack[sp++] = static_cast<uint32_t>(c.y);
-                stack[sp++] = static_cast<uint32_t>(c.x);
+    const float eps = scene_eps(lo, hi);
+    for (uint32_t i0 = blockIdx.x * kGB + (threadIdx.x & ~31u); i0 < f; i0 += gridDim.x * kGB) {
+        const bool on = i0 + lane < f;
+        FlatItem it{};
+        bool is_leaf = false;
+        if (on) {
+            it = items[i0 + lane];
+            is_leaf = leaf[it.node] != 0;
+        }
+        const uint32_t mi = __ballot_sync(~0u, on && !is_leaf), ml = __ballot_sync(~0u, is_leaf);
+        uint32_t at = 0;
+        if (lane == 0) {
+            if (mi)
+                at = atomicAdd(&lvl[level + 1], 2u * __popc(mi));
+            if (ml) {
+                atomicAdd(&leaf_stats[0], static_cast<unsigned long long>(__popc(ml)));
+                atomicAdd(&leaf_stats[1], static_cast<unsigned long long>(__popc(ml)) * level);
             }
         }
-        atomicAdd(&leaf_stats[0], 1ull);
-    } else {
-        // depth-first preorder slots, as the host builder lays nodes out: the k-th interior node in
-        // preorder keeps its children at 1 + 2k and 2 + 2k
-        link = 1 + 2 * it.pre;
-        count = 0;
-        int2 c = child[it.node];
-        next[2 * iscan[i]] = FlatItem{static_cast<uint32_t>(c.x), link, it.tri_start, it.pre + 1};
-        next[2 * iscan[i] + 1] =
-            FlatItem{static_cast<uint32_t>(c.y), link + 1, it.tri_start + ntris[c.x], it.pre + 1 + icount[c.x]};
+        at = __shfl_sync(~0u, at, 0) + 2u * __popc(mi & ((1u << lane) - 1u));
+        if (!on)
+            continue;
+        uint32_t link, count;
+        if (is_leaf) {
+            link = it.tri_start;
+            count = ntris[it.node];
+            // the leaf's triangles, left to right
+            uint32_t stack[kLeafStack];
+            int sp = 0, k = 0;
+            stack[sp++] = it.node;
+            while (sp > 0) {
+                uint32_t x = stack[--sp];
+                if (x < n) {
+                    uint32_t t = order[x];
+                    uint4 g = tidx[t];
+                    float4 p0 = vpos[g.x], p1 = vpos[g.y], p2 = vpos[g.z];
+                    size_t r = 3 * static_cast<size_t>(it.tri_start + k);
+                    tri[r] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(t));
+                    tri[r + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z,
+                                             k + 1 == static_cast<int>(count) ? 1.0f : 0.0f); // the leaf's last record
+                    tri[r + 2] = make_float4(p2.x - p0.x, p2.y - p0.y, p2.z - p0.z, 0.0f);
+                    k++;
+                } else if (sp + 2 <= kLeafStack) {
+                    int2 c = child[x];
+                    stack[sp++] = static_cast<uint32_t>(c.y);
+                    stack[sp++] = static_cast<uint32_t>(c.x);
+                }
+            }
+        } else {
+            // depth-first preorder slots, as the host builder lays nodes out: the k-th interior node in
+            // preorder keeps its children at 1 + 2k and 2 + 2k
+            link = 1 + 2 * it.pre;
+            count = 0;
+            int2 c = child[it.node];
+            if (at + 1 < 2 * n) { // a malformed tree is refused before a write could leave the buffers
+                next[at] = FlatItem{static_cast<uint32_t>(c.x), link, it.tri_start, it.pre + 1};
+                next[at + 1] =
+                    FlatItem{static_cast<uint32_t>(c.y), link + 1, it.tri_start + ntris[c.x], it.pre + 1 + icount[c.x]};
+            }
+        }
+        if (it.slot >= 2 * n)
+            continue;
+        const float4 b0 = blo[it.node], b1 = bhi[it.node];
+        nlo[it.slot] = make_float4(inflate_lo(b0.x, eps), inflate_lo(b0.y, eps), inflate_lo(b0.z, eps),
+                                   __uint_as_float(link));
+        nhi[it.slot] = make_float4(inflate_hi(b1.x, eps), inflate_hi(b1.y, eps), inflate_hi(b1.z, eps),
+                                   __uint_as_float(count));
     }
-    nlo[it.slot] = make_float4(inflate_lo(b0.x, eps), inflate_lo(b0.y, eps), inflate_lo(b0.z, eps),
-                               __uint_as_float(link));
-    nhi[it.slot] = make_float4(inflate_hi(b1.x, eps), inflate_hi(b1.y, eps), inflate_hi(b1.z, eps),
-                               __uint_as_float(count));
 }
 
 inline uint32_t blocks(uint64_t n, int per) { return n ? static_cast<uint32_t>((n + per - 1) / per) : 1u; }
@@ -626,16 +748,24 @@ struct Carver {
     }
 };
 
+// A level of the collapse: its frontier's length and the first node and triangle positions of the
+// next level (level l reads state[l] and makes state[l + 1]).
+struct WideState {
+    uint32_t f, next_base, tri_running;
+};
 struct Scratch {
     uint32_t *red, *keys0, *vals0, *keys1, *vals1, *hist, *sums, *total;
     float4 *tlo, *thi, *blo, *bhi;
     int2 *child;
-    uint32_t *clus0, *clus1, *mflag, *kflag, *mscan, *kscan, *parent, *counter, *ntris, *icount;
+    uint32_t *clus0, *clus1, *parent, *counter, *ntris, *icount;
+    uint64_t *scan, *tile_sums; // two counts per word (PLOC rounds, eight-wide levels)
+    PlocState *ploc;            // the rounds' two states
+    uint32_t *lvl;              // items per level of the flattening
+    WideState *wstate;          // per level of the collapse
     int32_t *nn;
     float *cost;
     uint8_t *leaf;
     FlatItem *fa, *fb;
-    uint32_t *iflag;
     unsigned long long *leaf_stats;
     WideItem *wa, *wb;   // eight-wide collapse: frontiers,
     uint32_t *wslots;    // 8 chosen children per frontier node,
@@ -664,10 +794,11 @@ Scratch carve(void *base, uint32_t n, size_t *bytes) {
     s.child = c.take<int2>(nodes);
     s.clus0 = c.take<uint32_t>(n);
     s.clus1 = c.take<uint32_t>(n);
-    s.mflag = c.take<uint32_t>(n);
-    s.kflag = c.take<uint32_t>(n);
-    s.mscan = c.take<uint32_t>(n);
-    s.kscan = c.take<uint32_t>(n);
+    s.scan = c.take<uint64_t>(n);
+    s.tile_sums = c.take<uint64_t>(blocks(n, kScanTile) + 1);
+    s.ploc = c.take<PlocState>(2);
+    s.lvl = c.take<uint32_t>(kLevels);
+    s.wstate = c.take<WideState>(kLevels);
     s.nn = c.take<int32_t>(n);
     s.parent = c.take<uint32_t>(nodes);
     s.counter = c.take<uint32_t>(nodes);
@@ -677,7 +808,6 @@ Scratch carve(void *base, uint32_t n, size_t *bytes) {
     s.leaf = c.take<uint8_t>(nodes);
     s.fa = c.take<FlatItem>(nodes);
     s.fb = c.take<FlatItem>(nodes);
-    s.iflag = c.take<uint32_t>(nodes);
     s.leaf_stats = c.take<unsigned long long>(2);
     s.wa = c.take<WideItem>(n);
     s.wb = c.take<WideItem>(n);
@@ -711,116 +841,172 @@ __device__ __forceinline__ float wide_area(float4 lo, float4 hi) {
 // Children of one wide node in slot order (binary node ids, kNone for an empty slot).
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
-__device__ void wide_children(uint32_t bn, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi, uint32_t slots[8]) {
-    uint32_t ch[8];
-    int n = 0;
-    if (__float_as_uint(nhi[bn].w) == 0) {
-        uint32_t l = __float_as_uint(nlo[bn].w);
-        ch[0] = l;
-        ch[1] = l + 1;
-        n = 2;
-        while (n < 8) {
-            int best = -1;
-            float best_area = -1.0f;
-            for (int i = 0; i < n; i++)
-                if (__float_as_uint(nhi[ch[i]].w) == 0) {
-                    float a = wide_area(nlo[ch[i]], nhi[ch[i]]);
-                    if (a > best_area) {
-                        best = i;
-                        best_area = a;
-                    }
-                }
-            if (best < 0)
-                break;
-            uint32_t l = __float_as_uint(nlo[ch[best]].w);
-            ch[best] = l;
-            ch[n++] = l + 1;
+__global__ void k_wide_start(WideItem *items, WideState *state) {
+    items[0] = WideItem{0, 0};
+    state[0] = WideState{1, 1, 0};
+}
+
+// Eight lanes per wide node, one child each (a thread per node with its children and costs in local
+// memory took 731 us over the nine levels of the 1.3M-triangle scene, this 313): the child with the largest area is opened until there
+// are eight (or none is interior), then children take octant slots greedily by the cost of the octant
+// they lie in, the cheapest (child, slot) first. Ties: the lowest child, then the lowest slot.
+__global__ void __launch_bounds__(kGB)
+    k_wide_plan(WideState const *state, WideItem const *items, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
+                uint32_t *slots_out, uint64_t *counts) {
+    const uint32_t f = state->f, lane = threadIdx.x & 31u, li = lane & 7u, g0 = lane & ~7u;
+    for (uint32_t i0 = (blockIdx.x * kGB + (threadIdx.x & ~31u)) / 8; i0 < f; i0 += gridDim.x * (kGB / 8)) {
+        const uint32_t i = i0 + lane / 8;
+        const bool on = i < f;
+        uint32_t id = kNone, n = 0, link = 0, cnt = 1;
+        float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+        if (on) {
+            const uint32_t bn = items[i].bn;
+            lo = nlo[bn], hi = nhi[bn];
+            const bool interior = __float_as_uint(hi.w) == 0;
+            n = interior ? 2u : 1u; // a root that is a leaf is its own child
+            id = li < n ? (interior ? __float_as_uint(lo.w) + li : bn) : kNone;
         }
-    } else {
-        ch[0] = bn; // a root that is a leaf
-        n = 1;
-    }
-    float ulo[3] = {INFINITY, INFINITY, INFINITY}, uhi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = 0; i < n; i++) {
-        float4 a = nlo[ch[i]], b = nhi[ch[i]];
-        ulo[0] = a.x < ulo[0] ? a.x : ulo[0];
-        ulo[1] = a.y < ulo[1] ? a.y : ulo[1];
-        ulo[2] = a.z < ulo[2] ? a.z : ulo[2];
-        uhi[0] = uhi[0] < b.x ? b.x : uhi[0];
-        uhi[1] = uhi[1] < b.y ? b.y : uhi[1];
-        uhi[2] = uhi[2] < b.z ? b.z : uhi[2];
-    }
-    float cost[8][8];
-    for (int i = 0; i < n; i++) {
-        float4 a = nlo[ch[i]], b = nhi[ch[i]];
-        float lo[3] = {a.x, a.y, a.z}, hi[3] = {b.x, b.y, b.z};
+        bool fetch = id != kNone;
+        for (int step = 0; step < 7; step++) {
+            if (fetch) {
+                lo = nlo[id], hi = nhi[id];
+                link = __float_as_uint(lo.w);
+                cnt = __float_as_uint(hi.w);
+            }
+            // the interior child with the largest area, the lowest of equals
+            float area = id != kNone && cnt == 0 ? wide_area(lo, hi) : -1.0f;
+            uint32_t at = li;
+            for (int k = 4; k > 0; k >>= 1) {
+                float a2 = __shfl_xor_sync(~0u, area, k);
+                uint32_t l2 = __shfl_xor_sync(~0u, at, k);
+                if (a2 > area || (a2 == area && l2 < at)) {
+                    area = a2;
+                    at = l2;
+                }
+            }
+            const bool open = on && n < 8 && n > 1 && area > -1.0f;
+            const uint32_t l = __shfl_sync(~0u, link, g0 + at);
+            fetch = open && (li == at || li == n);
+            if (fetch)
+                id = li == at ? l : l + 1;
+            n += open;
+        }
+        // (seven rounds: six openings and the fetch of the last pair)
+        const bool have = id != kNone;
+        float ulo[3] = {INFINITY, INFINITY, INFINITY}, uhi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        const float blo[3] = {lo.x, lo.y, lo.z}, bhi[3] = {hi.x, hi.y, hi.z};
+        float off[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            if (have) {
+                ulo[a] = blo[a];
+                uhi[a] = bhi[a];
+            }
+            for (int k = 4; k > 0; k >>= 1) {
+                ulo[a] = fminf(ulo[a], __shfl_xor_sync(~0u, ulo[a], k));
+                uhi[a] = fmaxf(uhi[a], __shfl_xor_sync(~0u, uhi[a], k));
+            }
+            off[a] = 0.5f * (blo[a] + bhi[a]) - 0.5f * (ulo[a] + uhi[a]);
+        }
+        float cost[8];
+#pragma unroll
         for (int s = 0; s < 8; s++) {
             float c = 0;
-            for (int ax = 0; ax < 3; ax++) {
-                float off = 0.5f * (lo[ax] + hi[ax]) - 0.5f * (ulo[ax] + uhi[ax]);
-                c += (s >> ax & 1) ? -off : off;
-            }
-            cost[i][s] = c;
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+                c += (s >> a & 1) ? -off[a] : off[a];
+            cost[s] = c;
         }
-    }
-    int slot_of[8], child_in[8];
-    for (int i = 0; i < 8; i++)
-        slot_of[i] = child_in[i] = -1;
-    for (int k = 0; k < n; k++) {
-        int bi = -1, bs = -1;
-        float bc = INFINITY;
-        for (int i = 0; i < n; i++) {
-            if (slot_of[i] >= 0)
-                continue;
-            for (int s = 0; s < (n <= 4 ? 4 : 8); s++)
-                if (child_in[s] < 0 && (bi < 0 || cost[i][s] < bc)) {
-                    bi = i;
+        uint32_t open_slots = n <= 4 ? 0xFu : 0xFFu, slot = kNone;
+        for (uint32_t k = 0; k < 8; k++) {
+            const bool want = have && slot == kNone;
+            float bc = INFINITY;
+            uint32_t bs = 8;
+#pragma unroll
+            for (uint32_t s = 0; s < 8; s++)
+                if (want && (open_slots >> s & 1u) && (bs == 8 || cost[s] < bc)) {
+                    bc = cost[s] == cost[s] ? cost[s] : INFINITY; // boxes near the float range: any order will do
                     bs = s;
-                    bc = cost[i][s];
                 }
+            uint32_t at = want ? li : 8 + li;
+            for (int o = 4; o > 0; o >>= 1) {
+                float c2 = __shfl_xor_sync(~0u, bc, o);
+                uint32_t a2 = __shfl_xor_sync(~0u, at, o);
+                if (a2 < 8 && (at >= 8 || c2 < bc || (c2 == bc && a2 < at))) {
+                    bc = c2;
+                    at = a2;
+                }
+            }
+            const uint32_t taken = __shfl_sync(~0u, bs, g0 + (at & 7u));
+            if (at < 8) {
+                if (li == at)
+                    slot = taken;
+                open_slots &= ~(1u << taken);
+            }
         }
-        slot_of[bi] = bs;
-        child_in[bs] = bi;
+        uint32_t used = have ? 1u << slot : 0u, ni = have && cnt == 0, nt = have ? cnt : 0u;
+        for (int k = 4; k > 0; k >>= 1) {
+            used |= __shfl_xor_sync(~0u, used, k);
+            ni += __shfl_xor_sync(~0u, ni, k);
+            nt += __shfl_xor_sync(~0u, nt, k);
+        }
+        if (on) {
+            if (have)
+                slots_out[8 * static_cast<size_t>(i) + slot] = id;
+            if (!(used >> li & 1u))
+                slots_out[8 * static_cast<size_t>(i) + li] = kNone;
+            if (li == 0)
+                counts[i] = static_cast<uint64_t>(nt) << 32 | ni;
+        }
     }
-    for (int s = 0; s < 8; s++)
-        slots[s] = child_in[s] < 0 ? kNone : ch[child_in[s]];
 }
 
-__global__ void k_wide_plan(WideItem const *items, uint32_t f, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
-                            uint32_t *slots_out, uint32_t *n_int, uint32_t *n_tri) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= f)
-        return;
-    uint32_t slots[8];
-    wide_children(items[i].bn, nlo, nhi, slots);
-    uint32_t ni = 0, nt = 0;
-    for (int s = 0; s < 8; s++) {
-        slots_out[8 * static_cast<size_t>(i) + s] = slots[s];
-        if (slots[s] == kNone)
-            continue;
-        uint32_t cnt = __float_as_uint(nhi[slots[s]].w);
-        if (cnt == 0)
-            ni++;
-        else
-            nt += cnt;
+// Scan of a level's (triangles, interior children), tile by tile, then the tile totals.
+__global__ void __launch_bounds__(1024) k_wide_tiles(WideState const *state, uint64_t *counts, uint64_t *sums) {
+    __shared__ uint64_t sh[32];
+    const uint32_t f = state->f;
+    for (uint32_t tile = blockIdx.x; tile * kScanTile < f; tile += gridDim.x) {
+        uint32_t base = tile * kScanTile + threadIdx.x * kScanItems;
+        uint64_t v[kScanItems], t = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            v[k] = base + k < f ? counts[base + k] : 0;
+            t += v[k];
+        }
+        uint64_t incl = block_inclusive<1024>(t, sh);
+        uint64_t run = incl - t;
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            if (base + k < f)
+                counts[base + k] = run;
+            run += v[k];
+        }
+        if (threadIdx.x == 1023)
+            sums[tile] = incl;
     }
-    n_int[i] = ni;
-    n_tri[i] = nt;
 }
 
-__global__ void k_wide_emit(WideItem const *items, uint32_t f, uint32_t const *slots_in, uint32_t const *int_scan,
-                            uint32_t const *tri_scan, uint32_t next_base, uint32_t tri_running, NodeHalf<const float4> nlo,
-                            NodeHalf<const float4> nhi, float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide,
-                            WideItem *next) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= f)
-        return;
+__global__ void __launch_bounds__(1024) k_wide_sums(WideState const *state, WideState *next, uint64_t *sums) {
+    __shared__ uint64_t sh[32];
+    WideState s = *state;
+    const uint64_t total = scan_totals(sums, s.f ? (s.f - 1) / kScanTile + 1 : 0, sh);
+    if (threadIdx.x == 0)
+        *next = WideState{static_cast<uint32_t>(total), s.next_base + static_cast<uint32_t>(total),
+                          s.tri_running + static_cast<uint32_t>(total >> 32)};
+}
+
+__device__ __forceinline__ void wide_emit_node(WideState const &st, WideItem const &item, uint32_t i,
+                                               uint32_t const *slots_in, uint64_t at, uint32_t n,
+                                               NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
+                                               float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide,
+                                               WideItem *next) {
+    const uint32_t int_at = static_cast<uint32_t>(at);
     uint32_t words[24];
     for (int k = 0; k < 24; k++)
         words[k] = 0;
     float slo[8][3], shi[8][3];
     uint32_t present = 0, imask = 0, leaves = 0, counts = 0;
-    uint32_t child_base = next_base + int_scan[i], tri_base = tri_running + tri_scan[i];
+    uint32_t child_base = st.next_base + int_at, tri_base = st.tri_running + static_cast<uint32_t>(at >> 32);
     uint32_t rank = 0, toff = 0;
     uint32_t meta[2] = {0, 0};
     for (int s = 0; s < 8; s++) {
@@ -837,7 +1023,8 @@ __global__ void k_wide_emit(WideItem const *items, uint32_t f, uint32_t const *s
         uint32_t cnt = __float_as_uint(b.w);
         if (cnt == 0) {
             imask |= 1u << s;
-            next[int_scan[i] + rank] = WideItem{c, child_base + rank};
+            if (int_at + rank < n)
+                next[int_at + rank] = WideItem{c, child_base + rank};
             rank++;
         } else {
             meta[s >> 2] |= toff << (8 * (s & 3));
@@ -861,11 +1048,20 @@ __global__ void k_wide_emit(WideItem const *items, uint32_t f, uint32_t const *s
     words[7] = meta[1];
     words[20] = counts;
     words[21] = leaves;
-    uint4 *dst = wide + 6 * static_cast<size_t>(items[i].wn);
+    uint4 *dst = wide + 6 * static_cast<size_t>(item.wn);
     for (int q = 0; q < 6; q++)
         dst[q] = make_uint4(words[4 * q], words[4 * q + 1], words[4 * q + 2], words[4 * q + 3]);
 }
 
+__global__ void __launch_bounds__(kGB)
+    k_wide_emit(WideState const *state, WideItem const *items, uint32_t const *slots_in, uint64_t const *scan,
+                uint64_t const *sums, uint32_t n, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
+                float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide, WideItem *next) {
+    const uint32_t f = state->f;
+    for (uint32_t i = blockIdx.x * kGB + threadIdx.x; i < f; i += gridDim.x * kGB)
+        wide_emit_node(*state, items[i], i, slots_in, scan[i] + sums[i / kScanTile], n, nlo, nhi, tri_bin, tri_wide,
+                       step_min, wide, next);
+}
 } // namespace
 
 size_t gpu_build_scratch_bytes(uint32_t num_tris) {
@@ -899,44 +1095,43 @@ cudaError_t gpu_build_sah_pairs(GpuBuildIn const &in, GpuBuildOut &out, cudaStre
     uint32_t *order = vin; // sorted position -> triangle
     k_gather_leaves<<<blocks(n, kGB), kGB, 0, st>>>(order, s.tlo, s.thi, n, s.blo, s.bhi, s.clus0);
     // 2. PLOC rounds
-    uint32_t m = n, base = n;
-    uint32_t *ca = s.clus0, *cb = s.clus1;
-    int rounds = 0;
-    while (m > 1) {
-        if (m <= static_cast<uint32_t>(kPlocSmall)) {
-            // the remaining rounds in one block
-            k_ploc_finish<<<1, kPlocSmallThreads, 0, st>>>(ca, m, base, s.blo, s.bhi, s.child, s.total + 2);
-            cudaError_t e = cudaMemcpyAsync(host, s.total + 2, 4, cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess)
-                e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess)
-                return e;
-            if (host[0] == 0)
-                return cudaErrorUnknown; // no mutual pair (non-finite boxes): host build
-            base = host[0];
-            m = 1;
-            break;
+    k_ploc_start<<<1, 1, 0, st>>>(s.ploc, n);
+    auto *hs = static_cast<PlocState *>(in.host_pinned);
+    PlocState now{n, n, 0, 0, 0};
+    for (uint32_t r = 0; now.m > static_cast<uint32_t>(kPlocSmall);) {
+        const uint32_t m0 = now.m, g = blocks(now.m, kGB), tiles = blocks(now.m, kScanTile);
+        for (int k = 0; k < kPlocBatch; k++, r++) {
+            PlocState *cur = s.ploc + (r & 1), *nxt = s.ploc + (r & 1 ^ 1);
+            k_ploc_nn<<<g, kGB, 0, st>>>(cur, s.clus0, s.clus1, s.blo, s.bhi, s.nn);
+            k_ploc_tiles<<<tiles, 1024, 0, st>>>(cur, s.nn, s.scan, s.tile_sums);
+            k_ploc_sums<<<1, 1024, 0, st>>>(cur, nxt, s.tile_sums);
+            k_ploc_apply<<<g, kGB, 0, st>>>(cur, s.clus0, s.clus1, s.nn, s.scan, s.tile_sums, s.blo, s.bhi, s.child);
         }
-        if (++rounds > 100000)
-            return cudaErrorUnknown; // no progress: the caller falls back to the host build
-        uint32_t g = blocks(m, kGB);
-        k_ploc_nn<<<g, kGB, 0, st>>>(ca, m, s.blo, s.bhi, s.nn);
-        k_ploc_flags<<<g, kGB, 0, st>>>(s.nn, m, s.mflag, s.kflag);
-        cudaMemcpyAsync(s.mscan, s.mflag, 4 * static_cast<size_t>(m), cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(s.kscan, s.kflag, 4 * static_cast<size_t>(m), cudaMemcpyDeviceToDevice, st);
-        scan(s.mscan, m, s.sums, s.total, st);
-        scan(s.kscan, m, s.sums, s.total + 1, st);
-        k_ploc_apply<<<g, kGB, 0, st>>>(ca, cb, s.nn, m, s.mscan, s.kscan, s.mflag, s.kflag, base, s.blo, s.bhi,
-                                        s.child);
-        cudaMemcpyAsync(host, s.total, 8, cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = cudaMemcpyAsync(hs, s.ploc + (r & 1), sizeof(PlocState), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess)
+            return e;
+        now = *hs;
+        if (now.stuck || now.m >= m0)
+            return cudaErrorUnknown; // no mutual pair (non-finite boxes): host build
+    }
+    uint32_t base = now.base;
+    if (now.m > 1) { // the remaining rounds in one block
+        cudaError_t e = cudaFuncSetAttribute(k_ploc_finish, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(kPlocFinishShared));
+        if (e != cudaSuccess)
+            return e;
+        k_ploc_finish<<<1, kPlocSmallThreads, kPlocFinishShared, st>>>(now.cur ? s.clus1 : s.clus0, now.m, base, s.blo,
+                                                                       s.bhi, s.child, s.total + 2);
+        e = cudaMemcpyAsync(host, s.total + 2, 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(st);
         if (e != cudaSuccess)
             return e;
         if (host[0] == 0)
             return cudaErrorUnknown; // no mutual pair (non-finite boxes): host build
-        base += host[0];
-        m = host[1];
-        std::swap(ca, cb);
+        base = host[0];
     }
     uint32_t num_nodes = base, root = num_nodes - 1;
     // 3. leaf collapse
@@ -946,48 +1141,41 @@ cudaError_t gpu_build_sah_pairs(GpuBuildIn const &in, GpuBuildOut &out, cudaStre
     cudaMemsetAsync(s.counter, 0, 4 * static_cast<size_t>(num_nodes), st);
     k_collapse<<<blocks(n, kGB), kGB, 0, st>>>(n, s.child, s.parent, s.blo, s.bhi, s.counter, s.ntris, s.icount, s.cost,
                                                s.leaf, in.max_leaf, in.tri_cost, in.node_cost);
-    // 4. flatten level by level
-    FlatItem first{root, 0, 0, 0};
-    cudaMemcpyAsync(s.fa, &first, sizeof(first), cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(s.leaf_stats, 0, 16, st);
-    uint32_t f = 1, slot_base = 1, depth = 0;
-    uint64_t leaf_depth_sum = 0;
-    FlatItem *fa = s.fa, *fb = s.fb;
-    while (f > 0) {
-        depth++;
-        // a level never holds more nodes than there are triangles; anything else is a malformed
-        // tree, which is refused before a write could leave the buffers
-        if (f > n || slot_base > 2ull * n)
-            return cudaErrorUnknown;
-        if (depth > in.max_depth) { // deeper than the traversal stack: the host builds instead
-            out.ok = false;
-            return cudaSuccess;
-        }
-        uint32_t g = blocks(f, kGB);
-        k_flat_flags<<<g, kGB, 0, st>>>(fa, f, s.leaf, s.iflag);
-        scan(s.iflag, f, s.sums, s.total, st);
-        k_flat_emit<<<g, kGB, 0, st>>>(fa, f, s.iflag, n, s.child, s.leaf, s.ntris, s.icount, s.blo, s.bhi, order,
-                                       in.tidx, in.vpos, s.red, in.nlo, in.nhi, in.tri, fb, s.leaf_stats);
-        cudaMemcpyAsync(host, s.total, 4, cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess)
-            return e;
-        uint32_t interior = host[0];
-        leaf_depth_sum += static_cast<uint64_t>(f - interior) * (depth - 1);
-        slot_base += 2 * interior;
-        f = 2 * interior;
-        std::swap(fa, fb);
+    // 4. flatten level by level, one level more than the traversal stack allows
+    k_flat_start<<<1, 64, 0, st>>>(s.fa, s.lvl, s.leaf_stats, root);
+    const uint32_t levels = std::min<uint32_t>(in.max_depth, kLevels - 2);
+    for (uint32_t l = 0; l < levels; l++) {
+        const uint32_t g = static_cast<uint32_t>(std::min<uint64_t>(blocks(uint64_t(1) << std::min(l, 31u), kGB),
+                                                                    std::min<uint32_t>(blocks(n, kGB), grid_cap)));
+        k_flat_level<<<g, kGB, 0, st>>>(l & 1 ? s.fb : s.fa, l & 1 ? s.fa : s.fb, s.lvl, l, n, s.child, s.leaf, s.ntris,
+                                        s.icount, s.blo, s.bhi, order, in.tidx, in.vpos, s.red, in.nlo, in.nhi, in.tri,
+                                        s.leaf_stats);
     }
-    out.num_nodes = slot_base;
-    unsigned long long leaves = 0;
-    cudaError_t e = cudaMemcpyAsync(host, s.leaf_stats, 8, cudaMemcpyDeviceToHost, st);
+    uint32_t lvl[kLevels], stats[4 + 6];
+    cudaError_t e = cudaMemcpyAsync(lvl, s.lvl, sizeof(lvl), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(host + 2, s.red, 24, cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(stats, s.leaf_stats, 16, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(stats + 4, s.red, 24, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(st);
     if (e != cudaSuccess)
         return e;
-    std::memcpy(&leaves, host, 8);
+    uint32_t slots = 0, depth = 0;
+    for (; depth < levels && lvl[depth]; depth++) {
+        if (lvl[depth] > n || slots + lvl[depth] > 2ull * n)
+            return cudaErrorUnknown; // a malformed tree
+        slots += lvl[depth];
+    }
+    if (depth == levels && lvl[depth]) { // deeper than the traversal stack: the host builds instead
+        out.ok = false;
+        return cudaSuccess;
+    }
+    out.num_nodes = slots;
+    unsigned long long leaves = 0, leaf_depth_sum = 0;
+    host = stats + 2;
+    std::memcpy(&leaf_depth_sum, stats + 2, 8);
+    std::memcpy(&leaves, stats, 8);
     for (int a = 0; a < 3; a++) {
         uint32_t lo = host[2 + a], hi = host[5 + a];
         uint32_t ul = (lo & 0x80000000u) ? (lo & 0x7FFFFFFFu) : ~lo;
@@ -998,7 +1186,7 @@ cudaError_t gpu_build_sah_pairs(GpuBuildIn const &in, GpuBuildOut &out, cudaStre
     out.num_leaves = static_cast<uint32_t>(leaves);
     out.max_depth = depth;
     out.avg_leaf_depth = leaves ? static_cast<double>(leaf_depth_sum) / static_cast<double>(leaves) : 0.0;
-    out.ploc_rounds = static_cast<uint32_t>(rounds);
+    out.ploc_rounds = now.rounds;
     out.ok = depth <= in.max_depth;
     return cudaGetLastError();
 }
@@ -1014,41 +1202,50 @@ cudaError_t gpu_collapse_wide(GpuWideIn const &in, GpuWideOut &out, cudaStream_t
         return cudaSuccess;
     size_t bytes = 0;
     Scratch s = carve(in.scratch, n, &bytes);
-    uint32_t *host = static_cast<uint32_t *>(in.host_pinned);
     double step_min = wide_step_min(in.max_abs);
-    WideItem root{0, 0};
-    cudaError_t e = cudaMemcpyAsync(s.wa, &root, sizeof(root), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess)
-        return e;
-    uint32_t f = 1, next_base = 1, tri_running = 0, depth = 0, level_first = 0;
-    WideItem *wa = s.wa, *wb = s.wb;
-    while (f > 0) {
-        if (++depth > in.max_depth || depth >= 32 || f > n || next_base > n + 1) {
-            out.ok = false; // too deep for the eight-wide stack: keep the binary tree
-            return cudaSuccess;
+    k_wide_start<<<1, 1, 0, st>>>(s.wa, s.wstate);
+    // the levels follow each other without the host, which looks after kWideBatch of them and then
+    // for the few more that a deep tree has
+    constexpr uint32_t kWideBatch = 10;
+    const uint32_t levels = std::min<uint32_t>(in.max_depth, 31);
+    const uint32_t cap = 8 * in.num_sms;
+    WideState ws[kLevels];
+    uint32_t depth = 0;
+    for (uint32_t l = 0; l < levels;) {
+        const uint32_t to = std::min<uint32_t>(l + kWideBatch, levels);
+        for (; l < to; l++) {
+            const uint64_t most = std::min<uint64_t>(n, uint64_t(1) << std::min<uint32_t>(3 * l, 32));
+            WideItem *wa = l & 1 ? s.wb : s.wa, *wb = l & 1 ? s.wa : s.wb;
+            WideState *cur = s.wstate + l;
+            k_wide_plan<<<std::min<uint32_t>(blocks(8 * most, kGB), cap), kGB, 0, st>>>(cur, wa, in.nlo, in.nhi, s.wslots,
+                                                                                       s.scan);
+            k_wide_tiles<<<std::min<uint32_t>(blocks(most, kScanTile), cap), 1024, 0, st>>>(cur, s.scan, s.tile_sums);
+            k_wide_sums<<<1, 1024, 0, st>>>(cur, cur + 1, s.tile_sums);
+            k_wide_emit<<<std::min<uint32_t>(blocks(most, kGB), cap), kGB, 0, st>>>(
+                cur, wa, s.wslots, s.scan, s.tile_sums, n, in.nlo, in.nhi, in.tri, s.tri_tmp, step_min, in.wide, wb);
         }
-        out.level_start[depth - 1] = level_first; // this level's nodes are [level_first, next_base)
-        level_first = next_base;
-        uint32_t g = blocks(f, kGB);
-        k_wide_plan<<<g, kGB, 0, st>>>(wa, f, in.nlo, in.nhi, s.wslots, s.mscan, s.kscan);
-        scan(s.mscan, f, s.sums, s.total, st);
-        scan(s.kscan, f, s.sums, s.total + 1, st);
-        k_wide_emit<<<g, kGB, 0, st>>>(wa, f, s.wslots, s.mscan, s.kscan, next_base, tri_running, in.nlo, in.nhi,
-                                       in.tri, s.tri_tmp, step_min, in.wide, wb);
-        e = cudaMemcpyAsync(host, s.total, 8, cudaMemcpyDeviceToHost, st);
+        cudaError_t e = cudaMemcpyAsync(ws, s.wstate, sizeof(WideState) * (l + 1), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess)
             e = cudaStreamSynchronize(st);
         if (e != cudaSuccess)
             return e;
-        next_base += host[0];
-        tri_running += host[1];
-        f = host[0];
-        std::swap(wa, wb);
+        for (; depth < l && ws[depth].f; depth++) {
+            if (ws[depth].f > n || ws[depth].next_base > n + 1)
+                return cudaErrorUnknown; // a malformed tree
+            out.level_start[depth] = ws[depth].next_base - ws[depth].f;
+        }
+        if (ws[depth].f == 0)
+            break;
     }
-    if (tri_running != n)
+    if (ws[depth].f) {
+        out.ok = false; // too deep for the eight-wide stack: keep the binary tree
+        return cudaSuccess;
+    }
+    const uint32_t next_base = ws[depth].next_base;
+    if (ws[depth].tri_running != n)
         return cudaErrorUnknown;
     // the triangle records move to the wide order only now that the collapse succeeded
-    e = cudaMemcpyAsync(in.tri, s.tri_tmp, 48 * static_cast<size_t>(n), cudaMemcpyDeviceToDevice, st);
+    cudaError_t e = cudaMemcpyAsync(in.tri, s.tri_tmp, 48 * static_cast<size_t>(n), cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess)
         return e;
     out.num_nodes = next_base;

@@ -28,7 +28,7 @@ struct GpuBuildOut {
 };
 
 size_t gpu_build_scratch_bytes(uint32_t num_tris);
-// Synchronises `st` once per clustering round and per level. cudaErrorUnknown: no progress
+// Synchronises `st` every few clustering rounds and at the end. cudaErrorUnknown: no progress
 // (non-finite boxes); the caller builds on the host instead.
 cudaError_t gpu_build_sah_pairs(GpuBuildIn const &in, GpuBuildOut &out, cudaStream_t st);
 
@@ -42,7 +42,7 @@ struct GpuWideIn {
     float max_abs;           // largest |coordinate| of the vertices and the camera
     uint32_t max_depth;      // levels the eight-wide stack allows
     void *scratch;           // gpu_build_scratch_bytes(num_tris) bytes
-    void *host_pinned;       // 8 bytes of pinned host memory
+    int num_sms;
     uint4 *wide;             // room for num_tris nodes of 96 bytes
 };
 struct GpuWideOut {
