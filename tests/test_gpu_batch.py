@@ -79,3 +79,20 @@ def test_batch_wavefront_equals_separate_renders(ctx):
         ref = ctx.render(p)
         close = np.abs(img - ref) <= np.maximum(1e-4 * np.abs(ref), 1e-5)
         assert close.mean() >= 0.999, close.mean()
+
+
+@pytest.mark.parametrize("integrator", [abi.INTEGRATOR_WAVEFRONT, abi.INTEGRATOR_MEGAKERNEL])
+@pytest.mark.parametrize("n", [1, 2, 40])
+def test_batch_of_uneven_scenes_built_on_every_core(ctx, n, integrator):
+    """Fewer and more scenes than cores, of 12 to 3,000 triangles: each image is its scene's own."""
+    layout = abi.BVH_WIDE if integrator == abi.INTEGRATOR_WAVEFRONT else abi.BVH_SAH
+    scenes = [S.soup((12, 3000, 400, 57)[k % 4], seed=k + 1, width=16, height=16) for k in range(n)]
+    params = [default_params(abi.MODE_MIS, 16, 16, 2, seed=k + 9, max_depth=4, rr_start=3) for k in range(n)]
+    for p in params:
+        p.integrator = integrator
+    imgs, _ = render_batch(ctx, scenes, params)
+    for k in {0, 1 % n, n - 1}:
+        ctx.upload(scenes[k], layout=layout)
+        ref = ctx.render(params[k])
+        close = np.abs(imgs[k] - ref) <= np.maximum(1e-4 * np.abs(ref), 1e-5)
+        assert close.mean() >= 0.999, (k, close.mean())

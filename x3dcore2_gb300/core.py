@@ -105,8 +105,8 @@ class Context:
 
     def pipeline_frame(self, cfg, width, height, want_rgba=False):
         """One pipeline frame: (8-bit RGBA pixels (h, w, 4), float image or None)."""
-        px = np.zeros((height, width, 4), np.uint8)
-        rgba = np.zeros((height, width, 4), np.float32) if want_rgba else None
+        px = np.empty((height, width, 4), np.uint8)
+        rgba = np.empty((height, width, 4), np.float32) if want_rgba else None
         self._check(self.lib.e8g_pipeline_frame(self.h, C.byref(cfg), width, height, _ptr(px),
                                                 None if rgba is None else _ptr(rgba)), "e8g_pipeline_frame")
         return px, rgba
@@ -171,7 +171,7 @@ class Context:
 
     # ---- rendering ----------------------------------------------------------------------
     def render(self, params):
-        out = np.zeros((params.height, params.width, 4), np.float32)
+        out = np.empty((params.height, params.width, 4), np.float32)
         self._check(self.lib.e8g_render(self.h, C.byref(params), _ptr(out)), "e8g_render")
         return out
 
@@ -236,7 +236,7 @@ class Context:
 
     # ---- differentiable rendering -------------------------------------------------------
     def forward(self, params):
-        out = np.zeros((params.height, params.width, 4), np.float32)
+        out = np.empty((params.height, params.width, 4), np.float32)
         self._check(self.lib.e8g_forward(self.h, C.byref(params), _ptr(out)), "e8g_forward")
         return out
 
@@ -259,7 +259,7 @@ def render_batch(ctx, scenes, params):
     items = (abi.BatchItem * n)()
     outs = []
     for k, (sc, p) in enumerate(zip(scenes, params)):
-        img = np.zeros((p.height, p.width, 4), np.float32)
+        img = np.empty((p.height, p.width, 4), np.float32)
         outs.append(img)
         items[k].scene = C.pointer(sc.desc)
         items[k].params = p

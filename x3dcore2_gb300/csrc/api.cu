@@ -826,7 +826,7 @@ e8g_status e8g_render(e8g_ctx *c, e8g_render_params const *p, float *rgba_out) {
     cudaError_t e = c->b_img.reserve(bytes);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "image buffer");
-    s = render_image(c, p, static_cast<float *>(c->b_img.ptr), nullptr);
+    s = render_image(c, p, static_cast<float *>(c->b_img.ptr), nullptr, 0, rgba_out);
     if (s != E8G_OK)
         return s;
     e = cudaMemcpyAsync(rgba_out, c->b_img.ptr, bytes, cudaMemcpyDeviceToHost, c->stream);

@@ -132,8 +132,12 @@ e8g_status build_tree(e8g_ctx *c);
 e8g_status sync_host_vertices(e8g_ctx *c);
 
 // Renders an image into d_rgba (device). counts (host, 3 values) requests the instrumented run.
+// host_out: where the caller copies the image next (its pages are made present meanwhile).
 e8g_status render_image(e8g_ctx *c, e8g_render_params const *p, float *d_rgba, unsigned long long *counts,
-                        uint64_t prior_spp = 0);
+                        uint64_t prior_spp = 0, float *host_out = nullptr);
+// Makes the pages of a large host output present while the GPU works on what goes there. Fresh pages
+// (a new array's) otherwise fault one by one under the copy.
+void populate_host(void *out, size_t bytes);
 // Wavefront integrator over the image or a path list (E8G_MODE_MIS).
 e8g_status run_wavefront(e8g_ctx *c, RenderArgs const &A, float4 *accum, float *path_rgb, uint32_t capacity,
                          uint32_t bounces, uint32_t threshold, BatchDev const *B = nullptr,

@@ -10,23 +10,67 @@
 #include "api_internal.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
+#include <exception>
+#include <memory>
+#include <mutex>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 namespace e8g {
 namespace {
 
-struct staged {
-    std::vector<unsigned char> bytes;
-    size_t put(void const *src, size_t n) {
-        size_t off = (bytes.size() + 255) & ~static_cast<size_t>(255);
-        bytes.resize(off + std::max<size_t>(n, 16));
-        if (n)
-            std::memcpy(bytes.data() + off, src, n);
+// Offsets of arrays in one allocation, each at a multiple of 256 bytes.
+struct layout_of {
+    size_t size = 0;
+    size_t put(size_t n) {
+        size_t off = (size + 255) & ~static_cast<size_t>(255);
+        size = off + std::max<size_t>(n, 16);
         return off;
     }
-    template <class T> size_t put(std::vector<T> const &v) { return put(v.data(), v.size() * sizeof(T)); }
+    template <class T> size_t put(std::vector<T> const &v) { return put(v.size() * sizeof(T)); }
 };
+
+// fn(k) for every scene, spread over the machine's cores; the scenes with most triangles start first, so
+// that none of them is left for the end. An exception of a call is thrown again here once every thread
+// has stopped; threads that cannot be started are done without.
+template <class F> void for_scenes(e8g_batch_item const *items, uint32_t n, F &&fn) {
+    std::vector<uint32_t> order(n);
+    for (uint32_t k = 0; k < n; k++)
+        order[k] = k;
+    auto tris = [&](uint32_t k) { return items[k].scene->mesh_tri_offset[items[k].scene->num_meshes]; };
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return tris(a) > tris(b); });
+    std::atomic<uint32_t> next{0};
+    std::mutex lock;
+    std::exception_ptr error;
+    auto work = [&] {
+        for (uint32_t i; (i = next.fetch_add(1)) < n;) {
+            try {
+                fn(order[i]);
+            } catch (...) {
+                std::lock_guard<std::mutex> hold(lock);
+                if (!error)
+                    error = std::current_exception();
+                next = n;
+            }
+        }
+    };
+    const uint32_t most = std::min<uint32_t>(n, std::max(1u, std::thread::hardware_concurrency()));
+    std::vector<std::thread> threads;
+    threads.reserve(most);
+    try {
+        while (threads.size() + 1 < most)
+            threads.emplace_back(work);
+    } catch (std::system_error const &) {
+    }
+    work();
+    for (std::thread &t : threads)
+        t.join();
+    if (error)
+        std::rethrow_exception(error);
+}
 
 } // namespace
 } // namespace e8g
@@ -61,8 +105,8 @@ extern "C" e8g_status e8g_batch_render(e8g_ctx *c, e8g_batch_item const *items, 
         return fail(c, E8G_ERR_CANCELLED, "batch cancelled");
     cudaSetDevice(c->device);
     c->prog_spp = 0; // the batch reuses the accumulator
-    // host: pack, build, stage
-    staged st;
+    // host: pack, build, stage, a scene to a core
+    layout_of lay;
     struct offs {
         size_t nodes, wide, tri, tidx, vpos, vnrm, vtx, mesh_mat, mesh_light, mesh_toff, mesh_area, tri_cum, mats, light_mesh,
             light_rad, light_cum, light_pnorm;
@@ -74,56 +118,89 @@ extern "C" e8g_status e8g_batch_render(e8g_ctx *c, e8g_batch_item const *items, 
     uint32_t rng_kinds = 0;
     for (uint32_t k = 0; k < n; k++)
         rng_kinds |= 1u << items[k].params.rng;
+    std::unique_ptr<unsigned char[]> stage;
+    size_t recs = 0, pp = 0, px = 0, scene_rec = 0;
     try {
-        for (uint32_t k = 0; k < n; k++)
-            pack_scene(*items[k].scene, packs[k]);
         bvh_build_opts bo;
         bo.layout = use_wf ? 2u : 0u;
-        for (uint32_t k = 0; k < n; k++)
+        std::vector<std::vector<float>> nodes(n); // SAH pairs as the device keeps them
+        auto build = [&](uint32_t k) {
             build_scene_bvh(packs[k], bo);
-        for (uint32_t k = 0; k < n && use_wf; k++)
-            if (packs[k].layout != 2) { // a tree too deep for the wide stack: SAH pairs for all
-                use_wf = false;
-                bo.layout = 0;
-                for (uint32_t j = 0; j < n; j++)
-                    build_scene_bvh(packs[j], bo);
-            }
+            interleave_nodes(packs[k].bvh, nodes[k]);
+        };
+        for_scenes(items, n, [&](uint32_t k) {
+            pack_scene(*items[k].scene, packs[k]);
+            build(k);
+        });
+        if (use_wf && std::any_of(packs.begin(), packs.end(), [](packed_scene const &p) { return p.layout != 2; })) {
+            use_wf = false; // a tree too deep for the wide stack: SAH pairs for all
+            bo.layout = 0;
+            for_scenes(items, n, build);
+        }
         for (uint32_t k = 0; k < n; k++) {
             packed_scene &p = packs[k];
             offs &o = off[k];
-            std::vector<float> nodes;
-            interleave_nodes(p.bvh, nodes);
-            o.nodes = st.put(nodes);
-            o.wide = st.put(p.wide);
-            o.tri = st.put(p.tri);
-            o.tidx = st.put(p.tidx);
-            o.vpos = st.put(p.vpos);
-            o.vnrm = st.put(p.vnrm);
-            o.vtx = st.put(p.vtx);
-            o.mesh_mat = st.put(p.mesh_mat);
-            o.mesh_light = st.put(p.mesh_light);
-            o.mesh_toff = st.put(p.mesh_toff);
-            o.mesh_area = st.put(p.mesh_area);
-            o.tri_cum = st.put(p.tri_cum);
-            o.mats = st.put(p.mats);
-            o.light_mesh = st.put(p.light_mesh);
-            o.light_rad = st.put(p.light_rad);
-            o.light_cum = st.put(p.light_cum);
-            o.light_pnorm = st.put(p.light_pnorm);
+            o.nodes = lay.put(nodes[k]);
+            o.wide = lay.put(p.wide);
+            o.tri = lay.put(p.tri);
+            o.tidx = lay.put(p.tidx);
+            o.vpos = lay.put(p.vpos);
+            o.vnrm = lay.put(p.vnrm);
+            o.vtx = lay.put(p.vtx);
+            o.mesh_mat = lay.put(p.mesh_mat);
+            o.mesh_light = lay.put(p.mesh_light);
+            o.mesh_toff = lay.put(p.mesh_toff);
+            o.mesh_area = lay.put(p.mesh_area);
+            o.tri_cum = lay.put(p.tri_cum);
+            o.mats = lay.put(p.mats);
+            o.light_mesh = lay.put(p.light_mesh);
+            o.light_rad = lay.put(p.light_rad);
+            o.light_cum = lay.put(p.light_cum);
+            o.light_pnorm = lay.put(p.light_pnorm);
             args[k] = make_args(&items[k].params);
             path_prefix[k + 1] = path_prefix[k] + args[k].total_paths;
             pix_prefix[k + 1] = pix_prefix[k] + static_cast<uint64_t>(items[k].params.width) * items[k].params.height;
         }
+        recs = lay.put(args);
+        pp = lay.put(path_prefix);
+        px = lay.put(pix_prefix);
+        scene_rec = lay.put(n * sizeof(DevScene));
+        stage.reset(new unsigned char[lay.size]);
+        auto put = [&](size_t at, auto const &v) {
+            if (!v.empty())
+                std::memcpy(stage.get() + at, v.data(), v.size() * sizeof(v[0]));
+        };
+        for_scenes(items, n, [&](uint32_t k) {
+            packed_scene const &p = packs[k];
+            offs const &o = off[k];
+            put(o.nodes, nodes[k]);
+            put(o.wide, p.wide);
+            put(o.tri, p.tri);
+            put(o.tidx, p.tidx);
+            put(o.vpos, p.vpos);
+            put(o.vnrm, p.vnrm);
+            put(o.vtx, p.vtx);
+            put(o.mesh_mat, p.mesh_mat);
+            put(o.mesh_light, p.mesh_light);
+            put(o.mesh_toff, p.mesh_toff);
+            put(o.mesh_area, p.mesh_area);
+            put(o.tri_cum, p.tri_cum);
+            put(o.mats, p.mats);
+            put(o.light_mesh, p.light_mesh);
+            put(o.light_rad, p.light_rad);
+            put(o.light_cum, p.light_cum);
+            put(o.light_pnorm, p.light_pnorm);
+        });
+        put(recs, args);
+        put(pp, path_prefix);
+        put(px, pix_prefix);
     } catch (std::bad_alloc const &) {
         return fail(c, E8G_ERR_OUT_OF_MEMORY, "host allocation failed while packing the batch");
+    } catch (std::system_error const &x) {
+        return fail(c, E8G_ERR_INTERNAL, std::string("building the batch's trees: ") + x.what());
     }
-    size_t recs = st.put(args);
-    size_t pp = st.put(path_prefix);
-    size_t px = st.put(pix_prefix);
-    size_t scene_rec = (st.bytes.size() + 255) & ~static_cast<size_t>(255);
-    st.bytes.resize(scene_rec + n * sizeof(DevScene));
     uint64_t total_pix = pix_prefix[n];
-    cudaError_t e = c->b_batch.reserve(st.bytes.size());
+    cudaError_t e = c->b_batch.reserve(lay.size);
     if (e == cudaSuccess)
         e = c->b_fh.reserve(total_pix * sizeof(FirstHit));
     if (e == cudaSuccess)
@@ -169,7 +246,7 @@ extern "C" e8g_status e8g_batch_render(e8g_ctx *c, e8g_batch_item const *items, 
             S.bmax[i] = p.bmax[i];
         }
         S.cam = p.cam;
-        std::memcpy(st.bytes.data() + scene_rec + k * sizeof(DevScene), &S, sizeof(DevScene));
+        std::memcpy(stage.get() + scene_rec + k * sizeof(DevScene), &S, sizeof(DevScene));
     }
     BatchDev B{};
     B.scenes = reinterpret_cast<DevScene const *>(base + scene_rec);
@@ -178,7 +255,7 @@ extern "C" e8g_status e8g_batch_render(e8g_ctx *c, e8g_batch_item const *items, 
     B.pix_prefix = reinterpret_cast<uint64_t const *>(base + px);
     B.n = n;
     B.total_paths = path_prefix[n];
-    e = cudaMemcpyAsync(base, st.bytes.data(), st.bytes.size(), cudaMemcpyHostToDevice, c->stream);
+    e = cudaMemcpyAsync(base, stage.get(), lay.size, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "batch upload");
     // device: one first-hit launch, one persistent integrator launch, one resolve

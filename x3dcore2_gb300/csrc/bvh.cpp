@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 #include <future>
+#include <system_error>
 #include <thread>
 
 namespace e8g {
@@ -53,7 +54,7 @@ struct builder {
     std::vector<tmp_node> nodes;
     std::atomic<uint32_t> next{0};
     std::atomic<uint32_t> max_depth{0};
-    uint32_t parallel_cutoff = 1u << 15;
+    uint32_t parallel_cutoff = 1u << 15; // larger subtrees are built by two threads
 
     uint32_t alloc() { return next.fetch_add(1); }
 
@@ -89,38 +90,76 @@ struct builder {
             float ext = cb.hi[a] - cb.lo[a];
             if (!(ext > 0))
                 continue;
-            box bins[64];
-            uint32_t cnt[64] = {0};
+            // Only occupied bins are swept, and in a node of fewer triangles than bins only they are set up:
+            // a split beside an empty bin costs what the one before it costs.
+            struct bin_box {
+                float lo[3], hi[3];
+            } bins[64];
+            uint32_t cnt[64];
+            uint64_t occ = 0;
             float k = nb / ext;
-            for (uint32_t i = start; i < end; i++) {
-                uint32_t id = ids[i];
-                uint32_t bi = std::min<uint32_t>(nb - 1, static_cast<uint32_t>((pc[3 * id + a] - cb.lo[a]) * k));
-                bins[bi].grow(pb[id]);
-                cnt[bi]++;
+            auto bin_of = [&](uint32_t id) {
+                return std::min<uint32_t>(nb - 1, static_cast<uint32_t>((pc[3 * id + a] - cb.lo[a]) * k));
+            };
+            auto grow_bin = [](bin_box &d, box const &t) {
+                for (int x = 0; x < 3; x++) {
+                    d.lo[x] = std::min(d.lo[x], t.lo[x]);
+                    d.hi[x] = std::max(d.hi[x], t.hi[x]);
+                }
+            };
+            if (count >= nb) {
+                for (uint32_t i = 0; i < nb; i++) {
+                    bins[i] = {{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
+                    cnt[i] = 0;
+                }
+                for (uint32_t i = start; i < end; i++) {
+                    uint32_t id = ids[i], bi = bin_of(id);
+                    grow_bin(bins[bi], pb[id]);
+                    cnt[bi]++;
+                }
+                for (uint32_t i = 0; i < nb; i++)
+                    occ |= uint64_t(cnt[i] ? 1 : 0) << i;
+            } else {
+                for (uint32_t i = start; i < end; i++) {
+                    uint32_t id = ids[i], bi = bin_of(id);
+                    if (occ >> bi & 1u) {
+                        grow_bin(bins[bi], pb[id]);
+                        cnt[bi]++;
+                    } else {
+                        occ |= uint64_t(1) << bi;
+                        std::memcpy(bins[bi].lo, pb[id].lo, sizeof(bins[bi].lo));
+                        std::memcpy(bins[bi].hi, pb[id].hi, sizeof(bins[bi].hi));
+                        cnt[bi] = 1;
+                    }
+                }
             }
-            float right_area[64];
-            uint32_t right_cnt[64];
+            uint8_t at[64]; // the occupied bins, in order
+            int n_occ = 0;
+            for (uint64_t m = occ; m; m &= m - 1)
+                at[n_occ++] = static_cast<uint8_t>(__builtin_ctzll(m));
+            auto grow = [&](box &acc, int bin) {
+                for (int x = 0; x < 3; x++) {
+                    acc.lo[x] = std::min(acc.lo[x], bins[bin].lo[x]);
+                    acc.hi[x] = std::max(acc.hi[x], bins[bin].hi[x]);
+                }
+            };
+            float right_area[64]; // of the occupied bins from the j-th on
             box acc;
-            uint32_t c = 0;
-            for (int i = static_cast<int>(nb) - 1; i > 0; i--) {
-                acc.grow(bins[i]);
-                c += cnt[i];
-                right_area[i] = acc.area();
-                right_cnt[i] = c;
+            for (int j = n_occ - 1; j > 0; j--) {
+                grow(acc, at[j]);
+                right_area[j] = acc.area();
             }
             box lacc;
             uint32_t lc = 0;
-            for (uint32_t i = 0; i + 1 < nb; i++) {
-                lacc.grow(bins[i]);
-                lc += cnt[i];
-                if (lc == 0 || right_cnt[i + 1] == 0)
-                    continue;
-                float cost = o.node_cost + o.tri_cost * (lacc.area() * lc + right_area[i + 1] * right_cnt[i + 1]) /
+            for (int j = 0; j + 1 < n_occ; j++) {
+                grow(lacc, at[j]);
+                lc += cnt[at[j]];
+                float cost = o.node_cost + o.tri_cost * (lacc.area() * lc + right_area[j + 1] * (count - lc)) /
                                                std::max(parent_area, 1e-30f);
                 if (cost < best_cost) {
                     best_cost = cost;
                     best_axis = a;
-                    best_bin = i + 1;
+                    best_bin = at[j] + 1u;
                 }
             }
         }
@@ -147,9 +186,15 @@ struct builder {
         nodes[n].child[0] = static_cast<int32_t>(l);
         nodes[n].child[1] = static_cast<int32_t>(r);
         if (count > parallel_cutoff) {
-            auto fut = std::async(std::launch::async, [this, l, start, mid, depth] { build(l, start, mid, depth + 1); });
+            std::future<void> fut;
+            try {
+                fut = std::async(std::launch::async, [this, l, start, mid, depth] { build(l, start, mid, depth + 1); });
+            } catch (std::system_error const &) { // no thread to be had
+                build(l, start, mid, depth + 1);
+            }
             build(r, mid, end, depth + 1);
-            fut.get();
+            if (fut.valid())
+                fut.get();
         } else {
             build(l, start, mid, depth + 1);
             build(r, mid, end, depth + 1);
@@ -181,6 +226,8 @@ flat_bvh build_bvh(float const *pos, uint32_t const *tris, uint32_t num_tris, bv
         scene.grow(tb);
     }
     b.nodes.resize(2 * static_cast<size_t>(num_tris) + 1);
+    // about eight threads at work in a small tree too, down to subtrees of some milliseconds
+    b.parallel_cutoff = std::min(1u << 15, std::max(1u << 12, num_tris / 8));
     uint32_t root = b.alloc();
     b.build(root, 0, num_tris, 0);
     uint32_t n_tmp = b.next.load();

@@ -167,30 +167,38 @@ wide_bvh collapse_wide(flat_bvh const &b, float const *pos, uint32_t const *tris
         for (int i = 0; i < 8; i++)
             slot_of[i] = child_in[i] = -1;
         float cost[8][8];
-        for (int i = 0; i < n; i++)
+        const int slots = n <= 4 ? 4 : 8;
+        int row_best[8]; // child i's cheapest free slot, the first of equal ones
+        auto find_best = [&](int i) {
+            int bs = -1;
+            for (int s = 0; s < slots; s++)
+                if (child_in[s] < 0 && (bs < 0 || cost[i][s] < cost[i][bs]))
+                    bs = s;
+            row_best[i] = bs;
+        };
+        for (int i = 0; i < n; i++) {
+            float off[3];
+            for (int a = 0; a < 3; a++)
+                off[a] = 0.5f * (ch[i].b.lo[a] + ch[i].b.hi[a]) - 0.5f * (u.lo[a] + u.hi[a]);
             for (int s = 0; s < 8; s++) {
                 float c = 0;
-                for (int a = 0; a < 3; a++) {
-                    float off = 0.5f * (ch[i].b.lo[a] + ch[i].b.hi[a]) - 0.5f * (u.lo[a] + u.hi[a]);
-                    c += (s >> a & 1) ? -off : off;
-                }
+                for (int a = 0; a < 3; a++)
+                    c += (s >> a & 1) ? -off[a] : off[a];
                 cost[i][s] = c;
             }
+            find_best(i);
+        }
         for (int k = 0; k < n; k++) {
-            int bi = -1, bs = -1;
-            float bc = INFINITY;
-            for (int i = 0; i < n; i++) {
-                if (slot_of[i] >= 0)
-                    continue;
-                for (int s = 0; s < (n <= 4 ? 4 : 8); s++)
-                    if (child_in[s] < 0 && (bi < 0 || cost[i][s] < bc)) {
-                        bi = i;
-                        bs = s;
-                        bc = cost[i][s];
-                    }
-            }
+            int bi = -1;
+            for (int i = 0; i < n; i++)
+                if (slot_of[i] < 0 && (bi < 0 || cost[i][row_best[i]] < cost[bi][row_best[bi]]))
+                    bi = i;
+            const int bs = row_best[bi];
             slot_of[bi] = bs;
             child_in[bs] = bi;
+            for (int i = 0; i < n; i++)
+                if (slot_of[i] < 0 && row_best[i] == bs)
+                    find_best(i);
         }
         // quantization grid and child boxes
         uint32_t words[kWideWords] = {0};

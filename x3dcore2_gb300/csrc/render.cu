@@ -5,11 +5,14 @@
 #include "wavefront.h"
 
 #include <algorithm>
+#include <cerrno>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <map>
 #include <string>
+#include <sys/mman.h>
+#include <unistd.h>
 
 namespace e8g {
 
@@ -477,8 +480,26 @@ e8g_status run_wavefront_concurrent(e8g_ctx *c, RenderArgs const &A, float4 *acc
     return E8G_OK;
 }
 
+void populate_host(void *out, size_t bytes) {
+#if defined(MADV_POPULATE_WRITE)
+    if (bytes < (size_t(1) << 20))
+        return;
+    // whole pages only; contents stay, and where the kernel refuses the pages fault as before
+    const auto page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
+    const uintptr_t lo = (reinterpret_cast<uintptr_t>(out) + page - 1) / page * page;
+    const uintptr_t hi = (reinterpret_cast<uintptr_t>(out) + bytes) / page * page;
+    const int saved = errno;
+    if (hi > lo)
+        (void)madvise(reinterpret_cast<void *>(lo), hi - lo, MADV_POPULATE_WRITE);
+    errno = saved;
+#else
+    (void)out;
+    (void)bytes;
+#endif
+}
+
 e8g_status render_image(e8g_ctx *c, e8g_render_params const *p, float *d_rgba, unsigned long long *counts,
-                        uint64_t prior_spp) {
+                        uint64_t prior_spp, float *host_out) {
     if (counts && p->mode == E8G_MODE_REF_LT2)
         return fail(c, E8G_ERR_UNSUPPORTED, "traversal counters cover every integrator but bidirect_lt2");
     nvtx_range range("e8g render");
@@ -528,6 +549,8 @@ e8g_status render_image(e8g_ctx *c, e8g_render_params const *p, float *d_rgba, u
         if (e != cudaSuccess)
             return cuda_fail(c, e, "counter readback");
     }
+    if (host_out)
+        populate_host(host_out, npix * 16);
     e = cudaEventSynchronize(c->ev1);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "render");
