@@ -658,17 +658,18 @@ constexpr int kWalkBlock = 512;
 template <class R>
 __global__ void __launch_bounds__(kWalkBlock, 1024 / kWalkBlock)
     k_bdw_walk(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh, BdwChunk C, WfSlots W,
-               uint64_t const *range, uint32_t *ext_n, uint32_t *busy) {
+               uint64_t const *range, WfLive const *live, uint32_t *ext_n, uint32_t *busy) {
     const uint64_t mix = splitmix64(A.seed);
+    const WfVisit visit = wf_visit(W, *live);
     const uint32_t max_len = C.max_len;
     const uint64_t first = range[0];
     const uint32_t count = static_cast<uint32_t>(range[1]);
     const uint32_t lane = lane_id();
     uint32_t busy_local = 0;
-    for (uint32_t s0 = blockIdx.x * blockDim.x; s0 < W.capacity; s0 += gridDim.x * blockDim.x) {
+    for (uint32_t s0 = blockIdx.x * blockDim.x; s0 < visit.n; s0 += gridDim.x * blockDim.x) {
         __syncthreads();
-        const uint32_t s = s0 + threadIdx.x;
-        const bool in = s < W.capacity;
+        const bool in = s0 + threadIdx.x < visit.n;
+        const uint32_t s = visit.list && in ? visit.list[s0 + threadIdx.x] : s0 + threadIdx.x;
         const uint32_t st = in ? W.state[s] : kWkEmpty;
         uint32_t stage = st & 3u, len = (st >> 2) & 31u, clen = (st >> 7) & 31u;
         uint32_t path = 0, pixel = 0, sample = 0, light = 0;
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(kWalkBlock, 1024 / kWalkBlock)
         __syncthreads();
         // once the chunk's path counter has passed its last path (it only grows), no slot takes a
         // path for the rest of the chunk: the tail bounces skip the refill atomics
-        bool emitted = false, paths_left = __ldcg(W.next_path) < count;
+        bool emitted = false, paths_left = !visit.list && __ldcg(W.next_path) < count;
         for (int round = 0; round < kWalkRounds; round++) {
             // a new path for every empty slot, one atomic per warp and draw; a path whose camera ray
             // left the scene has no camera vertex and contributes nothing, so the lane draws again
@@ -842,6 +843,8 @@ __global__ void __launch_bounds__(kWalkBlock, 1024 / kWalkBlock)
                 if (E8G_CHK(S.check, q < W.capacity, kChkQueue, q)) {
                     W.ext_o[q] = make_float4(org.x, org.y, org.z, __uint_as_float(s));
                     W.ext_d[q] = make_float4(dir.x, dir.y, dir.z, 0.0f);
+                    if (visit.next)
+                        visit.next[q] = s;
                 }
                 W.state[s] = stage | len << 2 | clen << 7;
                 W.sid[s] = path;
@@ -1144,9 +1147,11 @@ int bdpt_walk_grid(uint32_t slots, int num_sms) {
 void launch_bdpt_walk(DevScene const &S, RenderArgs const &A, FirstHit const *fh, BdwChunk const &C,
                       WfSlots const &W, uint64_t const *range, int grid, cudaStream_t st) {
     if (A.rng == E8G_RNG_MINSTD)
-        k_bdw_walk<RngMinstd><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_ext_count_ptr(W), wf_busy_ptr(W));
+        k_bdw_walk<RngMinstd><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_live_ptr(W), wf_ext_count_ptr(W),
+                                                              wf_busy_ptr(W));
     else
-        k_bdw_walk<RngPhilox><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_ext_count_ptr(W), wf_busy_ptr(W));
+        k_bdw_walk<RngPhilox><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_live_ptr(W), wf_ext_count_ptr(W),
+                                                              wf_busy_ptr(W));
 }
 
 void launch_bdpt_eval(DevScene const &S, float4 *accum, float *path_rgb, BdwChunk const &C, WfSlots const &Q,

@@ -23,6 +23,18 @@ struct WfCounters { // mirrors the device Counters of wavefront.cu
     uint32_t shadow_n, ext_n, busy, pad[3];
 };
 
+// Device memory for `pools` slot arrays of Q slots each, with the lists of occupied slots unless the
+// context has a memory limit (what fitted it still fits) or their allocation fails. *bytes: of one pool.
+cudaError_t reserve_slots(e8g_ctx *c, uint32_t Q, size_t pools, bool *live, size_t *bytes) {
+    for (*live = c->budget.cap == 0;; *live = false) {
+        *bytes = (wf_total_bytes(Q, *live) + 255) & ~static_cast<size_t>(255);
+        cudaError_t e = c->b_wf.reserve(pools == 1 ? wf_total_bytes(Q, *live) : pools * *bytes);
+        if (e == cudaSuccess || !*live)
+            return e;
+        cudaGetLastError();
+    }
+}
+
 // The split form of E8G_MODE_BDPT_POWER. Paths go in chunks (at most 2^26, and at most 32 GiB or
 // half the free device memory for subpaths, connection lists and shadow queue; fewer when the
 // memory limit refuses that: every chunk ends with a tail of walk bounces, and the 1280x720,
@@ -85,10 +97,12 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
     BdwChunk C = carve(static_cast<char *>(c->b_bdw.ptr), chunk, &Q, &range, &need);
     // the walk's slots
     const uint32_t slots = static_cast<uint32_t>(std::min<uint64_t>((chunk + 255) / 256 * 256, 1u << 23));
-    e = c->b_wf.reserve(wf_total_bytes(slots));
+    bool live = false;
+    size_t slot_bytes = 0;
+    e = reserve_slots(c, slots, 1, &live, &slot_bytes);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "bidirectional walk slots");
-    WfSlots W = wf_carve(c->b_wf.ptr, slots);
+    WfSlots W = wf_carve(c->b_wf.ptr, slots, live);
     // refill threshold of the trace kernels (threshold 8 against 16: 42.3 against 43.0 ms per
     // 1280x720, 32-spp frame)
     const uint32_t threshold = c->dev.layout == 0 || c->dev.layout == 2 ? 8u : 0u;
@@ -103,7 +117,7 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
     if (e != cudaSuccess)
         return cuda_fail(c, e, "bidirectional walk capture");
     for (uint32_t k = 0; k < kBounces; k++) {
-        wf_enqueue_reset(W, c->stream);
+        wf_enqueue_reset(W, range, c->stream);
         launch_bdpt_walk(c->dev, A, fh, C, W, range, grid_walk, c->stream);
         wf_enqueue_trace(c->dev, A, W, nullptr, nullptr, grid_trace, threshold, c->stream);
     }
@@ -262,10 +276,12 @@ e8g_status run_wavefront(e8g_ctx *c, RenderArgs const &A, float4 *accum, float *
         threshold = 16; // the many-scene form always traces with dynamic fetch
     uint64_t want = std::max<uint64_t>(total, 1024);
     uint32_t Q = static_cast<uint32_t>(std::min<uint64_t>(capacity, (want + 255) / 256 * 256));
-    cudaError_t e = c->b_wf.reserve(wf_total_bytes(Q));
+    bool live = false;
+    size_t slot_bytes = 0;
+    cudaError_t e = reserve_slots(c, Q, 1, &live, &slot_bytes);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "wavefront slots");
-    WfSlots W = wf_carve(c->b_wf.ptr, Q);
+    WfSlots W = wf_carve(c->b_wf.ptr, Q, live);
     e = wf_init(W, c->stream);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "wavefront init");
@@ -354,8 +370,9 @@ e8g_status run_wavefront_concurrent(e8g_ctx *c, RenderArgs const &A, float4 *acc
     uint64_t want = std::max<uint64_t>(total, 2048);
     uint32_t Qh = static_cast<uint32_t>(std::min<uint64_t>(capacity / 2, (want / 2 + 255) / 256 * 256));
     Qh = std::max<uint32_t>(Qh, 256);
-    size_t pool = (wf_total_bytes(Qh) + 255) & ~static_cast<size_t>(255);
-    cudaError_t e = c->b_wf.reserve(2 * pool);
+    bool live = false;
+    size_t pool = 0;
+    cudaError_t e = reserve_slots(c, Qh, 2, &live, &pool);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "wavefront slots");
     if (!c->stream2) {
@@ -367,8 +384,8 @@ e8g_status run_wavefront_concurrent(e8g_ctx *c, RenderArgs const &A, float4 *acc
         if (e != cudaSuccess)
             return cuda_fail(c, e, "second stream");
     }
-    WfSlots WA = wf_carve(c->b_wf.ptr, Qh);
-    WfSlots WB = wf_carve(static_cast<char *>(c->b_wf.ptr) + pool, Qh);
+    WfSlots WA = wf_carve(c->b_wf.ptr, Qh, live);
+    WfSlots WB = wf_carve(static_cast<char *>(c->b_wf.ptr) + pool, Qh, live);
     WB.next_path = WA.next_path;
     e = wf_init(WA, c->stream);
     if (e == cudaSuccess)

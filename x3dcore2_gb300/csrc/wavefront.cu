@@ -35,7 +35,7 @@ struct Counters {
     uint32_t shadow_n, ext_n;      // queue lengths of the current bounce
     uint32_t busy;                 // slots holding a path after the last shade
     uint32_t shadow_head, ext_head; // next queue entry to hand out (dynamic fetch)
-    uint32_t pad;
+    WfLive live;                    // the slots this bounce visits
 };
 
 __device__ __forceinline__ void emit_to(RenderArgs const &A, float4 *accum, float *path_rgb, uint32_t out, float3 c) {
@@ -95,11 +95,14 @@ __global__ void __launch_bounds__(THREADS, MINB)
     // Read once per thread: once the path counter has passed the last path (it only grows), no
     // slot can be refilled for the rest of the frame, and the tail bounces skip the refill atomics
     // (one per warp and slot group on a single address).
-    const bool paths_left = __ldcg(W.next_path) < total_paths;
+    const WfVisit visit = wf_visit(W, cnt->live);
+    const bool paths_left = !visit.list && __ldcg(W.next_path) < total_paths;
     uint32_t busy_local = 0;
-    for (uint32_t s0 = blockIdx.x * blockDim.x; s0 < W.capacity; s0 += gridDim.x * blockDim.x) {
+    for (uint32_t s0 = blockIdx.x * blockDim.x; s0 < visit.n; s0 += gridDim.x * blockDim.x) {
         uint32_t s = s0 + threadIdx.x;
-        bool in = s < W.capacity;
+        bool in = s < visit.n;
+        if (visit.list && in)
+            s = visit.list[s];
         uint32_t state = in ? W.state[s] : kEmpty;
         uint32_t sid = 0, pixel = 0, sample = 0, out = 0;
         float3 beta = f3(0, 0, 0), p = f3(0, 0, 0), n = f3(0, 0, 0), o = f3(0, 0, 0);
@@ -290,6 +293,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
         if (push_ext) {
             W.ext_o[eq] = make_float4(p.x, p.y, p.z, __uint_as_float(s));
             W.ext_d[eq] = make_float4(-o.x, -o.y, -o.z, __uint_as_float(sid));
+            if (visit.next)
+                visit.next[eq] = s;
         }
         if (in) {
             W.state[s] = state;
@@ -517,7 +522,12 @@ __global__ void __launch_bounds__(kBlock, kWfTraceBlocks)
     }
 }
 
-__global__ void k_wf_reset(Counters *cnt) {
+// total: paths in all, or range[1] (device memory) when range is given.
+__global__ void k_wf_reset(Counters *cnt, unsigned long long const *next_path, uint64_t total, uint64_t const *range,
+                           bool lists) {
+    cnt->live.listed = lists && __ldcg(next_path) >= (range ? range[1] : total) ? 1u : 0u;
+    cnt->live.n = cnt->ext_n;
+    cnt->live.turn ^= 1u;
     cnt->shadow_n = 0;
     cnt->ext_n = 0;
     cnt->busy = 0;
@@ -529,7 +539,7 @@ __global__ void k_wf_reset(Counters *cnt) {
 
 // Lays the slot arrays and queues out from `base` (each array 256-byte aligned) and returns
 // the bytes used in *total; with a null base it only measures (all pointers null).
-static WfSlots carve(char *base, uint32_t capacity, size_t *total) {
+static WfSlots carve(char *base, uint32_t capacity, bool live, size_t *total) {
     WfSlots W{};
     W.capacity = capacity;
     size_t off = 0;
@@ -555,20 +565,21 @@ static WfSlots carve(char *base, uint32_t capacity, size_t *total) {
     W.ext_d = reinterpret_cast<float4 *>(take(Q * 16));
     W.vp = reinterpret_cast<float4 *>(take(Q * 16));
     W.vn = reinterpret_cast<float4 *>(take(Q * 16));
+    W.live = live ? reinterpret_cast<uint32_t *>(take(2 * Q * 4)) : nullptr;
     W.counters = take(sizeof(Counters));
     W.next_path = base ? &reinterpret_cast<Counters *>(W.counters)->next_path : nullptr;
     *total = off;
     return W;
 }
 
-WfSlots wf_carve(void *base, uint32_t capacity) {
+WfSlots wf_carve(void *base, uint32_t capacity, bool live) {
     size_t total = 0;
-    return carve(static_cast<char *>(base), capacity, &total);
+    return carve(static_cast<char *>(base), capacity, live, &total);
 }
 
-size_t wf_total_bytes(uint32_t capacity) {
+size_t wf_total_bytes(uint32_t capacity, bool live) {
     size_t total = 0;
-    carve(nullptr, capacity, &total);
+    carve(nullptr, capacity, live, &total);
     return total;
 }
 
@@ -654,7 +665,7 @@ void wf_enqueue_bounce(DevScene const &S, RenderArgs const &A, FirstHit const *f
     mark(0);
     if (!B && shade_split(shade_variant))
         k_wf_complete<<<shade_grid, 256, 0, st>>>(S, A, W, cnt, accum, path_rgb);
-    k_wf_reset<<<1, 1, 0, st>>>(cnt);
+    k_wf_reset<<<1, 1, 0, st>>>(cnt, W.next_path, total_paths, nullptr, W.live != nullptr);
     if (B) { // the many-scene form shades with the first block shape
         if (A.rng == E8G_RNG_MINSTD)
             k_wf_shade<RngMinstd, true, 256, 4, false><<<shade_grid, 256, 0, st>>>(S, A, *B, fh, W, cnt, accum, nullptr,
@@ -689,7 +700,7 @@ void wf_enqueue_shade(DevScene const &S, RenderArgs const &A, FirstHit const *fh
     auto *cnt = reinterpret_cast<Counters *>(W.counters);
     if (shade_split(shade_variant))
         k_wf_complete<<<shade_grid, 256, 0, st>>>(S, A, W, cnt, accum, path_rgb);
-    k_wf_reset<<<1, 1, 0, st>>>(cnt);
+    k_wf_reset<<<1, 1, 0, st>>>(cnt, W.next_path, total_paths, nullptr, W.live != nullptr);
     if (A.rng == E8G_RNG_MINSTD)
         launch_shade<RngMinstd>(shade_variant, shade_grid, st, S, A, fh, W, cnt, accum, path_rgb, total_paths);
     else
@@ -722,7 +733,10 @@ uint32_t *wf_busy_ptr(WfSlots const &W) { return &reinterpret_cast<Counters *>(W
 size_t wf_counters_bytes() { return sizeof(Counters); }
 uint32_t *wf_shadow_count_ptr(WfSlots const &W) { return &reinterpret_cast<Counters *>(W.counters)->shadow_n; }
 uint32_t *wf_ext_count_ptr(WfSlots const &W) { return &reinterpret_cast<Counters *>(W.counters)->ext_n; }
-void wf_enqueue_reset(WfSlots const &W, cudaStream_t st) { k_wf_reset<<<1, 1, 0, st>>>(reinterpret_cast<Counters *>(W.counters)); }
+WfLive const *wf_live_ptr(WfSlots const &W) { return &reinterpret_cast<Counters *>(W.counters)->live; }
+void wf_enqueue_reset(WfSlots const &W, uint64_t const *range, cudaStream_t st) {
+    k_wf_reset<<<1, 1, 0, st>>>(reinterpret_cast<Counters *>(W.counters), W.next_path, 0, range, W.live != nullptr);
+}
 unsigned long long *wf_next_ptr(WfSlots const &W) { return &reinterpret_cast<Counters *>(W.counters)->next_path; }
 
 } // namespace e8g

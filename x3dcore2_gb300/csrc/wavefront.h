@@ -13,10 +13,34 @@ struct WfSlots {
     float4 *sh_o, *sh_d, *sh_c; // shadow queue: origin | out, direction | tmax, contribution
     float4 *ext_o, *ext_d;      // extension queue: origin | slot, direction
     float4 *vp, *vn;            // split form: completed vertex (position | mesh, normal | depth)
+    uint32_t *live;             // slots that hold a path: two lists, written in turn (WfLive); or null
     void *counters;
     unsigned long long *next_path; // the path counter refills draw from (shared by the pools of a
                                    // concurrent wavefront; the pool's own counter otherwise)
 };
+
+// Which slots a bounce visits, set by k_wf_reset. While paths are left every slot is: an empty one takes
+// a path. After the last path was taken (listed), only those on the list that the bounce before
+// wrote, one entry for each extension ray: the warps of the last bounces, and of every bounce but the
+// first of a render that fits the slots, are full (1280x720, 32-spp bidirectional frame: its walk's last
+// ten bounces ran with 10 of 32 lanes).
+struct WfLive {
+    uint32_t listed; // visit the list
+    uint32_t n;      // its length
+    uint32_t turn;   // the list being written; the other one is visited
+};
+struct WfVisit {
+    uint32_t const *list; // null: every slot
+    uint32_t n;           // entries or slots
+    uint32_t *next;       // the list being written, at the extension queue's positions
+};
+__device__ __forceinline__ WfVisit wf_visit(WfSlots const &W, WfLive const &l) {
+    WfVisit v;
+    v.list = l.listed ? W.live + static_cast<size_t>(l.turn ^ 1u) * W.capacity : nullptr;
+    v.n = l.listed ? l.n : W.capacity;
+    v.next = W.live ? W.live + static_cast<size_t>(l.turn) * W.capacity : nullptr;
+    return v;
+}
 
 // A path's stream kept in a slot between bounces: minstd keeps its state word, Philox the number
 // of draws taken (its 4-word block is regenerated on resume).
@@ -60,8 +84,9 @@ template <> struct RngSlot<RngPhilox> {
     }
 };
 
-size_t wf_total_bytes(uint32_t capacity);
-WfSlots wf_carve(void *base, uint32_t capacity);
+// live: with the lists of occupied slots (8 bytes a slot).
+size_t wf_total_bytes(uint32_t capacity, bool live);
+WfSlots wf_carve(void *base, uint32_t capacity, bool live);
 cudaError_t wf_init(WfSlots const &W, cudaStream_t st);
 int wf_trace_blocks_per_sm(uint32_t layout, uint32_t threshold);
 // threshold > 0: trace kernels refill idle lanes with new rays during traversal once that many
@@ -83,8 +108,10 @@ uint32_t *wf_busy_ptr(WfSlots const &W);
 size_t wf_counters_bytes();
 uint32_t *wf_shadow_count_ptr(WfSlots const &W);
 uint32_t *wf_ext_count_ptr(WfSlots const &W);
-// Zeroes the queue lengths, fetch heads and busy count (not the path counter) before a bounce.
-void wf_enqueue_reset(WfSlots const &W, cudaStream_t st);
+WfLive const *wf_live_ptr(WfSlots const &W);
+// Before a bounce: chooses the slots it visits and zeroes the queue lengths, fetch heads and busy count
+// (not the path counter). range: device memory, range[1] the number of paths.
+void wf_enqueue_reset(WfSlots const &W, uint64_t const *range, cudaStream_t st);
 
 // The split form of E8G_MODE_BDPT_POWER (bdpt.cu). The walk: one bounce over the slots of W
 // (advance every slot's path by one subpath vertex, refill finished slots from the chunk), whose
