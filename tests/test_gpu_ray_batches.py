@@ -90,3 +90,17 @@ def test_hit_records_equal_hit_arrays(ctx, layout, n):
     assert np.array_equal(g["t"], raw[:, 0]) and np.array_equal(g["b"], raw[:, 3:])
     assert np.array_equal(g["mesh"], raw[:, 1].view(np.int32)) and np.array_equal(g["tri"], raw[:, 2].view(np.int32))
     assert n == 1 or (g["mesh"] < 0).any()
+
+
+@pytest.mark.parametrize("n", [11_915, 11_916, 15_887, 15_888])
+def test_batches_around_the_pinned_limit(ctx, n):
+    """512 KiB hold the rays and hits of 11,915 closest-hit queries and of 15,887 any-hit ones: beyond
+    that the batch goes through device memory. Both give what the first rays alone give."""
+    ctx.upload(S.soup(500, seed=3, width=64, height=64), layout=abi.BVH_SAH)
+    rays = random_rays(n, -1.0, 1.0, seed=5)
+    tmin, tmax = np.full(n, 1e-4, np.float32), np.linspace(0.01, 2.0, n, dtype=np.float32)
+    hit, occ = ctx.trace_closest(rays), ctx.trace_any(rays, tmin, tmax)
+    for lo, hi in ((0, 4000), (n - 4000, n)):
+        part = ctx.trace_closest(rays[lo:hi])
+        assert all(np.array_equal(hit[k][lo:hi], part[k]) for k in part)
+        assert np.array_equal(occ[lo:hi], ctx.trace_any(rays[lo:hi], tmin[lo:hi], tmax[lo:hi]))

@@ -496,7 +496,9 @@ e8g_status e8g_create(e8g_ctx **out, e8g_device_opts const *opts) {
     if (e == cudaSuccess)
         e = c->b_work.reserve(64);
     if (e == cudaSuccess)
-        e = cudaMallocHost(&c->host_pinned, 64);
+        e = cudaMallocHost(&c->host_pinned, 64 + kHostIo);
+    if (e == cudaSuccess)
+        c->host_io = static_cast<char *>(c->host_pinned) + 64;
 #if defined(E8G_CHECKS)
     if (e == cudaSuccess)
         e = c->b_check.reserve(8);
@@ -707,6 +709,19 @@ static e8g_status trace_closest_host(e8g_ctx *c, e8g_ray const *rays, uint32_t n
         return fail(c, E8G_ERR_INVALID_ARG, "NULL buffers");
     cudaSetDevice(c->device);
     size_t rb = static_cast<size_t>(n) * sizeof(e8g_ray), hb = static_cast<size_t>(n) * sizeof(e8g_hit);
+    if (rb + hb <= kHostIo) {
+        auto *out = reinterpret_cast<float *>(c->host_io + rb);
+        std::memcpy(c->host_io, rays, rb);
+        launch_trace_closest(c->dev, reinterpret_cast<float const *>(c->host_io), n,
+                             arrays ? hit_arrays(out, n) : hit_records(out), c->num_sms, c->stream);
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess)
+            return cuda_fail(c, e, "trace_closest");
+        std::memcpy(hits, out, hb);
+        return read_checks(c);
+    }
     cudaError_t e = c->b_io0.reserve(rb);
     if (e == cudaSuccess)
         e = c->b_io1.reserve(hb);
@@ -717,6 +732,7 @@ static e8g_status trace_closest_host(e8g_ctx *c, e8g_ray const *rays, uint32_t n
     auto *out = static_cast<float *>(c->b_io1.ptr);
     launch_trace_closest(c->dev, static_cast<float const *>(c->b_io0.ptr), n,
                          arrays ? hit_arrays(out, n) : hit_records(out), c->num_sms, c->stream);
+    populate_host(hits, hb);
     e = cudaMemcpyAsync(hits, out, hb, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
@@ -742,6 +758,22 @@ e8g_status e8g_trace_any(e8g_ctx *c, e8g_ray const *rays, float const *t_min, fl
         return fail(c, E8G_ERR_INVALID_ARG, "NULL buffers");
     cudaSetDevice(c->device);
     size_t rb = static_cast<size_t>(n) * sizeof(e8g_ray), tb = static_cast<size_t>(n) * sizeof(float);
+    if (rb + 2 * tb + n <= kHostIo) {
+        char *base = c->host_io;
+        auto *out = reinterpret_cast<uint8_t *>(base + rb + 2 * tb);
+        std::memcpy(base, rays, rb);
+        std::memcpy(base + rb, t_min, tb);
+        std::memcpy(base + rb + tb, t_max, tb);
+        launch_trace_any(c->dev, reinterpret_cast<float const *>(base), reinterpret_cast<float const *>(base + rb),
+                         reinterpret_cast<float const *>(base + rb + tb), n, out, c->num_sms, c->stream);
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess)
+            return cuda_fail(c, e, "trace_any");
+        std::memcpy(occluded, out, n);
+        return read_checks(c);
+    }
     cudaError_t e = c->b_io0.reserve(rb + 2 * tb + n);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "trace_any buffers");
@@ -756,6 +788,7 @@ e8g_status e8g_trace_any(e8g_ctx *c, e8g_ray const *rays, float const *t_min, fl
     if (e != cudaSuccess)
         return cuda_fail(c, e, "trace_any upload");
     launch_trace_any(c->dev, reinterpret_cast<float const *>(base), dtmin, dtmax, n, docc, c->num_sms, c->stream);
+    populate_host(occluded, n);
     e = cudaMemcpyAsync(occluded, docc, n, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);

@@ -197,7 +197,7 @@ e8g_status e8g_pipeline_frame(e8g_ctx *c, e8g_pipeline_config const *cfg, uint32
         bool reset = !c->pipe_valid || !same_config(c->pipe_cfg, *cfg) || c->prog_spp == 0;
         s = e8g_render_progressive(c, &p, reset ? 1 : 0, d_rgba, nullptr);
     } else {
-        s = render_image(c, &p, d_rgba, nullptr, 0, rgba_out);
+        s = render_image(c, &p, d_rgba, nullptr, 0, rgba_out, pixels);
     }
     if (s != E8G_OK)
         return s;

@@ -499,7 +499,7 @@ e8g_status run_wavefront_concurrent(e8g_ctx *c, RenderArgs const &A, float4 *acc
 
 void populate_host(void *out, size_t bytes) {
 #if defined(MADV_POPULATE_WRITE)
-    if (bytes < (size_t(1) << 20))
+    if (!out || bytes < (size_t(1) << 17))
         return;
     // whole pages only; contents stay, and where the kernel refuses the pages fault as before
     const auto page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
@@ -516,7 +516,7 @@ void populate_host(void *out, size_t bytes) {
 }
 
 e8g_status render_image(e8g_ctx *c, e8g_render_params const *p, float *d_rgba, unsigned long long *counts,
-                        uint64_t prior_spp, float *host_out) {
+                        uint64_t prior_spp, void *rgba_out, void *pixels_out) {
     if (counts && p->mode == E8G_MODE_REF_LT2)
         return fail(c, E8G_ERR_UNSUPPORTED, "traversal counters cover every integrator but bidirect_lt2");
     nvtx_range range("e8g render");
@@ -566,8 +566,8 @@ e8g_status render_image(e8g_ctx *c, e8g_render_params const *p, float *d_rgba, u
         if (e != cudaSuccess)
             return cuda_fail(c, e, "counter readback");
     }
-    if (host_out)
-        populate_host(host_out, npix * 16);
+    populate_host(rgba_out, npix * 16);
+    populate_host(pixels_out, npix * 4);
     e = cudaEventSynchronize(c->ev1);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "render");
