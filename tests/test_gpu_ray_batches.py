@@ -104,3 +104,44 @@ def test_batches_around_the_pinned_limit(ctx, n):
         part = ctx.trace_closest(rays[lo:hi])
         assert all(np.array_equal(hit[k][lo:hi], part[k]) for k in part)
         assert np.array_equal(occ[lo:hi], ctx.trace_any(rays[lo:hi], tmin[lo:hi], tmax[lo:hi]))
+
+
+def edge_rays(sc, n, seed):
+    """Rays of which half are aimed at vertices and at points of edges, where two triangles lie at the
+    same distance, and some along an axis."""
+    r = np.random.default_rng(seed)
+    tri = sc.world_triangles().astype(np.float64)
+    t = tri[r.integers(0, len(tri), n)]
+    w = r.uniform(0, 1, (n, 1))
+    aim = np.where(r.random((n, 1)) < 0.3, t[:, 0], t[:, 0] * w + t[:, 1] * (1 - w))
+    aim = np.where(r.random((n, 1)) < 0.5, aim, r.uniform(-1, 1, (n, 3)))
+    o = r.uniform(-1, 1, (n, 3))
+    d = aim - o
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    d[: n // 16] = np.eye(3)[r.integers(0, 3, n // 16)]
+    return np.concatenate([o, d], axis=1).astype(np.float32)
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("scene", ["soup", "ico", "cornell", "doubled", "one"])
+def test_warp_per_ray_equals_lane_per_ray(ctx, layout, scene):
+    """Small batches give each ray a warp, large ones a lane: the same rays have the same hits in both,
+    bit for bit, also where two triangles lie at one distance."""
+    r = np.random.default_rng(1)
+    sc = {"soup": lambda: S.soup(3000, seed=2, width=64, height=64),
+          "ico": lambda: S.displaced_icosphere(level=4, seed=3, num_materials=8, width=64, height=64),
+          "cornell": lambda: S.cornell(64, 64),
+          "doubled": lambda: mesh_scene(np.repeat(r.uniform(-1, 1, (40, 3, 3)), 9, axis=0)),
+          "one": lambda: mesh_scene(r.uniform(-1, 1, (1, 3, 3)))}[scene]()
+    ctx.upload(sc, layout=layout)
+    n, copies = 3001, 30  # more than four rays for every warp the GPU holds in one call of all copies
+    rays = edge_rays(sc, n, seed=4)
+    tmin = r.choice(np.array([1e-4, 0.0, -1.0, 0.5], np.float32), n)
+    tmax = r.choice(np.array([0.25, 1.0, 1e-5, np.inf], np.float32), n)
+    many = ctx.trace_closest(np.tile(rays, (copies, 1)))
+    occ = ctx.trace_any(np.tile(rays, (copies, 1)), np.tile(tmin, copies), np.tile(tmax, copies))
+    for lo, hi in ((0, n), (0, 1), (5, 38)):
+        few = ctx.trace_closest(rays[lo:hi])
+        for k in few:
+            assert np.array_equal(few[k].view(np.uint32), np.ascontiguousarray(many[k][lo:hi]).view(np.uint32)), k
+        assert np.array_equal(ctx.trace_any(rays[lo:hi], tmin[lo:hi], tmax[lo:hi]), occ[lo:hi])
