@@ -85,8 +85,11 @@ struct RenderArgs {
 };
 
 // Map a path index to (pixel, sample) and its output slot: the list index (explicit lists), the
-// pixel (image accumulation) or sample * W * H + pixel (per-sample images). Consecutive path
-// indices cover 8x4 pixel tiles, one warp per tile, so a warp's first hits are neighbours.
+// pixel (image accumulation) or sample * W * H + pixel (per-sample images). 32 consecutive path
+// indices cover an 8x4 pixel tile, so a warp's first hits are neighbours; the tile's samples follow
+// each other, so the paths on their way at one time start in a small part of the image and share
+// the nodes around it (with all tiles of one sample after the other, the 1080p, 16-spp frame of the
+// 1.3M-triangle scene takes 18.3 ms against 16.9, the 64-spp wavefront 55.4 against 52.6).
 // Returns false for padding lanes outside the image.
 __device__ __forceinline__ bool path_coords(RenderArgs const &A, uint64_t idx, uint32_t &pixel, uint32_t &sample,
                                             uint32_t &out) {
@@ -96,9 +99,9 @@ __device__ __forceinline__ bool path_coords(RenderArgs const &A, uint64_t idx, u
         out = static_cast<uint32_t>(idx);
         return true;
     }
-    uint32_t s = static_cast<uint32_t>(idx / A.paths_per_sample);
-    uint32_t j = static_cast<uint32_t>(idx - static_cast<uint64_t>(s) * A.paths_per_sample);
-    uint32_t tile = j >> 5, w = j & 31u;
+    const uint64_t j = idx >> 5;
+    const uint32_t tile = static_cast<uint32_t>(j / A.spp), s = static_cast<uint32_t>(j - static_cast<uint64_t>(tile) * A.spp);
+    const uint32_t w = static_cast<uint32_t>(idx) & 31u;
     uint32_t x = (tile % A.tiles_x) * 8 + (w & 7u), y = (tile / A.tiles_x) * 4 + (w >> 3);
     if (x >= A.width || y >= A.height)
         return false;
