@@ -79,6 +79,37 @@ E8G_BOX_HD void wide_grid_floor_ceil(float v, float org, float inv, float &fl, f
         cl += 1.0f;
 }
 
+// One axis of a node's quantization grid from the children's union: the grid starts one step below it and
+// 253 steps cover it, so no child box is clamped to the grid's ends and every quantized plane lies at
+// least one step outside the (already pushed-out) child box: the slack absorbs the rounding of the
+// traversal's plane arithmetic. inv_step: 2^-e (dividing by the step 2^e is this exact product); returns
+// the exponent byte.
+E8G_BOX_HD uint32_t wide_grid_axis(float u_lo, float u_hi, double step_min, float &org, float &inv_step) {
+    double ext = static_cast<double>(u_hi) - static_cast<double>(u_lo);
+    double want = ext / 251.0;
+    want = want > step_min ? want : step_min;
+    int e = wide_exponent(want);
+    inv_step = ldexpf(1.0f, -e);
+    double l = static_cast<double>(u_lo) - ldexp(1.0, e);
+    float f = static_cast<float>(l);
+    if (static_cast<double>(f) > l)
+        f = nextafterf(f, -INFINITY);
+    org = f;
+    return static_cast<uint32_t>(e + 127);
+}
+
+// The quantized planes of one child box on one axis.
+E8G_BOX_HD void wide_grid_planes(float lo, float hi, float org, float inv_step, uint32_t &qlo, uint32_t &qhi) {
+    float fl, cl, unused;
+    wide_grid_floor_ceil(lo, org, inv_step, fl, unused);
+    wide_grid_floor_ceil(hi, org, inv_step, unused, cl);
+    float ql = fl - 1.0f, qh = cl + 1.0f;
+    ql = ql < 0.0f ? 0.0f : (ql > 255.0f ? 255.0f : ql);
+    qh = qh < 0.0f ? 0.0f : (qh > 255.0f ? 255.0f : qh);
+    qlo = static_cast<uint32_t>(ql);
+    qhi = static_cast<uint32_t>(qh);
+}
+
 // Fills a node's grid and quantized child boxes: words[0..2] (grid origin), the exponent bytes of
 // words[3] (the interior mask byte is left alone) and words[8..19]. lo/hi hold the pushed-out
 // boxes of the eight slots; only slots in `present` are used.
@@ -93,26 +124,11 @@ E8G_BOX_HD void wide_quantize(float const lo[8][3], float const hi[8][3], uint32
             u_hi[a] = u_hi[a] < hi[s][a] ? hi[s][a] : u_hi[a];
         }
     }
-    // The grid starts one step below the children's union and 253 steps cover it, so no child box
-    // is clamped to the grid's ends and every quantized plane lies at least one step outside the
-    // (already pushed-out) child box: the slack absorbs the rounding of the traversal's plane
-    // arithmetic.
-    float inv_step[3]; // 2^-e: dividing by the step 2^e is this exact product
-    float org[3];
+    float inv_step[3], org[3];
     uint32_t ebytes = 0;
     for (int a = 0; a < 3; a++) {
-        double ext = static_cast<double>(u_hi[a]) - static_cast<double>(u_lo[a]);
-        double want = ext / 251.0;
-        want = want > step_min ? want : step_min;
-        int e = wide_exponent(want);
-        inv_step[a] = ldexpf(1.0f, -e);
-        ebytes |= static_cast<uint32_t>(e + 127) << (8 * a);
-        double l = static_cast<double>(u_lo[a]) - ldexp(1.0, e);
-        float f = static_cast<float>(l);
-        if (static_cast<double>(f) > l)
-            f = nextafterf(f, -INFINITY);
-        org[a] = f;
-        words[a] = box_f2u(f);
+        ebytes |= wide_grid_axis(u_lo[a], u_hi[a], step_min, org[a], inv_step[a]) << (8 * a);
+        words[a] = box_f2u(org[a]);
     }
     words[3] = (words[3] & 0xFF000000u) | ebytes;
     uint32_t qb[12] = {0};
@@ -120,15 +136,11 @@ E8G_BOX_HD void wide_quantize(float const lo[8][3], float const hi[8][3], uint32
         if (!(present >> s & 1))
             continue;
         for (int a = 0; a < 3; a++) {
-            float fl, cl, unused;
-            wide_grid_floor_ceil(lo[s][a], org[a], inv_step[a], fl, unused);
-            wide_grid_floor_ceil(hi[s][a], org[a], inv_step[a], unused, cl);
-            float ql = fl - 1.0f, qh = cl + 1.0f;
-            ql = ql < 0.0f ? 0.0f : (ql > 255.0f ? 255.0f : ql);
-            qh = qh < 0.0f ? 0.0f : (qh > 255.0f ? 255.0f : qh);
+            uint32_t ql, qh;
+            wide_grid_planes(lo[s][a], hi[s][a], org[a], inv_step[a], ql, qh);
             // byte s of plane a (lo) and plane 3 + a (hi); 8 bytes per plane, little endian
-            qb[2 * a + (s >> 2)] |= static_cast<uint32_t>(ql) << (8 * (s & 3));
-            qb[2 * (3 + a) + (s >> 2)] |= static_cast<uint32_t>(qh) << (8 * (s & 3));
+            qb[2 * a + (s >> 2)] |= ql << (8 * (s & 3));
+            qb[2 * (3 + a) + (s >> 2)] |= qh << (8 * (s & 3));
         }
     }
     for (int k = 0; k < 12; k++)

@@ -16,13 +16,13 @@
 // 4. Top-down, one launch per level: every node of the level writes its 32-byte record (boxes
 //    pushed out exactly as the host builder pushes them out, bvh_boxes.h) at its depth-first
 //    preorder slot (the host builder's order: children adjacent, the k-th interior node's at 1 + 2k,
-//    from interior-node counts of the subtrees), leaves write their triangles' records.
+//    from interior-node counts of the subtrees); then a thread per triangle writes its record.
 // Every byte of the tree is deterministic: scans decide the clusters' and wide nodes' positions, and the
 // flattening's items carry theirs (only the order of a level's work list comes from an atomic).
 // Counts stay on the device: rounds and levels follow each other in the stream with grids for the
 // most they can hold, and the host reads back every few rounds and at the end. 525 launches and about
 // 70 reads made 5.7 ms of the 1.3M-triangle scene's eight-wide build; it is 236 launches, a dozen
-// reads and 3.1 ms (pairs 4.3 -> 2.3).
+// reads and 2.9 ms (pairs 4.3 -> 2.1).
 #include "bvh_boxes.h"
 #include "gpu_build.h"
 #include "launch.h"
@@ -41,7 +41,6 @@ constexpr int kScanItems = 4;     // elements per thread in the device-wide scan
 constexpr int kScanTile = 1024 * kScanItems;
 constexpr int kPlocRadius = 24;
 constexpr int kLevels = 40;       // entries of the per-level states (trees are at most 32 levels deep)
-constexpr int kLeafStack = 16;    // subtree walk of a leaf (at most 15 triangles)
 
 __device__ __forceinline__ uint32_t ord_key(float f) {
     uint32_t u = __float_as_uint(f);
@@ -147,74 +146,65 @@ __global__ void __launch_bounds__(kGB) k_sort_hist(uint32_t const *keys, uint32_
     hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x]; // digit-major
 }
 
-// Stable scatter of one tile: the tile is sorted by the digit in shared memory with eight stable
-// one-bit splits, then every key goes to its digit's global offset plus its rank in the tile.
+// Stable scatter of one tile: every key's rank among the equal digits before it (a warp matches 32 keys
+// at a time and keeps its own digit counts), one scan of the tile's digit counts, the tile put in
+// digit order in shared memory and written from there in runs. Eight one-bit splits with a block scan
+// each took 50 us a pass of 1.3M keys, this 21.
 __global__ void __launch_bounds__(kGB)
     k_sort_scatter(uint32_t const *kin, uint32_t const *vin, uint32_t *kout, uint32_t *vout, uint32_t n, int shift,
                    uint32_t const *offs) {
     __shared__ uint32_t sk[kSortTile], sv[kSortTile];
+    __shared__ uint32_t counts[kGB / 32][256]; // per warp and digit: the count, then where the warp's keys start
+    __shared__ uint32_t start[256];
     __shared__ uint32_t sh[32];
-    __shared__ uint32_t start[257];
-    uint32_t base = blockIdx.x * kSortTile;
-    uint32_t valid = min(static_cast<uint32_t>(kSortTile), n - base);
+    static_assert(kGB == 256, "a thread per digit");
+    const uint32_t base = blockIdx.x * kSortTile, lane = threadIdx.x & 31u, warp = threadIdx.x / 32;
+    const uint32_t valid = min(static_cast<uint32_t>(kSortTile), n - base);
+    for (int w = 0; w < kGB / 32; w++)
+        counts[w][threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
 #pragma unroll
     for (int k = 0; k < kSortItems; k++) {
-        uint32_t p = k * kGB + threadIdx.x;
-        sk[p] = p < valid ? kin[base + p] : 0xFFFFFFFFu; // padding sorts last and is never written
-        sv[p] = p < valid ? vin[base + p] : 0u;
+        const uint32_t p = warp * (32 * kSortItems) + k * 32 + lane;
+        const bool in = p < valid;
+        key[k] = in ? kin[base + p] : 0;
+        val[k] = in ? vin[base + p] : 0;
+        const uint32_t d = (key[k] >> shift) & 255u;
+        const uint32_t peers = __match_any_sync(~0u, in ? d : 256u);
+        const uint32_t before = in ? counts[warp][d] : 0;
+        rank[k] = before + __popc(peers & ((1u << lane) - 1u));
+        __syncwarp();
+        if (in && lane == 31u - __clz(peers)) // the last of the equal digits
+            counts[warp][d] = rank[k] + 1;
+        __syncwarp();
     }
     __syncthreads();
-    uint32_t key[kSortItems], val[kSortItems];
+    uint32_t sum = 0;
+    for (int w = 0; w < kGB / 32; w++) {
+        const uint32_t c = counts[w][threadIdx.x];
+        counts[w][threadIdx.x] = sum;
+        sum += c;
+    }
+    start[threadIdx.x] = block_inclusive<kGB>(sum, sh) - sum;
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < kSortItems; k++) {
-        key[k] = sk[threadIdx.x * kSortItems + k];
-        val[k] = sv[threadIdx.x * kSortItems + k];
-    }
-    __syncthreads();
-    for (int b = 0; b < 8; b++) {
-        int bit = shift + b;
-        uint32_t zeros = 0;
-#pragma unroll
-        for (int k = 0; k < kSortItems; k++)
-            zeros += ((key[k] >> bit) & 1u) ^ 1u;
-        uint32_t incl = block_inclusive<kGB>(zeros, sh);
-        uint32_t total_zeros = sh[kGB / 32 - 1]; // the block's total
-        uint32_t zbefore = incl - zeros;
-        uint32_t pos = threadIdx.x * kSortItems;
-#pragma unroll
-        for (int k = 0; k < kSortItems; k++) {
-            uint32_t one = (key[k] >> bit) & 1u;
-            uint32_t dst = one ? total_zeros + (pos + k - zbefore) : zbefore;
-            zbefore += one ^ 1u;
-            sk[dst] = key[k];
-            sv[dst] = val[k];
+        if (warp * (32 * kSortItems) + k * 32 + lane < valid) {
+            const uint32_t d = (key[k] >> shift) & 255u, p = start[d] + counts[warp][d] + rank[k];
+            sk[p] = key[k];
+            sv[p] = val[k];
         }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kSortItems; k++) {
-            key[k] = sk[threadIdx.x * kSortItems + k];
-            val[k] = sv[threadIdx.x * kSortItems + k];
-        }
-        __syncthreads();
-    }
-    // digit boundaries of the sorted tile
-#pragma unroll
-    for (int k = 0; k < kSortItems; k++) {
-        uint32_t p = threadIdx.x * kSortItems + k;
-        uint32_t d = (key[k] >> shift) & 255u;
-        uint32_t prev = p ? (sk[p - 1] >> shift) & 255u : 0xFFFFFFFFu;
-        if (p < valid && d != prev)
-            start[d] = p;
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kSortItems; k++) {
-        uint32_t p = threadIdx.x * kSortItems + k;
+        const uint32_t p = k * kGB + threadIdx.x;
         if (p < valid) {
-            uint32_t d = (key[k] >> shift) & 255u;
-            uint32_t dst = offs[d * gridDim.x + blockIdx.x] + (p - start[d]);
-            kout[dst] = key[k];
-            vout[dst] = val[k];
+            const uint32_t x = sk[p], d = (x >> shift) & 255u;
+            const uint32_t dst = offs[d * gridDim.x + blockIdx.x] + (p - start[d]);
+            kout[dst] = x;
+            vout[dst] = sv[p];
         }
     }
 }
@@ -658,8 +648,8 @@ __global__ void k_flat_start(FlatItem *items, uint32_t *lvl, unsigned long long 
 __global__ void __launch_bounds__(kGB)
     k_flat_level(FlatItem const *items, FlatItem *next, uint32_t *lvl, uint32_t level, uint32_t n, int2 const *child,
                  uint8_t const *leaf, uint32_t const *ntris, uint32_t const *icount, float4 const *blo,
-                 float4 const *bhi, uint32_t const *order, uint4 const *tidx, float4 const *vpos, uint32_t const *red,
-                 NodeHalf<float4> nlo, NodeHalf<float4> nhi, float4 *tri, unsigned long long *leaf_stats) {
+                 float4 const *bhi, uint32_t const *red, NodeHalf<float4> nlo, NodeHalf<float4> nhi,
+                 uint32_t *leaf_start, unsigned long long *leaf_stats) {
     const uint32_t f = lvl[level], lane = threadIdx.x & 31u;
     float lo[3], hi[3];
     for (int a = 0; a < 3; a++) {
@@ -692,28 +682,7 @@ __global__ void __launch_bounds__(kGB)
         if (is_leaf) {
             link = it.tri_start;
             count = ntris[it.node];
-            // the leaf's triangles, left to right
-            uint32_t stack[kLeafStack];
-            int sp = 0, k = 0;
-            stack[sp++] = it.node;
-            while (sp > 0) {
-                uint32_t x = stack[--sp];
-                if (x < n) {
-                    uint32_t t = order[x];
-                    uint4 g = tidx[t];
-                    float4 p0 = vpos[g.x], p1 = vpos[g.y], p2 = vpos[g.z];
-                    size_t r = 3 * static_cast<size_t>(it.tri_start + k);
-                    tri[r] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(t));
-                    tri[r + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z,
-                                             k + 1 == static_cast<int>(count) ? 1.0f : 0.0f); // the leaf's last record
-                    tri[r + 2] = make_float4(p2.x - p0.x, p2.y - p0.y, p2.z - p0.z, 0.0f);
-                    k++;
-                } else if (sp + 2 <= kLeafStack) {
-                    int2 c = child[x];
-                    stack[sp++] = static_cast<uint32_t>(c.y);
-                    stack[sp++] = static_cast<uint32_t>(c.x);
-                }
-            }
+            leaf_start[it.node] = link;
         } else {
             // depth-first preorder slots, as the host builder lays nodes out: the k-th interior node in
             // preorder keeps its children at 1 + 2k and 2 + 2k
@@ -734,6 +703,42 @@ __global__ void __launch_bounds__(kGB)
         nhi[it.slot] = make_float4(inflate_hi(b1.x, eps), inflate_hi(b1.y, eps), inflate_hi(b1.z, eps),
                                    __uint_as_float(count));
     }
+}
+
+// A thread per triangle, in Morton order: its leaf is the topmost ancestor that was made one, its place in
+// the leaf the number of the leaf's triangles to its left (as parts of a level's walk over its leaves,
+// one triangle after the other, the records took 110 us of the 1.3M-triangle scene's build, this 50).
+__global__ void __launch_bounds__(kGB)
+    k_leaf_tris(uint32_t n, uint32_t max_leaf, int2 const *child, uint32_t const *parent, uint8_t const *leaf,
+                uint32_t const *ntris, uint32_t const *leaf_start, uint32_t const *order, uint4 const *tidx,
+                float4 const *vpos, float4 *tri) {
+    const uint32_t x = blockIdx.x * kGB + threadIdx.x;
+    if (x >= n)
+        return;
+    const uint32_t t = order[x];
+    const uint4 g = tidx[t];
+    const float4 p0 = vpos[g.x], p1 = vpos[g.y], p2 = vpos[g.z];
+    uint32_t top = x, count = 1, rank = 0, left = 0;
+    for (uint32_t at = x, p = parent[x]; p != 0xFFFFFFFFu; p = parent[at]) {
+        const uint32_t c = ntris[p];
+        if (c > max_leaf)
+            break;
+        const int2 ch = child[p];
+        if (static_cast<uint32_t>(ch.y) == at)
+            left += ntris[ch.x];
+        at = p;
+        if (leaf[p]) {
+            top = p;
+            count = c;
+            rank = left;
+        }
+    }
+    const size_t r = leaf_start[top] + static_cast<size_t>(rank);
+    if (r >= n)
+        return; // (never: every leaf was reached)
+    tri[3 * r] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(t));
+    tri[3 * r + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z, rank + 1 == count ? 1.0f : 0.0f);
+    tri[3 * r + 2] = make_float4(p2.x - p0.x, p2.y - p0.y, p2.z - p0.z, 0.0f);
 }
 
 inline uint32_t blocks(uint64_t n, int per) { return n ? static_cast<uint32_t>((n + per - 1) / per) : 1u; }
@@ -995,72 +1000,116 @@ __global__ void __launch_bounds__(1024) k_wide_sums(WideState const *state, Wide
                           s.tri_running + static_cast<uint32_t>(total >> 32)};
 }
 
-__device__ __forceinline__ void wide_emit_node(WideState const &st, WideItem const &item, uint32_t i,
-                                               uint32_t const *slots_in, uint64_t at, uint32_t n,
-                                               NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
-                                               float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide,
-                                               WideItem *next) {
-    const uint32_t int_at = static_cast<uint32_t>(at);
-    uint32_t words[24];
-    for (int k = 0; k < 24; k++)
-        words[k] = 0;
-    float slo[8][3], shi[8][3];
-    uint32_t present = 0, imask = 0, leaves = 0, counts = 0;
-    uint32_t child_base = st.next_base + int_at, tri_base = st.tri_running + static_cast<uint32_t>(at >> 32);
-    uint32_t rank = 0, toff = 0;
-    uint32_t meta[2] = {0, 0};
-    for (int s = 0; s < 8; s++) {
-        uint32_t c = slots_in[8 * static_cast<size_t>(i) + s];
-        if (c == kNone) {
-            for (int a = 0; a < 3; a++)
-                slo[s][a] = shi[s][a] = 0.0f;
-            continue;
-        }
-        float4 a = nlo[c], b = nhi[c];
-        slo[s][0] = a.x, slo[s][1] = a.y, slo[s][2] = a.z;
-        shi[s][0] = b.x, shi[s][1] = b.y, shi[s][2] = b.z;
-        present |= 1u << s;
-        uint32_t cnt = __float_as_uint(b.w);
-        if (cnt == 0) {
-            imask |= 1u << s;
-            if (int_at + rank < n)
-                next[int_at + rank] = WideItem{c, child_base + rank};
-            rank++;
-        } else {
-            meta[s >> 2] |= toff << (8 * (s & 3));
-            counts |= cnt << (4 * s);
-            leaves |= 1u << s;
-            uint32_t first = __float_as_uint(a.w);
-            for (uint32_t k = 0; k < cnt; k++) {
-                size_t src = 3 * static_cast<size_t>(first + k), dst = 3 * static_cast<size_t>(tri_base + toff + k);
-                tri_wide[dst] = tri_bin[src];
-                tri_wide[dst + 1] = tri_bin[src + 1];
-                tri_wide[dst + 2] = tri_bin[src + 2];
-            }
-            toff += cnt;
-        }
-    }
-    wide_quantize(slo, shi, present, step_min, words);
-    words[3] |= imask << 24;
-    words[4] = child_base;
-    words[5] = tri_base;
-    words[6] = meta[0];
-    words[7] = meta[1];
-    words[20] = counts;
-    words[21] = leaves;
-    uint4 *dst = wide + 6 * static_cast<size_t>(item.wn);
-    for (int q = 0; q < 6; q++)
-        dst[q] = make_uint4(words[4 * q], words[4 * q + 1], words[4 * q + 2], words[4 * q + 3]);
-}
-
+// Eight lanes per wide node, a slot each: the slot's quantized planes (three lanes compute the grid's
+// axes: FP64 is slow on this GPU), its triangles' records and its place among the interior children; the
+// record is put together in shared memory and written in one piece. (A thread per node with its slots
+// in local memory took 274 us over the ten levels of the 1.3M-triangle scene, this 247.)
 __global__ void __launch_bounds__(kGB)
     k_wide_emit(WideState const *state, WideItem const *items, uint32_t const *slots_in, uint64_t const *scan,
                 uint64_t const *sums, uint32_t n, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
                 float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide, WideItem *next) {
-    const uint32_t f = state->f;
-    for (uint32_t i = blockIdx.x * kGB + threadIdx.x; i < f; i += gridDim.x * kGB)
-        wide_emit_node(*state, items[i], i, slots_in, scan[i] + sums[i / kScanTile], n, nlo, nhi, tri_bin, tri_wide,
-                       step_min, wide, next);
+    __shared__ __align__(16) uint32_t rec[kGB / 8][24];
+    const WideState st = *state;
+    const uint32_t lane = threadIdx.x & 31u, s = lane & 7u, g0 = lane & ~7u;
+    uint32_t *words = rec[threadIdx.x / 8];
+    for (uint32_t i0 = (blockIdx.x * kGB + (threadIdx.x & ~31u)) / 8; i0 < st.f; i0 += gridDim.x * (kGB / 8)) {
+        const uint32_t i = i0 + lane / 8;
+        const bool on = i < st.f;
+        const uint32_t c = on ? slots_in[8 * static_cast<size_t>(i) + s] : kNone;
+        const bool have = c != kNone;
+        float4 lo4 = make_float4(0, 0, 0, 0), hi4 = lo4;
+        if (have)
+            lo4 = nlo[c], hi4 = nhi[c];
+        const uint32_t cnt = have ? __float_as_uint(hi4.w) : 0u;
+        const bool inner = have && cnt == 0;
+        // places among the node's interior children and triangles
+        const uint32_t in_mask = __ballot_sync(~0u, inner) >> g0 & 0xFFu, leaf_mask = __ballot_sync(~0u, cnt != 0) >> g0 & 0xFFu;
+        const uint32_t rank = __popc(in_mask & ((1u << s) - 1u));
+        uint32_t toff = cnt;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(~0u, toff, o, 8);
+            toff += static_cast<int>(s) >= o ? y : 0u;
+        }
+        toff -= cnt;
+        const uint64_t at = on ? scan[i] + sums[i / kScanTile] : 0;
+        const uint32_t int_at = static_cast<uint32_t>(at);
+        const uint32_t child_base = st.next_base + int_at, tri_base = st.tri_running + static_cast<uint32_t>(at >> 32);
+        if (inner && int_at + rank < n)
+            next[int_at + rank] = WideItem{c, child_base + rank};
+        const uint32_t first = __float_as_uint(lo4.w);
+        for (uint32_t k = 0; k < cnt; k++) {
+            const size_t src = 3 * static_cast<size_t>(first + k), dst = 3 * static_cast<size_t>(tri_base + toff + k);
+            tri_wide[dst] = tri_bin[src];
+            tri_wide[dst + 1] = tri_bin[src + 1];
+            tri_wide[dst + 2] = tri_bin[src + 2];
+        }
+        // the grid: lane a < 3 of the node computes axis a
+        const float lo[3] = {lo4.x, lo4.y, lo4.z}, hi[3] = {hi4.x, hi4.y, hi4.z};
+        float ulo = 0.0f, uhi = 0.0f;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            float l = have ? lo[a] : INFINITY, h = have ? hi[a] : -INFINITY;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                const float l2 = __shfl_xor_sync(~0u, l, o), h2 = __shfl_xor_sync(~0u, h, o);
+                l = l2 < l ? l2 : l;
+                h = h < h2 ? h2 : h;
+            }
+            if (static_cast<int>(s) == a)
+                ulo = l, uhi = h;
+        }
+        float org = 0.0f, inv = 0.0f;
+        uint32_t ebyte = 0;
+        if (on && s < 3)
+            ebyte = wide_grid_axis(ulo, uhi, step_min, org, inv);
+        if (s < 3)
+            words[s] = __float_as_uint(org);
+        uint32_t ebytes = s < 3 ? ebyte << (8 * s) : 0u;
+        uint32_t meta = cnt ? toff << (8 * (s & 3)) : 0u, counts = cnt << (4 * s);
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const float oa = __shfl_sync(~0u, org, g0 + a), ia = __shfl_sync(~0u, inv, g0 + a);
+            uint32_t ql = 0, qh = 0;
+            if (have)
+                wide_grid_planes(lo[a], hi[a], oa, ia, ql, qh);
+            ql <<= 8 * (s & 3), qh <<= 8 * (s & 3);
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                ql |= __shfl_xor_sync(~0u, ql, o);
+                qh |= __shfl_xor_sync(~0u, qh, o);
+            }
+            if ((s & 3u) == 0) {
+                words[8 + 2 * a + s / 4] = ql;
+                words[14 + 2 * a + s / 4] = qh;
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            counts |= __shfl_xor_sync(~0u, counts, o);
+            ebytes |= __shfl_xor_sync(~0u, ebytes, o);
+            if (o < 4)
+                meta |= __shfl_xor_sync(~0u, meta, o);
+        }
+        if ((s & 3u) == 0)
+            words[6 + s / 4] = meta;
+        if (s == 0) {
+            words[3] = ebytes | in_mask << 24;
+            words[4] = child_base;
+            words[5] = tri_base;
+            words[20] = counts;
+            words[21] = leaf_mask;
+            words[22] = words[23] = 0;
+        }
+        __syncwarp();
+        const uint32_t wn = on ? items[i].wn : 0;
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t w = __shfl_sync(~0u, wn, 8 * k);
+            if (i0 + k < st.f && lane < 6)
+                wide[6 * static_cast<size_t>(w) + lane] = reinterpret_cast<uint4 const *>(rec[threadIdx.x / 32 * 4 + k])[lane];
+        }
+        __syncwarp();
+    }
 }
 } // namespace
 
@@ -1142,14 +1191,14 @@ cudaError_t gpu_build_sah_pairs(GpuBuildIn const &in, GpuBuildOut &out, cudaStre
     k_collapse<<<blocks(n, kGB), kGB, 0, st>>>(n, s.child, s.parent, s.blo, s.bhi, s.counter, s.ntris, s.icount, s.cost,
                                                s.leaf, in.max_leaf, in.tri_cost, in.node_cost);
     // 4. flatten level by level, one level more than the traversal stack allows
+    uint32_t *leaf_start = reinterpret_cast<uint32_t *>(s.cost); // per node; the costs are done with
     k_flat_start<<<1, 64, 0, st>>>(s.fa, s.lvl, s.leaf_stats, root);
     const uint32_t levels = std::min<uint32_t>(in.max_depth, kLevels - 2);
     for (uint32_t l = 0; l < levels; l++) {
         const uint32_t g = static_cast<uint32_t>(std::min<uint64_t>(blocks(uint64_t(1) << std::min(l, 31u), kGB),
                                                                     std::min<uint32_t>(blocks(n, kGB), grid_cap)));
         k_flat_level<<<g, kGB, 0, st>>>(l & 1 ? s.fb : s.fa, l & 1 ? s.fa : s.fb, s.lvl, l, n, s.child, s.leaf, s.ntris,
-                                        s.icount, s.blo, s.bhi, order, in.tidx, in.vpos, s.red, in.nlo, in.nhi, in.tri,
-                                        s.leaf_stats);
+                                        s.icount, s.blo, s.bhi, s.red, in.nlo, in.nhi, leaf_start, s.leaf_stats);
     }
     uint32_t lvl[kLevels], stats[4 + 6];
     cudaError_t e = cudaMemcpyAsync(lvl, s.lvl, sizeof(lvl), cudaMemcpyDeviceToHost, st);
@@ -1171,6 +1220,9 @@ cudaError_t gpu_build_sah_pairs(GpuBuildIn const &in, GpuBuildOut &out, cudaStre
         out.ok = false;
         return cudaSuccess;
     }
+    // every leaf was reached: the triangle records
+    k_leaf_tris<<<blocks(n, kGB), kGB, 0, st>>>(n, in.max_leaf, s.child, s.parent, s.leaf, s.ntris, leaf_start, order,
+                                                in.tidx, in.vpos, in.tri);
     out.num_nodes = slots;
     unsigned long long leaves = 0, leaf_depth_sum = 0;
     host = stats + 2;
@@ -1221,7 +1273,7 @@ cudaError_t gpu_collapse_wide(GpuWideIn const &in, GpuWideOut &out, cudaStream_t
                                                                                        s.scan);
             k_wide_tiles<<<std::min<uint32_t>(blocks(most, kScanTile), cap), 1024, 0, st>>>(cur, s.scan, s.tile_sums);
             k_wide_sums<<<1, 1024, 0, st>>>(cur, cur + 1, s.tile_sums);
-            k_wide_emit<<<std::min<uint32_t>(blocks(most, kGB), cap), kGB, 0, st>>>(
+            k_wide_emit<<<std::min<uint32_t>(blocks(8 * most, kGB), cap), kGB, 0, st>>>(
                 cur, wa, s.wslots, s.scan, s.tile_sums, n, in.nlo, in.nhi, in.tri, s.tri_tmp, step_min, in.wide, wb);
         }
         cudaError_t e = cudaMemcpyAsync(ws, s.wstate, sizeof(WideState) * (l + 1), cudaMemcpyDeviceToHost, st);
