@@ -22,7 +22,7 @@
 // Counts stay on the device: rounds and levels follow each other in the stream with grids for the
 // most they can hold, and the host reads back every few rounds and at the end. 525 launches and about
 // 70 reads made 5.7 ms of the 1.3M-triangle scene's eight-wide build; it is 236 launches, a dozen
-// reads and 2.9 ms (pairs 4.3 -> 2.1).
+// reads and 2.8 ms (pairs 4.3 -> 2.1).
 #include "bvh_boxes.h"
 #include "gpu_build.h"
 #include "launch.h"
@@ -1001,15 +1001,16 @@ __global__ void __launch_bounds__(1024) k_wide_sums(WideState const *state, Wide
 }
 
 // Eight lanes per wide node, a slot each: the slot's quantized planes (three lanes compute the grid's
-// axes: FP64 is slow on this GPU), its triangles' records and its place among the interior children; the
+// axes), its triangles' records and its place among the interior children; the
 // record is put together in shared memory and written in one piece. (A thread per node with its slots
-// in local memory took 274 us over the ten levels of the 1.3M-triangle scene, this 247.)
+// in local memory took 274 us over the ten levels of the 1.3M-triangle scene, this 147.)
 __global__ void __launch_bounds__(kGB)
     k_wide_emit(WideState const *state, WideItem const *items, uint32_t const *slots_in, uint64_t const *scan,
                 uint64_t const *sums, uint32_t n, NodeHalf<const float4> nlo, NodeHalf<const float4> nhi,
                 float4 const *tri_bin, float4 *tri_wide, double step_min, uint4 *wide, WideItem *next) {
     __shared__ __align__(16) uint32_t rec[kGB / 8][24];
     const WideState st = *state;
+    const int e_min = wide_exponent(step_min);
     const uint32_t lane = threadIdx.x & 31u, s = lane & 7u, g0 = lane & ~7u;
     uint32_t *words = rec[threadIdx.x / 8];
     for (uint32_t i0 = (blockIdx.x * kGB + (threadIdx.x & ~31u)) / 8; i0 < st.f; i0 += gridDim.x * (kGB / 8)) {
@@ -1062,7 +1063,7 @@ __global__ void __launch_bounds__(kGB)
         float org = 0.0f, inv = 0.0f;
         uint32_t ebyte = 0;
         if (on && s < 3)
-            ebyte = wide_grid_axis(ulo, uhi, step_min, org, inv);
+            ebyte = wide_grid_axis(ulo, uhi, step_min, e_min, org, inv);
         if (s < 3)
             words[s] = __float_as_uint(org);
         uint32_t ebytes = s < 3 ? ebyte << (8 * s) : 0u;
