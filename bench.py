@@ -860,11 +860,11 @@ def main():
     if best_integ == "wavefront":
         # the dominant kernel is the trace kernel: every traversal byte is fetched there
         dom_ms, dom_launches = rb["trace_ms"], rb["trace_launches_per_step"]
-        dom_name = ("k_wf_trace_wide_both (extension and shadow rays of a bounce, eight-wide tree)" if best_lay == "wide"
-                    else "k_wf_trace_dyn (extension and shadow rays, SAH pairs)")
+        dom_name = ("k_wf_trace_both (extension and shadow rays of a bounce, eight-wide tree)" if best_lay == "wide"
+                    else "k_wf_trace_both (extension and shadow rays, SAH pairs)")
     else:
         dom_ms, dom_launches = loop_ms, 1
-        dom_name = {"plain": "k_plain (baseline per-path kernel)", "megakernel": "k_mega (megakernel)"}[best_integ]
+        dom_name = {"plain": "k_plain (baseline per-path kernel)", "megakernel": "k_mega_pool (megakernel)"}[best_integ]
     achieved = alg_bytes / (dom_ms / 1000.0) / 1e9
     achieved_loop = alg_bytes / (loop_ms / 1000.0) / 1e9
     shade_traffic = None

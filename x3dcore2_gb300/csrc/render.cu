@@ -106,6 +106,7 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
     // refill threshold of the trace kernels (threshold 8 against 16: 42.3 against 43.0 ms per
     // 1280x720, 32-spp frame)
     const uint32_t threshold = c->dev.layout == 0 || c->dev.layout == 2 ? 8u : 0u;
+    const uint32_t traces = wf_trace_launches(c->dev.layout, threshold);
     const int grid_walk = bdpt_walk_grid(slots, c->num_sms);
     const int grid_eval = persistent_grid(c, bdpt_eval_blocks_per_sm());
     const int grid_trace = persistent_grid(c, wf_trace_blocks_per_sm(c->dev.layout, threshold));
@@ -158,7 +159,7 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
                 e = cudaMemcpyAsync(host_conn, C.conn_n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
             if (e == cudaSuccess)
                 e = cudaStreamSynchronize(c->stream);
-            c->launches += 4 * kBounces;
+            c->launches += (2 + traces) * kBounces; // reset, walk, trace(s)
             if (e == cudaSuccess && host->busy == 0 && host->next_path >= C.count)
                 break;
         }
@@ -176,7 +177,7 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
                 break;
             launch_bdpt_eval(c->dev, accum, path_rgb, C, Q, q0, n, grid_eval, c->stream);
             wf_enqueue_trace(c->dev, A, Q, accum, path_rgb, grid_trace, threshold, c->stream);
-            c->launches += 3;
+            c->launches += 1 + traces;
             e = cudaGetLastError();
         }
     }
@@ -300,7 +301,7 @@ e8g_status run_wavefront(e8g_ctx *c, RenderArgs const &A, float4 *accum, float *
             return cuda_fail(c, e, "kernel timing events");
         c->kt_events.push_back(ev);
     }
-    uint32_t traces_per_bounce = layout == 2 && threshold > 0 ? 1u : 2u;
+    const uint32_t traces_per_bounce = wf_trace_launches(layout, threshold);
     e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "wavefront capture");
@@ -332,7 +333,7 @@ e8g_status run_wavefront(e8g_ctx *c, RenderArgs const &A, float4 *accum, float *
             e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess)
             break;
-        c->launches += (layout == 2 && threshold > 0 ? 3 : 4) * bounces; // reset, shade, trace(s)
+        c->launches += (2 + traces_per_bounce) * bounces; // reset, shade, trace(s)
         if (timed) { // the replay has finished: read its bounces' event pairs
             for (uint32_t k = 0; k < bounces; k++) {
                 float a = 0, b = 0;
@@ -451,7 +452,7 @@ e8g_status run_wavefront_concurrent(e8g_ctx *c, RenderArgs const &A, float4 *acc
     }
     auto *host = static_cast<WfCounters *>(c->host_pinned); // [0]: pool A, [1]: pool B
     uint64_t max_replays = ((total + 2 * Qh - 1) / (2 * Qh) + 1) * (kHardDepth + 3) / bounces + 16;
-    uint32_t traces_per_bounce = layout == 2 && threshold > 0 ? 1u : 2u;
+    const uint32_t traces_per_bounce = wf_trace_launches(layout, threshold);
     uint64_t r = 0;
     bool cancelled = false;
     for (; r < max_replays; r++) {

@@ -89,6 +89,10 @@ size_t wf_total_bytes(uint32_t capacity, bool live);
 WfSlots wf_carve(void *base, uint32_t capacity, bool live);
 cudaError_t wf_init(WfSlots const &W, cudaStream_t st);
 int wf_trace_blocks_per_sm(uint32_t layout, uint32_t threshold);
+// Trace kernels that a bounce launches: one for both queues on the two fast trees, else one for each.
+inline uint32_t wf_trace_launches(uint32_t layout, uint32_t threshold) {
+    return threshold > 0 && (layout == 0 || layout == 2) ? 1u : 2u;
+}
 // threshold > 0: trace kernels refill idle lanes with new rays during traversal once that many
 // lanes of a warp are idle; 0: one ray per thread.
 // B: the scene table of a many-scene wavefront (eight-wide trees, threshold > 0), or null.
