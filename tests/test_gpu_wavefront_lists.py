@@ -11,7 +11,9 @@ from x3dcore2_gb300.core import default_params
 pytestmark = pytest.mark.gpu
 
 # width, height, samples, slots, bounces per graph: 8x4-pixel tiles pad each sample to whole warps
-SIZES = [(32, 32, 1, 1024, 1), (37, 29, 1, 1024, 3), (2, 2, 1, 1024, 2), (64, 64, 3, 1024, 5), (64, 64, 3, 16384, 2)]
+SIZES = [(32, 32, 1, 1024, 1), (37, 29, 1, 1024, 3), (2, 2, 1, 1024, 2), (64, 64, 3, 1024, 5), (64, 64, 3, 16384, 2),
+         # lists are kept from 155,649 slots on (1,024 for each of 152 SMs)
+         (500, 400, 1, 1 << 18, 2), (500, 400, 2, 160000, 3), (512, 304, 1, 155648, 1), (512, 304, 2, 155649, 1)]
 
 
 def _close(a, b):
@@ -42,7 +44,7 @@ def test_wavefront_with_lists_equals_megakernel(ctx, w, h, spp, slots, bounces, 
 
 
 @pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE])
-@pytest.mark.parametrize("w,h,spp", [(2, 2, 1), (37, 29, 1), (64, 64, 3)])
+@pytest.mark.parametrize("w,h,spp", [(2, 2, 1), (37, 29, 1), (64, 64, 3), (512, 304, 1), (500, 400, 2)])
 def test_split_bdpt_with_lists_equals_the_one_thread_form(ctx, w, h, spp, layout):
     ctx.upload(S.cornell(w, h), layout=layout)
     p = default_params(abi.MODE_BDPT_POWER, w, h, spp, seed=6, bdpt_max_len=8)

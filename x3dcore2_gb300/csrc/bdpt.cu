@@ -641,7 +641,11 @@ enum : uint32_t { kWkEmpty = 0, kWkCam = 1, kWkLight = 2 };
 constexpr int kWalkRounds = 4; // paths a slot may start and finish without a ray in one bounce
 constexpr int kWalkDraws = 8;  // paths without a first hit a slot may pass over in one round
 
-constexpr int kWalkBlock = 512;
+// Threads of a walk block: 512, or 128 where the slots do not fill the GPU with blocks of 512 and a block's
+// barriers would wait for more warps than an SM needs (Cornell room, 120x100, 2 spp: 0.58 -> 0.53 ms; a
+// 2,000-triangle soup, 100x80, 4 spp: 1.39 -> 1.33; at 240,000 paths both take 1.62).
+constexpr int kWalkBlock = 512, kWalkBlockSmall = 128;
+inline bool walk_small(uint32_t slots, int num_sms) { return slots < static_cast<uint32_t>(num_sms) * kWalkBlock * 2; }
 
 // One bounce of the walk over every slot. range: the chunk's first path index and path count
 // (device memory, so one captured graph serves every chunk). W.next_path: the chunk's path
@@ -655,12 +659,12 @@ constexpr int kWalkBlock = 512;
 // same part of it, so that a fetched line serves all of them: blocks of 256 threads without barriers
 // 36.0 ms per frame, with one / three barriers per group of slots 34.2 / 33.7, blocks of 512 33.2 /
 // 33.0, of 1024 33.0.
-template <class R>
-__global__ void __launch_bounds__(kWalkBlock, 1024 / kWalkBlock)
+template <class R, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     k_bdw_walk(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh, BdwChunk C, WfSlots W,
                uint64_t const *range, WfLive const *live, uint32_t *ext_n, uint32_t *busy) {
     const uint64_t mix = splitmix64(A.seed);
-    const WfVisit visit = wf_visit(W, *live);
+    const WfVisit visit = wf_visit(W, live);
     const uint32_t max_len = C.max_len;
     const uint64_t first = range[0];
     const uint32_t count = static_cast<uint32_t>(range[1]);
@@ -1138,20 +1142,20 @@ int bdpt_eval_blocks_per_sm() {
     return n > 0 ? n : 1;
 }
 
-// Two rounds of the resident blocks, or a block per group of slots.
-int bdpt_walk_grid(uint32_t slots, int num_sms) {
-    return static_cast<int>(std::min<uint64_t>((slots + kWalkBlock - 1) / kWalkBlock,
-                                               static_cast<uint64_t>(num_sms) * 2 * (1024 / kWalkBlock)));
-}
-
 void launch_bdpt_walk(DevScene const &S, RenderArgs const &A, FirstHit const *fh, BdwChunk const &C,
-                      WfSlots const &W, uint64_t const *range, int grid, cudaStream_t st) {
-    if (A.rng == E8G_RNG_MINSTD)
-        k_bdw_walk<RngMinstd><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_live_ptr(W), wf_ext_count_ptr(W),
-                                                              wf_busy_ptr(W));
+                      WfSlots const &W, uint64_t const *range, int num_sms, cudaStream_t st) {
+    const int block = walk_small(W.capacity, num_sms) ? kWalkBlockSmall : kWalkBlock;
+    // two rounds of the resident blocks, or a block per group of slots
+    const int grid = static_cast<int>(std::min<uint64_t>((W.capacity + block - 1) / block,
+                                                         static_cast<uint64_t>(num_sms) * 2 * (1024 / block)));
+    auto go = [&](auto *kern) {
+        kern<<<grid, block, 0, st>>>(S, A, fh, C, W, range, wf_live_ptr(W), wf_ext_count_ptr(W), wf_busy_ptr(W));
+    };
+    if (block == kWalkBlock)
+        A.rng == E8G_RNG_MINSTD ? go(k_bdw_walk<RngMinstd, kWalkBlock>) : go(k_bdw_walk<RngPhilox, kWalkBlock>);
     else
-        k_bdw_walk<RngPhilox><<<grid, kWalkBlock, 0, st>>>(S, A, fh, C, W, range, wf_live_ptr(W), wf_ext_count_ptr(W),
-                                                              wf_busy_ptr(W));
+        A.rng == E8G_RNG_MINSTD ? go(k_bdw_walk<RngMinstd, kWalkBlockSmall>)
+                                : go(k_bdw_walk<RngPhilox, kWalkBlockSmall>);
 }
 
 void launch_bdpt_eval(DevScene const &S, float4 *accum, float *path_rgb, BdwChunk const &C, WfSlots const &Q,

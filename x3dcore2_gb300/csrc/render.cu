@@ -24,9 +24,11 @@ struct WfCounters { // mirrors the device Counters of wavefront.cu
 };
 
 // Device memory for `pools` slot arrays of Q slots each, with the lists of occupied slots unless the
-// context has a memory limit (what fitted it still fits) or their allocation fails. *bytes: of one pool.
+// context has a memory limit (what fitted it still fits) or their allocation fails; nor where every slot
+// has a resident thread of its own, which visits it in no time (there the lists' loads lengthened each
+// bounce: 120x100, 2-spp bidirectional frame 1.00 -> 1.04 ms). *bytes: of one pool.
 cudaError_t reserve_slots(e8g_ctx *c, uint32_t Q, size_t pools, bool *live, size_t *bytes) {
-    for (*live = c->budget.cap == 0;; *live = false) {
+    for (*live = c->budget.cap == 0 && Q > static_cast<uint32_t>(c->num_sms) * 1024;; *live = false) {
         *bytes = (wf_total_bytes(Q, *live) + 255) & ~static_cast<size_t>(255);
         cudaError_t e = c->b_wf.reserve(pools == 1 ? wf_total_bytes(Q, *live) : pools * *bytes);
         if (e == cudaSuccess || !*live)
@@ -107,7 +109,6 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
     // 1280x720, 32-spp frame)
     const uint32_t threshold = c->dev.layout == 0 || c->dev.layout == 2 ? 8u : 0u;
     const uint32_t traces = wf_trace_launches(c->dev.layout, threshold);
-    const int grid_walk = bdpt_walk_grid(slots, c->num_sms);
     const int grid_eval = persistent_grid(c, bdpt_eval_blocks_per_sm());
     const int grid_trace = persistent_grid(c, wf_trace_blocks_per_sm(c->dev.layout, threshold));
     auto const *fh = static_cast<FirstHit const *>(c->b_fh.ptr);
@@ -119,7 +120,7 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
         return cuda_fail(c, e, "bidirectional walk capture");
     for (uint32_t k = 0; k < kBounces; k++) {
         wf_enqueue_reset(W, range, c->stream);
-        launch_bdpt_walk(c->dev, A, fh, C, W, range, grid_walk, c->stream);
+        launch_bdpt_walk(c->dev, A, fh, C, W, range, c->num_sms, c->stream);
         wf_enqueue_trace(c->dev, A, W, nullptr, nullptr, grid_trace, threshold, c->stream);
     }
     e = cudaStreamEndCapture(c->stream, &graph);

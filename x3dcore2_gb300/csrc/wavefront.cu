@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
     // Read once per thread: once the path counter has passed the last path (it only grows), no
     // slot can be refilled for the rest of the frame, and the tail bounces skip the refill atomics
     // (one per warp and slot group on a single address).
-    const WfVisit visit = wf_visit(W, cnt->live);
+    const WfVisit visit = wf_visit(W, &cnt->live);
     const bool paths_left = !visit.list && __ldcg(W.next_path) < total_paths;
     uint32_t busy_local = 0;
     for (uint32_t s0 = blockIdx.x * blockDim.x; s0 < visit.n; s0 += gridDim.x * blockDim.x) {
@@ -525,9 +525,11 @@ __global__ void __launch_bounds__(kBlock, kWfTraceBlocks)
 // total: paths in all, or range[1] (device memory) when range is given.
 __global__ void k_wf_reset(Counters *cnt, unsigned long long const *next_path, uint64_t total, uint64_t const *range,
                            bool lists) {
-    cnt->live.listed = lists && __ldcg(next_path) >= (range ? range[1] : total) ? 1u : 0u;
-    cnt->live.n = cnt->ext_n;
-    cnt->live.turn ^= 1u;
+    if (lists) {
+        cnt->live.listed = __ldcg(next_path) >= (range ? range[1] : total) ? 1u : 0u;
+        cnt->live.n = cnt->ext_n;
+        cnt->live.turn ^= 1u;
+    }
     cnt->shadow_n = 0;
     cnt->ext_n = 0;
     cnt->busy = 0;

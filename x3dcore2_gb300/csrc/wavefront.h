@@ -34,11 +34,16 @@ struct WfVisit {
     uint32_t n;           // entries or slots
     uint32_t *next;       // the list being written, at the extension queue's positions
 };
-__device__ __forceinline__ WfVisit wf_visit(WfSlots const &W, WfLive const &l) {
-    WfVisit v;
-    v.list = l.listed ? W.live + static_cast<size_t>(l.turn ^ 1u) * W.capacity : nullptr;
-    v.n = l.listed ? l.n : W.capacity;
-    v.next = W.live ? W.live + static_cast<size_t>(l.turn) * W.capacity : nullptr;
+__device__ __forceinline__ WfVisit wf_visit(WfSlots const &W, WfLive const *live) {
+    WfVisit v{nullptr, W.capacity, nullptr};
+    if (W.live) {
+        const WfLive l = *live;
+        if (l.listed) {
+            v.list = W.live + static_cast<size_t>(l.turn ^ 1u) * W.capacity;
+            v.n = l.n;
+        }
+        v.next = W.live + static_cast<size_t>(l.turn) * W.capacity;
+    }
     return v;
 }
 
@@ -124,10 +129,9 @@ void wf_enqueue_reset(WfSlots const &W, uint64_t const *range, cudaStream_t st);
 // list into the shadow queue of Q (its counters zeroed beforehand, sh_* arrays sized for n
 // entries), which wf_enqueue_trace then drains.
 void launch_bdpt_walk(DevScene const &S, RenderArgs const &A, FirstHit const *fh, BdwChunk const &C,
-                      WfSlots const &W, uint64_t const *range, int grid, cudaStream_t st);
+                      WfSlots const &W, uint64_t const *range, int num_sms, cudaStream_t st);
 void launch_bdpt_eval(DevScene const &S, float4 *accum, float *path_rgb, BdwChunk const &C, WfSlots const &Q,
                       uint32_t first, uint32_t n, int grid, cudaStream_t st);
-int bdpt_walk_grid(uint32_t slots, int num_sms);
 int bdpt_eval_blocks_per_sm();
 unsigned long long *wf_next_ptr(WfSlots const &W);
 // The two halves of a bounce, for pools that interleave on two streams (concurrent wavefront):
