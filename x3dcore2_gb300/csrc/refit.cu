@@ -160,40 +160,54 @@ __global__ void k_parents_pairs(NodeHalf<const float4> nlo, NodeHalf<const float
     parent[link + 1] = i;
 }
 
-__device__ __forceinline__ void store_pair_node(NodeHalf<float4> nlo, NodeHalf<float4> nhi, uint32_t n, float const lo[3],
-                                                float const hi[3], float eps, float4 *ex_lo, float4 *ex_hi) {
-    ex_lo[n] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-    ex_hi[n] = make_float4(hi[0], hi[1], hi[2], 0.0f);
-    float lw = nlo[n].w, hw = nhi[n].w; // link and count stay
-    nlo[n] = make_float4(inflate_lo(lo[0], eps), inflate_lo(lo[1], eps), inflate_lo(lo[2], eps), lw);
-    nhi[n] = make_float4(inflate_hi(hi[0], eps), inflate_hi(hi[1], eps), inflate_hi(hi[2], eps), hw);
-}
-
+// Exact boxes bottom-up: at every parent the last child to arrive unions its own box, still in registers,
+// with its sibling's and carries on. Bound by the chain of one step (the counter's release, which waits for
+// the box just written, and the sibling's box); link and parent are fetched before the counter, and the
+// node records are written by a kernel of their own: with them in the chain the 1.3M-triangle scene's
+// walk took 352 us, now 127 and 21 for k_store_pairs.
 __global__ void __launch_bounds__(kRefitBlock)
-    k_refit_pairs(NodeHalf<float4> nlo, NodeHalf<float4> nhi, uint32_t nn, float4 const *tlo, float4 const *thi, uint32_t const *parent,
-                  uint32_t *counter, float4 *ex_lo, float4 *ex_hi, uint32_t const *red) {
+    k_refit_pairs(NodeHalf<const float4> nlo, NodeHalf<const float4> nhi, uint32_t nn, float4 const *tlo,
+                  float4 const *thi, uint32_t const *parent, uint32_t *counter, float4 *ex_lo, float4 *ex_hi) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nn)
         return;
     uint32_t count = __float_as_uint(nhi[i].w);
     if (count == 0)
         return;
-    float eps = scene_eps_of(red);
     float lo[3], hi[3];
     range_box(tlo, thi, __float_as_uint(nlo[i].w), count, lo, hi);
-    store_pair_node(nlo, nhi, i, lo, hi, eps, ex_lo, ex_hi);
-    uint32_t n = parent[i];
+    ex_lo[i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+    ex_hi[i] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+    uint32_t cur = i, n = parent[i];
     while (n != 0xFFFFFFFFu) {
+        const uint32_t c = __float_as_uint(nlo[n].w), up = parent[n];
         if (arrive(&counter[n]) == 0)
             return; // the sibling's thread finishes this node
-        uint32_t c = __float_as_uint(nlo[n].w);
-        float4 a0 = __ldcg(&ex_lo[c]), a1 = __ldcg(&ex_hi[c]);
-        float4 b0 = __ldcg(&ex_lo[c + 1]), b1 = __ldcg(&ex_hi[c + 1]);
+        const uint32_t sib = cur == c ? c + 1 : c;
+        const float4 s0 = __ldcg(&ex_lo[sib]), s1 = __ldcg(&ex_hi[sib]);
+        const float4 m0 = make_float4(lo[0], lo[1], lo[2], 0.0f), m1 = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        const float4 a0 = cur == c ? m0 : s0, a1 = cur == c ? m1 : s1, b0 = cur == c ? s0 : m0, b1 = cur == c ? s1 : m1;
         lo[0] = fminf(a0.x, b0.x), lo[1] = fminf(a0.y, b0.y), lo[2] = fminf(a0.z, b0.z);
         hi[0] = fmaxf(a1.x, b1.x), hi[1] = fmaxf(a1.y, b1.y), hi[2] = fmaxf(a1.z, b1.z);
-        store_pair_node(nlo, nhi, n, lo, hi, eps, ex_lo, ex_hi);
-        n = parent[n];
+        ex_lo[n] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+        ex_hi[n] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        cur = n;
+        n = up;
     }
+}
+
+// The node records from the exact boxes; link and count stay.
+__global__ void __launch_bounds__(kRefitBlock)
+    k_store_pairs(NodeHalf<float4> nlo, NodeHalf<float4> nhi, uint32_t nn, float4 const *ex_lo, float4 const *ex_hi,
+                  uint32_t const *red) {
+    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= nn)
+        return;
+    const float eps = scene_eps_of(red);
+    const float4 lo = ex_lo[n], hi = ex_hi[n];
+    const float lw = nlo[n].w, hw = nhi[n].w;
+    nlo[n] = make_float4(inflate_lo(lo.x, eps), inflate_lo(lo.y, eps), inflate_lo(lo.z, eps), lw);
+    nhi[n] = make_float4(inflate_hi(hi.x, eps), inflate_hi(hi.y, eps), inflate_hi(hi.z, eps), hw);
 }
 
 // ------------------------------------------------------------------- eight-wide ----
@@ -344,10 +358,12 @@ void launch_refit(DevScene const &S, RefitScratch const &R, uint32_t nv, float c
                                                                               count, R.tlo, R.thi, R.ex_lo, R.ex_hi,
                                                                               R.red, cam_abs);
         }
-    } else
-        k_refit_pairs<<<blocks_for(nn), kRefitBlock, 0, st>>>(NodeHalf<float4>{const_cast<float4 *>(S.nlo.p)}, NodeHalf<float4>{const_cast<float4 *>(S.nhi.p)},
-                                                                nn, R.tlo, R.thi, R.parent, R.counter, R.ex_lo,
-                                                                R.ex_hi, R.red);
+    } else {
+        const NodeHalf<float4> nlo{const_cast<float4 *>(S.nlo.p)}, nhi{const_cast<float4 *>(S.nhi.p)};
+        k_refit_pairs<<<blocks_for(nn), kRefitBlock, 0, st>>>(S.nlo, S.nhi, nn, R.tlo, R.thi, R.parent, R.counter,
+                                                              R.ex_lo, R.ex_hi);
+        k_store_pairs<<<blocks_for(nn), kRefitBlock, 0, st>>>(nlo, nhi, nn, R.ex_lo, R.ex_hi, R.red);
+    }
 }
 
 namespace {
