@@ -658,7 +658,7 @@ inline bool walk_small(uint32_t slots, int num_sms) { return slots < static_cast
 // runs some tens of kilobytes of code per group of slots. The barriers keep a block's warps in the
 // same part of it, so that a fetched line serves all of them: blocks of 256 threads without barriers
 // 36.0 ms per frame, with one / three barriers per group of slots 34.2 / 33.7, blocks of 512 33.2 /
-// 33.0, of 1024 33.0.
+// 33.0, of 1024 33.0. Lists of the occupied slots (WfLive) and paths numbered tile by tile: 28.7.
 template <class R, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     k_bdw_walk(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh, BdwChunk C, WfSlots W,

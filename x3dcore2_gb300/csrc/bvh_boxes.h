@@ -109,8 +109,8 @@ E8G_BOX_HD uint32_t wide_grid_axis_double(float u_lo, float u_hi, double step_mi
 }
 
 // The same result in single precision (the double form's divisions and differences run at about two a
-// cycle on each SM: 100 of the 247 us that the 1.3M-triangle scene's eight-wide emission took). The exponent follows from the
-// single-precision quotient unless its mantissa lies within 16 ulps, several times its rounding, of a
+// cycle on each SM: 100 of the 247 us that the 1.3M-triangle scene's eight-wide emission took). The
+// exponent follows from the single-precision quotient unless its mantissa lies within 16 ulps, several times its rounding, of a
 // power of two; the origin is the difference rounded down, from its exact error (Knuth's TwoSum), equal
 // to the double form's while the difference is exact in double (exponents close enough). Anything else
 // takes the double form.

@@ -13,7 +13,7 @@
 //
 // Measured on one GB300, device time of the integrator: the 1080p, 16-spp MIS frame of that scene
 // 26.3 (k_mega) -> 18.8 ms on the pairs and 30.8 -> 19.1 on the eight-wide tree, the 720p lt1 frame
-// 11.4 -> 8.1, a 1080p one-sample unidirectional frame 0.97 -> 0.90, the Cornell room at 256 x 256,
+// 11.4 -> 8.1 (with paths numbered tile by tile since: 16.9, 17.4 and 6.2), a 1080p one-sample unidirectional frame 0.97 -> 0.90, the Cornell room at 256 x 256,
 // 16 spp 1.21 -> 0.91, a 50,000-triangle soup 4.13 -> 2.67. What bounds it now: issue slots (0.5 per
 // cycle and scheduler) shared with memory latency at 28 warps per SM; three quarters of the time is
 // tracing.

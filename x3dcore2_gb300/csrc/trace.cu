@@ -467,10 +467,9 @@ void launch_first_hits_rays(DevScene const &S, float const *rays6, uint32_t n, F
 void launch_camera_rays(DevScene const &S, uint32_t w, uint32_t h, float *rays6, cudaStream_t st) {
     k_camera_rays<<<blocks(w * h, 256), 256, 0, st>>>(S, w, h, rays6);
 }
-// Rays per warp: an equal share of the batch for every resident warp. A small batch then has few rays
-// in each warp, whose steps follow each other sooner than 32 lanes' would: a closest-hit and an
-// any-hit query of 1,500 rays against a 1,000-triangle soup take 250 us in 47 warps and 179 us with a
-// warp each (of 1,000,003 rays against the 327,690-triangle icosphere 0.85 ms).
+// A warp per ray for batches of at most kWarpRays rays per resident warp, else an equal share of the batch
+// for every resident warp (a closest-hit and an any-hit query of 1,000,003 rays against the
+// 327,690-triangle icosphere 0.83 ms).
 template <bool ANY>
 static void trace_rays(DevScene const &S, float const *rays6, float const *tmin, float const *tmax, uint32_t n,
                        HitOut const &hits, uint8_t *occ, int num_sms, cudaStream_t st) {
