@@ -145,3 +145,36 @@ def test_warp_per_ray_equals_lane_per_ray(ctx, layout, scene):
         for k in few:
             assert np.array_equal(few[k].view(np.uint32), np.ascontiguousarray(many[k][lo:hi]).view(np.uint32)), k
         assert np.array_equal(ctx.trace_any(rays[lo:hi], tmin[lo:hi], tmax[lo:hi]), occ[lo:hi])
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("far", [3e8, 4e8, 1e12, 1e18])
+def test_axis_parallel_rays_far_from_the_origin(ctx, layout, far):
+    """Sheets across the z axis around x = far, and rays along it whose other components are zero or tiny:
+    the planes' distances leave the float range there. The linear layout, which tests every triangle,
+    says what is hit; closest hits and shadow rays, a warp and a lane per ray."""
+    r = np.random.default_rng(7)
+    side = far * 1e-3
+    tris = []
+    for z in range(1, 9):
+        for i in range(6):
+            for j in range(6):
+                x0, x1 = far + side * (i / 3 - 1), far + side * ((i + 1) / 3 - 1)
+                y0, y1 = side * (j / 3 - 1), side * ((j + 1) / 3 - 1)
+                tris += [[[x0, y0, z], [x1, y0, z], [x1, y1, z]], [[x0, y0, z], [x1, y1, z], [x0, y1, z]]]
+    sc = mesh_scene(tris)
+    n, copies = 3000, 30
+    o = np.stack([far + side * r.uniform(-0.9, 0.9, n), side * r.uniform(-0.9, 0.9, n), r.integers(0, 9, n) + 0.5], axis=1)
+    tiny = np.array([0.0, -0.0, 1e-35, -1e-31, 1e-29])
+    d = np.stack([r.choice(tiny, n), r.choice(tiny, n), r.choice([-1.0, 1.0], n)], axis=1)
+    rays = np.concatenate([o, d], axis=1).astype(np.float32)
+    tmin = np.full(n, 1e-4, np.float32)
+    tmax = r.choice(np.array([0.25, 2.0, 1000.0, np.inf], np.float32), n)
+    ctx.upload(sc, layout=abi.BVH_LINEAR)
+    want, occ = ctx.trace_closest(rays), ctx.trace_any(rays, tmin, tmax)
+    assert (want["mesh"] == 0).mean() > 0.8 and 0.2 < occ.mean() < 0.9
+    ctx.upload(sc, layout=layout)
+    for k in (1, copies):
+        got = ctx.trace_closest(np.tile(rays, (k, 1)))
+        assert np.array_equal(got["mesh"], np.tile(want["mesh"], k)) and np.array_equal(got["t"], np.tile(want["t"], k))
+        assert np.array_equal(ctx.trace_any(np.tile(rays, (k, 1)), np.tile(tmin, k), np.tile(tmax, k)), np.tile(occ, k))
