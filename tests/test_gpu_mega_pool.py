@@ -89,3 +89,89 @@ def test_backward_is_the_one_path_per_lane_kernels(lib, kind, depth, rr, layout)
     assert np.abs(wa).sum() > 0
     np.testing.assert_allclose(da, wa, rtol=1e-3, atol=1e-6 * np.abs(wa).max())
     assert np.linalg.norm(dr - wr) <= 1e-3 * max(np.linalg.norm(wr), 1e-12)
+
+
+@pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE])
+@pytest.mark.parametrize("mode,depth", [(abi.MODE_MIS, 6), (abi.MODE_REF_LT1, 0), (abi.MODE_REF_UNI, 0)])
+@pytest.mark.parametrize("kind", ["cornell", "soup"])
+def test_image_adds_a_path_once(ctx, kind, mode, depth, layout):
+    """A pixel of two samples is the sum of its two paths' radiances rounded once, bit for bit, however many
+    contributions each has (halving is exact)."""
+    w, h = 1027, 1023
+    sc = S.cornell(w, h) if kind == "cornell" else S.soup(20_000, seed=3, width=w, height=h)
+    ctx.upload(sc, layout=layout)
+    p = default_params(mode, w, h, 2, seed=11, max_depth=depth, rr_start=3)
+    px = np.tile(np.arange(w * h, dtype=np.uint32), 2)
+    paths = ctx.render_paths(plain(p), px, np.repeat(np.arange(2, dtype=np.uint32), w * h))
+    want = paths.astype(np.float64).reshape(2, h, w, 3).sum(axis=0).astype(np.float32) * np.float32(0.5)
+    assert want.sum() > 0
+    assert np.array_equal(ctx.render(p)[..., :3], want)
+
+
+@pytest.mark.parametrize("mode,depth", [(abi.MODE_MIS, 6), (abi.MODE_REF_LT1, 0), (abi.MODE_REF_UNI, 0)])
+@pytest.mark.parametrize("kind", ["cornell", "soup"])
+def test_a_path_is_the_same_in_a_short_and_a_long_list(ctx, kind, mode, depth):
+    """Long lists run over the pools, short ones a path per lane: the same bits for every path, those that start
+    on a light (here one that reflects) among them."""
+    w, h = 1024, 512
+    sc = S.cornell(w, h) if kind == "cornell" else S.soup(20_000, seed=3, width=w, height=h)
+    for light in sc.lights[:sc.num_lights]:
+        sc.mesh_mat[light.mesh] = sc.mesh_mat[0]
+    ctx.upload(sc)
+    p = default_params(mode, w, h, 4, seed=11, max_depth=depth, rr_start=3)
+    px, smp = np.tile(np.arange(w * h, dtype=np.uint32), 4), np.repeat(np.arange(4, dtype=np.uint32), w * h)
+    long = ctx.render_paths(p, px, smp)
+    for k in range(3):
+        at = slice(k * 300_007, (k + 1) * 300_007)
+        short = ctx.render_paths(p, px[at], smp[at])
+        assert short.sum() > 0
+        assert np.array_equal(long[at].view(np.uint32), short.view(np.uint32))
+
+
+@pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE])
+@pytest.mark.parametrize("mode,depth", [(abi.MODE_MIS, 6), (abi.MODE_REF_LT1, 0)])
+@pytest.mark.parametrize("spp,slots", [(16, 640), (32, 1024)])
+def test_larger_pools(lib, spp, slots, mode, depth, layout):
+    """Renders long enough for 640 and for all 1,024 slots a block (128 bytes each, seven blocks an SM), at an
+    odd size: a pixel is a sum of at most 32 equal terms in any order."""
+    import torch
+
+    from x3dcore2_gb300.core import Context
+    w, h = 1023, 577
+    p = default_params(mode, w, h, spp, seed=11, max_depth=depth, rr_start=3)
+    with Context(0) as c:
+        c.set_memory_limit(64 << 30)
+        c.upload(S.soup(20_000, seed=3, width=w, height=h), layout=layout)
+        c.render(p)
+        lanes = c.memory_used()
+        c.set_memory_limit(0)
+        got = c.render(p)
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        assert sms != 152 or c.memory_used() - lanes == sms * 7 * slots * 128
+        np.testing.assert_allclose(got, c.render(plain(p)), rtol=RTOL, atol=1e-12)
+        p.firefly = 1  # sample images of single paths, which are the same bits, and the same clamp
+        np.testing.assert_allclose(c.render(p), c.render(plain(p)), rtol=RTOL, atol=1e-12)
+
+
+@pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE])
+def test_backward_with_its_most_slots(lib, layout):
+    """512 slots a block (twice a small render's) against the one-path-per-lane kernel; tolerance as above."""
+    from x3dcore2_gb300.core import Context
+    grew = []
+    for w, h, spp in ((257, 255, 16), (513, 511, 32)):
+        p = default_params(abi.MODE_MIS, w, h, spp, seed=5, max_depth=6, rr_start=3)
+        dl = np.random.default_rng(2).uniform(0.5, 1.0, (h, w, 3)).astype(np.float32)
+        with Context(0) as c:
+            c.set_memory_limit(64 << 30)
+            c.upload(S.displaced_icosphere(level=5, seed=2, num_materials=16, width=w, height=h), layout=layout)
+            c.forward(p)
+            wa, wr = c.backward(dl)
+            lanes = c.memory_used()
+            c.set_memory_limit(0)
+            c.forward(p)
+            da, dr = c.backward(dl)
+            grew.append(c.memory_used() - lanes)
+        assert np.abs(wa).sum() > 0
+        np.testing.assert_allclose(da, wa, rtol=1e-3, atol=1e-6 * np.abs(wa).max())
+        assert np.linalg.norm(dr - wr) <= 1e-3 * max(np.linalg.norm(wr), 1e-12)
+    assert grew[1] == 2 * grew[0] > 0

@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kBlock) k_adjoint(DevScene S, RenderArgs A, Fi
 // ray left the scene gathers nothing after it); a path's end adds the list. A path that made more
 // vertices than the list holds starts over in its slot and adds the later scatters directly, its
 // radiance being known.
-// Slot arrays after those of mega_pool.cuh: the radiance (w: 1 on the second walk), the last scatter
+// Slot arrays beside those of mega_pool.cuh (kPoolRad's w: 1 on the second walk): the last scatter
 // (x: material, y: its d ln f / d r, z: the light sample's d ln f / d r), and the list's entries,
 // (radiance, d ln f / d r) and the materials four to an array; the second walk keeps the path's whole
 // radiance in the first entry.
@@ -293,7 +293,7 @@ __device__ __forceinline__ void add_grad_warp(GradAcc &g, bool on, int32_t mi, f
     }
 }
 
-enum { kAdjL = kPoolArrays, kAdjScat, kAdjRec, kAdjMat = kAdjRec + kScatterList, kAdjArrays = kAdjMat + kScatterList / 4 };
+enum { kAdjScat = kPoolArrays, kAdjRec, kAdjMat = kAdjRec + kScatterList, kAdjArrays = kAdjMat + kScatterList / 4 };
 
 __device__ __forceinline__ float3 pixel_grad(float const *dl_dimage, uint32_t pixel, float inv_spp) {
     float const *d = dl_dimage + 3 * static_cast<size_t>(pixel);
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kBlock, kAdjBlocks)
             uint32_t made = 0; // vertices made so far, and scatters with a vertex after them
             uint32_t nl = 0;   // list entries to add: the path ended
             if (back) {
-                const float4 ids = P[kPoolIds * slots + s], l4 = P[kAdjL * slots + s];
+                const float4 ids = P[kPoolIds * slots + s], l4 = P[kPoolRad * slots + s];
                 pixel = __float_as_uint(ids.x);
                 sample = __float_as_uint(ids.y);
                 rad = xyz(l4);
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(kBlock, kAdjBlocks)
                 P[kPoolPos * slots + s] = make_float4(v.p.x, v.p.y, v.p.z, 0.0f);
                 P[kPoolIds * slots + s] = make_float4(__uint_as_float(pixel), __uint_as_float(sample), 0.0f,
                                                       __uint_as_float(RngSlot<RngPhilox>::store(rng)));
-                P[kAdjL * slots + s] = make_float4(rad.x, rad.y, rad.z, second ? 1.0f : 0.0f);
+                P[kPoolRad * slots + s] = make_float4(rad.x, rad.y, rad.z, second ? 1.0f : 0.0f);
                 P[kAdjScat * slots + s] = make_float4(__int_as_float(mi), dl_scat, dl_light, 0.0f);
             }
             if (open) { // kRayEnd: no extension ray, the path ends once its shadow ray is back
@@ -459,8 +459,7 @@ __global__ void __launch_bounds__(kBlock, kAdjBlocks)
         const uint32_t ne = Q.n_ext, n = ne + Q.n_sh;
         if (n == 0 && Q.over && !more)
             break;
-        pool_trace<LAYOUT>(S, L, P, slots, Q, ne, n, stk, keep,
-                           [&](uint32_t slot, bool visible) { return visible ? kRayHit : kRayNone; });
+        pool_trace<LAYOUT>(S, L, P, slots, Q, ne, n, stk, keep);
         __syncthreads();
         if (threadIdx.x == 0)
             Q.n_ext = Q.n_sh = Q.head = 0;

@@ -35,27 +35,13 @@ constexpr uint32_t kPoolSlots = 1024;
 // Idle lanes of a warp that wait for each other before they take new rays (4 / 8 / 16: within 2%).
 constexpr uint32_t kPoolRefill = 8;
 
-// State of a slot's ray: none, on its way (or queued), back with its hit; kRayEnd: no extension ray, but
-// an end still to be handled (the backward's).
+// State of a slot's ray. Extension: no path, on its way (or queued), back with its hit; kRayEnd: the path
+// has none and ends once its shadow ray is back. Shadow: none or occluded, on its way, unoccluded.
 enum : uint8_t { kRayNone = 0, kRayOut = 1, kRayHit = 2, kRayEnd = 3 };
 
-// A block's slots: arrays of float4, kPoolSlots each.
-enum { kPoolIds = 0, kPoolBeta, kPoolDir, kPoolHit, kPoolPos, kPoolShDir, kPoolShAdd, kPoolArrays };
-
-// One contribution of a path to the image (or to its entry of the per-path output, which the host
-// zeroed); nothing when it is exactly zero.
-__device__ __forceinline__ void pool_add(float4 *accum, float *path_rgb, uint32_t out, float3 c) {
-    if (c.x == 0.0f && c.y == 0.0f && c.z == 0.0f)
-        return;
-    if (path_rgb) {
-        float *o = path_rgb + 3 * static_cast<size_t>(out);
-        atomicAdd(o, c.x);
-        atomicAdd(o + 1, c.y);
-        atomicAdd(o + 2, c.z);
-    } else {
-        atomicAdd(&accum[out], make_float4(c.x, c.y, c.z, 0.0f));
-    }
-}
+// A block's slots: arrays of float4, `slots` each. kPoolRad: the radiance the path has gathered, without
+// the shadow ray on its way; kPoolShAdd: with it (in the backward, the light sample's term alone).
+enum { kPoolIds = 0, kPoolBeta, kPoolDir, kPoolHit, kPoolPos, kPoolShDir, kPoolShAdd, kPoolRad, kPoolArrays };
 
 struct PoolVertex {
     float3 beta, p, n, o;
@@ -204,10 +190,9 @@ struct PoolLane {
 
 // Traces the block's queue: ne extension rays, then shadow rays, n in all. A warp leaves when the
 // queue is empty and at most `keep` of its rays are on their way, after 16 steps at least.
-// shadow_done(slot, visible) takes a finished shadow ray and gives its slot's new shadow state.
-template <int LAYOUT, class F>
+template <int LAYOUT>
 __device__ __forceinline__ void pool_trace(DevScene const &S, PoolLane &L, float4 *P, uint32_t slots, PoolQueue &Q,
-                                           uint32_t ne, uint32_t n, uint32_t *stk, uint32_t keep, F &&shadow_done) {
+                                           uint32_t ne, uint32_t n, uint32_t *stk, uint32_t keep) {
     const uint32_t lane = lane_id();
     const WideView WV{S.wnodes, S.tri, S.nnodes, S.ntris, S.check};
     // the ray's state in locals for the loop (as members of L they stay in local memory)
@@ -262,7 +247,7 @@ __device__ __forceinline__ void pool_trace(DevScene const &S, PoolLane &L, float
                 P[kPoolHit * slots + cur] = make_float4(h.t, __uint_as_float(h.tri), h.b1, h.b2);
                 Q.ext_st[cur] = kRayHit;
             } else {
-                Q.sh_st[cur] = shadow_done(cur, h.tri == 0xFFFFFFFFu);
+                Q.sh_st[cur] = h.tri == 0xFFFFFFFFu ? kRayHit : kRayNone;
             }
             cur = kPoolNone;
         }
@@ -306,6 +291,25 @@ __device__ __forceinline__ bool pool_complete(DevScene const &S, float4 hv, floa
     v.mesh = nv.mesh;
     v.depth = __float_as_uint(dd.w) + 1u;
     return true;
+}
+
+__device__ __forceinline__ bool pool_nonzero(float3 a) { return a.x != 0.0f || a.y != 0.0f || a.z != 0.0f; }
+
+// A path's radiance (kPoolRad) to its pixel, or to its entry of the per-path output (which the host zeroed):
+// once a path, so that a pixel's sum is rounded once a sample, and lt1's first-hit emission last, as the
+// reference adds it (w: whether there is one). Against an atomic for every term, which rounded a pixel's sum two
+// to six times a sample: 1080p, 16-spp frame of the 1.3M-triangle icosphere, pairs, MIS / lt1 / uni 16.9 / 14.1 /
+// 8.0 -> 16.9 / 14.2 / 8.5 ms, eight-wide 17.0 / 14.2 / 7.8 -> 16.2 / 13.4 / 7.9.
+template <int MODE>
+__device__ __forceinline__ void pool_finish(DevScene const &S, RenderArgs const &A, FirstHit const *fh, float4 *accum,
+                                            float *path_rgb, uint32_t pixel, uint32_t out, float4 rad) {
+    float3 L = xyz(rad);
+    if (MODE == E8G_MODE_REF_LT1 && rad.w != 0.0f) {
+        const FirstHit f = fh[pixel];
+        L = add(L, light_radiance(S, __float_as_int(f.n.w), neg(xyz(f.d)), xyz(f.n)));
+    }
+    if (pool_nonzero(L))
+        emit(A, accum, path_rgb, out, L);
 }
 
 // Starts a path at its cached first hit. False when the camera ray has none.
@@ -358,23 +362,33 @@ __global__ void __launch_bounds__(kBlock, kPoolBlocks)
         for (uint32_t s0 = 0; s0 < slots; s0 += kBlock) {
             __syncthreads();
             const uint32_t s = s0 + threadIdx.x;
-            bool at_vertex = false, fresh = false;
+            bool at_vertex = false;
             PoolVertex v;
             R rng;
             uint32_t pixel = 0, sample = 0, out = 0;
-            float3 add = f3(0, 0, 0);
-            const uint32_t es = Q.ext_st[s];
-            const bool open = es != kRayOut && Q.sh_st[s] == kRayNone;
-            if (open && es == kRayHit) {
-                float4 hv = P[kPoolHit * slots + s], ids = P[kPoolIds * slots + s];
-                if (__float_as_uint(hv.y) != 0xFFFFFFFFu) {
-                    at_vertex = pool_complete<MODE>(S, hv, P[kPoolDir * slots + s], P[kPoolBeta * slots + s], v, add);
-                    if (at_vertex) {
-                        pixel = __float_as_uint(ids.x);
-                        sample = __float_as_uint(ids.y);
-                        out = __float_as_uint(ids.z);
-                        rng = RngSlot<R>::load(A, pixel, sample, __float_as_uint(ids.w));
+            const uint32_t es = Q.ext_st[s], sh = Q.sh_st[s];
+            const bool open = es != kRayOut && sh != kRayOut;
+            if (open && es != kRayNone) { // a path whose rays are back
+                const float4 ids = P[kPoolIds * slots + s];
+                float3 hit = f3(0, 0, 0); // emission at the vertex
+                if (es == kRayHit) {
+                    const float4 hv = P[kPoolHit * slots + s];
+                    at_vertex = __float_as_uint(hv.y) != 0xFFFFFFFFu &&
+                                pool_complete<MODE>(S, hv, P[kPoolDir * slots + s], P[kPoolBeta * slots + s], v, hit);
+                    if (at_vertex)
+                        rng = RngSlot<R>::load(A, __float_as_uint(ids.x), __float_as_uint(ids.y), __float_as_uint(ids.w));
+                }
+                const bool grew = sh == kRayHit || (MODE == E8G_MODE_MIS && pool_nonzero(hit));
+                if (!at_vertex || grew) {
+                    float4 rad = P[(sh == kRayHit ? kPoolShAdd : kPoolRad) * slots + s];
+                    if (MODE == E8G_MODE_MIS) {
+                        const float3 r = add(xyz(rad), hit);
+                        rad = make_float4(r.x, r.y, r.z, 0.0f);
                     }
+                    if (at_vertex)
+                        P[kPoolRad * slots + s] = rad;
+                    else
+                        pool_finish<MODE>(S, A, fh, accum, path_rgb, __float_as_uint(ids.x), __float_as_uint(ids.z), rad);
                 }
             }
             // a path for every free slot; paths without a first hit end at once
@@ -390,9 +404,12 @@ __global__ void __launch_bounds__(kBlock, kPoolBlocks)
                         if (pool_start(f, v)) {
                             rng = RngSlot<R>::fresh(A, mix, pixel, sample);
                             int32_t light = __float_as_int(f.n.w);
-                            if ((MODE == E8G_MODE_MIS || MODE == E8G_MODE_REF_LT1) && light >= 0)
-                                add = light_radiance(S, light, v.o, v.n);
-                            at_vertex = fresh = true;
+                            const float3 rad =
+                                MODE == E8G_MODE_MIS && light >= 0 ? light_radiance(S, light, v.o, v.n) : f3(0, 0, 0);
+                            P[kPoolIds * slots + s] =
+                                make_float4(__uint_as_float(pixel), __uint_as_float(sample), __uint_as_float(out), 0.0f);
+                            P[kPoolRad * slots + s] = make_float4(rad.x, rad.y, rad.z, light >= 0 ? 1.0f : 0.0f);
+                            at_vertex = true;
                             want = false;
                         }
                     }
@@ -401,32 +418,46 @@ __global__ void __launch_bounds__(kBlock, kPoolBlocks)
             __syncthreads();
             bool shadow = false, extend = false;
             if (at_vertex) {
-                pool_add(accum, path_rgb, out, add);
                 PoolRays q;
                 pool_shade<MODE>(S, A, v, rng, q);
-                if (MODE != E8G_MODE_MIS)
-                    pool_add(accum, path_rgb, out, q.add);
                 shadow = q.shadow;
                 extend = q.extend;
                 if (extend) {
                     P[kPoolBeta * slots + s] = make_float4(v.beta.x, v.beta.y, v.beta.z, q.pdf);
                     P[kPoolDir * slots + s] = make_float4(q.i.x, q.i.y, q.i.z, __uint_as_float(v.depth));
                 }
-                if (shadow) {
-                    P[kPoolShDir * slots + s] = make_float4(q.sd.x, q.sd.y, q.sd.z, q.st);
-                    P[kPoolShAdd * slots + s] = make_float4(q.vis.x, q.vis.y, q.vis.z, __uint_as_float(q.occ_nan));
+                const bool plus = MODE != E8G_MODE_MIS && pool_nonzero(q.add), ends = !shadow && !extend;
+                if (shadow || plus || ends) {
+                    // read again: held over the shading it would be spilled
+                    float4 rad = P[kPoolRad * slots + s];
+                    if (plus) {
+                        const float3 r = add(xyz(rad), q.add);
+                        P[kPoolRad * slots + s] = rad = make_float4(r.x, r.y, r.z, rad.w);
+                    }
+                    if (shadow) {
+                        const float3 r = add(xyz(rad), q.vis);
+                        P[kPoolShAdd * slots + s] = make_float4(r.x, r.y, r.z, rad.w);
+                        if (MODE == E8G_MODE_REF_LT1 && q.occ_nan) {
+                            const float nan = __uint_as_float(0x7FFFFFFFu);
+                            P[kPoolRad * slots + s] = make_float4(q.occ_nan & 1u ? nan : rad.x, q.occ_nan & 2u ? nan : rad.y,
+                                                                  q.occ_nan & 4u ? nan : rad.z, rad.w);
+                        }
+                    }
+                    if (ends) {
+                        const float4 ids = P[kPoolIds * slots + s];
+                        pool_finish<MODE>(S, A, fh, accum, path_rgb, __float_as_uint(ids.x), __float_as_uint(ids.z), rad);
+                    }
                 }
-                if (shadow || extend) {
+                if (shadow)
+                    P[kPoolShDir * slots + s] = make_float4(q.sd.x, q.sd.y, q.sd.z, q.st);
+                if (!ends) {
                     P[kPoolPos * slots + s] = make_float4(v.p.x, v.p.y, v.p.z, 0.0f);
-                    if (fresh)
-                        P[kPoolIds * slots + s] = make_float4(__uint_as_float(pixel), __uint_as_float(sample),
-                                                              __uint_as_float(out), __uint_as_float(RngSlot<R>::store(rng)));
-                    else if (extend)
-                        reinterpret_cast<uint32_t *>(&P[kPoolIds * slots + s])[3] = RngSlot<R>::store(rng);
+                    if (extend)
+                        reinterpret_cast<float *>(&P[kPoolIds * slots + s])[3] = __uint_as_float(RngSlot<R>::store(rng));
                 }
             }
             if (open) {
-                Q.ext_st[s] = extend ? kRayOut : kRayNone;
+                Q.ext_st[s] = extend ? kRayOut : shadow ? kRayEnd : kRayNone;
                 Q.sh_st[s] = shadow ? kRayOut : kRayNone;
             }
             pool_push(Q, s, extend, shadow);
@@ -435,19 +466,7 @@ __global__ void __launch_bounds__(kBlock, kPoolBlocks)
         const uint32_t ne = Q.n_ext, n = ne + Q.n_sh;
         if (n == 0 && Q.over && !out_rays)
             break;
-        pool_trace<LAYOUT>(S, L, P, slots, Q, ne, n, stk, keep, [&](uint32_t slot, bool visible) {
-            float4 c = P[kPoolShAdd * slots + slot];
-            float3 add = f3(0, 0, 0);
-            if (visible) {
-                add = xyz(c);
-            } else if (MODE == E8G_MODE_REF_LT1 && __float_as_uint(c.w)) {
-                uint32_t f = __float_as_uint(c.w);
-                float nan = __uint_as_float(0x7FFFFFFFu);
-                add = f3(f & 1u ? nan : 0.0f, f & 2u ? nan : 0.0f, f & 4u ? nan : 0.0f);
-            }
-            pool_add(accum, path_rgb, __float_as_uint(P[kPoolIds * slots + slot].z), add);
-            return kRayNone;
-        });
+        pool_trace<LAYOUT>(S, L, P, slots, Q, ne, n, stk, keep);
         __syncthreads();
         if (threadIdx.x == 0)
             Q.n_ext = Q.n_sh = Q.head = 0;
