@@ -338,7 +338,9 @@ e8g_status e8g_scene_validate(const e8g_scene_desc *desc, char *msg, size_t msg_
 /* Caps the device memory the context's buffers may hold (0 = no limit, the default). An upload,
  * build or render that would need more fails with E8G_ERR_OUT_OF_MEMORY, as a failed cudaMalloc
  * does, and the context stays usable: a failed upload or build leaves no scene or no tree (the
- * next render reports E8G_ERR_NO_SCENE or E8G_ERR_NOT_BUILT) until one succeeds. For callers
+ * next render reports E8G_ERR_NO_SCENE or E8G_ERR_NOT_BUILT) until one succeeds. Path pools and slot
+ * lists, which only make renders faster, are not allocated under a limit; those of earlier calls give way to
+ * whatever needs their room (also without a limit, when the device is full). For callers
  * with a memory budget, and for testing the out-of-memory paths. */
 e8g_status e8g_set_memory_limit(e8g_ctx *ctx, uint64_t bytes);
 /* Device memory the context's buffers hold now. */

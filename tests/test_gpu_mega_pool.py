@@ -175,3 +175,39 @@ def test_backward_with_its_most_slots(lib, layout):
         np.testing.assert_allclose(da, wa, rtol=1e-3, atol=1e-6 * np.abs(wa).max())
         assert np.linalg.norm(dr - wr) <= 1e-3 * max(np.linalg.norm(wr), 1e-12)
     assert grew[1] == 2 * grew[0] > 0
+
+
+@pytest.mark.parametrize("what", ["render", "wavefront", "backward"])
+def test_a_limit_set_later_takes_back_the_pools_room(lib, what):
+    """What fits a limit does not depend on when it was set: path pools and slot lists of an earlier call give
+    way to the buffers of a later one."""
+    from x3dcore2_gb300.core import Context
+    w, h = 1027, 1023
+    sc = S.displaced_icosphere(level=5, seed=2, num_materials=16, width=w, height=h)
+    p = default_params(abi.MODE_MIS, w, h, 2, seed=5, max_depth=6, rr_start=3)
+    if what == "wavefront":
+        p.integrator = abi.INTEGRATOR_WAVEFRONT
+    dl = np.ones((h, w, 3), np.float32)
+    r = np.random.default_rng(1)
+    rays = np.concatenate([r.uniform(-2, 2, (1_500_000, 3)), r.normal(0, 1, (1_500_000, 3))], axis=1).astype(np.float32)
+
+    def call(c):
+        if what != "backward":
+            return c.render(p)
+        c.forward(p)
+        return c.backward(dl)[0]
+
+    with Context(0) as c:
+        c.set_memory_limit(64 << 30)
+        c.upload(sc)
+        want = call(c)
+        hits = c.trace_closest(rays)
+        need = c.memory_used()
+    with Context(0) as c:
+        c.upload(sc)
+        call(c)
+        more = c.memory_used()
+        c.set_memory_limit(need)
+        got = c.trace_closest(rays)
+        assert np.array_equal(got["t"], hits["t"]) and more + 44 * len(rays) > need >= c.memory_used()
+        np.testing.assert_allclose(call(c), want, rtol=1e-3, atol=1e-6 * np.abs(want).max())

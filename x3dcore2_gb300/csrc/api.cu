@@ -80,10 +80,26 @@ void dev_buffer::release() {
 cudaError_t dev_buffer::reserve(size_t n) {
     if (n <= bytes)
         return cudaSuccess;
-    if (budget && budget->cap && budget->used - bytes + n > budget->cap)
+    auto refused = [&] { return budget && budget->cap && budget->used - bytes + n > budget->cap; };
+    auto give_back = [&] { // (cudaFree waits for the kernels that use them)
+        bool freed = false;
+        for (int k = 0; budget && k < 2; k++) {
+            dev_buffer *s = budget->spare[k];
+            if (s && s != this && s->ptr) {
+                s->release();
+                freed = true;
+            }
+        }
+        return freed;
+    };
+    if (refused() && !(give_back() && !refused()))
         return cudaErrorMemoryAllocation;
     release();
     cudaError_t e = cudaMalloc(&ptr, n);
+    if (e == cudaErrorMemoryAllocation && give_back()) {
+        cudaGetLastError();
+        e = cudaMalloc(&ptr, n);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError(); // not sticky: keep it out of later launch checks
         ptr = nullptr;
@@ -480,6 +496,8 @@ e8g_status e8g_create(e8g_ctx **out, e8g_device_opts const *opts) {
     c->device = dev;
     for (dev_buffer *b : c->all_buffers())
         b->budget = &c->budget;
+    c->budget.spare[0] = &c->b_pool;
+    c->budget.spare[1] = &c->b_live;
     cudaError_t e = cudaSetDevice(dev);
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);

@@ -15,10 +15,14 @@
 
 namespace e8g {
 
-// Device memory a context may hold (e8g_set_memory_limit): cap 0 = no limit.
+struct dev_buffer;
+
+// Device memory a context may hold (e8g_set_memory_limit): cap 0 = no limit. spare: buffers that only make
+// calls faster; when another one does not fit, in the limit or on the device, they are freed first.
 struct mem_budget {
     size_t cap = 0;
     size_t used = 0;
+    dev_buffer *spare[2] = {nullptr, nullptr};
 };
 
 struct dev_buffer {
@@ -26,8 +30,8 @@ struct dev_buffer {
     size_t bytes = 0;
     mem_budget *budget = nullptr;
     // Grows the buffer to n bytes (contents not kept). A request beyond the context's memory
-    // limit fails with cudaErrorMemoryAllocation before anything is freed; a failed cudaMalloc
-    // leaves the buffer empty.
+    // limit fails with cudaErrorMemoryAllocation before anything but the spare buffers is freed; a
+    // failed cudaMalloc leaves the buffer empty.
     cudaError_t reserve(size_t n);
     void release();
 };
@@ -63,7 +67,8 @@ struct e8g_ctx {
     e8g::dev_buffer b_fh, b_accum, b_work, b_img, b_io0, b_io1, b_counts;
     // wavefront queues and adjoint state
     e8g::dev_buffer b_wf, b_grad, b_ff, b_batch; // b_ff: firefly per-sample images; b_batch: staged batch scenes
-    e8g::dev_buffer b_pool; // path slots of the pooled megakernel
+    e8g::dev_buffer b_pool; // path slots of the pooled megakernel and backward (spare)
+    e8g::dev_buffer b_live; // lists of the wavefront's occupied slots (spare)
     e8g::dev_buffer b_bdw; // subpaths and connection lists of the split bidirectional form
     e8g_render_params fwd_params{};
     bool have_forward = false;
@@ -107,7 +112,7 @@ struct e8g_ctx {
         return {&b_nodes, &b_wide, &b_tri, &b_tidx, &b_vpos, &b_vnrm, &b_vtx, &b_mesh_mat, &b_mesh_light, &b_mesh_toff,
                 &b_mesh_area, &b_tri_cum, &b_mats, &b_light_mesh, &b_light_rad, &b_light_cum, &b_light_pnorm,
                 &b_fh, &b_accum, &b_work, &b_img, &b_io0, &b_io1, &b_counts, &b_wf, &b_grad, &b_ff, &b_batch,
-                &b_refit, &b_vpos0, &b_vnrm0, &b_gbuild, &b_pipe, &b_check, &b_bdw, &b_pool};
+                &b_refit, &b_vpos0, &b_vnrm0, &b_gbuild, &b_pipe, &b_check, &b_bdw, &b_pool, &b_live};
     }
 };
 

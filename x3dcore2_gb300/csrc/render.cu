@@ -23,18 +23,24 @@ struct WfCounters { // mirrors the device Counters of wavefront.cu
     uint32_t shadow_n, ext_n, busy, pad[3];
 };
 
-// Device memory for `pools` slot arrays of Q slots each, with the lists of occupied slots unless the
-// context has a memory limit (what fitted it still fits) or their allocation fails; nor where every slot
-// has a resident thread of its own, which visits it in no time (there the lists' loads lengthened each
-// bounce: 120x100, 2-spp bidirectional frame 1.00 -> 1.04 ms). *bytes: of one pool.
-cudaError_t reserve_slots(e8g_ctx *c, uint32_t Q, size_t pools, bool *live, size_t *bytes) {
-    for (*live = c->budget.cap == 0 && Q > static_cast<uint32_t>(c->num_sms) * 1024;; *live = false) {
-        *bytes = (wf_total_bytes(Q, *live) + 255) & ~static_cast<size_t>(255);
-        cudaError_t e = c->b_wf.reserve(pools == 1 ? wf_total_bytes(Q, *live) : pools * *bytes);
-        if (e == cudaSuccess || !*live)
-            return e;
+// Device memory for `pools` (one or two) slot arrays of Q slots each in W, with the lists of occupied slots
+// unless the context has a memory limit (what fitted it still fits) or their allocation fails; nor where
+// every slot has a resident thread of its own, which visits it in no time (there the lists' loads lengthened
+// each bounce: 120x100, 2-spp bidirectional frame 1.00 -> 1.04 ms).
+cudaError_t reserve_slots(e8g_ctx *c, uint32_t Q, size_t pools, WfSlots *W) {
+    const size_t bytes = (wf_total_bytes(Q) + 255) & ~static_cast<size_t>(255);
+    cudaError_t e = c->b_wf.reserve(pools == 1 ? wf_total_bytes(Q) : pools * bytes);
+    if (e != cudaSuccess)
+        return e;
+    bool lists = c->budget.cap == 0 && Q > static_cast<uint32_t>(c->num_sms) * 1024;
+    if (lists && c->b_live.reserve(pools * 2 * sizeof(uint32_t) * Q) != cudaSuccess) {
         cudaGetLastError();
+        lists = false;
     }
+    for (size_t k = 0; k < pools; k++)
+        W[k] = wf_carve(static_cast<char *>(c->b_wf.ptr) + k * bytes, Q,
+                        lists ? static_cast<uint32_t *>(c->b_live.ptr) + k * 2 * static_cast<size_t>(Q) : nullptr);
+    return cudaSuccess;
 }
 
 // The split form of E8G_MODE_BDPT_POWER. Paths go in chunks (at most 2^26, and at most 32 GiB or
@@ -99,12 +105,10 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
     BdwChunk C = carve(static_cast<char *>(c->b_bdw.ptr), chunk, &Q, &range, &need);
     // the walk's slots
     const uint32_t slots = static_cast<uint32_t>(std::min<uint64_t>((chunk + 255) / 256 * 256, 1u << 23));
-    bool live = false;
-    size_t slot_bytes = 0;
-    e = reserve_slots(c, slots, 1, &live, &slot_bytes);
+    WfSlots W{};
+    e = reserve_slots(c, slots, 1, &W);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "bidirectional walk slots");
-    WfSlots W = wf_carve(c->b_wf.ptr, slots, live);
     // refill threshold of the trace kernels (threshold 8 against 16: 42.3 against 43.0 ms per
     // 1280x720, 32-spp frame)
     const uint32_t threshold = c->dev.layout == 0 || c->dev.layout == 2 ? 8u : 0u;
@@ -195,7 +199,8 @@ e8g_status run_bdpt_split(e8g_ctx *c, RenderArgs const &A, float4 *accum, float 
 
 // Whether the megakernel runs over block-local path pools: an estimator and a tree that kernel
 // has, and its slots allocated. A context with a memory limit keeps the kernel without slots, so
-// that what fitted the limit still fits; so does one whose allocation fails.
+// that what fitted the limit still fits (slots allocated before the limit was set are spare: they give way
+// to whatever needs their room); so does one whose allocation fails.
 bool use_mega_pool(e8g_ctx *c, e8g_render_params const *p, RenderArgs const &A) {
     if (p->integrator == E8G_INTEGRATOR_PLAIN || c->budget.cap != 0 || !mega_pool_takes(c->dev, A))
         return false;
@@ -278,12 +283,10 @@ e8g_status run_wavefront(e8g_ctx *c, RenderArgs const &A, float4 *accum, float *
         threshold = 16; // the many-scene form always traces with dynamic fetch
     uint64_t want = std::max<uint64_t>(total, 1024);
     uint32_t Q = static_cast<uint32_t>(std::min<uint64_t>(capacity, (want + 255) / 256 * 256));
-    bool live = false;
-    size_t slot_bytes = 0;
-    cudaError_t e = reserve_slots(c, Q, 1, &live, &slot_bytes);
+    WfSlots W{};
+    cudaError_t e = reserve_slots(c, Q, 1, &W);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "wavefront slots");
-    WfSlots W = wf_carve(c->b_wf.ptr, Q, live);
     e = wf_init(W, c->stream);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "wavefront init");
@@ -372,9 +375,8 @@ e8g_status run_wavefront_concurrent(e8g_ctx *c, RenderArgs const &A, float4 *acc
     uint64_t want = std::max<uint64_t>(total, 2048);
     uint32_t Qh = static_cast<uint32_t>(std::min<uint64_t>(capacity / 2, (want / 2 + 255) / 256 * 256));
     Qh = std::max<uint32_t>(Qh, 256);
-    bool live = false;
-    size_t pool = 0;
-    cudaError_t e = reserve_slots(c, Qh, 2, &live, &pool);
+    WfSlots pools[2];
+    cudaError_t e = reserve_slots(c, Qh, 2, pools);
     if (e != cudaSuccess)
         return cuda_fail(c, e, "wavefront slots");
     if (!c->stream2) {
@@ -386,8 +388,7 @@ e8g_status run_wavefront_concurrent(e8g_ctx *c, RenderArgs const &A, float4 *acc
         if (e != cudaSuccess)
             return cuda_fail(c, e, "second stream");
     }
-    WfSlots WA = wf_carve(c->b_wf.ptr, Qh, live);
-    WfSlots WB = wf_carve(static_cast<char *>(c->b_wf.ptr) + pool, Qh, live);
+    WfSlots WA = pools[0], WB = pools[1];
     WB.next_path = WA.next_path;
     e = wf_init(WA, c->stream);
     if (e == cudaSuccess)

@@ -541,7 +541,7 @@ __global__ void k_wf_reset(Counters *cnt, unsigned long long const *next_path, u
 
 // Lays the slot arrays and queues out from `base` (each array 256-byte aligned) and returns
 // the bytes used in *total; with a null base it only measures (all pointers null).
-static WfSlots carve(char *base, uint32_t capacity, bool live, size_t *total) {
+static WfSlots carve(char *base, uint32_t capacity, size_t *total) {
     WfSlots W{};
     W.capacity = capacity;
     size_t off = 0;
@@ -567,21 +567,22 @@ static WfSlots carve(char *base, uint32_t capacity, bool live, size_t *total) {
     W.ext_d = reinterpret_cast<float4 *>(take(Q * 16));
     W.vp = reinterpret_cast<float4 *>(take(Q * 16));
     W.vn = reinterpret_cast<float4 *>(take(Q * 16));
-    W.live = live ? reinterpret_cast<uint32_t *>(take(2 * Q * 4)) : nullptr;
     W.counters = take(sizeof(Counters));
     W.next_path = base ? &reinterpret_cast<Counters *>(W.counters)->next_path : nullptr;
     *total = off;
     return W;
 }
 
-WfSlots wf_carve(void *base, uint32_t capacity, bool live) {
+WfSlots wf_carve(void *base, uint32_t capacity, uint32_t *live) {
     size_t total = 0;
-    return carve(static_cast<char *>(base), capacity, live, &total);
+    WfSlots W = carve(static_cast<char *>(base), capacity, &total);
+    W.live = live;
+    return W;
 }
 
-size_t wf_total_bytes(uint32_t capacity, bool live) {
+size_t wf_total_bytes(uint32_t capacity) {
     size_t total = 0;
-    carve(nullptr, capacity, live, &total);
+    carve(nullptr, capacity, &total);
     return total;
 }
 

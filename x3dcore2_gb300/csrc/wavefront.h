@@ -89,9 +89,9 @@ template <> struct RngSlot<RngPhilox> {
     }
 };
 
-// live: with the lists of occupied slots (8 bytes a slot).
-size_t wf_total_bytes(uint32_t capacity, bool live);
-WfSlots wf_carve(void *base, uint32_t capacity, bool live);
+size_t wf_total_bytes(uint32_t capacity);
+// live: memory for the lists of occupied slots (two entries a slot), or null.
+WfSlots wf_carve(void *base, uint32_t capacity, uint32_t *live);
 cudaError_t wf_init(WfSlots const &W, cudaStream_t st);
 int wf_trace_blocks_per_sm(uint32_t layout, uint32_t threshold);
 // Trace kernels that a bounce launches: one for both queues on the two fast trees, else one for each.
