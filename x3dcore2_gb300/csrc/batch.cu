@@ -8,15 +8,12 @@
 // graph) when every item asks for E8G_INTEGRATOR_WAVEFRONT with E8G_MODE_MIS and one stream kind,
 // else the persistent megakernel on SAH-pair trees (k_mega_batch).
 #include "api_internal.h"
+#include "host_threads.h"
 
 #include <algorithm>
-#include <atomic>
 #include <cstring>
-#include <exception>
 #include <memory>
-#include <mutex>
 #include <system_error>
-#include <thread>
 #include <vector>
 
 namespace e8g {
@@ -34,42 +31,14 @@ struct layout_of {
 };
 
 // fn(k) for every scene, spread over the machine's cores; the scenes with most triangles start first, so
-// that none of them is left for the end. An exception of a call is thrown again here once every thread
-// has stopped; threads that cannot be started are done without.
+// that none of them is left for the end.
 template <class F> void for_scenes(e8g_batch_item const *items, uint32_t n, F &&fn) {
     std::vector<uint32_t> order(n);
     for (uint32_t k = 0; k < n; k++)
         order[k] = k;
     auto tris = [&](uint32_t k) { return items[k].scene->mesh_tri_offset[items[k].scene->num_meshes]; };
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return tris(a) > tris(b); });
-    std::atomic<uint32_t> next{0};
-    std::mutex lock;
-    std::exception_ptr error;
-    auto work = [&] {
-        for (uint32_t i; (i = next.fetch_add(1)) < n;) {
-            try {
-                fn(order[i]);
-            } catch (...) {
-                std::lock_guard<std::mutex> hold(lock);
-                if (!error)
-                    error = std::current_exception();
-                next = n;
-            }
-        }
-    };
-    const uint32_t most = std::min<uint32_t>(n, std::max(1u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> threads;
-    threads.reserve(most);
-    try {
-        while (threads.size() + 1 < most)
-            threads.emplace_back(work);
-    } catch (std::system_error const &) {
-    }
-    work();
-    for (std::thread &t : threads)
-        t.join();
-    if (error)
-        std::rethrow_exception(error);
+    for_each_on_cores(order, fn);
 }
 
 } // namespace
