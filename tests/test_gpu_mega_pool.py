@@ -130,9 +130,9 @@ def test_a_path_is_the_same_in_a_short_and_a_long_list(ctx, kind, mode, depth):
 
 @pytest.mark.parametrize("layout", [abi.BVH_SAH, abi.BVH_WIDE])
 @pytest.mark.parametrize("mode,depth", [(abi.MODE_MIS, 6), (abi.MODE_REF_LT1, 0)])
-@pytest.mark.parametrize("spp,slots", [(16, 640), (32, 1024)])
-def test_larger_pools(lib, spp, slots, mode, depth, layout):
-    """Renders long enough for 640 and for all 1,024 slots a block (128 bytes each, seven blocks an SM), at an
+@pytest.mark.parametrize("spp,slots", [(1, 128), (16, 640), (32, 1024)])
+def test_smaller_and_larger_pools(lib, spp, slots, mode, depth, layout):
+    """Renders for the fewest slots a block, for 640 and for all 1,024 (128 bytes each, seven blocks an SM), at an
     odd size: a pixel is a sum of at most 32 equal terms in any order."""
     import torch
 

@@ -41,10 +41,18 @@ void launch_megakernel(DevScene const &S, RenderArgs const &A, FirstHit const *f
 }
 
 // The estimators with a random walk on their default streams, on the two fast trees, from 2^19 paths
-// on (five per lane of the GPU): below that the pools hardly refill and k_mega is as fast or faster
-// (640 x 360, 1 spp: 0.49 ms against 0.58; 16 spp of 256 x 256: 1.21 against 0.91).
+// on (four per lane of the pools); below that the pools hardly refill and k_mega is as fast or faster.
+// Where the two break even depends on how long paths are. One-sample frames of 541,000 / 1.07M / 2.07M paths, k_mega
+// against pools, ms, on the pairs: a 50,000-triangle soup in a closed room MIS 1.51 / 2.53 / 4.55 against
+// 1.22 / 1.81 / 2.81, lt1 1.34 / 2.31 / 4.13 against 1.09 / 1.49 / 2.31; the 1.3M-triangle icosphere, an open
+// scene whose paths have one or two rays, MIS 0.67 / 1.06 / 1.90 against 0.81 / 1.13 / 1.71, lt1 0.59 / 0.97 /
+// 1.79 against 0.66 / 0.98 / 1.44. On the eight-wide tree the pools win in both (541,000 paths: 1.76 against
+// 1.10, 0.70 against 0.60). The unidirectional estimator has no shadow rays to fill lanes with and starts
+// later on the pairs (541,000 / 1.07M / 1.44M paths: soup 0.81 / 1.42 / 1.87 against 0.81 / 1.12 / 1.33, icosphere
+// 0.39 / 0.56 / 0.75 against 0.51 / 0.67 / 0.79).
 bool mega_pool_takes(DevScene const &S, RenderArgs const &A) {
-    return (S.layout == 0 || S.layout == 2) && A.total_paths >= (1u << 19) &&
+    const uint64_t least = S.layout == 0 && A.mode == E8G_MODE_REF_UNI ? 5u << 18 : 1u << 19;
+    return (S.layout == 0 || S.layout == 2) && A.total_paths >= least &&
            ((A.mode == E8G_MODE_MIS && A.rng == E8G_RNG_PHILOX) ||
             ((A.mode == E8G_MODE_REF_LT1 || A.mode == E8G_MODE_REF_UNI) && A.rng == E8G_RNG_MINSTD));
 }

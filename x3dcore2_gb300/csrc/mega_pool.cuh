@@ -478,11 +478,15 @@ __global__ void __launch_bounds__(kBlock, kPoolBlocks)
 
 // Slots per block: about sixteen paths each, since a pool that the render fills only a few times
 // spends its time in the end, when slots run empty (2 M paths: 256 / 512 / 1024 slots 0.89 / 0.92 /
-// 1.05 ms; 33 M: 19.9 / 19.4 / 18.8).
+// 1.05 ms; 33 M: 19.9 / 19.4 / 18.8). At least 256, and 128 below 2^20 paths. With 128 / 256 slots, pairs,
+// 541,000 paths of a one-sample frame: 0.81 / 0.86 ms (1.3M-triangle icosphere), 1.21 / 1.26 (50,000-triangle
+// soup), backward 0.71 / 0.82 (327,690 triangles) and 1.24 / 1.24; 1.07M paths: 1.09 / 1.11 and 1.85 / 1.79;
+// 2.07M: 1.77 / 1.70 and 3.01 / 2.81. The eight-wide tree alike.
 inline uint32_t pool_slots(RenderArgs const &A, int num_sms) {
     const uint64_t per_block = A.total_paths / (static_cast<uint64_t>(num_sms) * kPoolBlocks);
     const uint64_t want = (per_block / 16 + kBlock - 1) / kBlock * kBlock;
-    return static_cast<uint32_t>(std::min<uint64_t>(std::max<uint64_t>(want, 256), kPoolSlots));
+    const uint64_t least = A.total_paths < (1u << 20) ? 128 : 256;
+    return static_cast<uint32_t>(std::min<uint64_t>(std::max<uint64_t>(want, least), kPoolSlots));
 }
 
 // Rays a warp may leave the trace phase with (0 / 8 / 16: 21.8 / 18.8 / 18.9 ms per 16-spp frame); in a
