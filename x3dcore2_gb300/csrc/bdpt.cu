@@ -413,17 +413,14 @@ __global__ void __launch_bounds__(kBlock, COUNT || LAYOUT < 0 ? 1 : kBdptBlocks)
             R rng;
             seed_path(rng, A, mix, pixel, sample);
             FirstHit f = fh[pixel];
-            uint32_t clen = 0;
-            int32_t mesh = __float_as_int(f.p.w);
-            if (mesh >= 0 && max_len != 0) { // sample_path with the cached first hit (:127-137)
-                cam[0].v = neg(xyz(f.d));
-                cam[0].dens = 1.0f;
-                cam[0].p = xyz(f.p);
-                cam[0].n = xyz(f.n);
-                cam[0].mesh = mesh;
-                cam[0].light = __float_as_int(f.n.w);
-                clen = sample_subpath<LAYOUT, COUNT>(S, rng, cam, 1, max_len, stk, &cnt);
-            }
+            // sample_path with the cached first hit (:127-137), which every path taken has
+            cam[0].v = neg(xyz(f.d));
+            cam[0].dens = 1.0f;
+            cam[0].p = xyz(f.p);
+            cam[0].n = xyz(f.n);
+            cam[0].mesh = __float_as_int(f.p.w);
+            cam[0].light = __float_as_int(f.n.w);
+            const uint32_t clen = sample_subpath<LAYOUT, COUNT>(S, rng, cam, 1, max_len, stk, &cnt);
             // sample_illum_source (:754-767), area_light::sample_emssion (light.cpp:26-32)
             float pmf;
             int light = sample_light(S, rng, pmf);
@@ -435,7 +432,7 @@ __global__ void __launch_bounds__(kBlock, COUNT || LAYOUT < 0 ? 1 : kBdptBlocks)
             if (COUNT)
                 cnt.rays++;
             Hit h = trace_call<LAYOUT, COUNT>(S, em.p, w, 1e-4f, 1000.0f, false, stk, &cnt); // sample_path from r0 (:109-120)
-            if (h.tri != 0xFFFFFFFFu && max_len != 0) {
+            if (h.tri != 0xFFFFFFFFu) {
                 Vert v0 = make_vert(S, h);
                 if (!(dot(v0.n, neg(w)) <= 0.0f)) {
                     lp[0].v = neg(w);
@@ -462,55 +459,47 @@ __global__ void __launch_bounds__(kBlock, COUNT || LAYOUT < 0 ? 1 : kBdptBlocks)
 }
 
 // Both subpaths of one path (the draw order of k_bdpt_power): the camera subpath from the cached
-// first hit f, then the light pick, the emission point and direction and the light subpath.
-// Returns the light's index; clen = 0 when the camera ray missed.
+// first hit f (a valid one; max_len at least 1), then the light pick, the emission point and direction and
+// the light subpath. Returns the light's index.
 template <int LAYOUT, bool COUNT, class R>
 __device__ __forceinline__ int sample_subpaths(DevScene const &S, R &rng, FirstHit const &f, uint32_t max_len, BV *cam,
                                                BV *lp, uint32_t &clen, uint32_t &llen, uint32_t *stk,
                                                TraceCounters *cnt) {
-    int32_t mesh = __float_as_int(f.p.w);
-    float3 o0 = neg(xyz(f.d));
-    clen = 0;
-    llen = 0;
-    if (mesh >= 0 && max_len) {
-        cam[0].p = xyz(f.p);
-        cam[0].n = xyz(f.n);
-        cam[0].mesh = mesh;
-        cam[0].beta = f3(1.0f, 1.0f, 1.0f);
-        cam[0].fwd = 1.0f;
-        cam[0].rev = 0.0f;
-        clen = bdp_walk<LAYOUT, COUNT>(S, rng, cam, 1, max_len, o0, stk, cnt);
-    }
+    cam[0].p = xyz(f.p);
+    cam[0].n = xyz(f.n);
+    cam[0].mesh = __float_as_int(f.p.w);
+    cam[0].beta = f3(1.0f, 1.0f, 1.0f);
+    cam[0].fwd = 1.0f;
+    cam[0].rev = 0.0f;
+    clen = bdp_walk<LAYOUT, COUNT>(S, rng, cam, 1, max_len, neg(xyz(f.d)), stk, cnt);
     float pmf;
     int light = sample_light(S, rng, pmf);
     uint32_t lmesh = __ldg(&S.light_mesh[light]);
     Surf em = mesh_sample(S, lmesh, rng, true);
     float3 w = cos_hemisphere(em.n, rng);
     float pdf_w = dot(em.n, w) / kPi;
-    if (max_len) {
-        lp[0].p = em.p;
-        lp[0].n = em.n;
-        lp[0].mesh = static_cast<int32_t>(lmesh);
-        lp[0].fwd = pmf * em.area_dens;
-        lp[0].rev = 0.0f;
-        float ib = 1.0f / lp[0].fwd;
-        lp[0].beta = f3(ib, ib, ib);
-        llen = 1;
-        if (pdf_w > 0.0f && max_len > 1) {
-            if (COUNT)
-                cnt->rays++;
-            Hit h = trace_call<LAYOUT, COUNT>(S, em.p, w, 1e-4f, 1000.0f, false, stk, cnt);
-            if (h.tri != 0xFFFFFFFFu) {
-                Vert v0 = make_vert(S, h);
-                if (dot(v0.n, neg(w)) > 0.0f) {
-                    lp[1].p = v0.p;
-                    lp[1].n = v0.n;
-                    lp[1].mesh = v0.mesh;
-                    lp[1].beta = scale(light_rad(S, light), dot(em.n, w) / (pdf_w * lp[0].fwd));
-                    lp[1].fwd = to_area(pdf_w, em.p, lp[1].p, lp[1].n);
-                    lp[1].rev = 0.0f;
-                    llen = bdp_walk<LAYOUT, COUNT>(S, rng, lp, 2, max_len, neg(w), stk, cnt);
-                }
+    lp[0].p = em.p;
+    lp[0].n = em.n;
+    lp[0].mesh = static_cast<int32_t>(lmesh);
+    lp[0].fwd = pmf * em.area_dens;
+    lp[0].rev = 0.0f;
+    float ib = 1.0f / lp[0].fwd;
+    lp[0].beta = f3(ib, ib, ib);
+    llen = 1;
+    if (pdf_w > 0.0f && max_len > 1) {
+        if (COUNT)
+            cnt->rays++;
+        Hit h = trace_call<LAYOUT, COUNT>(S, em.p, w, 1e-4f, 1000.0f, false, stk, cnt);
+        if (h.tri != 0xFFFFFFFFu) {
+            Vert v0 = make_vert(S, h);
+            if (dot(v0.n, neg(w)) > 0.0f) {
+                lp[1].p = v0.p;
+                lp[1].n = v0.n;
+                lp[1].mesh = v0.mesh;
+                lp[1].beta = scale(light_rad(S, light), dot(em.n, w) / (pdf_w * lp[0].fwd));
+                lp[1].fwd = to_area(pdf_w, em.p, lp[1].p, lp[1].n);
+                lp[1].rev = 0.0f;
+                llen = bdp_walk<LAYOUT, COUNT>(S, rng, lp, 2, max_len, neg(w), stk, cnt);
             }
         }
     }
@@ -539,8 +528,7 @@ __global__ void __launch_bounds__(kBlock, COUNT || LAYOUT < 0 ? 1 : kBdptBlocks)
             FirstHit f = fh[pixel];
             uint32_t clen, llen;
             int light = sample_subpaths<LAYOUT, COUNT>(S, rng, f, max_len, cam, lp, clen, llen, stk, &cnt);
-            float3 L = clen ? connect_power<LAYOUT, COUNT>(S, cam, clen, lp, llen, max_len, neg(xyz(f.d)), light, stk, &cnt)
-                            : f3(0, 0, 0);
+            float3 L = connect_power<LAYOUT, COUNT>(S, cam, clen, lp, llen, max_len, neg(xyz(f.d)), light, stk, &cnt);
             if (path_rgb) {
                 path_rgb[3 * static_cast<size_t>(out)] = L.x;
                 path_rgb[3 * static_cast<size_t>(out) + 1] = L.y;
