@@ -303,7 +303,9 @@ e8g_status e8g_trace_any(e8g_ctx *ctx, const e8g_ray *rays, const float *t_min, 
 e8g_status e8g_trace_closest_dev(e8g_ctx *ctx, const e8g_ray *d_rays, uint32_t n, e8g_hit *d_hits,
                                  void *stream);
 
-/* Image render: rgba_out is host memory of width*height*4 floats (alpha = 1). */
+/* Image render: rgba_out is host memory of width*height*4 floats (alpha = 1). A pixel's samples are added in the
+ * order their paths end, so an image of several samples can differ in its last bits from call to
+ * call; the radiance of one unidirectional path (e8g_render_paths) does not. */
 e8g_status e8g_render(e8g_ctx *ctx, const e8g_render_params *params, float *rgba_out);
 /* Same, writing a device buffer; the caller synchronises. */
 e8g_status e8g_render_dev(e8g_ctx *ctx, const e8g_render_params *params, float *d_rgba_out,

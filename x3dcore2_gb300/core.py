@@ -151,6 +151,8 @@ class Context:
         return out
 
     def trace_closest(self, rays):
+        """Closest hits as a dict of arrays (t, mesh, tri, b); the four are views of one buffer, so keeping one
+        keeps its memory."""
         rays = np.ascontiguousarray(rays, np.float32).reshape(-1, 6)
         n = len(rays)
         # the device writes the arrays; splitting (n, 5) records here took ten times the query

@@ -19,8 +19,8 @@ namespace {
 // One out-of-line traversal for a kernel's five call sites: inlined, with every layout behind a
 // run-time test, they overflowed the instruction cache (7.7 of 15 stall cycles per instruction in
 // k_bdpt_ref, 166 registers): with it, eight blocks per SM and no walk for paths without a camera
-// vertex that frame takes 3.2 ms against 7.3. LAYOUT -1: the scene's layout at run time (the reference's tree, the linear layout, and
-// the counted runs).
+// vertex that frame takes 3.2 ms against 7.3. LAYOUT -1: the scene's layout at run time (the reference's tree,
+// the linear layout, and the counted runs).
 template <int LAYOUT, bool COUNT>
 __device__ __noinline__ Hit trace_call(DevScene const &S, float3 o, float3 d, float tmin, float tmax, bool any,
                                        uint32_t *stk, TraceCounters *cnt) {
@@ -642,11 +642,13 @@ inline bool walk_small(uint32_t slots, int num_sms) { return slots < static_cast
 // The materials' code is out of line and the kernel held to 64 registers (32 warps per SM): the walk
 // stalled on instruction fetch with it inlined, and at 24 warps per SM (80 registers, no spills) it
 // took 52.1 ms per 1280x720, 32-spp frame against 47.6 ms.
-// It is bound by instruction fetch (9.7 of 22 stall cycles per instruction waited for it): every warp
-// runs some tens of kilobytes of code per group of slots. The barriers keep a block's warps in the
-// same part of it, so that a fetched line serves all of them: blocks of 256 threads without barriers
-// 36.0 ms per frame, with one / three barriers per group of slots 34.2 / 33.7, blocks of 512 33.2 /
-// 33.0, of 1024 33.0. Lists of the occupied slots (WfLive) and paths numbered tile by tile: 28.7.
+// It is bound by the latency of its fetches (18.7 and 7.7 of the stall cycles per issue in the first and third
+// bounce) and by divergence (12 of 32 lanes in the third). Every warp runs some tens of kilobytes of code per
+// group of slots, and without the barriers instruction fetch came first (9.7 of 22 stall cycles): they keep a
+// block's warps in the same part of the code, so that a fetched line serves all of them (0.9 to 1.7 cycles now,
+// 3.6 to 5.6 at the barriers). Blocks of 256 threads without barriers 36.0 ms per frame, with one / three
+// barriers per group of slots 34.2 / 33.7, blocks of 512 33.2 / 33.0, of 1024 33.0. Lists of the occupied
+// slots (WfLive) and paths numbered tile by tile: 28.7.
 template <class R, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     k_bdw_walk(DevScene S, RenderArgs A, FirstHit const *__restrict__ fh, BdwChunk C, WfSlots W,

@@ -8,15 +8,15 @@
 // warps trace the extension and shadow rays of all slots from a queue in shared memory, a lane
 // taking the next ray as soon as its own is done. Rays still on their way when the queue is empty
 // stay in their lanes over the next shading phase, so no block waits for its longest ray. No phase
-// leaves the kernel: no launches, no host synchronisation, and small renders keep the GPU as busy
-// as large ones.
+// leaves the kernel: no launches, no host synchronisation. Renders that fill the slots only once or twice
+// gain nothing and stay with k_mega (mega_pool_takes).
 //
-// Measured on one GB300, device time of the integrator: the 1080p, 16-spp MIS frame of that scene
-// 26.3 (k_mega) -> 18.8 ms on the pairs and 30.8 -> 19.1 on the eight-wide tree, the 720p lt1 frame
-// 11.4 -> 8.1 (with paths numbered tile by tile since: 16.9, 17.4 and 6.2), a 1080p one-sample unidirectional frame 0.97 -> 0.90, the Cornell room at 256 x 256,
-// 16 spp 1.21 -> 0.91, a 50,000-triangle soup 4.13 -> 2.67. What bounds it now: issue slots (0.5 per
-// cycle and scheduler) shared with memory latency at 28 warps per SM; three quarters of the time is
-// tracing.
+// Measured on one GB300, device time of the integrator, k_mega -> pools: the 1080p, 16-spp MIS frame of that
+// scene 26.3 -> 16.9 ms on the pairs and 30.8 -> 16.2 on the eight-wide tree, its one-sample frame 1.90 -> 1.71 and
+// 2.15 -> 1.47, 1.07M paths of the Cornell room 0.72 -> 0.61 and 0.84 -> 0.54, a one-sample 1080p frame of a
+// 50,000-triangle soup 4.55 -> 2.81 and 5.40 -> 2.70. What bounds it now (pairs, 8 spp): issue slots (0.48 per cycle and
+// scheduler, 15.1 of 32 lanes) and the latency of fetches (6.3 of the stall cycles per issue) at 28 warps per
+// SM; three quarters of the time is tracing.
 #pragma once
 
 #include "mega.cuh"
@@ -28,7 +28,8 @@ namespace e8g {
 
 namespace {
 
-// Blocks per SM (72 registers): 6 / 7 / 8 blocks take 21.5 / 19.6 / 20.0 ms per 16-spp frame.
+// Blocks per SM (72 registers): 6 / 7 / 8 blocks took 21.5 / 19.6 / 20.0 ms per 16-spp frame (before paths were
+// numbered tile by tile).
 constexpr int kPoolBlocks = 7;
 // Slots per block at most (pool_slots).
 constexpr uint32_t kPoolSlots = 1024;
@@ -489,9 +490,10 @@ inline uint32_t pool_slots(RenderArgs const &A, int num_sms) {
     return static_cast<uint32_t>(std::min<uint64_t>(std::max<uint64_t>(want, least), kPoolSlots));
 }
 
-// Rays a warp may leave the trace phase with (0 / 8 / 16: 21.8 / 18.8 / 18.9 ms per 16-spp frame); in a
-// tiny tree rays are short and of one length, and leaving slots out of the next shading costs more
-// than their wait (Cornell: 0.91 ms with 0, 0.96 with 8).
+// Rays a warp may leave the trace phase with: 0 / 8 / 16 / 24 take 1.99 / 1.70 / 1.74 / 1.79 ms in a one-sample
+// 1080p frame of 1.3M triangles, 3.19 / 2.81 / 2.83 / 2.91 in one of a 50,000-triangle soup and 1.18 / 1.15 / 1.20 / 1.25
+// with 20,000 triangles. In a tiny tree rays are short and of one length, and leaving slots out of the next
+// shading costs more than their wait (Cornell: 0.91 ms with 0, 0.96 with 8).
 inline uint32_t pool_keep(DevScene const &S) { return S.nnodes >= 1024 ? 8u : 0u; }
 
 template <int LAYOUT>
